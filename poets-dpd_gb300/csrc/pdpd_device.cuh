@@ -69,7 +69,10 @@ __device__ __forceinline__ float min_dist_sqr_f()
 
 __device__ __forceinline__ int wrap_index(int i, int L)
 {
-    i %= L;
+    if (i >= L) i -= L;
+    if (i < 0) i += L;
+    if ((unsigned)i < (unsigned)L) return i;
+    i %= L;  // more than one box away
     return i < 0 ? i + L : i;
 }
 

@@ -232,7 +232,8 @@ __device__ __forceinline__ void pair_accumulate(float dx, float dy, float dz, fl
                                                 uint32_t hj, float2 pp, uint32_t th_lo,
                                                 uint32_t th_hi, float scale, float F[3])
 {
-    const float inv_r = rsqrtf(r2);
+    float inv_r;  // r2 >= 1e-18: normal, so flushing subnormals changes nothing and saves the scaling around them
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv_r) : "f"(r2));
     const float r = __fmul_rn(r2, inv_r);
     const float wr = __fsub_rn(1.0f, r);
     const float ex = __fmul_rn(dx, inv_r), ey = __fmul_rn(dy, inv_r), ez = __fmul_rn(dz, inv_r);
@@ -826,17 +827,17 @@ int launch_begin32(const KArgs &a, cudaStream_t s)
 // blocks per SM (variants 8 and 9), within the 16-bit staged indices of the list entries.
 uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max)
 {
-    if (variant != 8 && variant != 9) return 2047u;  // variant 6: its bricks stay far below
+    if (variant != 8 && variant != 9) return 2046u;  // variant 6: its bricks stay far below
     int dev = 0, smem_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
-        return 2047u;
+        return 2046u;
     const uint32_t hm = variant == 9 ? home_max : 0u;
     const BrickLayout L = brick_layout(hc_max, 0, npair, brick_variant_threads(variant), hm);
-    // per staged bead: position and velocity (32 B), and for the half shell its home index
-    const int per_bead = variant == 9 ? 34 : 32;
-    const int budget = smem_sm / 2 - 1024 - (int)L.bytes - 64;
-    return (uint32_t)std::max(64, std::min(65535, budget / per_bead));
+    const int per_bead = (int)(variant == 9 ? HALF_BEAD_BYTES : FULL_BEAD_BYTES);
+    const int budget = smem_sm / 2 - 1024 - (int)L.bytes - 128;  // (each part is rounded up to 16 bytes)
+    const int most = variant == 9 ? 65535 : (int)FULL_MAX_STAGED;
+    return (uint32_t)std::max(64, std::min(most, budget / per_bead)) & ~1u;
 }
 
 // Set up the brick kernel for a brick shape: opt in to the shared memory it needs and

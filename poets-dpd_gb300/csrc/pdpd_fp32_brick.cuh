@@ -32,7 +32,7 @@ constexpr int BRICK_THREADS = 128;       // threads per block of variant 6
 constexpr int BRICK_THREADS_WIDE = 512;  // threads per block of variant 8 (larger bricks)
 constexpr int HALF_THREADS = 384;        // threads per block of variant 9
 constexpr int BRICK_MAX_WARPS = BRICK_THREADS_WIDE / 32;
-constexpr int BLIST_MAX = 32;            // list capacity of the full-shell row walk
+constexpr int SEG_MAX = 9;               // walk segments kept per thread before an evaluation
 constexpr int HLIST_MAX = 32;            // list capacity of the half-shell walk
 constexpr int BRICK_MAX_ROWS = 64;
 constexpr uint16_t NOT_HOME = 0xffffu;
@@ -43,6 +43,7 @@ struct BrickHeader {
     uint32_t home_rows[BRICK_MAX_ROWS + 1];
     uint32_t next;    // the block's next brick
     uint32_t cursor;  // half shell: the next home bead a warp takes
+    uint32_t total;   // full shell: staged beads of the brick
 };
 
 // A block's next brick: after its first (blockIdx.x), blocks take bricks from a shared
@@ -56,15 +57,20 @@ __device__ __forceinline__ uint32_t brick_fetch(const KArgs &a, BrickHeader &H)
     return H.next;
 }
 
-// Shared-memory layout of one block: header, pair table, hstart[HC+1], hslot[HC], hlo[HC],
-// pos[maxb], vel[maxb], list[cap][threads]; the half shell adds hidx[maxb] (home index of a
-// staged bead, NOT_HOME for a halo bead), hsi[home_max] (staged index of a home bead) and
-// acc[6][home_max] (fixed-point force sums of the home beads: per axis a word of the terms'
-// low 16 bits and a word of their high parts, so that 32-bit atomics add them exactly).
+// Shared-memory layout of one block.
+//   Full shell (variants 6 and 8): header, pair table, hstart[rows][HZ + 1] (16 bits), hslot[HC],
+//   then per staged bead, beads in pairs (2k, 2k + 1): xy = {x, x', y, y'} per pair, zf = the
+//   bead's z in brick coordinates, vel = {v, hash}, zc = {z offset, halo cell}; then
+//   seg[SEG_MAX][threads].
+//   Half shell: header, pair table, hstart[HC+1], hslot[HC], hlo[HC], pos[maxb], vel[maxb],
+//   list[cap][threads], hidx[maxb] (home index of a staged bead, NOT_HOME for a halo bead),
+//   hsi[home_max] (staged index of a home bead) and acc[6][home_max] (fixed-point force sums of
+//   the home beads: per axis a word of the terms' low 16 bits and a word of their high parts, so
+//   that 32-bit atomics add them exactly).
 struct BrickLayout {
-    uint32_t hc_max, maxb, home_max, list_cap;
+    uint32_t hc_max, maxb, home_max;
     uint32_t off_pair, off_hstart, off_hslot, off_hlo, off_pos, off_vel, off_list, off_hidx, off_hsi,
-        off_acc, bytes;
+        off_acc, off_zf, off_zc, bytes;
 };
 
 inline uint32_t brick_variant_threads(int variant)
@@ -72,40 +78,46 @@ inline uint32_t brick_variant_threads(int variant)
     return variant == 8 ? BRICK_THREADS_WIDE : (variant == 9 ? HALF_THREADS : BRICK_THREADS);
 }
 
+// Bytes of shared memory per staged bead.
+constexpr uint32_t FULL_BEAD_BYTES = 36, HALF_BEAD_BYTES = 34;
+
 // npair: the largest n_types^2 of the attached worlds (the staged pair table); home_max: the
 // home-bead capacity of the half-shell variant (0 for the full-shell variants).
 __host__ __device__ inline BrickLayout brick_layout(uint32_t hc_max, uint32_t maxb, uint32_t npair,
                                                     uint32_t threads, uint32_t home_max)
 {
-    BrickLayout L;
+    BrickLayout L{};
     L.hc_max = hc_max;
     L.maxb = maxb;
     L.home_max = home_max;
-    L.list_cap = home_max ? HLIST_MAX : BLIST_MAX;
     uint32_t off = (uint32_t)((sizeof(BrickHeader) + 15) & ~size_t(15));
-    L.off_pair = off;
-    off += 8 * npair;
-    off = (off + 15) & ~15u;
-    L.off_hstart = off;
-    off += 4 * (hc_max + 1);
-    L.off_hslot = off;
-    off += 4 * hc_max;
-    L.off_hlo = off;
-    off += 2 * hc_max;
-    off = (off + 15) & ~15u;
-    L.off_pos = off;
-    off += 16 * maxb;
-    L.off_vel = off;
-    off += 16 * maxb;
-    L.off_list = off;
-    off += 2 * L.list_cap * threads;
-    L.off_hidx = off;
-    if (home_max) off += 2 * maxb;
-    L.off_hsi = off;
-    if (home_max) off += 2 * home_max;
-    off = (off + 15) & ~15u;
-    L.off_acc = off;
-    if (home_max) off += 24 * home_max;
+    auto take = [&](uint32_t bytes) {
+        const uint32_t at = off;
+        off = (off + bytes + 15) & ~15u;
+        return at;
+    };
+    L.off_pair = take(8 * npair);
+    if (home_max) {
+        L.off_hstart = take(4 * (hc_max + 1));
+        L.off_hslot = take(4 * hc_max);
+        L.off_hlo = take(2 * hc_max);
+        L.off_pos = take(16 * maxb);
+        L.off_vel = take(16 * maxb);
+        L.off_list = take(2 * HLIST_MAX * threads);
+        L.off_hidx = take(2 * maxb);
+        L.off_hsi = take(2 * home_max);
+        L.off_acc = take(24 * home_max);
+    } else {
+        maxb = (maxb + 3) & ~3u;
+        L.off_hstart = take(3 * hc_max);  // 16 bits for HZ + 1 <= 4/3 HZ entries of each row
+        L.off_hslot = take(4 * hc_max);
+        L.off_hlo = take(4 * (hc_max / 3));  // the rows' bases (HZ >= 3)
+        L.off_pos = take(8 * maxb);
+        L.off_zf = take(4 * maxb);
+        L.off_vel = take(16 * maxb);
+        L.off_zc = take(8 * maxb);
+        L.off_list = take(4 * (SEG_MAX + 1) * threads);
+    }
     L.bytes = off;
     return L;
 }
@@ -128,38 +140,6 @@ __device__ __forceinline__ int home_row_of(const uint32_t *rows, int nr, uint32_
     return lo;
 }
 
-// Evaluate list entries [0, n) of this thread in order, adding to F (variants 6 and 8): an
-// entry is a staged index of an in-range neighbour, and the neighbour direction is the
-// difference of the two beads' staged halo cells (vi is the home bead's staged velocity); the
-// separation is recomputed exactly as the walk computed it.
-template <int T>
-__device__ __forceinline__ void brick_rows_eval(const float4 *__restrict__ spos,
-                                                const float4 *__restrict__ svel,
-                                                const uint16_t *__restrict__ list, int n,
-                                                const float4 pi, const float4 vi,
-                                                const float2 *pair, uint32_t nt, uint32_t th_lo,
-                                                uint32_t th_hi, float scale, float F[3])
-{
-    const uint32_t hi = __float_as_uint(pi.w);
-    const uint32_t ti = min(hi >> 28, nt - 1u);
-    const uint32_t hc = staged_cell(vi);
-    const int hx = (int)(hc & 255u), hy = (int)((hc >> 8) & 255u), hz = (int)(hc >> 16);
-    for (int k = 0; k < n; k++) {
-        const uint32_t j = list[k * T + threadIdx.x];
-        const float4 pj = spos[j];
-        const float4 vj = svel[j];
-        const uint32_t cj = staged_cell(vj);
-        const float ax = __fsub_rn(pi.x, (float)((int)(cj & 255u) - hx));
-        const float ay = __fsub_rn(pi.y, (float)((int)((cj >> 8) & 255u) - hy));
-        const float az = __fsub_rn(pi.z, (float)((int)(cj >> 16) - hz));
-        float dx, dy, dz;
-        const float r2 = pair_r2(ax, ay, az, pj, dx, dy, dz);
-        const uint32_t hj = __float_as_uint(pj.w);
-        pair_accumulate(dx, dy, dz, r2, vi, vj, hi, hj, pair[ti * nt + min(hj >> 28, nt - 1u)],
-                        th_lo, th_hi, scale, F);
-    }
-}
-
 // 16-byte asynchronous global-to-shared copy (cp.async, no register round trip) and the wait
 // for all of this thread's copies.  Both addresses are 16-byte aligned (float4 arrays).
 __device__ __forceinline__ void cp_async16(float4 *dst_shared, const float4 *src_global)
@@ -173,7 +153,7 @@ __device__ __forceinline__ void cp_async_wait_all()
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Halo setup and staging of one brick, block-wide (ends with __syncthreads):
+// Half shell: halo setup and staging of one brick, block-wide (ends with __syncthreads):
 //   hstart[hc] = first staged index of halo cell hc (hc = (hx * HY + hy) * HZ + hz, z fastest),
 //   hstart[HC] = total, hslot[hc] = its first slot in the sorted state, hlo[hc] = its beads in
 //   the lower z half, H.home_rows[r] = first home index of home (x, y) row r, and, if the halo
@@ -297,77 +277,216 @@ __device__ __forceinline__ void brick_halo_and_stage(const KArgs &a, const World
     n_home = H.home_rows[br.bx * br.by];
 }
 
-// Full-shell row walk of one staged home bead (variants 6 and 8): the 9 neighbour rows (dx, dy)
-// in order; a row's 3 cells (dz = -1, 0, +1) are one contiguous range of staged beads, trimmed
-// at its ends by the same conservative test as the per-cell loop (and by the far z half of an
-// end cell: a cell's beads with z offset < 0.5 come first, hlo counts them).  The warp pays the
-// longest row of its lanes 9 times instead of the longest cell 27 times.  The in-range
-// candidates (the reference's test, update_bead_pair, on the walk's separation) go to this
-// thread's list, as staged indices, in the direction order; room for a
-// whole row is made before the row (the list is evaluated into F first when it could
-// overflow), so the candidate loop has no capacity check and no branch.  Returns the number
-// of entries left in the list.
-template <int T>
-__device__ __forceinline__ int brick_rows_collect(const float4 *__restrict__ spos,
-                                                  const float4 *__restrict__ svel,
-                                                  uint16_t *__restrict__ list, int cap,
-                                                  const uint32_t *__restrict__ hstart,
-                                                  const uint16_t *__restrict__ hlo, int HY, int HZ,
-                                                  int hx, int hy, int hz, const float4 pi,
-                                                  const float4 vi, const float2 *pair, uint32_t nt,
-                                                  uint32_t th_lo, uint32_t th_hi, float scale,
-                                                  float F[3])
+// Two FP32 values per 64-bit register, one instruction for both (sm_100 packed FP32: each half
+// rounded as the scalar operation).
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi)
 {
-    const float PRUNE = 1.0001f;
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// The same for all lanes of a warp at t = t0 + lane: the lanes compare the row starts with t0,
+// and each lane moves on from the row that this gives.
+__device__ __forceinline__ int home_row_near(const uint32_t *rows, int nr, uint32_t t0, uint32_t t)
+{
+    const int lane = threadIdx.x & 31;
+    int r = -1;
+    for (int q = 0; q < nr; q += 32)
+        r += __popc(__ballot_sync(0xffffffffu, q + lane < nr && rows[q + lane] <= t0));
+    while (r + 1 < nr && rows[r + 1] <= t) r++;
+    return r;
+}
+
+// The staged beads of a full-shell brick (BrickLayout): xy[2k] .. is the pair (2k, 2k + 1).
+struct Staged {
+    const ulonglong2 *xy;  // per pair {x, x'}, {y, y'}: offsets inside their cells
+    const uint64_t *zf;    // per pair {z, z'} in brick coordinates (halo cell + offset, rounded)
+    const float4 *vel;     // velocity, hash
+    const float2 *zc;      // z offset, halo cell code hx | hy << 8 | hz << 16
+};
+
+constexpr float WALK_R2 = 1.0001f;
+constexpr uint32_t SEG_BEADS = 20;      // candidates of one walk segment
+constexpr uint32_t SEG_BASE = 0xfffu;   // low 12 bits of a segment: its first pair
+constexpr uint32_t FULL_MAX_STAGED = 2 * SEG_BASE;
+
+// A halo coordinate (byte k of the code) as a float: the byte becomes the low mantissa bits of
+// 2^23 + v, and the difference of two of these is exact.
+template <int K> __device__ __forceinline__ float code_axis(uint32_t code)
+{
+    return __uint_as_float(__byte_perm(code, 0x4B000000u, 0x7440 + K));
+}
+
+// Evaluate the n_cand candidates of this thread's walk segments in order, adding to F: a
+// segment is 20 candidates' in-range bits (bit 31 the first) over the index of their first
+// staged pair, and has at least one bit.  The walk's test is conservative; the exact one (the
+// reference's update_bead_pair) is here, on the separation of the other full-shell paths.  The
+// direction is the difference of the two beads' halo cells.  The next segment is read ahead, so
+// that moving on to it takes no branch (segs has an entry more than the walk fills).
+template <int T>
+__device__ __forceinline__ void segs_eval(const Staged &st, const uint32_t *__restrict__ segs, int n_cand,
+                                          const float4 pi, const float4 vi, uint32_t code,
+                                          const float2 *pair, uint32_t nt, uint32_t th_lo, uint32_t th_hi,
+                                          float scale, float F[3])
+{
     const float min2 = min_dist_sqr_f();
-    const float azm = __fsub_rn(pi.z, -1.0f), azp = __fsub_rn(pi.z, 1.0f);
-    const float gzm = pi.z, gzp = 1.0f - pi.z;
-    // gaps to the far halves of the end cells: the lower half of the cell below (z offsets
-    // < 0.5) and the upper half of the cell above (>= 0.5)
-    const float gzm2 = pi.z + 0.5f, gzp2 = 1.5f - pi.z;
-    int n = 0;
-#pragma unroll 1
-    for (int rr = 0; rr < 9; rr++) {
-        const int ddx = rr / 3 - 1, ddy = rr - (rr / 3) * 3 - 1;
-        const float gx = slab_gap(pi.x, ddx), gy = slab_gap(pi.y, ddy);
-        const float gxy = gx * gx + gy * gy;
-        if (gxy >= PRUNE) continue;
-        const int rowc = ((hx + ddx) * HY + (hy + ddy)) * HZ + hz;
-        const uint32_t c1 = hstart[rowc], c2 = hstart[rowc + 1];
-        const uint32_t c0 = hstart[rowc - 1], c3 = hstart[rowc + 2];
-        const uint32_t j0 = gxy + gzm * gzm >= PRUNE ? c1 : (gxy + gzm2 * gzm2 >= PRUNE ? c0 + hlo[rowc - 1] : c0);
-        const uint32_t j1 = gxy + gzp * gzp >= PRUNE ? c2 : (gxy + gzp2 * gzp2 >= PRUNE ? c2 + hlo[rowc + 1] : c3);
-        const float ax = __fsub_rn(pi.x, (float)ddx), ay = __fsub_rn(pi.y, (float)ddy);
-        if (n + (int)(j1 - j0) > cap) {  // room for the whole row, or evaluate the list first
-            brick_rows_eval<T>(spos, svel, list, n, pi, vi, pair, nt, th_lo, th_hi, scale, F);
-            n = 0;
+    const uint32_t hi = __float_as_uint(pi.w);
+    const float2 *row = pair + (hi >> 28) * nt;
+    const float cx = code_axis<0>(code), cy = code_axis<1>(code), cz = code_axis<2>(code);
+    const float *xy = (const float *)st.xy;
+    uint32_t w = 0, next = segs[0];
+    for (; n_cand > 0; n_cand--) {
+        if (w <= SEG_BASE) {  // no candidate left in the segment
+            w = next;
+            segs += T;
         }
-        if ((int)(j1 - j0) <= cap) {
-#pragma unroll 2
-            for (uint32_t j = j0; j < j1; j++) {
-                const float4 pj = spos[j];
-                const float az = j < c1 ? azm : (j < c2 ? pi.z : azp);
-                float dx, dy, dz;
-                const float r2 = pair_r2(ax, ay, az, pj, dx, dy, dz);
-                list[n * T + threadIdx.x] = (uint16_t)j;
-                n += (r2 < 1.0f && r2 >= min2) ? 1 : 0;
-            }
-        } else {
-            for (uint32_t j = j0; j < j1; j++) {
-                const float4 pj = spos[j];
-                const float az = j < c1 ? azm : (j < c2 ? pi.z : azp);
-                float dx, dy, dz;
-                const float r2 = pair_r2(ax, ay, az, pj, dx, dy, dz);
-                list[n * T + threadIdx.x] = (uint16_t)j;
-                n += (r2 < 1.0f && r2 >= min2) ? 1 : 0;
-                if (n == cap) {
-                    brick_rows_eval<T>(spos, svel, list, n, pi, vi, pair, nt, th_lo, th_hi, scale, F);
-                    n = 0;
+        next = segs[0];
+        uint32_t b;
+        asm("bfind.u32 %0, %1;" : "=r"(b) : "r"(w));
+        const uint32_t j = 2 * (w & SEG_BASE) + 31 - b;
+        w ^= 1u << b;
+        const float *pj = xy + 2 * j - (j & 1u);
+        const float2 zc = st.zc[j];
+        const float4 vj = st.vel[j];
+        const uint32_t cj = __float_as_uint(zc.y);
+        const float dx = __fsub_rn(__fsub_rn(pi.x, __fsub_rn(code_axis<0>(cj), cx)), pj[0]);
+        const float dy = __fsub_rn(__fsub_rn(pi.y, __fsub_rn(code_axis<1>(cj), cy)), pj[2]);
+        const float dz = __fsub_rn(__fsub_rn(pi.z, __fsub_rn(code_axis<2>(cj), cz)), zc.x);
+        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+        if (r2 < 1.0f && r2 >= min2) {
+            const uint32_t hj = __float_as_uint(vj.w);
+            pair_accumulate(dx, dy, dz, r2, vi, vj, hi, hj, row[hj >> 28], th_lo, th_hi, scale, F);
+        }
+    }
+}
+
+// The evaluation as a call, for the rare bead whose segments do not fit (several rows of more
+// than 20 candidates): returns the new F.
+template <int T>
+__device__ __noinline__ float3 segs_eval_call(Staged st, const uint32_t *segs, int n_cand, float4 pi, float4 vi,
+                                              uint32_t code, const float2 *pair, uint32_t nt, uint32_t th_lo,
+                                              uint32_t th_hi, float scale, float3 F3)
+{
+    float F[3] = {F3.x, F3.y, F3.z};
+    segs_eval<T>(st, segs, n_cand, pi, vi, code, pair, nt, th_lo, th_hi, scale, F);
+    return make_float3(F[0], F[1], F[2]);
+}
+
+// The in-range bits of the nv <= SEG_BEADS candidates from staged index p (even), the first in
+// bit 31: two candidates per packed FP32 instruction, the sign of r^2 - WALK_R2 shifted into
+// the mask, four candidates a turn (those past nv are masked out).
+__device__ __forceinline__ uint32_t walk_mask(const Staged &st, uint32_t p, uint32_t nv, uint64_t nx, uint64_t ny,
+                                              uint64_t nz, uint64_t m_r2)
+{
+    const ulonglong2 *xy = st.xy + (p >> 1);
+    const uint64_t *zf = st.zf + (p >> 1);
+    uint32_t m = 0, done = 0;
+#pragma unroll 1
+    do {
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            const ulonglong2 a = xy[q];
+            const uint64_t dx = add_f32x2(a.x, nx), dy = add_f32x2(a.y, ny), dz = add_f32x2(zf[q], nz);
+            const uint64_t r = fma_f32x2(dz, dz, fma_f32x2(dy, dy, fma_f32x2(dx, dx, m_r2)));
+            m = __funnelshift_l((uint32_t)r, m, 1);
+            m = __funnelshift_l((uint32_t)(r >> 32), m, 1);
+        }
+        xy += 2;
+        zf += 2;
+        done += 4;
+    } while (done < nv);
+    return (m << (32 - done)) & (uint32_t)((int)0x80000000 >> (int)(nv - 1));
+}
+
+// Full-shell pair forces of one staged home bead (variants 6 and 8), at staged index si.
+//
+// The 9 neighbour rows (dx, dy) in order; a row's 3 cells (dz = -1, 0, +1) are one contiguous
+// range of staged beads, a whole end cell left out where its nearest face is >= 1 away.  The
+// kernel is bound by instruction issue, so the walk spends as few instructions per candidate as
+// it can: it tests two candidates per packed instruction, on z in brick coordinates (no choice
+// of the direction per candidate), and keeps the results as bits instead of list entries: 13
+// instructions for two candidates, where a loop that tested each exactly and stored list
+// entries took about 36.  The test is conservative (brick coordinates below 36 are rounded to
+// 2^-19, so r^2 of a pair in range is off by < 1.2e-5) and the exact one follows in segs_eval,
+// so the pairs evaluated and their order are those of the other full-shell paths.  A candidate
+// of a left-out cell and the filler of an odd row fail the test.  A lane whose row lies out of
+// reach walks it all the same: the warp takes as long as its longest lane.  Force pass of the
+// 128^3 box: 1.14 -> 0.94 ms per step, 186 -> 140 warp instructions per bead.
+template <int T>
+__device__ __forceinline__ void rows_forces(const Staged &st, uint32_t *__restrict__ segs, int cap,
+                                            const uint16_t *__restrict__ hstart, int HY, int HZ1, uint32_t code,
+                                            uint32_t si, const float4 pi, const float4 vi, const float2 *pair,
+                                            uint32_t nt, uint32_t th_lo, uint32_t th_hi, float scale, float F[3])
+{
+    const int hx = (int)(code & 255u), hy = (int)((code >> 8) & 255u), hz = (int)(code >> 16);
+    const float gzm = pi.z, gzp = 1.0f - pi.z;
+    const float below = WALK_R2 - gzm * gzm, above = WALK_R2 - gzp * gzp;
+    const float zi = -((const float *)st.zf)[si];
+    const uint64_t nz = f32x2(zi, zi), m_r2 = f32x2(-WALK_R2, -WALK_R2);
+    const uint16_t *h = hstart + ((hx - 1) * HY + (hy - 1)) * HZ1 + hz;
+    uint32_t *out = segs;
+    const uint32_t *const full = segs + (cap - 3) * T;  // room for the first segments of three rows
+    int n_cand = 0;
+#pragma unroll 1
+    for (int ddx = -1; ddx <= 1; ddx++) {
+        const float gx = slab_gap(pi.x, ddx), nax = (float)ddx - pi.x;
+        const uint64_t nx = f32x2(nax, nax);
+#pragma unroll
+        for (int ddy = -1; ddy <= 1; ddy++) {
+            const float gy = slab_gap(pi.y, ddy);
+            const float gxy = gx * gx + gy * gy;
+            const uint32_t j1 = h[gxy >= above ? 1 : 2];
+            uint32_t p = h[gxy >= below ? 0 : -1] & ~1u;
+            h += HZ1;
+            const float nay = (float)ddy - pi.y;
+            const uint64_t ny = f32x2(nay, nay);
+            while (p < j1) {
+                uint32_t m = walk_mask(st, p, min(j1 - p, SEG_BEADS), nx, ny, nz, m_r2);
+                if (ddy == 0 && ddx == 0 && si - p < SEG_BEADS) m &= ~(0x80000000u >> (si - p));  // not itself
+                if (m) {
+                    *out = m | (p >> 1);
+                    out += T;
+                    n_cand += __popc(m);
+                }
+                p += SEG_BEADS;
+                if (p < j1 && out > full) {
+                    const float3 G = segs_eval_call<T>(st, segs, n_cand, pi, vi, code, pair, nt, th_lo, th_hi, scale,
+                                                       make_float3(F[0], F[1], F[2]));
+                    F[0] = G.x;
+                    F[1] = G.y;
+                    F[2] = G.z;
+                    out = segs;
+                    n_cand = 0;
                 }
             }
         }
+        h += (HY - 3) * HZ1;
+        if (ddx < 1 && out > full) {
+            const float3 G = segs_eval_call<T>(st, segs, n_cand, pi, vi, code, pair, nt, th_lo, th_hi, scale,
+                                               make_float3(F[0], F[1], F[2]));
+            F[0] = G.x;
+            F[1] = G.y;
+            F[2] = G.z;
+            out = segs;
+            n_cand = 0;
+        }
     }
-    return n;
+    segs_eval<T>(st, segs, n_cand, pi, vi, code, pair, nt, th_lo, th_hi, scale, F);
 }
 
 // One home bead of a brick whose halo does not fit in shared memory: pair forces gathered
@@ -390,6 +509,142 @@ __device__ __forceinline__ void brick_fallback_bead(const KArgs &a, const WorldD
     integrate32<FINAL>(a, w, s, c, ph, vh, F, err);
 }
 
+// Halo setup and staging of one brick for the full-shell kernels, block-wide (ends with
+// __syncthreads).  Rows (hx, hy) of halo cells, HZ cells each, start at even staged indices (a
+// filler far away pads an odd row), so a pair of staged beads never spans two rows:
+//   hstart[row * (HZ + 1) + z] = first staged index of halo cell (row, z), the last entry the
+//   row's end; hslot[row * HZ + z] = the cell's first slot in the sorted state;
+//   H.home_rows[r] = first home index of home row r; total = staged beads with the fillers.
+// If the halo fits (total <= maxb) the beads are staged; else hstart holds nothing of use.  Halo
+// coordinates lie in [-1, L] (bricks are cut at the box faces), so each wraps with one
+// conditional add or subtract.
+template <int T>
+__device__ __forceinline__ void brick_stage_rows(const KArgs &a, const WorldDev &w, const Brick &br,
+                                                 BrickHeader &H, uint16_t *hstart, uint32_t *hslot,
+                                                 uint32_t *rowbase, float *xy, float *zf, float4 *svel,
+                                                 float2 *zc, uint32_t maxb, uint32_t &total, uint32_t &n_home)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int HX = br.bx + 2, HY = br.by + 2, HZ = br.bz + 2, HZ1 = HZ + 1;
+    const int rows = HX * HY;
+    const int L0 = w.L[0], L1 = w.L[1], L2 = w.L[2];
+    auto row_cell0 = [&](int hx, int hy) {  // global cell (hx, hy, 0) of a halo row
+        int gx = br.x0 - 1 + hx, gy = br.y0 - 1 + hy;
+        gx += gx < 0 ? L0 : 0;
+        gx -= gx >= L0 ? L0 : 0;
+        gy += gy < 0 ? L1 : 0;
+        gy -= gy >= L1 ? L1 : 0;
+        return w.cell_base + ((uint32_t)gx * (uint32_t)L1 + (uint32_t)gy) * (uint32_t)L2;
+    };
+
+    // the counts of each row's cells, their prefix in the row, and the row's total: a warp
+    // takes as many whole rows as it has lanes for, one lane per cell
+    const int group = max(1, 32 / HZ);
+    const int sub = lane / HZ, z = lane - sub * HZ;  // (a row of 33 or 34 cells: two turns, below)
+    for (int r0 = warp * group; r0 < rows; r0 += (T / 32) * group) {
+        const int row = r0 + (HZ > 32 ? 0 : sub);
+        const int hx = row / HY, hy = row - hx * HY;
+        const bool act = (HZ > 32 || sub < group) && row < rows;
+        const uint32_t cell0 = act ? row_cell0(hx, hy) : 0u;
+        uint32_t carry = 0, first_home = 0;
+        for (int z0 = 0; z0 < HZ; z0 += 32) {
+            const int zz = HZ > 32 ? z0 + lane : z;
+            const bool on = act && zz < HZ;
+            uint32_t n = 0;
+            if (on) {
+                int gz = br.z0 - 1 + zz;
+                gz += gz < 0 ? L2 : 0;
+                gz -= gz >= L2 ? L2 : 0;
+                const uint32_t s0 = a.start[cell0 + (uint32_t)gz];
+                n = a.start[cell0 + (uint32_t)gz + 1] - s0;
+                hslot[row * HZ + zz] = s0;
+            }
+            uint32_t inc = n;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+                if ((HZ > 32 ? lane : z) >= off) inc += y;
+            }
+            inc += carry;
+            if (on) {
+                uint16_t *h = hstart + row * HZ1;
+                if (zz == 0) h[0] = 0;
+                h[zz + 1] = (uint16_t)inc;
+                if (zz == HZ - 1) rowbase[row] = inc;
+            }
+            if (z0 == 0) first_home = __shfl_sync(0xffffffffu, inc, HZ > 32 ? 0 : sub * HZ);
+            if (on && zz == br.bz && hx >= 1 && hx <= br.bx && hy >= 1 && hy <= br.by)
+                H.home_rows[(hx - 1) * br.by + (hy - 1)] = inc - first_home;
+            carry = HZ > 32 ? __shfl_sync(0xffffffffu, inc, 31) : 0u;
+        }
+    }
+    __syncthreads();
+    // warp 0: the rows' staged bases (even) and their total; warp 1: the home rows' prefix
+    if (warp < 2) {
+        uint32_t *v = warp == 0 ? rowbase : H.home_rows;
+        const int m = warp == 0 ? rows : br.bx * br.by;
+        uint32_t carry = 0;
+        for (int r0 = 0; r0 < m; r0 += 32) {
+            const int r = r0 + lane;
+            uint32_t c = r < m ? v[r] : 0u;
+            if (warp == 0) c = (c + 1u) & ~1u;
+            uint32_t inc = c;
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+                if (lane >= off) inc += y;
+            }
+            if (r < m) v[r] = carry + inc - c;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) {
+            if (warp == 0) H.total = carry;
+            else H.home_rows[m] = carry;
+        }
+    }
+    __syncthreads();
+    total = H.total;
+    n_home = H.home_rows[br.bx * br.by];
+    if (total <= maxb) {
+        // A row's slots are one run, or at a periodic wrap of z its first or last cell is a run of
+        // its own; a bead's halo cell follows from its stored cell.
+        const bool wrap_lo = br.z0 == 0, wrap_hi = br.z0 + br.bz == L2;
+        const float4 *pos = (const float4 *)a.posA, *vel = (const float4 *)a.velA;
+        int hx = warp / HY, hy = warp - hx * HY;
+        for (int row = warp; row < rows; row += T / 32) {
+            uint16_t *h = hstart + row * HZ1;
+            const uint32_t *hs = hslot + row * HZ;
+            const uint32_t base = rowbase[row], len = h[HZ];
+            const uint32_t n_lo = wrap_lo ? h[1] : 0u, end_mid = wrap_hi ? h[HZ - 1] : len;
+            const uint32_t s_lo = hs[0], s_mid = wrap_lo ? hs[1] - n_lo : s_lo, s_hi = hs[HZ - 1] - end_mid;
+            const uint32_t rowcell = (uint32_t)hx | ((uint32_t)hy << 8);
+            const int z_off = 1 - br.z0 - (int)row_cell0(hx, hy);
+            for (uint32_t k = lane; k < ((len + 1u) & ~1u); k += 32) {
+                const uint32_t j = base + k;
+                float4 p = make_float4(1.0e4f, 1.0e4f, 1.0e4f, 0.f);  // the filler
+                if (k < len) {
+                    const uint32_t slot = k + (k < n_lo ? s_lo : (k < end_mid ? s_mid : s_hi));
+                    p = pos[slot];
+                    const float4 v = vel[slot];
+                    int zz = (int)a.cellg[slot] + z_off;
+                    zz = k < n_lo ? 0 : (k < end_mid ? zz : HZ - 1);
+                    svel[j] = make_float4(v.x, v.y, v.z, p.w);
+                    zc[j] = make_float2(p.z, __uint_as_float(rowcell | ((uint32_t)zz << 16)));
+                    p.z += (float)zz;
+                }
+                float *q = xy + 2 * j - (j & 1u);
+                q[0] = p.x;
+                q[2] = p.y;
+                zf[j] = p.z;
+            }
+            __syncwarp();
+            for (int c = lane; c <= HZ; c += 32) h[c] = (uint16_t)(h[c] + base);
+            for (hy += T / 32; hy >= HY; hy -= HY) hx++;
+        }
+    }
+    __syncthreads();
+}
+
 // Full-shell brick kernel (variants 6 and 8): one thread per home bead.
 template <int FINAL, int T>
 __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_brick(KArgs a, BrickLayout lay)
@@ -397,16 +652,19 @@ __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BrickHeader &H = *reinterpret_cast<BrickHeader *>(smem_raw);
     float2 *spair = reinterpret_cast<float2 *>(smem_raw + lay.off_pair);
-    uint32_t *hstart = reinterpret_cast<uint32_t *>(smem_raw + lay.off_hstart);
+    uint16_t *hstart = reinterpret_cast<uint16_t *>(smem_raw + lay.off_hstart);
     uint32_t *hslot = reinterpret_cast<uint32_t *>(smem_raw + lay.off_hslot);
-    uint16_t *hlo = reinterpret_cast<uint16_t *>(smem_raw + lay.off_hlo);
-    float4 *spos = reinterpret_cast<float4 *>(smem_raw + lay.off_pos);
+    uint32_t *rowbase = reinterpret_cast<uint32_t *>(smem_raw + lay.off_hlo);
+    float *xy = reinterpret_cast<float *>(smem_raw + lay.off_pos);
+    float *zf = reinterpret_cast<float *>(smem_raw + lay.off_zf);
     float4 *svel = reinterpret_cast<float4 *>(smem_raw + lay.off_vel);
-    uint16_t *list = reinterpret_cast<uint16_t *>(smem_raw + lay.off_list);
+    float2 *zc = reinterpret_cast<float2 *>(smem_raw + lay.off_zc);
     const int tid = threadIdx.x;
+    uint32_t *segs = reinterpret_cast<uint32_t *>(smem_raw + lay.off_list) + tid;
+    const int cap = (a.list_capacity > 0 && a.list_capacity < SEG_MAX) ? max(3, a.list_capacity) : SEG_MAX;
+    const Staged st{reinterpret_cast<const ulonglong2 *>(xy), reinterpret_cast<const uint64_t *>(zf), svel, zc};
     if (tid == 0) H.wc.world = 0xffffffffu;
     __syncthreads();
-    const int cap = (a.list_capacity > 0 && a.list_capacity < BLIST_MAX) ? a.list_capacity : BLIST_MAX;
     for (uint32_t bi = blockIdx.x; bi < a.n_bricks; bi = brick_fetch(a, H)) {
         const Brick br = a.bricks[bi];
         load_world(a, br.world, H.wc, spair);
@@ -419,30 +677,32 @@ __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_
         const int HY = br.by + 2, HZ = br.bz + 2;
 
         uint32_t total = 0, n_home = 0;
-        brick_halo_and_stage<T>(a, w, br, H, hstart, hslot, hlo, spos, svel, lay.maxb, total, n_home);
+        brick_stage_rows<T>(a, w, br, H, hstart, hslot, rowbase, xy, zf, svel, zc, lay.maxb, total, n_home);
         const bool staged = total <= lay.maxb;
 
         uint32_t err = 0;
-        for (uint32_t t = tid; t < n_home; t += T) {
-            const int r = home_row_of(H.home_rows, br.bx * br.by, t);
+        for (uint32_t t0 = tid & ~31; t0 < n_home; t0 += T) {
+            const uint32_t t = t0 + (tid & 31);
+            const int r = home_row_near(H.home_rows, br.bx * br.by, t0, t);
+            if (t >= n_home) continue;
             const int lx = r / br.by, ly = r - lx * br.by;
-            const int hx = lx + 1, hy = ly + 1;
-            const int hc0 = (hx * HY + hy) * HZ + 1;
+            const int row = (lx + 1) * HY + (ly + 1);
             const uint32_t k = t - H.home_rows[r];
-            const uint32_t s = hslot[hc0] + k;
+            const uint32_t s = hslot[row * HZ + 1] + k;
             if (!staged) {  // halo larger than the shared-memory budget: gather from global memory
                 brick_fallback_bead<FINAL, 0>(a, w, spair, th_lo, th_hi, scale, s, err);
                 continue;
             }
-            const uint32_t si = hstart[hc0] + k;
-            int z = 0;
-            while (hstart[hc0 + z + 1] <= si) z++;
-            const float4 pi = spos[si], vi = svel[si];
+            const uint32_t si = hstart[row * (HZ + 1) + 1] + k;
+            const float *q = xy + 2 * si - (si & 1u);
+            const float2 z = zc[si];
+            const float4 vi = svel[si];
+            const float4 pi = make_float4(q[0], q[2], z.x, vi.w);
+            const uint32_t code = __float_as_uint(z.y);
             float F[3] = {0.f, 0.f, 0.f};
-            const int nl = brick_rows_collect<T>(spos, svel, list, cap, hstart, hlo, HY, HZ, hx, hy, z + 1, pi, vi,
-                                                 spair, nt, th_lo, th_hi, scale, F);
-            brick_rows_eval<T>(spos, svel, list, nl, pi, vi, spair, nt, th_lo, th_hi, scale, F);
-            const int c[3] = {br.x0 + lx, br.y0 + ly, br.z0 + z};
+            rows_forces<T>(st, segs, cap, hstart, HY, HZ + 1, code, si, pi, vi, spair, nt, th_lo, th_hi, scale, F);
+            const int c[3] = {br.x0 - 1 + (int)(code & 255u), br.y0 - 1 + (int)((code >> 8) & 255u),
+                              br.z0 - 1 + (int)(code >> 16)};
             integrate32<FINAL>(a, w, s, c, pi, vi, F, err);
         }
         if (err) atomicOr(&a.worlds[br.world].err, err);
