@@ -54,8 +54,10 @@ __global__ void k_place_terms(const uint32_t *__restrict__ pairs, uint32_t n_bon
     }
 }
 
-// Each bead's terms in (parameter, role) order: an insertion sort (a bead has a few terms).
-__global__ void k_sort_terms(uint32_t n, const uint32_t *__restrict__ row, BondTerm *terms)
+// Each bead's terms in (parameter, role) order: an insertion sort (a bead has a few terms); and
+// the row that each end of the flat lists has come to.
+__global__ void k_sort_terms(uint32_t n, const uint32_t *__restrict__ row, BondTerm *terms, uint32_t n_bonds,
+                             uint32_t *__restrict__ row_of)
 {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= n) return;
@@ -69,6 +71,12 @@ __global__ void k_sort_terms(uint32_t n, const uint32_t *__restrict__ row, BondT
             terms[y] = u;
         }
         terms[y] = v;
+    }
+    if (!row_of) return;
+    for (uint32_t x = r0; x < r1; x++) {
+        const BondTerm v = terms[x];
+        const uint32_t role = v.meta >> 8;
+        row_of[v.param < n_bonds ? 2 * v.param + role : 2 * n_bonds + 3 * (v.param - n_bonds) + role] = x;
     }
 }
 
@@ -97,7 +105,8 @@ __global__ void k_polymer_list(uint32_t n, const uint32_t *__restrict__ hash, co
 }  // namespace
 
 int launch_bond_tables(uint32_t n_beads, const uint32_t *pairs, uint32_t n_bonds, const uint32_t *triples,
-                       uint32_t n_angles, const uint32_t *hash, uint32_t *row, BondTerm *terms, uint32_t *bonded,
+                       uint32_t n_angles, const uint32_t *hash, uint32_t *row, BondTerm *terms, uint32_t *row_of,
+                       uint32_t *bonded,
                        uint32_t *n_bonded, uint32_t *scratch, uint32_t *pos, uint32_t *blocksums, cudaStream_t s)
 {
     int launches = 0;
@@ -113,7 +122,7 @@ int launch_bond_tables(uint32_t n_beads, const uint32_t *pairs, uint32_t n_bonds
         k_set_word<<<1, 1, 0, s>>>(row + n_beads, n_terms);
         cudaMemcpyAsync(scratch, row, sizeof(uint32_t) * (size_t)n_beads, cudaMemcpyDeviceToDevice, s);
         k_place_terms<<<gt, BT, 0, s>>>(pairs, n_bonds, triples, n_angles, scratch, terms);
-        k_sort_terms<<<gb, BT, 0, s>>>(n_beads, row, terms);
+        k_sort_terms<<<gb, BT, 0, s>>>(n_beads, row, terms, n_bonds, row_of);
         launches += 6;
     }
     if (n_beads) {

@@ -226,6 +226,42 @@ struct WorldHost {
     std::shared_ptr<V2Layout> v2;
 };
 
+// Room for the FP64 engine's pair lists of a world: candidates and the pairs its beads evaluate
+// themselves (half of those, and both sides of the pairs across the box's faces), at the world's
+// mean density with a margin for its fluctuations.  Beads that find no room are evaluated without
+// lists, with the same result.
+struct List64Room {
+    double entries = 0, pairs = 0;
+    // one buffer: cursors, a record per bead, entries, pairs, terms
+    size_t off_lrec() const { return 256; }
+    size_t off_list(size_t n_beads) const { return off_lrec() + up(8 * n_beads); }
+    size_t off_pairs(size_t n_beads) const { return off_list(n_beads) + up(4 * (size_t)entries); }
+    size_t off_term(size_t n_beads) const { return off_pairs(n_beads) + up(8 * (size_t)pairs); }
+    size_t bytes(size_t n_beads) const { return off_term(n_beads) + up(24 * (size_t)pairs); }
+    static size_t up(size_t n) { return (n + 255) & ~size_t(255); }
+    void add(double n, const int32_t box[3], bool asym)
+    {
+        const double near = 1.3 * 4.19 * n / ((double)box[0] * box[1] * box[2]);
+        double across = 0;
+        for (int k = 0; k < 3; k++) across += 0.375 / box[k];
+        entries += n * (near + 8);
+        pairs += n * (near * (asym ? 1.0 : 0.5 + 0.5 * std::min(1.0, across)) + 5);
+    }
+};
+
+bool asymmetric(const pdpd_world &w)
+{
+    const uint32_t nt = w.n_bead_types;
+    const uint64_t tables = w.cell_conservative ? (uint64_t)w.box[0] * w.box[1] * w.box[2] : 1;
+    const double *a = w.cell_conservative ? w.cell_conservative : w.conservative;
+    const double *g = w.cell_conservative ? w.cell_dissipative : w.dissipative;
+    for (uint64_t c = 0; c < tables; c++, a += nt * nt, g += nt * nt)
+        for (uint32_t i = 0; i < nt; i++)
+            for (uint32_t j = 0; j < i; j++)
+                if (a[i * nt + j] != a[j * nt + i] || g[i * nt + j] != g[j * nt + i]) return true;
+    return false;
+}
+
 struct ConfigEntry {
     const char *name;
     const char *desc;
@@ -297,6 +333,8 @@ struct pdpd_engine {
     DevBuf d_posA, d_velA, d_frc, d_posB, d_velB, d_frcB;
     DevBuf d_ids, d_cellg, d_slot_of_id, d_keyrank, d_tmp;
     DevBuf d_bond_row, d_bond_terms, d_bond_params, d_pair, d_hash, d_bonded, d_fbond, d_cellpair, d_posf, d_bterm, d_zlo, d_brick_next, d_hash_old;
+    DevBuf d_lists;   // FP64 pair lists (List64Room)
+    DevBuf d_row_of;  // FP64: CSR row of each end of the flat bond lists
     DevBuf d_staging[2];
     HostPinned h_staging[2];
     HostPinned h_meta;  // attach: the flat bond lists and parameter rows, written here and uploaded from here
@@ -359,7 +397,7 @@ struct pdpd_engine {
                           &d_keyrank, &d_tmp, &d_bond_row, &d_bond_terms, &d_bond_params,
                           &d_pair, &d_hash, &d_bonded, &d_fbond, &d_staging[0], &d_staging[1],
                           &d_v2err, &d_cellpair, &d_posf, &d_bterm, &d_zlo, &d_brick_next, &d_hash_old,
-                          &d_hostio, &d_inv, &d_blist, &d_scan};
+                          &d_hostio, &d_inv, &d_blist, &d_scan, &d_lists, &d_row_of};
         for (DevBuf *b : bufs) b->release();
         worlds.clear();
         attached = false;
@@ -487,6 +525,29 @@ struct pdpd_engine {
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];
     }
 
+    // Brick shape and block size of the FP64 list kernel, by the batch's cells per SM as for the
+    // FP32 kernels.
+    void list64_shape(int shape[3])
+    {
+        const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
+        static const int big[3] = {5, 8, 8}, mid[3] = {3, 4, 6}, small[3] = {2, 4, 4};
+        const int *b = per_sm >= 1300 ? big : (per_sm >= 200 ? mid : small);
+        args.block_threads = b == big ? 512 : 128;
+        if (b == big) {  // (a denser batch: smaller bricks, as default_shape)
+            static const int less[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {4, 4, 6}, {3, 4, 4}};
+            b = less[4];
+            for (const auto &c : less) {
+                const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
+                const double mean = max_density * hc;
+                if (mean + 5.0 * std::sqrt(mean) <= (double)list64_maxb_limit(512, hc)) {
+                    b = c;
+                    break;
+                }
+            }
+        }
+        for (int d = 0; d < 3; d++) shape[d] = b[d];
+    }
+
     // Staged beads a brick of hc halo cells should have room for: the mean halo population
     // of the densest world + 6 standard deviations (Poisson), at least 1.2x the mean, + 32.
     double staging_want(uint32_t hc) const
@@ -515,7 +576,9 @@ struct pdpd_engine {
         a.force_kernel = any_spatial() ? 1 : cfg_force_kernel;
         a.bricks = nullptr;
         a.n_bricks = 0;
-        if (fp64() || a.force_kernel == 1) return PDPD_OK;
+        if (fp64() ? !a.list : a.force_kernel == 1) return PDPD_OK;
+        int shape[3] = {cfg_brick[0], cfg_brick[1], cfg_brick[2]};
+        if (fp64()) list64_shape(shape);
         // Each axis of a world is cut into ceil(L / b) bricks of as equal extents as possible
         // (e.g. a side of 9 with b = 4 into 3 + 3 + 3, not 4 + 4 + 1): no extent exceeds the
         // configured one, and no thin remainder brick stages a halo for a few home cells.
@@ -528,8 +591,7 @@ struct pdpd_engine {
         };
         for (uint32_t i = 0; i < worlds.size(); i++) {
             const int32_t *L = worlds[i].dev.L;
-            const std::vector<int> cx = cuts(L[0], cfg_brick[0]), cy = cuts(L[1], cfg_brick[1]),
-                                   cz = cuts(L[2], cfg_brick[2]);
+            const std::vector<int> cx = cuts(L[0], shape[0]), cy = cuts(L[1], shape[1]), cz = cuts(L[2], shape[2]);
             for (size_t a0 = 0; a0 + 1 < cx.size(); a0++)
                 for (size_t a1 = 0; a1 + 1 < cy.size(); a1++)
                     for (size_t a2 = 0; a2 + 1 < cz.size(); a2++)
@@ -547,7 +609,16 @@ struct pdpd_engine {
         if (ce != cudaSuccess) return cuda_fail(ce, "brick table upload");
         a.bricks = d_bricks.as<Brick>();
         a.n_bricks = (uint32_t)bricks.size();
-        a.brick_hc_max = (uint32_t)(cfg_brick[0] + 2) * (cfg_brick[1] + 2) * (cfg_brick[2] + 2);
+        a.brick_hc_max = (uint32_t)(shape[0] + 2) * (shape[1] + 2) * (shape[2] + 2);
+        if (fp64()) {
+            const double most = (double)list64_maxb_limit(a.block_threads, a.brick_hc_max);
+            a.brick_maxb = (uint32_t)std::min(most, std::max(64.0, staging_want(a.brick_hc_max)));
+            const int rc = list64_setup(sm_count, a.block_threads, a.brick_hc_max, a.brick_maxb, &a.brick_grid);
+            if (rc) return fail(PDPD_E_CUDA, "list kernel setup: %s", cudaGetErrorString((cudaError_t)rc));
+            if (cfg_grid_blocks > 0) a.brick_grid = cfg_grid_blocks;
+            drop_graph();
+            return PDPD_OK;
+        }
         a.brick_npair = 1;
         for (const WorldHost &wh : worlds) a.brick_npair = std::max(a.brick_npair, wh.dev.n_types * wh.dev.n_types);
         // staged-bead capacity (staging_want) within the variant's limit; a fuller brick takes
@@ -1129,9 +1200,13 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         for (uint32_t k = 0; w.stationary && k < w.n_bead_types; k++)
             if (w.stationary[k]) d.stationary |= 1u << k;
         d.spatial = w.cell_conservative ? 1u : 0u;
+        d.asym = f64 && asymmetric(w) ? 1u : 0u;
         d.cellpair_base = 0;
         d.dt = w.dt;
         d.scale_inv_sqrt_dt = std::sqrt(24 * 1.0 / w.dt);  // pow_half(24 kT / dt)
+        d.hdt = w.dt * 0.5;
+        d.hdt2 = (w.dt * w.dt) * 0.5;
+        for (int k = 0; k < 3; k++) d.Ld[k] = (double)w.box[k];
         d.seed = w.seed;
         d.t = w.t;
         for (uint32_t b = 0; b < w.n_beads; b += TILE_BEADS)
@@ -1269,11 +1344,23 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     A(e->d_fbond, f64 ? 16 : sizeof(float4) * std::max<uint64_t>(1, nb));
     A(e->d_posf, f64 ? sizeof(float4) * std::max<uint64_t>(1, nb) : 16);
     A(e->d_bterm, f64 ? sizeof(double) * 4 * std::max<uint64_t>(1, n_terms) : 16);
+    A(e->d_row_of, f64 ? sizeof(uint32_t) * std::max<uint64_t>(1, n_terms) : 16);
     A(e->d_staging[0], sizeof(double) * 9 * nb);
     if (ce != cudaSuccess) {
         cudaGetLastError();
         e->release();
         return e->fail(PDPD_E_NOMEM, "device allocation failed: %s", cudaGetErrorString(ce));
+    }
+    // FP64: the pair lists, where they are addressable and there is memory for them (else the
+    // force pass runs without: same results, slower)
+    List64Room room;
+    bool lists = f64 && nb > 0 && nb < (1u << 25);
+    for (uint32_t i = 0; lists && i < n_worlds; i++)
+        if (ws[i].n_beads) room.add((double)ws[i].n_beads, ws[i].box, wdev[i].asym != 0);
+    lists = lists && room.entries < 2e9 && room.pairs < 1e9;
+    if (lists) {
+        lists = e->d_lists.alloc(room.bytes(nb)) == cudaSuccess;
+        if (!lists) cudaGetLastError();
     }
     // Host staging rows of the worlds that come from their descriptors: the whole batch in
     // slot order, or in a re-pack only the new worlds, packed (the kept worlds' rows stay on
@@ -1387,7 +1474,8 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         const uint32_t *d_pairs = e->d_blist.as<uint32_t>();
         e->launches += launch_bond_tables((uint32_t)nb, d_pairs, n_bond_par, d_pairs + 2 * (size_t)n_bond_par,
                                           n_angle_par, e->d_hash.as<uint32_t>(), e->d_bond_row.as<uint32_t>(),
-                                          e->d_bond_terms.as<BondTerm>(), e->d_bonded.as<uint32_t>(),
+                                          e->d_bond_terms.as<BondTerm>(),
+                                          f64 ? e->d_row_of.as<uint32_t>() : nullptr, e->d_bonded.as<uint32_t>(),
                                           e->d_scan.as<uint32_t>() + scan_blocks((uint32_t)nb),
                                           e->d_inv.as<uint32_t>(), e->d_slot_of_id.as<uint32_t>(),
                                           e->d_scan.as<uint32_t>(), s);
@@ -1437,13 +1525,30 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.cellpair = e->d_cellpair.p;
     a.bonded_ids = e->d_bonded.as<uint32_t>();
     a.n_bonded = 0;  // (known once the attach's kernels have run, below)
+    a.bond_list = e->d_blist.as<uint32_t>();
+    a.n_bonds = n_bond_par;
+    a.n_angles = n_angle_par;
+    a.row_of = e->d_row_of.as<uint32_t>();
+    a.hash = e->d_hash.as<uint32_t>();
     a.fbond = e->d_fbond.as<float4>();
     a.posf = f64 ? e->d_posf.as<float4>() : nullptr;
     a.zlo = f64 ? nullptr : e->d_zlo.as<uint16_t>();
-    a.brick_next = f64 ? nullptr : e->d_brick_next.as<uint32_t>();
+    a.brick_next = e->d_brick_next.as<uint32_t>();
     a.bterm = f64 ? e->d_bterm.p : nullptr;
     a.staging = e->d_staging[0].as<double>();
+    if (lists) {
+        char *at = e->d_lists.as<char>();
+        a.list_cursor = (unsigned long long *)at;
+        a.lrec = (uint2 *)(at + room.off_lrec());
+        a.list = (uint32_t *)(at + room.off_list(nb));
+        a.pair_i = (uint32_t *)(at + room.off_pairs(nb));
+        a.pair_j = a.pair_i + (size_t)room.pairs;
+        a.term = (double *)(at + room.off_term(nb));
+        a.list_cap = (uint32_t)room.entries;
+        a.pair_cap = (uint32_t)room.pairs;
+    }
     a.block_threads = 128;
+    a.pair_blocks = 32 * e->sm_count;
     int gb = e->cfg_grid_blocks > 0 ? e->cfg_grid_blocks : 16 * e->sm_count;
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;
@@ -2371,7 +2476,13 @@ size_t job_bytes(const pdpd_world &w, int precision)
     // sorted state A and B, ids / cells / ranks, two id-ordered staging rows, hashes
     const size_t per_bead = precision == PDPD_FP64 ? 424 : 296;
     const size_t cells = (size_t)w.box[0] * w.box[1] * w.box[2];
-    return per_bead * w.n_beads + 12 * cells +
+    size_t lists = 0;
+    if (precision == PDPD_FP64 && w.n_beads) {
+        List64Room room;
+        room.add((double)w.n_beads, w.box, asymmetric(w));
+        lists = room.bytes(w.n_beads);
+    }
+    return per_bead * w.n_beads + lists + 12 * cells +
            48 * (2 * (size_t)w.n_bonds + 3 * (size_t)w.n_angles) + 4096;
 }
 

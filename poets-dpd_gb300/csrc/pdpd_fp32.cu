@@ -15,6 +15,7 @@
 #include <cmath>
 
 #include "pdpd_device.cuh"
+#include "pdpd_walk.cuh"
 
 namespace pdpd {
 namespace {
@@ -195,12 +196,6 @@ constexpr int LIST_MAX = 48;
 __device__ __forceinline__ uint32_t pack_dir(int ddx, int ddy, int ddz)
 {
     return (uint32_t)(ddx + 1) | ((uint32_t)(ddy + 1) << 2) | ((uint32_t)(ddz + 1) << 4);
-}
-
-// Lower bound of the distance from offset o to the neighbour slab in direction d.
-__device__ __forceinline__ float slab_gap(float o, int d)
-{
-    return d == 0 ? 0.0f : (d < 0 ? o : 1.0f - o);
 }
 
 // Separation of a neighbour bead pj from a home position already shifted by the neighbour

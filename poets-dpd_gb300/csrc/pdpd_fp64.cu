@@ -9,12 +9,14 @@
 //
 // State per bead (sorted): pos = (x, y, z, hash as the low bits of w), vel = (v, 0),
 // frc = (f, 0).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
 
 #include "../../include/pdpd_gpu.h"
 #include "pdpd_device.cuh"
+#include "pdpd_walk.cuh"
 
 namespace pdpd {
 namespace {
@@ -50,7 +52,9 @@ __device__ __forceinline__ void load_world(const KArgs &a, uint32_t world, World
 }
 
 // update_pos (dpd_maths_core_half_step.hpp:22-49): x' = (x + v dt) + f (dt dt / 2), with the
-// reference's single periodic wrap.  Returns the global cell of x'.
+// reference's single periodic wrap.  Returns the global cell of x'.  The comparisons are made
+// on the bits (non-negative doubles order as their bits do): an FP64 comparison costs as much
+// as an FP64 addition, which is what the force pass is bound by.
 __device__ __forceinline__ uint32_t advance_position64(const WorldDev &w, double dt, double hdt2,
                                                        double x[3], const double v[3],
                                                        const double f[3], uint32_t &err)
@@ -58,20 +62,23 @@ __device__ __forceinline__ uint32_t advance_position64(const WorldDev &w, double
     int c[3];
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        const double L = (double)w.L[d];
+        const double L = w.Ld[d];
+        const long long Lb = __double_as_longlong(L);
         double xn = x[d] + v[d] * dt + f[d] * hdt2;
-        if (xn < 0) {
+        const long long b = __double_as_longlong(xn);
+        if (b < 0 && (b << 1) != 0) {  // xn < 0 (or a NaN, caught below)
             xn += L;
             if (xn == L) xn = 0;
-        } else if (xn >= L) {
+        } else if (b >= Lb) {  // xn >= L (or a NaN)
             xn -= L;
         }
-        if (!(xn >= 0.0 && xn < L)) {  // moved more than a box, or non-finite
+        const long long e = __double_as_longlong(xn);
+        if (!((e >= 0 && e < Lb) || (e << 1) == 0)) {  // moved more than a box, or non-finite
             err |= ERR_OUT_OF_BOX;
             xn = 0.0;
         }
         x[d] = xn;
-        c[d] = (int)floor(xn);
+        c[d] = (int)xn;  // = floor: xn >= 0
     }
     return w.cell_base + ((uint32_t)c[0] * (uint32_t)w.L[1] + (uint32_t)c[1]) * (uint32_t)w.L[2] +
            (uint32_t)c[2];
@@ -99,80 +106,76 @@ __device__ __forceinline__ void load_x(const Vec4d *__restrict__ pos, uint32_t s
     x[2] = p.z;
 }
 
-// Bond terms of one bead, one per row of its CSR (Hookean bonds, then angle bonds), each
-// evaluated exactly as update_hookean_bond / update_angle_bond
-// (naive_dpd_engine_half_step.hpp:426-483) and calc_angle_force
-// (dpd_maths_core_half_step.hpp:177-229), and stored with the sign it is added with: the
-// force kernel adds the rows in order after the pair forces (F - t == F + (-t) in IEEE
-// arithmetic), which is the reference's order of additions to the bead's force.
-__device__ void bond_terms64(const KArgs &a, const WorldDev &w, uint32_t id, const double xs[3],
-                             uint32_t &err)
+// Bond forces, one thread per Hookean bond or angle bond: each evaluated once, exactly as
+// update_hookean_bond / update_angle_bond (naive_dpd_engine_half_step.hpp:426-483) and
+// calc_angle_force (dpd_maths_core_half_step.hpp:177-229) do, and stored with the sign it is
+// added with at the CSR row of each of its beads (row_of): the force kernel adds a bead's rows in
+// order after the pair forces (F - t == F + (-t) in IEEE arithmetic), which is the reference's
+// order of additions to the bead's force.  (A thread per bead, evaluating each of its terms,
+// took 76 us for the 64^3 box: 2.4 times the terms, and warps that mix both kinds.)
+__device__ __forceinline__ void store_term64(const KArgs &a, uint32_t row, double x, double y, double z)
 {
-    Vec4d *out = (Vec4d *)a.bterm;
+    ((Vec4d *)a.bterm)[a.row_of[row]] = Vec4d{x, y, z, 0.0};
+}
+
+__device__ __forceinline__ void hookean64(const KArgs &a, const WorldDev &w, uint32_t k, uint32_t head,
+                                          uint32_t tail, uint32_t &err)
+{
     const Vec4d *pos = (const Vec4d *)a.posA;
-    const Vec4d *prm_tab = (const Vec4d *)a.bond_params;
-    const uint32_t r0 = a.bond_row[id], r1 = a.bond_row[id + 1];
-    for (uint32_t r = r0; r < r1; r++) {
-        const BondTerm bt = a.bond_terms[r];
-        const Vec4d prm = prm_tab[bt.param];
-        const uint32_t kind = bt.meta & 0xffu, role = bt.meta >> 8;
-        double xa[3], xb[3];
-        load_x(pos, a.slot_of_id[bt.a], xa);
-        if (kind == 0) {
-            const double *xh = role == 0 ? xs : xa;
-            const double *xt = role == 0 ? xa : xs;
-            double dx[3];
-            distance_from_to(w, xh, xt, dx);
-            const double dr = sqrt(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
-            if (dr > 2.0) err |= ERR_BOND_SNAPPED;
-            const double dr0 = prm.y - dr;
-            const double hookean_force = prm.x * dr0;
-            const double s = hookean_force / dr;
-            double t[3];
+    const Vec4d prm = ((const Vec4d *)a.bond_params)[k];
+    double xh[3], xt[3], dx[3];
+    load_x(pos, a.slot_of_id[head], xh);
+    load_x(pos, a.slot_of_id[tail], xt);
+    distance_from_to(w, xh, xt, dx);
+    const double dr = sqrt(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
+    if (dr > 2.0) err |= ERR_BOND_SNAPPED;
+    const double dr0 = prm.y - dr;
+    const double hookean_force = prm.x * dr0;
+    const double s = hookean_force / dr;
+    const double f[3] = {dx[0] * s, dx[1] * s, dx[2] * s};
+    store_term64(a, 2 * k, -f[0], -f[1], -f[2]);
+    store_term64(a, 2 * k + 1, f[0], f[1], f[2]);
+}
+
+__device__ __forceinline__ void angle64(const KArgs &a, const WorldDev &w, uint32_t g, const uint32_t *hmt)
+{
+    const Vec4d *pos = (const Vec4d *)a.posA;
+    const Vec4d prm = ((const Vec4d *)a.bond_params)[a.n_bonds + g];
+    double xh[3], xm[3], xt[3];
+    load_x(pos, a.slot_of_id[hmt[0]], xh);
+    load_x(pos, a.slot_of_id[hmt[1]], xm);
+    load_x(pos, a.slot_of_id[hmt[2]], xt);
+    double first[3], second[3];
+    distance_from_to(w, xh, xm, first);
+    distance_from_to(w, xm, xt, second);
+    const double r01 = sqrt(first[0] * first[0] + first[1] * first[1] + first[2] * first[2]);
+    const double r12 = sqrt(second[0] * second[0] + second[1] * second[1] + second[2] * second[2]);
+    const double kappa = prm.x, cos_theta0 = prm.y, sin_theta0 = prm.z;
+    double hf[3] = {0, 0, 0}, tf[3] = {0, 0, 0}, mf[3] = {0, 0, 0};
+    const double mag_product = r01 * r12;
+    if (mag_product > 0.0001) {
+        const double b1_mag_sq = r01 * r01;
+        const double b2_mag_sq = r12 * r12;
+        const double b1_dot_b2 = first[0] * second[0] + first[1] * second[1] + first[2] * second[2];
+        const double p1 = b1_dot_b2 / b1_mag_sq;
+        const double p2 = b1_dot_b2 / b2_mag_sq;
+        const double cos_phi_sq = p1 * p2;
+        double force_mag = kappa / mag_product;
+        if (fabs(b1_dot_b2) > 0.000001 && sin_theta0 > 0) {
+            const double inv_prefactor = 1.0 / sqrt(1.0 / cos_phi_sq - 1.0);
+            force_mag = force_mag * (cos_theta0 - sin_theta0 * inv_prefactor);
+        }
 #pragma unroll
-            for (int d = 0; d < 3; d++) {
-                const double fd = dx[d] * s;
-                t[d] = role == 0 ? -fd : fd;
-            }
-            out[r] = Vec4d{t[0], t[1], t[2], 0.0};
-        } else {
-            load_x(pos, a.slot_of_id[bt.b], xb);
-            const double *xh = role == 0 ? xs : xa;
-            const double *xm = role == 0 ? xa : (role == 1 ? xs : xb);
-            const double *xt = role == 2 ? xs : xb;
-            double first[3], second[3];
-            distance_from_to(w, xh, xm, first);
-            distance_from_to(w, xm, xt, second);
-            const double r01 = sqrt(first[0] * first[0] + first[1] * first[1] + first[2] * first[2]);
-            const double r12 = sqrt(second[0] * second[0] + second[1] * second[1] + second[2] * second[2]);
-            const double kappa = prm.x, cos_theta0 = prm.y, sin_theta0 = prm.z;
-            double hf[3] = {0, 0, 0}, tf[3] = {0, 0, 0}, mf[3] = {0, 0, 0};
-            const double mag_product = r01 * r12;
-            if (mag_product > 0.0001) {
-                const double b1_mag_sq = r01 * r01;
-                const double b2_mag_sq = r12 * r12;
-                const double b1_dot_b2 = first[0] * second[0] + first[1] * second[1] + first[2] * second[2];
-                const double p1 = b1_dot_b2 / b1_mag_sq;
-                const double p2 = b1_dot_b2 / b2_mag_sq;
-                const double cos_phi_sq = p1 * p2;
-                double force_mag = kappa / mag_product;
-                if (fabs(b1_dot_b2) > 0.000001 && sin_theta0 > 0) {
-                    const double inv_prefactor = 1.0 / sqrt(1.0 / cos_phi_sq - 1.0);
-                    force_mag = force_mag * (cos_theta0 - sin_theta0 * inv_prefactor);
-                }
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    hf[d] = (first[d] * p1 - second[d]) * force_mag;
-                    tf[d] = (first[d] - second[d] * p2) * force_mag;
-                    mf[d] = -(hf[d] + tf[d]);
-                }
-            }
-            double t[3];
-#pragma unroll
-            for (int d = 0; d < 3; d++) t[d] = role == 0 ? hf[d] : (role == 1 ? mf[d] : tf[d]);
-            out[r] = Vec4d{t[0], t[1], t[2], 0.0};
+        for (int d = 0; d < 3; d++) {
+            hf[d] = (first[d] * p1 - second[d]) * force_mag;
+            tf[d] = (first[d] - second[d] * p2) * force_mag;
+            mf[d] = -(hf[d] + tf[d]);
         }
     }
+    const uint32_t row = 2 * a.n_bonds + 3 * g;
+    store_term64(a, row, hf[0], hf[1], hf[2]);
+    store_term64(a, row + 1, mf[0], mf[1], mf[2]);
+    store_term64(a, row + 2, tf[0], tf[1], tf[2]);
 }
 
 constexpr int LIST_MAX = 32;
@@ -209,7 +212,6 @@ __device__ __forceinline__ PairTerms64 pair_terms64(double dx0, double dx1, doub
                                                     uint32_t th_hi, double scale_inv_sqrt_dt)
 {
     PairTerms64 q;
-    const double kappa = 0.0, r0 = 0.5;
     const double inv_dr = 1.0 / dr;
     const double dv0 = vh.x - vj.x, dv1 = vh.y - vj.y, dv2 = vh.z - vj.z;
     q.wr = 1.0 - dr;
@@ -223,9 +225,8 @@ __device__ __forceinline__ PairTerms64 pair_terms64(double dx0, double dx1, doub
     q.u = (double)hash_u(th_lo, th_hi, hh, hj);
     q.rand_scale = q.sqrt_gammap * scale_inv_sqrt_dt;
     q.rand = q.rand_scale * q.u;
-    const double dr0 = r0 - dr;
-    const double hookean_force = kappa * dr0;
-    q.scaled = q.con + q.diss + q.rand + hookean_force;
+    // (the reference also adds kappa (r0 - dr) with kappa = 0: a zero, which changes no sum)
+    q.scaled = q.con + q.diss + q.rand;
     return q;
 }
 
@@ -310,11 +311,6 @@ __device__ __forceinline__ void eval_list64(const KArgs &a, const WorldDev &w, c
                   h.hash, h.ti, s_pair, cp, h.hc, a.cellg, th_lo, th_hi, w.scale_inv_sqrt_dt, F);
 }
 
-__device__ __forceinline__ float slab_gap32(float o, int d)
-{
-    return d == 0 ? 0.0f : (d < 0 ? o : 1.0f - o);
-}
-
 // The neighbour walk of one bead: for each of the 27 directions in (-1..1)^3 order, for each
 // bead of that cell in id order (the reference's update_cell_forces order,
 // naive_dpd_engine_half_step.hpp:358-424), candidates are appended to the bead's list
@@ -338,15 +334,15 @@ __device__ __forceinline__ int walk64(const KArgs &a, const WorldDev &w, const V
     int n = 0;
     int dir[3];
     for (dir[0] = -1; dir[0] <= 1; dir[0]++) {
-        const float gx = slab_gap32(oh.x, dir[0]);
+        const float gx = slab_gap(oh.x, dir[0]);
         const float ax = oh.x - (float)dir[0];
         for (dir[1] = -1; dir[1] <= 1; dir[1]++) {
-            const float gy = slab_gap32(oh.y, dir[1]);
+            const float gy = slab_gap(oh.y, dir[1]);
             const float gxy = gx * gx + gy * gy;
             if (gxy >= PRUNE) continue;
             const float ay = oh.y - (float)dir[1];
             for (dir[2] = -1; dir[2] <= 1; dir[2]++) {
-                const float gz = slab_gap32(oh.z, dir[2]);
+                const float gz = slab_gap(oh.z, dir[2]);
                 if (gxy + gz * gz >= PRUNE) continue;
                 const float az = oh.z - (float)dir[2];
                 int op[3];
@@ -467,28 +463,81 @@ struct Balance64 {
     double f[3][TILE_BEADS];
 };
 
-// Bond terms of every polymer bead, one thread per bead (a compact list of the few bonded
-// beads), stored by CSR row for the force kernel: the lanes of a warp all do bond work,
-// instead of one or two lanes of a pair-force warp.
-__global__ void __launch_bounds__(128) k_bonds64(KArgs a)
+// Blocks [0, bond_blocks) take the Hookean bonds, the others the angle bonds (no warp mixes them).
+constexpr int BOND64_THREADS = 64;
+__global__ void __launch_bounds__(BOND64_THREADS) k_bonds64(KArgs a, uint32_t bond_blocks)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.n_bonded) return;
-    const uint32_t id = a.bonded_ids[k];
+    const bool angle = blockIdx.x >= bond_blocks;
+    const uint32_t k = (blockIdx.x - (angle ? bond_blocks : 0u)) * BOND64_THREADS + threadIdx.x;
+    if (k >= (angle ? a.n_angles : a.n_bonds)) return;
+    const uint32_t *ids = angle ? a.bond_list + 2 * (size_t)a.n_bonds + 3 * (size_t)k : a.bond_list + 2 * (size_t)k;
+    // (only polymer beads have bond forces, and their slots kept by id)
+    if ((a.hash[ids[0]] | a.hash[ids[1]] | (angle ? a.hash[ids[2]] : 0u)) & (1u << 27)) return;
+    const uint32_t id = ids[0];
     uint32_t lo = 0, hi = a.n_worlds;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) / 2;
         if (a.worlds[mid].bead_base <= id) lo = mid; else hi = mid;
     }
     const WorldDev &w = a.worlds[lo];
-    const Vec4d p = ((const Vec4d *)a.posA)[a.slot_of_id[id]];
-    const double x[3] = {p.x, p.y, p.z};
     uint32_t err = 0;
-    bond_terms64(a, w, id, x, err);
+    if (angle) angle64(a, w, k, ids);
+    else hookean64(a, w, k, ids[0], ids[1], err);
     if (err) atomicOr(&a.worlds[lo].err, err);
 }
 
-// Force pass of a tile of TILE_BEADS sorted beads, one thread per bead:
+// Bonds, update_mom and either the final write or the next update_pos with its cell count, for
+// one bead whose pair forces are in F.
+template <int FINAL>
+__device__ __forceinline__ void integrate64(const KArgs &a, const WorldDev &w, uint32_t world, uint32_t s,
+                                            double F[3])
+{
+    const double dt = w.dt, hdt = w.hdt, hdt2 = w.hdt2;
+    uint32_t err = 0;
+    const Vec4d ph = ((const Vec4d *)a.posA)[s];
+    const Vec4d vh = ((const Vec4d *)a.velA)[s];
+    const uint32_t hh = hash_of(ph);
+    double x[3] = {ph.x, ph.y, ph.z};
+    if (!(hh & (1u << 27))) {  // polymer bead: its bond terms, in CSR order
+        const uint32_t id = a.ids[s];
+        const Vec4d *bt = (const Vec4d *)a.bterm;
+#pragma unroll 1
+        for (uint32_t r = a.bond_row[id]; r < a.bond_row[id + 1]; r++) {
+            const Vec4d t = bt[r];
+            F[0] = F[0] + t.x;
+            F[1] = F[1] + t.y;
+            F[2] = F[2] + t.z;
+        }
+    }
+    // update_mom: v += f * half(dt); a stationary type's v and f are cleared instead
+    // (naive_dpd_engine_half_merge.hpp:387-394), so the next update_pos leaves it in place
+    double v[3] = {vh.x + F[0] * hdt, vh.y + F[1] * hdt, vh.z + F[2] * hdt};
+    if ((w.stationary >> (hh >> 28)) & 1u) {
+        v[0] = v[1] = v[2] = 0.0;
+        F[0] = F[1] = F[2] = 0.0;
+    }
+    if (FINAL) {
+        Vec4d vo = {v[0], v[1], v[2], 0.0};
+        Vec4d fo = {F[0], F[1], F[2], 0.0};
+        ((Vec4d *)a.velB)[s] = vo;
+        ((Vec4d *)a.frc)[s] = fo;
+        if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]))) err |= ERR_NONFINITE;
+    } else {
+        const uint32_t key = advance_position64(w, dt, hdt2, x, v, F, err);
+        const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+        Vec4d po = {x[0], x[1], x[2], ph.w};
+        Vec4d vo = {v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, 0.0};
+        ((Vec4d *)a.posB)[s] = po;
+        ((Vec4d *)a.velB)[s] = vo;
+        a.keyrank[s] = make_uint2(key, rank);
+    }
+    if (err) atomicOr(&a.worlds[world].err, err);
+}
+
+#include "pdpd_fp64_pairs.cuh"
+
+// Force pass without pair lists (pdpd_fp64_pairs.cuh), of a tile of TILE_BEADS sorted beads, one
+// thread per bead:
 //   1. each thread walks its bead's neighbours into its list;
 //   2. the lists are counting-sorted by length and thread t evaluates list perm[t], so the
 //      lanes of a warp evaluate lists of about the same length (the FP64 pipe executes an
@@ -561,45 +610,7 @@ __global__ void __launch_bounds__(TILE_BEADS) k_force64(KArgs a)
             F[0] = B.f[0][tid];
             F[1] = B.f[1][tid];
             F[2] = B.f[2][tid];
-            const double dt = w.dt, hdt = dt * 0.5, hdt2 = (dt * dt) * 0.5;
-            uint32_t err = 0;
-            const Vec4d ph = ((const Vec4d *)a.posA)[s];
-            const Vec4d vh = ((const Vec4d *)a.velA)[s];
-            const uint32_t hh = hash_of(ph);
-            double x[3] = {ph.x, ph.y, ph.z};
-            if (!(hh & (1u << 27))) {  // polymer bead: its bond terms, in CSR order
-                const uint32_t id = a.ids[s];
-                const Vec4d *bt = (const Vec4d *)a.bterm;
-                for (uint32_t r = a.bond_row[id]; r < a.bond_row[id + 1]; r++) {
-                    const Vec4d t = bt[r];
-                    F[0] = F[0] + t.x;
-                    F[1] = F[1] + t.y;
-                    F[2] = F[2] + t.z;
-                }
-            }
-            // update_mom: v += f * half(dt); a stationary type's v and f are cleared instead
-            // (naive_dpd_engine_half_merge.hpp:387-394), so the next update_pos leaves it in place
-            double v[3] = {vh.x + F[0] * hdt, vh.y + F[1] * hdt, vh.z + F[2] * hdt};
-            if ((w.stationary >> (hh >> 28)) & 1u) {
-                v[0] = v[1] = v[2] = 0.0;
-                F[0] = F[1] = F[2] = 0.0;
-            }
-            if (FINAL) {
-                Vec4d vo = {v[0], v[1], v[2], 0.0};
-                Vec4d fo = {F[0], F[1], F[2], 0.0};
-                ((Vec4d *)a.velB)[s] = vo;
-                ((Vec4d *)a.frc)[s] = fo;
-                if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]))) err |= ERR_NONFINITE;
-            } else {
-                const uint32_t key = advance_position64(w, dt, hdt2, x, v, F, err);
-                const uint32_t rank2 = atomicAdd(&a.cnt[key], 1u);
-                Vec4d po = {x[0], x[1], x[2], ph.w};
-                Vec4d vo = {v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, 0.0};
-                ((Vec4d *)a.posB)[s] = po;
-                ((Vec4d *)a.velB)[s] = vo;
-                a.keyrank[s] = make_uint2(key, rank2);
-            }
-            if (err) atomicOr(&a.worlds[tl.world].err, err);
+            integrate64<FINAL>(a, w, tl.world, s, F);
         }
         __syncthreads();  // the lists and B are reused by the next tile
     }
@@ -612,7 +623,7 @@ __global__ void __launch_bounds__(TILE_BEADS) k_begin64(KArgs a)
         const uint32_t s = tl.slot_begin + threadIdx.x;
         if (s >= tl.slot_end) continue;
         const WorldDev &w = a.worlds[tl.world];
-        const double dt = w.dt, hdt = dt * 0.5, hdt2 = (dt * dt) * 0.5;
+        const double dt = w.dt, hdt = w.hdt, hdt2 = w.hdt2;
         uint32_t err = 0;
         const Vec4d ph = ((const Vec4d *)a.posA)[s];
         const Vec4d vh = ((const Vec4d *)a.velA)[s];
@@ -707,15 +718,57 @@ int launch_pair_log64(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
 {
     int n = 0;
-    if (a.n_bonded > 0) {
-        k_bonds64<<<(a.n_bonded + 127) / 128, 128, 0, s>>>(a);
+    if (a.n_bonds + a.n_angles > 0) {
+        const uint32_t bb = (a.n_bonds + BOND64_THREADS - 1) / BOND64_THREADS;
+        const uint32_t ab = (a.n_angles + BOND64_THREADS - 1) / BOND64_THREADS;
+        k_bonds64<<<bb + ab, BOND64_THREADS, 0, s>>>(a, bb);
         n++;
+    }
+    if (a.list) {  // each pair once
+        const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb, (uint32_t)a.block_threads);
+        const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
+        if (a.block_threads == LIST64_WIDE)
+            k_list64<LIST64_WIDE><<<grid, LIST64_WIDE, L.bytes, s>>>(a, L);
+        else
+            k_list64<LIST64_NARROW><<<grid, LIST64_NARROW, L.bytes, s>>>(a, L);
+        const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
+        k_pairs64<<<std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s>>>(a);
+        const uint32_t parts = a.n_tiles * (TILE_BEADS / SUM64_BEADS);
+        if (a.n_tiles == 0) return n + 2;
+        if (final_step) k_sum64<1><<<parts, SUM64_THREADS, 0, s>>>(a);
+        else k_sum64<0><<<parts, SUM64_THREADS, 0, s>>>(a);
+        return n + 3;
     }
     if (final_step)
         k_force64<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
     else
         k_force64<0><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
     return n + 1;
+}
+
+// Largest staged-bead capacity of a k_list64 brick with two blocks per SM (large bricks).
+uint32_t list64_maxb_limit(int threads, uint32_t hc_max)
+{
+    int dev = 0, smem_sm = 0;
+    if (threads != LIST64_WIDE) return 2046u;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
+        return 2046u;
+    const int budget = smem_sm / 2 - 1024 - (int)list64_layout(hc_max, 0, (uint32_t)threads).bytes - 128;
+    return (uint32_t)std::max(64, std::min((int)FULL_MAX_STAGED, budget / (int)LIST64_BEAD_BYTES)) & ~1u;
+}
+
+int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int *grid)
+{
+    const int bytes = (int)list64_layout(hc_max, maxb, (uint32_t)threads).bytes;
+    void (*k)(KArgs, List64Layout) = threads == LIST64_WIDE ? k_list64<LIST64_WIDE> : k_list64<LIST64_NARROW>;
+    int nb = 0;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, bytes);
+    if (e != cudaSuccess) return (int)e;
+    if (nb < 1) return (int)cudaErrorInvalidConfiguration;
+    *grid = nb * sm_count;
+    return 0;
 }
 
 int launch_finish64(const KArgs &a, cudaStream_t s)

@@ -26,9 +26,13 @@ struct WorldDev {
     uint32_t spatial;     // 1: per-cell strengths at cellpair[cellpair_base + local cell * n_types^2]
     double dt;
     double scale_inv_sqrt_dt;  // sqrt(24 kT / dt), kT = 1 (dpd_maths_core.hpp:24)
+    double hdt, hdt2;          // dt / 2, dt dt / 2
+    double Ld[3];              // the box sides
     uint64_t seed;
     int64_t t;
     uint64_t cellpair_base;
+    uint32_t asym;        // 1: some strength a_ij or gamma_ij differs from a_ji or gamma_ji
+    uint32_t pad;
 };
 
 // A run of consecutive sorted bead slots of one world: the unit of work of the step
@@ -105,8 +109,12 @@ struct KArgs {
     const void *bond_params;   // float4 / Vec4d: (kappa, r0 | cos theta0, sin theta0, 0)
     const void *pair;          // float2 / Vec2d: (a_ij, sqrt(gamma_ij))
     const void *cellpair;      // float2 / Vec2d per (cell, type pair) of spatial worlds
-    const uint32_t *bonded_ids;  // ids of the beads that have bond terms (bond kernels)
+    const uint32_t *bonded_ids;  // ids of the beads that have bond terms (FP32 bond kernel)
     uint32_t n_bonded;
+    const uint32_t *bond_list;   // the batch's flat lists with global ids: n_bonds pairs, n_angles triples
+    uint32_t n_bonds, n_angles;
+    const uint32_t *row_of;      // CSR row of each end of the flat lists, in their order
+    const uint32_t *hash;        // BeadHash by bead id
     float4 *fbond;               // FP32: bond force of each bonded bead, by sorted slot
     float4 *posf;                // FP64: (x - floor(x), hash) in FP32, by sorted slot: the
                                  // neighbour walk's distance prefilter
@@ -128,8 +136,16 @@ struct KArgs {
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds
     uint32_t brick_home_max;  // half shell: home-bead capacity of one brick
-    uint32_t *brick_next;   // FP32: the brick queue's next free entry beyond the first
-                            // gridDim.x (zeroed by the sort, which precedes every force pass)
+    uint32_t *brick_next;   // the brick queue's next free entry beyond the first gridDim.x
+                            // (zeroed by the sort, which precedes every force pass)
+    // FP64 pair lists (pdpd_fp64_pairs.cuh; list null: not used)
+    uint2 *lrec;            // per slot: first list entry (~0: no list), entries
+    uint32_t *list;         // list_cap candidate entries
+    uint32_t *pair_i, *pair_j;  // pair_cap pairs: slot; other slot with direction and flag
+    double *term;           // 3 per pair
+    unsigned long long *list_cursor;  // entries and pairs taken (zeroed with brick_next)
+    uint32_t list_cap, pair_cap;
+    int pair_blocks;        // persistent grid of the pair kernel
 };
 
 // Kernel launchers.  Each returns the number of kernels it launched.
@@ -145,6 +161,9 @@ int launch_begin32(const KArgs &a, cudaStream_t s);
 int launch_force32(const KArgs &a, int final_step, cudaStream_t s);  // includes the bond kernel
 int launch_finish32(const KArgs &a, cudaStream_t s);
 int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
+// FP64 list kernel: staged-bead capacity of a brick, and its persistent grid (0 or a cudaError_t).
+uint32_t list64_maxb_limit(int threads, uint32_t hc_max);
+int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int *grid);
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);
@@ -211,10 +230,12 @@ void launch_scan(uint32_t *cnt, uint32_t n, uint32_t *blocksums, uint32_t *start
 // Attach (pdpd_bondcsr.cu): the per-bead bond CSR (row: n_beads + 1 offsets, terms) from the
 // batch's flat lists with global ids -- pairs (head, tail) of the Hookean bonds, parameter k
 // for bond k, and triples (head, middle, tail) of the angle bonds, parameter n_bonds + g for
-// angle g -- and the polymer beads' ids in id order (bonded; their number to *n_bonded).
+// angle g -- the CSR row of each end of each bond and angle (row_of: 2 per bond, then 3 per angle;
+// may be null), and the polymer beads' ids in id order (bonded; their number to *n_bonded).
 // Scratch: scratch and pos n_beads words each, blocksums scan_blocks(n_beads) words.
 int launch_bond_tables(uint32_t n_beads, const uint32_t *pairs, uint32_t n_bonds, const uint32_t *triples,
-                       uint32_t n_angles, const uint32_t *hash, uint32_t *row, BondTerm *terms, uint32_t *bonded,
+                       uint32_t n_angles, const uint32_t *hash, uint32_t *row, BondTerm *terms, uint32_t *row_of,
+                       uint32_t *bonded,
                        uint32_t *n_bonded, uint32_t *scratch, uint32_t *pos, uint32_t *blocksums, cudaStream_t s);
 
 // Device RNG on arrays (device pointers), for known-answer tests.
