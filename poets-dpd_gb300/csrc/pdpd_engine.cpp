@@ -249,6 +249,11 @@ struct List64Room {
     }
 };
 
+uint32_t bucket_room(double density)
+{
+    return (uint32_t)std::min(64.0, std::max(8.0, 4 * std::ceil((density + 5.5 * std::sqrt(density) + 3) / 4)));
+}
+
 bool asymmetric(const pdpd_world &w)
 {
     const uint32_t nt = w.n_bead_types;
@@ -331,7 +336,7 @@ struct pdpd_engine {
     // device arena
     DevBuf d_worlds, d_tiles, d_bricks, d_start, d_cnt, d_blocksums;
     DevBuf d_posA, d_velA, d_frc, d_posB, d_velB, d_frcB;
-    DevBuf d_ids, d_cellg, d_slot_of_id, d_keyrank, d_tmp;
+    DevBuf d_ids, d_cellg, d_slot_of_id, d_key, d_bucket, d_over_node, d_over_head;
     DevBuf d_bond_row, d_bond_terms, d_bond_params, d_pair, d_hash, d_bonded, d_fbond, d_cellpair, d_posf, d_bterm, d_zlo, d_brick_next, d_hash_old;
     DevBuf d_lists;   // FP64 pair lists (List64Room)
     DevBuf d_row_of;  // FP64: CSR row of each end of the flat bond lists
@@ -394,7 +399,7 @@ struct pdpd_engine {
         drop_graph();
         DevBuf *bufs[] = {&d_worlds, &d_tiles, &d_bricks, &d_start, &d_cnt, &d_blocksums, &d_posA, &d_velA,
                           &d_frc, &d_posB, &d_velB, &d_frcB, &d_ids, &d_cellg, &d_slot_of_id,
-                          &d_keyrank, &d_tmp, &d_bond_row, &d_bond_terms, &d_bond_params,
+                          &d_key, &d_bucket, &d_over_node, &d_over_head, &d_bond_row, &d_bond_terms, &d_bond_params,
                           &d_pair, &d_hash, &d_bonded, &d_fbond, &d_staging[0], &d_staging[1],
                           &d_v2err, &d_cellpair, &d_posf, &d_bterm, &d_zlo, &d_brick_next, &d_hash_old,
                           &d_hostio, &d_inv, &d_blist, &d_scan, &d_lists, &d_row_of};
@@ -417,13 +422,13 @@ struct pdpd_engine {
     int enqueue_begin(cudaStream_t s)
     {
         int n = fp64() ? launch_begin64(args, s) : launch_begin32(args, s);
-        n += launch_sort(args, fp64(), 0, 0, s);
+        n += launch_sort(args, fp64(), 0, 0, 1, s);
         return n;
     }
     int enqueue_step(cudaStream_t s)  // finish step t and start t+1
     {
         int n = fp64() ? launch_force64(args, 0, s) : launch_force32(args, 0, s);
-        n += launch_sort(args, fp64(), 1, 0, s);
+        n += launch_sort(args, fp64(), 1, 0, 1, s);
         return n;
     }
     int enqueue_final(cudaStream_t s)
@@ -1307,6 +1312,10 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         put(n_bond_par + g, p);
     });
 
+    // Room for the beads of a cell that a rebuild ranks from its bucket: the densest world's mean
+    // and 5.5 Poisson deviations (cells that hold more go through overflow lists).
+    const uint32_t bucket_k = bucket_room(max_density);
+
     // --- allocate
     const size_t P = payload_bytes(f64);
     cudaError_t ce = cudaSuccess;
@@ -1318,7 +1327,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     A(e->d_start, sizeof(uint32_t) * ((size_t)nc + 1));
     A(e->d_cnt, sizeof(uint32_t) * (size_t)nc);
     A(e->d_zlo, f64 ? 16 : sizeof(uint16_t) * std::max<size_t>(1, (size_t)nc));
-    A(e->d_brick_next, 16);
+    A(e->d_brick_next, 64);  // the brick queue's counter, then the overflow lists' state
     A(e->d_blocksums, sizeof(uint32_t) * (scan_blocks((uint32_t)nc) + 1));
     A(e->d_posA, P * nb);
     A(e->d_velA, P * nb);
@@ -1329,8 +1338,10 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     A(e->d_ids, sizeof(uint32_t) * nb);
     A(e->d_cellg, sizeof(uint32_t) * nb);
     A(e->d_slot_of_id, sizeof(uint32_t) * nb);
-    A(e->d_keyrank, sizeof(uint2) * nb);
-    A(e->d_tmp, sizeof(uint4) * nb);
+    A(e->d_key, sizeof(uint32_t) * nb);
+    A(e->d_bucket, sizeof(uint32_t) * bucket_k * (size_t)nc);
+    A(e->d_over_head, sizeof(uint64_t) * (size_t)nc);
+    A(e->d_over_node, sizeof(uint2) * nb);
     A(e->d_bond_row, sizeof(uint32_t) * (nb + 1));
     A(e->d_bond_terms, sizeof(BondTerm) * std::max<uint64_t>(1, n_terms));
     A(e->d_bond_params, (f64 ? sizeof(double) : sizeof(float)) * 4 * std::max<uint64_t>(1, n_bparams));
@@ -1486,6 +1497,8 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         ce = cudaMemcpyAsync(e->h_small.p, e->d_scan.as<uint32_t>() + scan_blocks((uint32_t)nb), sizeof(uint32_t),
                              cudaMemcpyDeviceToHost, s);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_cnt.p, 0, sizeof(uint32_t) * nc, s);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_over_head.p, 0, sizeof(uint64_t) * nc, s);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_brick_next.p, 0, 64, s);
     uint32_t total = (uint32_t)nb;  // start[n_cells] = total beads, fixed for the attach
     if (ce == cudaSuccess)
         ce = cudaMemcpyAsync(e->d_start.as<uint32_t>() + nc, &total, sizeof(uint32_t),
@@ -1516,8 +1529,12 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.ids = e->d_ids.as<uint32_t>();
     a.cellg = e->d_cellg.as<uint32_t>();
     a.slot_of_id = e->d_slot_of_id.as<uint32_t>();
-    a.keyrank = e->d_keyrank.as<uint2>();
-    a.tmp = e->d_tmp.as<uint4>();
+    a.key = e->d_key.as<uint32_t>();
+    a.bucket = e->d_bucket.as<uint32_t>();
+    a.bucket_k = bucket_k;
+    a.over = (Overflow *)(e->d_brick_next.as<char>() + 32);
+    a.over_head = e->d_over_head.as<unsigned long long>();
+    a.over_node = e->d_over_node.as<uint2>();
     a.bond_row = e->d_bond_row.as<uint32_t>();
     a.bond_terms = e->d_bond_terms.as<BondTerm>();
     a.bond_params = e->d_bond_params.p;
@@ -1571,7 +1588,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         ab.staging_n = (uint32_t)nb;
         e->launches += f64 ? launch_bin64(ab, hash_in, s) : launch_bin32(ab, hash_in, s);
     }
-    e->launches += launch_sort(a, f64, 0, 1, s);
+    e->launches += launch_sort(a, f64, 0, 1, 0, s);
     ce = cudaGetLastError();
     if (ce != cudaSuccess) {
         e->release();
@@ -1937,7 +1954,7 @@ int pdpd_run_intervals(pdpd_engine *e, int32_t interval_count, uint32_t interval
                 cudaMemcpyAsync(e->d_worlds.p, wv.data(), sizeof(WorldDev), cudaMemcpyHostToDevice, e->stream);
                 e->launches += e->fp64() ? launch_bin64(a, e->d_hash.as<uint32_t>(), e->stream)
                                          : launch_bin32(a, e->d_hash.as<uint32_t>(), e->stream);
-                e->launches += launch_sort(a, e->fp64(), 0, 1, e->stream);
+                e->launches += launch_sort(a, e->fp64(), 0, 1, 0, e->stream);
                 rc = pdpd_sync(e);
             }
             break;
@@ -2172,14 +2189,14 @@ int pdpd_profile_run(pdpd_engine *e, uint32_t n_steps, pdpd_phase_times *out)
     e->launches += f64 ? launch_begin64(e->args, s) : launch_begin32(e->args, s);
     size_t m1 = mark();
     spans.push_back({m0, m1, 2});
-    e->launches += launch_sort(e->args, f64, 0, 0, s);
+    e->launches += launch_sort(e->args, f64, 0, 0, 1, s);
     size_t m2 = mark();
     spans.push_back({m1, m2, 1});
     for (uint32_t i = 0; i + 1 < n_steps; i++) {
         size_t a = mark();
         e->launches += f64 ? launch_force64(e->args, 0, s) : launch_force32(e->args, 0, s);
         size_t b = mark();
-        e->launches += launch_sort(e->args, f64, 1, 0, s);
+        e->launches += launch_sort(e->args, f64, 1, 0, 1, s);
         size_t c = mark();
         spans.push_back({a, b, 0});
         spans.push_back({b, c, 1});
@@ -2414,7 +2431,7 @@ static int rebin_from_staging(pdpd_engine *e)
     a.staging = e->d_staging[0].as<double>();
     const uint32_t *hash_in = e->d_hash.as<uint32_t>();
     e->launches += e->fp64() ? launch_bin64(a, hash_in, e->stream) : launch_bin32(a, hash_in, e->stream);
-    e->launches += launch_sort(a, e->fp64(), 0, 1, e->stream);
+    e->launches += launch_sort(a, e->fp64(), 0, 1, 0, e->stream);
     cudaError_t ce = cudaGetLastError();
     if (ce != cudaSuccess) return e->cuda_fail(ce, "re-bin kernels");
     return e->check_device_errors();
@@ -2473,8 +2490,8 @@ struct Delivery {
 
 size_t job_bytes(const pdpd_world &w, int precision)
 {
-    // sorted state A and B, ids / cells / ranks, two id-ordered staging rows, hashes
-    const size_t per_bead = precision == PDPD_FP64 ? 424 : 296;
+    // sorted state A and B, ids / cells, two id-ordered staging rows, hashes
+    const size_t per_bead = precision == PDPD_FP64 ? 412 : 284;
     const size_t cells = (size_t)w.box[0] * w.box[1] * w.box[2];
     size_t lists = 0;
     if (precision == PDPD_FP64 && w.n_beads) {
@@ -2482,7 +2499,7 @@ size_t job_bytes(const pdpd_world &w, int precision)
         room.add((double)w.n_beads, w.box, asymmetric(w));
         lists = room.bytes(w.n_beads);
     }
-    return per_bead * w.n_beads + lists + 12 * cells +
+    return per_bead * w.n_beads + lists + (20 + 4 * bucket_room((double)w.n_beads / (double)cells)) * cells +
            48 * (2 * (size_t)w.n_bonds + 3 * (size_t)w.n_angles) + 4096;
 }
 

@@ -14,7 +14,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "pdpd_device.cuh"
+#include "pdpd_cells.cuh"
 #include "pdpd_walk.cuh"
 
 namespace pdpd {
@@ -71,11 +71,11 @@ __device__ __forceinline__ uint32_t advance_position(const WorldDev &w, float dt
            (uint32_t)nc[2];
 }
 
-// Arrival rank in the new cell with the z-half mark the sort orders by (bit 31: offset
-// z >= 0.5, compared exactly in FP32).
-__device__ __forceinline__ uint32_t zhalf_rank(uint32_t rank, float oz)
+// The upper z half of a cell, which the sort orders after the lower (offset z >= 0.5, compared
+// exactly in FP32).
+__device__ __forceinline__ uint32_t zhalf_bit(float oz)
 {
-    return rank | (oz >= 0.5f ? 0x80000000u : 0u);
+    return oz >= 0.5f ? 0x80000000u : 0u;
 }
 
 // Position of bead `slot` relative to a bead at (cell c, offset o), using the
@@ -115,7 +115,7 @@ __device__ __forceinline__ void min_image(const WorldDev &w, float d[3])
 __device__ __noinline__ void bond_forces32(const KArgs &a, const WorldDev &w, uint32_t id, const int c[3],
                               const float o[3], float F[3], uint32_t &err)
 {
-    const float4 *pos = (const float4 *)a.posA;
+    const float4 *pos = (const float4 *)a.posB;
     const float4 *prm_tab = (const float4 *)a.bond_params;
     const uint32_t r0 = a.bond_row[id], r1 = a.bond_row[id + 1];
     for (uint32_t r = r0; r < r1; r++) {
@@ -123,7 +123,7 @@ __device__ __noinline__ void bond_forces32(const KArgs &a, const WorldDev &w, ui
         const float4 prm = prm_tab[bt.param];
         const uint32_t kind = bt.meta & 0xffu, role = bt.meta >> 8;
         float ra[3], rb[3] = {0.f, 0.f, 0.f};
-        rel_pos(w, pos, a.cellg, a.slot_of_id[bt.a], c, o, ra);
+        rel_pos(w, pos, a.key, a.slot_of_id[bt.a], c, o, ra);
         if (kind == 0) {
             // Hookean: dx = tail - head; head gets -f, tail +f, f = dx * kappa (r0 - r) / r.
             float dx[3];
@@ -137,7 +137,7 @@ __device__ __noinline__ void bond_forces32(const KArgs &a, const WorldDev &w, ui
 #pragma unroll
             for (int d = 0; d < 3; d++) F[d] += sign * (dx[d] * s);
         } else {
-            rel_pos(w, pos, a.cellg, a.slot_of_id[bt.b], c, o, rb);
+            rel_pos(w, pos, a.key, a.slot_of_id[bt.b], c, o, rb);
             float xh[3], xm[3], xt[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
@@ -371,8 +371,9 @@ __device__ __forceinline__ void integrate32(const KArgs &a, const WorldDev &w, u
 {
     const float dt = (float)w.dt, hdt = 0.5f * dt, hdt2 = 0.5f * dt * dt;
     float o[3] = {ph.x, ph.y, ph.z};
-    if (!(__float_as_uint(ph.w) & (1u << 27))) {  // polymer bead: its bond force, from k_bonds32
-        const float4 fb = a.fbond[s];
+    const uint32_t id = a.ids[s];
+    if (!(__float_as_uint(ph.w) & (1u << 27))) {  // polymer bead: its bond force (bonds32)
+        const float4 fb = a.fbond[id];
         F[0] = __fadd_rn(F[0], fb.x);
         F[1] = __fadd_rn(F[1], fb.y);
         F[2] = __fadd_rn(F[2], fb.z);
@@ -386,26 +387,26 @@ __device__ __forceinline__ void integrate32(const KArgs &a, const WorldDev &w, u
         F[0] = F[1] = F[2] = 0.f;
     }
     if (FINAL) {
-        ((float4 *)a.velB)[s] = make_float4(v[0], v[1], v[2], 0.f);
+        ((float4 *)a.velB)[s] = make_float4(v[0], v[1], v[2], id_word32(id));
         ((float4 *)a.frc)[s] = make_float4(F[0], F[1], F[2], 0.f);
         if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]))) err |= ERR_NONFINITE;
     } else {
         const uint32_t key = advance_position(w, dt, hdt2, c, o, v, F, err);
-        const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+        cell_arrive(a, key, id | zhalf_bit(o[2]));
         ((float4 *)a.posB)[s] = make_float4(o[0], o[1], o[2], ph.w);
         ((float4 *)a.velB)[s] = make_float4(__fmaf_rn(F[0], hdt, v[0]), __fmaf_rn(F[1], hdt, v[1]),
-                                            __fmaf_rn(F[2], hdt, v[2]), 0.f);
-        a.keyrank[s] = make_uint2(key, zhalf_rank(rank, o[2]));
+                                            __fmaf_rn(F[2], hdt, v[2]), id_word32(id));
+        a.key[s] = key;
     }
 }
 
-// Bond forces of every polymer bead (monomer bit of the hash clear), one thread per bead,
-// written by sorted slot for the force kernel to add.  Running them here, on a compact list
-// of the few bonded beads, keeps their dependent partner lookups out of the pair kernel's
-// warps.
-__global__ void __launch_bounds__(128) k_bonds32(KArgs a)
+// Bond forces of every polymer bead (monomer bit of the hash clear), one thread per bead, by id
+// for the force kernel to add: on a compact list of the few bonded beads, so that their
+// dependent partner lookups stay out of the pair kernel's warps, and from the advanced, not yet
+// re-sorted state (slot_of_id is that of the sorted state it came from), so that it runs in the
+// launch of the cells' prefix sum.
+__device__ __forceinline__ void bonds32(const KArgs &a, uint32_t k)
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= a.n_bonded) return;
     const uint32_t id = a.bonded_ids[k];
     uint32_t lo = 0, hi = a.n_worlds;
@@ -415,15 +416,23 @@ __global__ void __launch_bounds__(128) k_bonds32(KArgs a)
     }
     const WorldDev &w = a.worlds[lo];
     const uint32_t s = a.slot_of_id[id];
-    const float4 p = ((const float4 *)a.posA)[s];
+    const float4 p = ((const float4 *)a.posB)[s];
     int c[3];
-    decode_cell(a.cellg[s] - w.cell_base, w.L, c[0], c[1], c[2]);
+    decode_cell(a.key[s] - w.cell_base, w.L, c[0], c[1], c[2]);
     const float o[3] = {p.x, p.y, p.z};
     float F[3] = {0.f, 0.f, 0.f};
     uint32_t err = 0;
     bond_forces32(a, w, id, c, o, F, err);
-    a.fbond[s] = make_float4(F[0], F[1], F[2], 0.f);
+    a.fbond[id] = make_float4(F[0], F[1], F[2], 0.f);
     if (err) atomicOr(&a.worlds[lo].err, err);
+}
+
+// The cells' prefix sum (blocks [0, nb)) and the bond forces.
+template <bool ONE_PASS>
+__global__ void __launch_bounds__(SCAN_THREADS) k_cells32(KArgs a, uint32_t nb, int tick)
+{
+    if (blockIdx.x < nb) scan_cells<ONE_PASS>(a, tick);
+    else bonds32(a, (blockIdx.x - nb) * SCAN_THREADS + threadIdx.x);
 }
 
 // Thread-per-bead pair forces straight from global memory, summed one pair at a time in the
@@ -742,11 +751,13 @@ __global__ void __launch_bounds__(TILE_BEADS) k_begin32(KArgs a)
         const float v[3] = {st ? 0.f : vh.x, st ? 0.f : vh.y, st ? 0.f : vh.z};
         const float F[3] = {st ? 0.f : fh.x, st ? 0.f : fh.y, st ? 0.f : fh.z};
         const uint32_t key = advance_position(w, dt, hdt2, c, o, v, F, err);
-        const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+        const uint32_t id = a.ids[s];
+        cell_arrive(a, key, id | zhalf_bit(o[2]));
         ((float4 *)a.posB)[s] = make_float4(o[0], o[1], o[2], ph.w);
-        ((float4 *)a.velB)[s] = st ? make_float4(vh.x, vh.y, vh.z, 0.f)
-                                   : make_float4(v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, 0.f);
-        a.keyrank[s] = make_uint2(key, zhalf_rank(rank, o[2]));
+        ((float4 *)a.velB)[s] = st ? make_float4(vh.x, vh.y, vh.z, id_word32(id))
+                                   : make_float4(v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt,
+                                                 id_word32(id));
+        a.key[s] = key;
         if (err) atomicOr(&a.worlds[tl.world].err, err);
     }
 }
@@ -784,12 +795,11 @@ __global__ void k_bin32(KArgs a, const uint32_t *__restrict__ hash_in)
     }
     if (err) atomicOr(&a.worlds[lo].err, err);
     const uint32_t key = w.cell_base + ((uint32_t)c[0] * (uint32_t)w.L[1] + (uint32_t)c[1]) * (uint32_t)w.L[2] + (uint32_t)c[2];
-    const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+    cell_arrive(a, key, g | zhalf_bit(o[2]));
     ((float4 *)a.posB)[g] = make_float4(o[0], o[1], o[2], __uint_as_float(hash_in[g]));
-    ((float4 *)a.velB)[g] = make_float4((float)st[field], (float)st[field + 1], (float)st[field + 2], 0.f);
+    ((float4 *)a.velB)[g] = make_float4((float)st[field], (float)st[field + 1], (float)st[field + 2], id_word32(g));
     ((float4 *)a.frcB)[g] = make_float4((float)st[2 * field], (float)st[2 * field + 1], (float)st[2 * field + 2], 0.f);
-    a.ids[g] = g;
-    a.keyrank[g] = make_uint2(key, zhalf_rank(rank, o[2]));
+    a.key[g] = key;
 }
 
 __global__ void k_finish32(KArgs a)
@@ -865,19 +875,16 @@ int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint3
     return 0;
 }
 
-static int launch_pair_forces32(const KArgs &a, int final_step, cudaStream_t s);
-
-int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
+int launch_cells32(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
-    int n = 0;
-    if (a.n_bonded > 0) {
-        k_bonds32<<<(a.n_bonded + 127) / 128, 128, 0, s>>>(a);
-        n++;
-    }
-    return n + launch_pair_forces32(a, final_step, s);
+    const uint32_t nb = scan_blocks(a.n_cells);
+    const uint32_t bb = bonds ? (a.n_bonded + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    if (scan_one_pass(a.n_cells)) k_cells32<true><<<nb + bb, SCAN_THREADS, 0, s>>>(a, nb, tick);
+    else k_cells32<false><<<nb + bb, SCAN_THREADS, 0, s>>>(a, nb, tick);
+    return 1;
 }
 
-static int launch_pair_forces32(const KArgs &a, int final_step, cudaStream_t s)
+int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
 {
     if (a.force_kernel != 1 && a.n_bricks > 0) {
         const int v = a.force_kernel;

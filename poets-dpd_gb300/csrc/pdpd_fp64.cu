@@ -15,7 +15,7 @@
 #include <mutex>
 
 #include "../../include/pdpd_gpu.h"
-#include "pdpd_device.cuh"
+#include "pdpd_cells.cuh"
 #include "pdpd_walk.cuh"
 
 namespace pdpd {
@@ -106,7 +106,8 @@ __device__ __forceinline__ void load_x(const Vec4d *__restrict__ pos, uint32_t s
     x[2] = p.z;
 }
 
-// Bond forces, one thread per Hookean bond or angle bond: each evaluated once, exactly as
+// Bond forces, one thread per Hookean bond or angle bond, from the advanced, not yet re-sorted
+// state (slot_of_id is that of the sorted state it came from): each evaluated once, exactly as
 // update_hookean_bond / update_angle_bond (naive_dpd_engine_half_step.hpp:426-483) and
 // calc_angle_force (dpd_maths_core_half_step.hpp:177-229) do, and stored with the sign it is
 // added with at the CSR row of each of its beads (row_of): the force kernel adds a bead's rows in
@@ -121,7 +122,7 @@ __device__ __forceinline__ void store_term64(const KArgs &a, uint32_t row, doubl
 __device__ __forceinline__ void hookean64(const KArgs &a, const WorldDev &w, uint32_t k, uint32_t head,
                                           uint32_t tail, uint32_t &err)
 {
-    const Vec4d *pos = (const Vec4d *)a.posA;
+    const Vec4d *pos = (const Vec4d *)a.posB;
     const Vec4d prm = ((const Vec4d *)a.bond_params)[k];
     double xh[3], xt[3], dx[3];
     load_x(pos, a.slot_of_id[head], xh);
@@ -139,7 +140,7 @@ __device__ __forceinline__ void hookean64(const KArgs &a, const WorldDev &w, uin
 
 __device__ __forceinline__ void angle64(const KArgs &a, const WorldDev &w, uint32_t g, const uint32_t *hmt)
 {
-    const Vec4d *pos = (const Vec4d *)a.posA;
+    const Vec4d *pos = (const Vec4d *)a.posB;
     const Vec4d prm = ((const Vec4d *)a.bond_params)[a.n_bonds + g];
     double xh[3], xm[3], xt[3];
     load_x(pos, a.slot_of_id[hmt[0]], xh);
@@ -463,12 +464,9 @@ struct Balance64 {
     double f[3][TILE_BEADS];
 };
 
-// Blocks [0, bond_blocks) take the Hookean bonds, the others the angle bonds (no warp mixes them).
-constexpr int BOND64_THREADS = 64;
-__global__ void __launch_bounds__(BOND64_THREADS) k_bonds64(KArgs a, uint32_t bond_blocks)
+// Thread k's bond or angle bond.
+__device__ __forceinline__ void bonds64(const KArgs &a, uint32_t k, bool angle)
 {
-    const bool angle = blockIdx.x >= bond_blocks;
-    const uint32_t k = (blockIdx.x - (angle ? bond_blocks : 0u)) * BOND64_THREADS + threadIdx.x;
     if (k >= (angle ? a.n_angles : a.n_bonds)) return;
     const uint32_t *ids = angle ? a.bond_list + 2 * (size_t)a.n_bonds + 3 * (size_t)k : a.bond_list + 2 * (size_t)k;
     // (only polymer beads have bond forces, and their slots kept by id)
@@ -486,6 +484,19 @@ __global__ void __launch_bounds__(BOND64_THREADS) k_bonds64(KArgs a, uint32_t bo
     if (err) atomicOr(&a.worlds[lo].err, err);
 }
 
+// The cells' prefix sum (blocks [0, nb)), the Hookean bonds (the next bb) and the angle bonds (no
+// warp mixes the two).
+template <bool ONE_PASS>
+__global__ void __launch_bounds__(SCAN_THREADS) k_cells64(KArgs a, uint32_t nb, uint32_t bb, int tick)
+{
+    if (blockIdx.x < nb) {
+        scan_cells<ONE_PASS>(a, tick);
+        return;
+    }
+    const bool angle = blockIdx.x - nb >= bb;
+    bonds64(a, (blockIdx.x - nb - (angle ? bb : 0u)) * SCAN_THREADS + threadIdx.x, angle);
+}
+
 // Bonds, update_mom and either the final write or the next update_pos with its cell count, for
 // one bead whose pair forces are in F.
 template <int FINAL>
@@ -498,8 +509,8 @@ __device__ __forceinline__ void integrate64(const KArgs &a, const WorldDev &w, u
     const Vec4d vh = ((const Vec4d *)a.velA)[s];
     const uint32_t hh = hash_of(ph);
     double x[3] = {ph.x, ph.y, ph.z};
+    const uint32_t id = a.ids[s];
     if (!(hh & (1u << 27))) {  // polymer bead: its bond terms, in CSR order
-        const uint32_t id = a.ids[s];
         const Vec4d *bt = (const Vec4d *)a.bterm;
 #pragma unroll 1
         for (uint32_t r = a.bond_row[id]; r < a.bond_row[id + 1]; r++) {
@@ -517,19 +528,19 @@ __device__ __forceinline__ void integrate64(const KArgs &a, const WorldDev &w, u
         F[0] = F[1] = F[2] = 0.0;
     }
     if (FINAL) {
-        Vec4d vo = {v[0], v[1], v[2], 0.0};
+        Vec4d vo = {v[0], v[1], v[2], id_word64(id)};
         Vec4d fo = {F[0], F[1], F[2], 0.0};
         ((Vec4d *)a.velB)[s] = vo;
         ((Vec4d *)a.frc)[s] = fo;
         if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]))) err |= ERR_NONFINITE;
     } else {
         const uint32_t key = advance_position64(w, dt, hdt2, x, v, F, err);
-        const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+        cell_arrive(a, key, id);
         Vec4d po = {x[0], x[1], x[2], ph.w};
-        Vec4d vo = {v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, 0.0};
+        Vec4d vo = {v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, id_word64(id)};
         ((Vec4d *)a.posB)[s] = po;
         ((Vec4d *)a.velB)[s] = vo;
-        a.keyrank[s] = make_uint2(key, rank);
+        a.key[s] = key;
     }
     if (err) atomicOr(&a.worlds[world].err, err);
 }
@@ -543,7 +554,7 @@ __device__ __forceinline__ void integrate64(const KArgs &a, const WorldDev &w, u
 //      lanes of a warp evaluate lists of about the same length (the FP64 pipe executes an
 //      instruction for the whole warp whatever its active lanes); every list is still
 //      summed by one thread in its own order, so the result is the same;
-//   3. each thread adds its bead's bond terms (k_bonds64) in CSR order, then update_mom and
+//   3. each thread adds its bead's bond terms (bonds64) in CSR order, then update_mom and
 //      either the final write or the next update_pos with its cell count.
 template <int FINAL>
 __global__ void __launch_bounds__(TILE_BEADS) k_force64(KArgs a)
@@ -634,13 +645,14 @@ __global__ void __launch_bounds__(TILE_BEADS) k_begin64(KArgs a)
         const double v[3] = {st ? 0.0 : vh.x, st ? 0.0 : vh.y, st ? 0.0 : vh.z};
         const double F[3] = {st ? 0.0 : fh.x, st ? 0.0 : fh.y, st ? 0.0 : fh.z};
         const uint32_t key = advance_position64(w, dt, hdt2, x, v, F, err);
-        const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+        const uint32_t id = a.ids[s];
+        cell_arrive(a, key, id);
         Vec4d po = {x[0], x[1], x[2], ph.w};
-        Vec4d vo = st ? Vec4d{vh.x, vh.y, vh.z, 0.0}
-                      : Vec4d{v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, 0.0};
+        Vec4d vo = st ? Vec4d{vh.x, vh.y, vh.z, id_word64(id)}
+                      : Vec4d{v[0] + F[0] * hdt, v[1] + F[1] * hdt, v[2] + F[2] * hdt, id_word64(id)};
         ((Vec4d *)a.posB)[s] = po;
         ((Vec4d *)a.velB)[s] = vo;
-        a.keyrank[s] = make_uint2(key, rank);
+        a.key[s] = key;
         if (err) atomicOr(&a.worlds[tl.world].err, err);
     }
 }
@@ -673,15 +685,14 @@ __global__ void k_bin64(KArgs a, const uint32_t *__restrict__ hash_in)
     }
     if (err) atomicOr(&a.worlds[lo].err, err);
     const uint32_t key = w.cell_base + ((uint32_t)c[0] * (uint32_t)w.L[1] + (uint32_t)c[1]) * (uint32_t)w.L[2] + (uint32_t)c[2];
-    const uint32_t rank = atomicAdd(&a.cnt[key], 1u);
+    cell_arrive(a, key, g);
     Vec4d po = {x[0], x[1], x[2], __longlong_as_double((long long)hash_in[g])};
-    Vec4d vo = {st[field], st[field + 1], st[field + 2], 0.0};
+    Vec4d vo = {st[field], st[field + 1], st[field + 2], id_word64(g)};
     Vec4d fo = {st[2 * field], st[2 * field + 1], st[2 * field + 2], 0.0};
     ((Vec4d *)a.posB)[g] = po;
     ((Vec4d *)a.velB)[g] = vo;
     ((Vec4d *)a.frcB)[g] = fo;
-    a.ids[g] = g;
-    a.keyrank[g] = make_uint2(key, rank);
+    a.key[g] = key;
 }
 
 __global__ void k_finish64(KArgs a)
@@ -715,15 +726,18 @@ int launch_pair_log64(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const
     return 1;
 }
 
+int launch_cells64(const KArgs &a, int tick, int bonds, cudaStream_t s)
+{
+    const uint32_t nb = scan_blocks(a.n_cells);
+    const uint32_t bb = bonds ? (a.n_bonds + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    const uint32_t ab = bonds ? (a.n_angles + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    if (scan_one_pass(a.n_cells)) k_cells64<true><<<nb + bb + ab, SCAN_THREADS, 0, s>>>(a, nb, bb, tick);
+    else k_cells64<false><<<nb + bb + ab, SCAN_THREADS, 0, s>>>(a, nb, bb, tick);
+    return 1;
+}
+
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
 {
-    int n = 0;
-    if (a.n_bonds + a.n_angles > 0) {
-        const uint32_t bb = (a.n_bonds + BOND64_THREADS - 1) / BOND64_THREADS;
-        const uint32_t ab = (a.n_angles + BOND64_THREADS - 1) / BOND64_THREADS;
-        k_bonds64<<<bb + ab, BOND64_THREADS, 0, s>>>(a, bb);
-        n++;
-    }
     if (a.list) {  // each pair once
         const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb, (uint32_t)a.block_threads);
         const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
@@ -734,16 +748,16 @@ int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
         k_pairs64<<<std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s>>>(a);
         const uint32_t parts = a.n_tiles * (TILE_BEADS / SUM64_BEADS);
-        if (a.n_tiles == 0) return n + 2;
+        if (a.n_tiles == 0) return 2;
         if (final_step) k_sum64<1><<<parts, SUM64_THREADS, 0, s>>>(a);
         else k_sum64<0><<<parts, SUM64_THREADS, 0, s>>>(a);
-        return n + 3;
+        return 3;
     }
     if (final_step)
         k_force64<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
     else
         k_force64<0><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
-    return n + 1;
+    return 1;
 }
 
 // Largest staged-bead capacity of a k_list64 brick with two blocks per SM (large bricks).

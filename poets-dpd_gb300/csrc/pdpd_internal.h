@@ -78,6 +78,12 @@ struct BondTerm {
     uint32_t param;
 };
 
+// Beads that found their cell's bucket full in this cell-list rebuild: their number, and the
+// epoch that tells this rebuild's lists from earlier ones.
+struct Overflow {
+    uint32_t count, epoch;
+};
+
 // Everything a step kernel needs.  Pointers are device pointers; the payload arrays are
 // float4 (FP32 engine) or Vec4d (FP64 engine).
 struct KArgs {
@@ -101,8 +107,13 @@ struct KArgs {
                          // the sort places first; not written for empty cells
     // advanced, not yet sorted state (B), indexed by the A slot it came from
     void *posB, *velB, *frcB;
-    uint2 *keyrank;      // (new global cell, arrival rank in that cell)
-    uint4 *tmp;          // (old slot, id, cell, 0) placed by provisional rank
+    uint32_t *key;       // new global cell
+    uint32_t *bucket;    // bucket_k (a multiple of 4) entries per cell: the ids of the beads that have
+                         // arrived in it, bit 31: the upper z half (FP32)
+    uint32_t bucket_k;
+    Overflow *over;      // beads that found their bucket full
+    unsigned long long *over_head;  // per cell: epoch << 32 | first node
+    uint2 *over_node;    // (entry, next node)
     // bonds
     const uint32_t *bond_row;  // n_beads+1 CSR rows by global id
     const BondTerm *bond_terms;
@@ -115,7 +126,7 @@ struct KArgs {
     uint32_t n_bonds, n_angles;
     const uint32_t *row_of;      // CSR row of each end of the flat lists, in their order
     const uint32_t *hash;        // BeadHash by bead id
-    float4 *fbond;               // FP32: bond force of each bonded bead, by sorted slot
+    float4 *fbond;               // FP32: bond force of each bonded bead, by id
     float4 *posf;                // FP64: (x - floor(x), hash) in FP32, by sorted slot: the
                                  // neighbour walk's distance prefilter
     void *bterm;                 // FP64: each bond term's force (Vec4d), by CSR row
@@ -158,7 +169,7 @@ struct KArgs {
 //   sort:   B -> A counting sort (pdpd_sort.cu)
 int launch_bin32(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
 int launch_begin32(const KArgs &a, cudaStream_t s);
-int launch_force32(const KArgs &a, int final_step, cudaStream_t s);  // includes the bond kernel
+int launch_force32(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish32(const KArgs &a, cudaStream_t s);
 int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
 // FP64 list kernel: staged-bead capacity of a brick, and its persistent grid (0 or a cudaError_t).
@@ -167,7 +178,14 @@ int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int 
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);
-int launch_sort(const KArgs &a, int fp64, int tick, int with_force, cudaStream_t s);
+// bonds: with the bond forces at the beads' new positions, for the force pass that follows.
+int launch_sort(const KArgs &a, int fp64, int tick, int with_force, int bonds, cudaStream_t s);
+// Its prefix sum of the cell counts, with the bond forces in the same launch; over more cells
+// than one kernel takes (scan_one_pass) it needs the chunks' sums first.
+bool scan_one_pass(uint32_t n_cells);
+void launch_cells_reduce(const KArgs &a, int tick, cudaStream_t s);
+int launch_cells32(const KArgs &a, int tick, int bonds, cudaStream_t s);
+int launch_cells64(const KArgs &a, int tick, int bonds, cudaStream_t s);
 
 // One record of the pair log (pdpd_log_pair_terms; the C ABI's pdpd_pair_terms has this
 // layout, with world-local ids): bead ids are global here.

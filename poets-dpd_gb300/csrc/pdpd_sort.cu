@@ -1,62 +1,41 @@
 // Cell-list rebuild: a counting sort of the advanced beads by their new cell.
 //
-// The step kernels have already counted each cell's arrivals (one atomicAdd per bead, which
-// also gives the bead a provisional rank inside its new cell).  Here:
-//   1. k_scan_reduce + k_scan_final: exclusive prefix sum of the counts -> start[] (and
-//      the counts are cleared for the next step);
-//   2. k_place: each bead writes (old slot, id, cell, z half) at start[cell] + provisional rank;
-//   3. k_canon: each placed bead re-ranks itself by (z half, bead id) inside its cell and
-//      moves its payload to start[cell] + that rank.
+// The step kernels have already counted each bead into its new cell and entered it in the
+// cell's bucket (cell_arrive, pdpd_cells.cuh).  Here:
+//   1. an exclusive prefix sum of the counts -> start[]: one kernel for up to 32K cells, two
+//      above; the launch also holds the bond forces of the next force pass (they need only the
+//      advanced positions, so their blocks run beside the few of the prefix sum);
+//   2. k_move: each bead ranks itself by (z half, bead id) among its cell's bucket and moves
+//      its payload to start[cell] + that rank; the counts are cleared for the next step.
 // The result is canonical: cells in index order, beads inside a cell in ascending bead id,
 // whatever order the atomics ran in.  That is the order in which the reference's cell lists
 // hold beads (naive_dpd_engine_half_step.hpp:276-293), so the FP64 force kernel adds pair
 // forces in the reference's order and the engine is deterministic run to run.  The FP32
-// engine marks beads whose cell offset z is >= 0.5 (bit 31 of the arrival rank): they follow
-// the lower-half beads of their cell, still in id order, and zlo[cell] counts the lower
-// half, so the FP32 neighbour walk can skip the far half of an end cell.
-#include "pdpd_device.cuh"
+// engine orders the beads whose cell offset z is >= 0.5 after the lower-half beads of their
+// cell, each half in id order, and zlo[cell] counts the lower half, so the half-shell walk can
+// skip the far half of an end cell.
+// (A first version placed the beads by arrival rank and re-ranked them in a second kernel: five
+// launches per step with the bond kernel in front of the force pass.  32^3 polymer box, per
+// step: 17 us of sort and 12 us of bonds.)
+#include <algorithm>
+
+#include "pdpd_cells.cuh"
 
 namespace pdpd {
-
-constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
-constexpr uint32_t SCAN_CHUNK = SCAN_THREADS * SCAN_ITEMS;
 
 uint32_t scan_blocks(uint32_t n_cells)
 {
     return (n_cells + SCAN_CHUNK - 1) / SCAN_CHUNK;
 }
 
-__device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t *sh)
+bool scan_one_pass(uint32_t n_cells)
 {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    uint32_t r = 0;
-    if (warp == 0) {
-        r = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0;
-        for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
-        if (lane == 0) sh[0] = r;
-    }
-    __syncthreads();
-    r = sh[0];
-    __syncthreads();
-    return r;
+    return scan_blocks(n_cells) <= SCAN_ONE_PASS;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__restrict__ cnt,
-                                                               uint32_t n, uint32_t *blocksums,
-                                                               WorldDev *worlds, uint32_t n_worlds,
-                                                               int tick, uint32_t *brick_next,
-                                                               unsigned long long *list_cursor)
+// The chunks' sums of cnt[0, n).
+__device__ __forceinline__ void reduce_chunk(const uint32_t *__restrict__ cnt, uint32_t n, uint32_t *blocksums)
 {
-    // the next force pass takes its bricks from a fresh queue, and room for its lists
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (brick_next) *brick_next = 0u;
-        if (list_cursor) list_cursor[0] = list_cursor[1] = 0ull;
-    }
     __shared__ uint32_t sh[32];
     const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
     uint32_t s = 0;
@@ -65,9 +44,23 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__
         if (base + k < n) s += cnt[base + k];
     s = block_sum(s, sh);
     if (threadIdx.x == 0) blocksums[blockIdx.x] = s;
-    // The force pass that produced these counts has finished: advance every world's t.
-    if (tick && blockIdx.x == 0)
-        for (uint32_t w = threadIdx.x; w < n_worlds; w += blockDim.x) worlds[w].t += 1;
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_cells_reduce(KArgs a, int tick)
+{
+    if (blockIdx.x == 0) rebuild_begin(a, tick);
+    reduce_chunk(a.cnt, a.n_cells, a.blocksums);
+}
+
+void launch_cells_reduce(const KArgs &a, int tick, cudaStream_t s)
+{
+    k_cells_reduce<<<scan_blocks(a.n_cells), SCAN_THREADS, 0, s>>>(a, tick);
+}
+
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__restrict__ cnt, uint32_t n,
+                                                               uint32_t *blocksums)
+{
+    reduce_chunk(cnt, n, blocksums);
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_final(uint32_t *__restrict__ cnt, uint32_t n,
@@ -79,54 +72,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_final(uint32_t *__restric
     uint32_t off = 0;
     for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) off += blocksums[b];
     off = block_sum(off, sh);
-
+    scan_chunk(cnt, n, blockIdx.x, off, start, sh);
     const uint32_t base = blockIdx.x * SCAN_CHUNK + threadIdx.x * SCAN_ITEMS;
-    uint32_t v[SCAN_ITEMS];
-    uint32_t tsum = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        v[k] = (base + k < n) ? cnt[base + k] : 0u;
-        tsum += v[k];
-    }
-    // Block-wide exclusive scan of the thread totals.
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    uint32_t inc = tsum;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) sh[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0;
-        uint32_t wi = w;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, wi, o);
-            if (lane >= o) wi += y;
-        }
-        sh[lane] = wi - w;  // exclusive warp offsets
-    }
-    __syncthreads();
-    uint32_t run = off + sh[warp] + (inc - tsum);
-#pragma unroll
-    for (int k = 0; k < SCAN_ITEMS; k++) {
-        if (base + k < n) {
-            start[base + k] = run;
-            cnt[base + k] = 0u;
-        }
-        run += v[k];
-    }
-}
-
-__global__ void k_place(uint32_t n, const uint2 *__restrict__ keyrank,
-                        const uint32_t *__restrict__ start, const uint32_t *__restrict__ ids,
-                        uint4 *__restrict__ tmp)
-{
-    uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    uint2 kr = keyrank[s];
-    uint32_t dst = start[kr.x] + (kr.y & 0x7fffffffu);
-    tmp[dst] = make_uint4(s, ids[s], kr.x, kr.y >> 31);
+    for (int k = 0; k < SCAN_ITEMS; k++)
+        if (base + k < n) cnt[base + k] = 0u;
 }
 
 // The bead hash carried in the w component of a position payload.
@@ -141,81 +90,87 @@ __device__ __forceinline__ uint32_t payload_hash(const Vec4d &p)
 
 // FP64 positions as FP32 offsets inside their cell (x - floor(x) is exact in FP64, the cell
 // being floor(x)), for the force kernel's distance prefilter; the hash rides along.
-__device__ __forceinline__ float4 offset_shadow(const float4 &p)
-{
-    return p;
-}
 __device__ __forceinline__ float4 offset_shadow(const Vec4d &p)
 {
     return make_float4((float)(p.x - floor(p.x)), (float)(p.y - floor(p.y)), (float)(p.z - floor(p.z)),
                        __uint_as_float(payload_hash(p)));
 }
 
-// slot_of_id is kept for polymer beads only (monomer bit of the hash clear): the bond kernels
-// look up bond partners through it; the codec walks slots and reads ids instead.
+__device__ __forceinline__ uint32_t z_half(const float4 &p) { return p.z >= 0.5f ? 0x80000000u : 0u; }
+__device__ __forceinline__ uint32_t z_half(const Vec4d &) { return 0u; }
+__device__ __forceinline__ void put_shadow(const KArgs &, uint32_t, const float4 &) {}
+__device__ __forceinline__ void put_shadow(const KArgs &a, uint32_t dst, const Vec4d &p) { a.posf[dst] = offset_shadow(p); }
+
+// Bound by memory: reads 8 (cell) + 32 (payload) bytes per bead in the old order, the cell's
+// bucket and start, and writes 40 in the new order, which is nearly the old one (a bead moves
+// little in a step), so both sides are nearly contiguous.  slot_of_id is kept for polymer beads
+// only (monomer bit of the hash clear): the bond kernels look up bond partners through it; the
+// codec walks slots and reads ids instead.
 template <class P>
-__global__ void k_canon(uint32_t n, const uint4 *__restrict__ tmp, const uint32_t *__restrict__ start,
-                        const P *__restrict__ pos_in, const P *__restrict__ vel_in,
-                        const P *__restrict__ frc_in, P *__restrict__ pos_out,
-                        P *__restrict__ vel_out, P *__restrict__ frc_out,
-                        uint32_t *__restrict__ ids_out, uint32_t *__restrict__ cellg_out,
-                        uint32_t *__restrict__ slot_of_id, float4 *__restrict__ shadow_out,
-                        uint16_t *__restrict__ zlo)
+__global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
 {
-    uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= n) return;
-    uint4 e = tmp[d];
-    uint32_t b = start[e.z], end = start[e.z + 1];
+    const uint32_t s = blockIdx.x * 256 + threadIdx.x;
+    if (s < a.n_cells) a.cnt[s] = 0u;
+    if (s >= a.n_beads) return;
+    const uint32_t key = a.key[s];
+    const P p = ((const P *)a.posB)[s], v = ((const P *)a.velB)[s];
+    const uint32_t id = payload_id(v), me = id | z_half(p);
+    const uint32_t b = a.start[key], n = a.start[key + 1] - b;
+    const uint32_t m = min(n, a.bucket_k);
+    const uint4 *bucket = (const uint4 *)(a.bucket + (size_t)key * a.bucket_k);
     uint32_t rank = 0, lo = 0;
-    for (uint32_t k = b; k < end; k++) {
-        const uint4 o = tmp[k];
-        rank += (o.w < e.w || (o.w == e.w && o.y < e.y)) ? 1u : 0u;
-        lo += o.w == 0u ? 1u : 0u;
+    for (uint32_t k = 0; k < m; k += 4) {
+        const uint4 q = bucket[k / 4];
+        const uint32_t o[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (uint32_t u = 0; u < 4; u++) {
+            const bool in = k + u < m;
+            rank += in && o[u] < me ? 1u : 0u;
+            lo += in && !(o[u] >> 31) ? 1u : 0u;
+        }
     }
-    if (zlo && rank == 0) zlo[e.z] = (uint16_t)min(lo, 0xffffu);
-    uint32_t dst = b + rank;
-    const P p = pos_in[e.x];
-    pos_out[dst] = p;
-    vel_out[dst] = vel_in[e.x];
-    if (frc_in) frc_out[dst] = frc_in[e.x];
-    ids_out[dst] = e.y;
-    cellg_out[dst] = e.z;
-    if (!(payload_hash(p) & (1u << 27))) slot_of_id[e.y] = dst;
-    if (shadow_out) shadow_out[dst] = offset_shadow(p);
+    if (n > m) {  // the cell's overflowing beads
+        const unsigned long long head = a.over_head[key];
+        uint32_t node = (uint32_t)(head >> 32) == a.over->epoch ? (uint32_t)head : 0xffffffffu;
+        while (node != 0xffffffffu) {
+            const uint2 o = a.over_node[node];
+            rank += o.x < me ? 1u : 0u;
+            lo += o.x >> 31 ? 0u : 1u;
+            node = o.y;
+        }
+    }
+    if (a.zlo && rank == 0) a.zlo[key] = (uint16_t)min(lo, 0xffffu);
+    const uint32_t dst = b + rank;
+    ((P *)a.posA)[dst] = p;
+    ((P *)a.velA)[dst] = v;
+    if (with_force) ((P *)a.frc)[dst] = ((const P *)a.frcB)[s];
+    a.ids[dst] = id;
+    a.cellg[dst] = key;
+    if (!(payload_hash(p) & (1u << 27))) a.slot_of_id[id] = dst;
+    put_shadow(a, dst, p);
 }
 
 void launch_scan(uint32_t *cnt, uint32_t n, uint32_t *blocksums, uint32_t *start, cudaStream_t s)
 {
     if (n == 0) return;
     const uint32_t nb = scan_blocks(n);
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(cnt, n, blocksums, nullptr, 0, 0, nullptr, nullptr);
+    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(cnt, n, blocksums);
     k_scan_final<<<nb, SCAN_THREADS, 0, s>>>(cnt, n, blocksums, start);
 }
 
-int launch_sort(const KArgs &a, int fp64, int tick, int with_force, cudaStream_t s)
+int launch_sort(const KArgs &a, int fp64, int tick, int with_force, int bonds, cudaStream_t s)
 {
-    const uint32_t nb = scan_blocks(a.n_cells);
-    k_scan_reduce<<<nb, SCAN_THREADS, 0, s>>>(a.cnt, a.n_cells, a.blocksums, a.worlds, a.n_worlds,
-                                              tick, a.brick_next, a.list_cursor);
-    k_scan_final<<<nb, SCAN_THREADS, 0, s>>>(a.cnt, a.n_cells, a.blocksums, a.start);
-    const int T = 256;
-    const uint32_t g = (a.n_beads + T - 1) / T;
-    if (a.n_beads == 0) return 2;
-    k_place<<<g, T, 0, s>>>(a.n_beads, a.keyrank, a.start, a.ids, a.tmp);
-    if (fp64) {
-        k_canon<Vec4d><<<g, T, 0, s>>>(a.n_beads, a.tmp, a.start, (const Vec4d *)a.posB,
-                                       (const Vec4d *)a.velB,
-                                       with_force ? (const Vec4d *)a.frcB : nullptr,
-                                       (Vec4d *)a.posA, (Vec4d *)a.velA, (Vec4d *)a.frc, a.ids,
-                                       a.cellg, a.slot_of_id, a.posf, nullptr);
-    } else {
-        k_canon<float4><<<g, T, 0, s>>>(a.n_beads, a.tmp, a.start, (const float4 *)a.posB,
-                                        (const float4 *)a.velB,
-                                        with_force ? (const float4 *)a.frcB : nullptr,
-                                        (float4 *)a.posA, (float4 *)a.velA, (float4 *)a.frc,
-                                        a.ids, a.cellg, a.slot_of_id, nullptr, a.zlo);
+    int n = 0;
+    if (!scan_one_pass(a.n_cells)) {
+        launch_cells_reduce(a, tick, s);
+        n++;
     }
-    return 4;
+    n += fp64 ? launch_cells64(a, tick, bonds, s) : launch_cells32(a, tick, bonds, s);
+    if (a.n_beads == 0) return n;
+    const uint32_t g = (std::max(a.n_beads, a.n_cells) + 255) / 256;
+    if (fp64) k_move<Vec4d><<<g, 256, 0, s>>>(a, with_force);
+    else k_move<float4><<<g, 256, 0, s>>>(a, with_force);
+    return n + 1;
 }
 
 __global__ void k_rng_eval(size_t n, const uint32_t *__restrict__ t, const uint64_t *__restrict__ seed,

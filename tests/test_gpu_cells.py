@@ -1,0 +1,61 @@
+"""The cell-list rebuild where it changes path: cells that hold as many beads as their bucket has
+room for, one more, and many more (the overflow lists), and cell counts at the edges of the
+one-kernel prefix sum (16 chunks of 2,048 cells)."""
+
+import numpy as np
+import pytest
+
+import oracle as O
+import pdpd_engine as E
+import pdpd_world as W
+
+pytestmark = pytest.mark.gpu
+
+
+def _clumps(counts, seed):
+    """A 6^3 box of density about 3 whose first cells hold the given numbers of beads."""
+    w = W.make_water(6, seed=seed, a=0.5, gamma=0.5, dt=0.001)
+    rng = np.random.default_rng(seed)
+    at = 0
+    for k, n in enumerate(counts):
+        cell = np.array([k // 6, k % 6, (3 * k) % 6], float)
+        w.x[at:at + n] = cell + 0.01 + 0.98 * rng.random((n, 3))
+        at += n
+    assert at <= w.n_beads
+    return w
+
+
+COUNTS = [15, 16, 17, 18, 33, 64, 65, 130]
+
+
+def _run(worlds, prec, steps):
+    eng = E.GB300DPDEngine(prec)
+    eng.AttachBatch(worlds)
+    eng.Run(steps)
+
+
+def test_full_and_overflowing_cells_fp64():
+    w = _clumps(COUNTS, 71)
+    o = O.OracleWorld(w)
+    o.run(3)
+    _run([w], "fp64", 3)
+    assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
+
+
+def test_full_and_overflowing_cells_fp32():
+    """Alone the clumped cells overflow their buckets; beside a dense world, which gives the
+    batch larger buckets, fewer do: the same state to the bit."""
+    a = _clumps(COUNTS, 72)
+    b, dense = a.copy(), W.make_water((3, 4, 3), seed=73, a=0.5, density=24, dt=0.001)
+    _run([a], "fp32", 3)
+    _run([dense, b], "fp32", 3)
+    assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
+
+
+@pytest.mark.parametrize("box", [(2, 2, 512), (32, 32, 32), (31, 33, 32), (32, 32, 33), (2, 5, 3277), (64, 64, 9)])
+def test_prefix_sum_edges(box):
+    w = W.make_water(box, seed=74, density=0.5)
+    o = O.OracleWorld(w)
+    o.run(2, nthreads=8)
+    _run([w], "fp64", 2)
+    assert np.array_equal(w.x, o.x) and np.array_equal(w.f, o.f)
