@@ -267,7 +267,7 @@ int pdpd_log_pair_terms(pdpd_engine *e, uint32_t world, const uint32_t *bead_ids
  *           of the n_steps steps makes it return PDPD_E_BEAD_LOST.
  * Limits: at most PDPD_NOALLOC_MAX_BEADS beads and PDPD_NOALLOC_MAX_CELLS cells; worlds with
  * Hookean or angle bonds are rejected (PDPD_E_UNSUPPORTED); larger worlds get PDPD_E_NOMEM.
- * Scratch memory is one fixed array inside the library (about 1.3 MB), held on every GPU that
+ * Scratch memory is one fixed array inside the library (about 2 MB), held on every GPU that
  * loads the library until the process exits.  The first call on a device looks up that
  * array's device address (cudaGetSymbolAddress); make that first call before any stream
  * capture begins.  Every call reuses the same array: calls that overlap on the GPU (on

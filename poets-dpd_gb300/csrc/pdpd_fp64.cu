@@ -803,7 +803,7 @@ int launch_finish64(const KArgs &a, cudaStream_t s)
 // on device arrays the caller owns, and keeps its own scratch -- the cell counts, cell
 // starts, arrival ranks and the canonical bead order of the counting sort -- in the
 // file-scope array g_noalloc_scratch below instead of allocating it.  Every GPU that loads
-// the library holds this array (about 1.3 MB) until the process exits.  All calls share
+// the library holds this array (about 2 MB) until the process exits.  All calls share
 // it: calls that overlap on the GPU (on different streams, or from different host threads
 // without ordering) race on it and corrupt each other's cell lists.
 //
@@ -824,7 +824,7 @@ struct NaScratch {
     uint32_t start[NA_MAX_CELLS + 1];
     uint2 keyrank[NA_MAX_BEADS];
     uint32_t tmp[NA_MAX_BEADS];
-    uint32_t order[NA_MAX_BEADS];
+    float4 pos[NA_MAX_BEADS];  // in cell order: offset in the cell (x - floor(x) in FP32), bead id
 };
 
 struct NaParams {
@@ -847,17 +847,18 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(pdpd::Na
 namespace pdpd {
 namespace {
 
-// Zeroes the cell counts before each step; the error word only before a call's first step,
-// so that a bead lost in any step of the call is still reported at its end.
-__global__ void k_na_clear(NaScratch *S, uint32_t n_cells, int clear_err)
+// Before a call's first step: zeroes the cell counts (each step's scan leaves them zero) and the
+// error word, so that a bead lost in any step of the call is reported at its end.
+__global__ void k_na_clear(NaScratch *S, uint32_t n_cells)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_cells) S->cnt[i] = 0u;
-    if (i == 0 && clear_err) S->err = 0u;
+    if (i == 0) S->err = 0u;
 }
 
-// update_pos (dpd_maths_core_half_step.hpp:22-49) and the bead's new cell and arrival rank.
-__global__ void k_na_update_pos(NaParams p, NaScratch *S, double *x, double *v, double *f)
+// update_pos (dpd_maths_core_half_step.hpp:22-49) and the bead's new cell and arrival rank; before
+// it (mom) the update_mom (:51-61) of the step before, the same bead's.
+__global__ void k_na_update_pos(NaParams p, NaScratch *S, double *x, double *v, double *f, int mom)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= p.n) return;
@@ -865,7 +866,10 @@ __global__ void k_na_update_pos(NaParams p, NaScratch *S, double *x, double *v, 
     int c[3];
     for (int d = 0; d < 3; d++) {
         const double L = (double)p.L[d];
-        double xn = x[3 * i + d] + v[3 * i + d] * dt + f[3 * i + d] * hdt2;
+        const double fd = f[3 * i + d];
+        double vd = v[3 * i + d];
+        if (mom) vd = vd + fd * hdt;
+        double xn = x[3 * i + d] + vd * dt + fd * hdt2;
         if (xn < 0) {
             xn += L;
             if (xn == L) xn = 0;
@@ -878,8 +882,7 @@ __global__ void k_na_update_pos(NaParams p, NaScratch *S, double *x, double *v, 
         }
         x[3 * i + d] = xn;
         c[d] = (int)floor(xn);
-        v[3 * i + d] = v[3 * i + d] + f[3 * i + d] * hdt;
-        f[3 * i + d] = 0.0;
+        v[3 * i + d] = vd + fd * hdt;
     }
     const uint32_t key = ((uint32_t)c[0] * (uint32_t)p.L[1] + (uint32_t)c[1]) * (uint32_t)p.L[2] + (uint32_t)c[2];
     const uint32_t rank = atomicAdd(&S->cnt[key], 1u);
@@ -907,6 +910,7 @@ __global__ void __launch_bounds__(1024) k_na_scan(NaScratch *S, uint32_t n_cells
     for (uint32_t k = b; k < e; k++) {
         S->start[k] = run;
         run += S->cnt[k];
+        S->cnt[k] = 0u;
     }
     if (threadIdx.x == 0) S->start[n_cells] = n;
 }
@@ -920,7 +924,7 @@ __global__ void k_na_place(NaScratch *S, uint32_t n)
 }
 
 // Canonical cell order: beads of a cell in ascending id, as the reference's cell lists.
-__global__ void k_na_canon(NaScratch *S, uint32_t n)
+__global__ void k_na_canon(NaScratch *S, uint32_t n, const double *__restrict__ x)
 {
     const uint32_t d = blockIdx.x * blockDim.x + threadIdx.x;
     if (d >= n) return;
@@ -929,78 +933,169 @@ __global__ void k_na_canon(NaScratch *S, uint32_t n)
     const uint32_t b = S->start[key], e = S->start[key + 1];
     uint32_t rank = 0;
     for (uint32_t k = b; k < e; k++) rank += S->tmp[k] < i ? 1u : 0u;
-    S->order[b + rank] = i;
+    float o[3];
+    for (int k = 0; k < 3; k++) o[k] = (float)(x[3 * i + k] - floor(x[3 * i + k]));
+    S->pos[b + rank] = make_float4(o[0], o[1], o[2], __uint_as_float(i));
 }
 
-// Pair forces (update_cell_forces + calc_force, naive_dpd_engine_half_step.hpp:300-424 and
-// dpd_maths_core_half_step.hpp:69-157), the same operations in the same order as
-// pair_forces64 / list_forces64.
-__global__ void k_na_forces(NaParams p, NaScratch *S, const double *__restrict__ x,
-                            const double *__restrict__ v, double *__restrict__ f,
-                            const uint32_t *__restrict__ hash)
+// One pair's term on bead i from bead j in direction dir (0..26, z fastest) of cell c: the
+// reference's separation, pair test and calc_force (naive_dpd_engine_half_step.hpp:181-196,
+// 404-411, dpd_maths_core_half_step.hpp:69-157); false when out of range.
+__device__ __forceinline__ bool na_pair(const NaParams &p, const double (*pair)[2], const double *__restrict__ x,
+                                        const double *__restrict__ v, const uint32_t *__restrict__ hash, uint32_t i,
+                                        uint32_t j, const int c[3], uint32_t dir, uint32_t th_lo, uint32_t th_hi,
+                                        double t[3])
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
+    const int d[3] = {(int)(dir / 9) - 1, (int)(dir / 3 % 3) - 1, (int)(dir % 3) - 1};
+    double dx[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int raw = c[k] + d[k];
+        const double delta = raw == p.L[k] ? (double)p.L[k] : (raw < 0 ? -(double)p.L[k] : 0.0);
+        dx[k] = x[3 * i + k] - (x[3 * j + k] + delta);
+    }
+    const double dr2 = dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2];
+    if (dr2 >= 1 || dr2 < (double)min_dist_sqr_f()) return false;
+    const Vec4d vi = {v[3 * i], v[3 * i + 1], v[3 * i + 2], 0.0}, vj = {v[3 * j], v[3 * j + 1], v[3 * j + 2], 0.0};
+    const uint32_t hi = hash[i], hj = hash[j];
+    const uint32_t pk = min(hi >> 28, p.nt - 1u) * p.nt + min(hj >> 28, p.nt - 1u);
+    const PairTerms64 q = pair_terms64(dx[0], dx[1], dx[2], sqrt(dr2), Vec2d{pair[pk][0], pair[pk][1]}, vi, vj, hi, hj,
+                                       th_lo, th_hi, p.scale_inv_sqrt_dt);
+    for (int k = 0; k < 3; k++) t[k] = q.e[k] * q.scaled;
+    return true;
+}
+
+// Visit the beads of direction (dx, dy, dz)'s cell that can be in range of the bead at offset o in
+// cell c: the conservative FP32 test of the engine's lists (walk_global64).
+template <class Visit>
+__device__ __forceinline__ void na_cell(const NaParams &p, const NaScratch *S, const int c[3], const float4 o,
+                                        uint32_t dir, Visit visit)
+{
+    const int d[3] = {(int)(dir / 9) - 1, (int)(dir / 3 % 3) - 1, (int)(dir % 3) - 1};
+    const float gx = slab_gap(o.x, d[0]), gy = slab_gap(o.y, d[1]), gz = slab_gap(o.z, d[2]);
+    if (gx * gx + gy * gy + gz * gz >= WALK_R2) return;
+    int op[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int raw = c[k] + d[k];
+        op[k] = raw < 0 ? raw + p.L[k] : (raw == p.L[k] ? 0 : raw);
+    }
+    const float ax = o.x - (float)d[0], ay = o.y - (float)d[1], az = o.z - (float)d[2];
+    const uint32_t nc = ((uint32_t)op[0] * (uint32_t)p.L[1] + (uint32_t)op[1]) * (uint32_t)p.L[2] + (uint32_t)op[2];
+    const uint32_t k1 = S->start[nc + 1];
+    for (uint32_t k = S->start[nc]; k < k1; k++) {
+        const float4 q = S->pos[k];
+        const float ex = ax - q.x, ey = ay - q.y, ez = az - q.z;
+        if (ex * ex + ey * ey + ez * ez < WALK_R2) visit(__float_as_uint(q.w));
+    }
+}
+
+// Pair forces of NA_BEADS beads, consecutive in cell order.  Eight lanes of a bead walk its 9
+// neighbour rows into lists (a row each, the first lane also the last row); the block's
+// candidates are then evaluated flat, a thread each, and a thread per bead and axis adds a
+// bead's terms in walk order, the reference's.  One thread per bead did all of this for itself,
+// a serial chain of FP64 latencies on 48 blocks: 458 us for the 16^3 box against 34 us.
+constexpr int NA_BEADS = 16, NA_LANES = 8, NA_THREADS = NA_BEADS * NA_LANES, NA_ROWS = 9;
+constexpr uint32_t NA_ROW_CAP = 24, NA_TERMS = 512;
+__global__ void __launch_bounds__(NA_THREADS) k_na_forces(const __grid_constant__ NaParams p, const NaScratch *S,
+                                                          const double *__restrict__ x, const double *__restrict__ v,
+                                                          double *__restrict__ f, const uint32_t *__restrict__ hash)
+{
+    __shared__ double s_pair[256][2];
+    __shared__ double s_t[3][NA_TERMS];
+    __shared__ uint32_t s_row[NA_BEADS * NA_ROWS][NA_ROW_CAP];  // bead, direction << 16
+    __shared__ uint32_t s_pre[NA_BEADS * NA_ROWS + 1];          // entry counts, then their prefix
+    __shared__ uint32_t s_id[NA_BEADS];
+    __shared__ int s_c[NA_BEADS][3];
+    __shared__ uint32_t s_long[NA_BEADS];  // a row of this bead does not fit
+    const int tid = threadIdx.x, b = tid / NA_LANES, sub = tid % NA_LANES;
+    for (uint32_t k = tid; k < p.nt * p.nt; k += NA_THREADS) {
+        s_pair[k][0] = p.pair[k][0];
+        s_pair[k][1] = p.pair[k][1];
+    }
+    if (tid < NA_BEADS) s_long[tid] = 0u;
+    __syncthreads();
+    const uint32_t h = blockIdx.x * NA_BEADS + b;
+    const bool act = h < p.n;
+    uint32_t i = 0;
+    int c[3] = {0, 0, 0};
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (act) {
+        o = S->pos[h];
+        i = __float_as_uint(o.w);
+        const uint32_t key = S->keyrank[i].x, yz = (uint32_t)p.L[1] * (uint32_t)p.L[2];
+        c[0] = (int)(key / yz);
+        c[1] = (int)(key / (uint32_t)p.L[2] % (uint32_t)p.L[1]);
+        c[2] = (int)(key % (uint32_t)p.L[2]);
+        if (sub == 0) {
+            s_id[b] = i;
+            for (int k = 0; k < 3; k++) s_c[b][k] = c[k];
+        }
+    }
+    for (int row = sub; row < NA_ROWS; row += NA_LANES) {
+        uint32_t n = 0, *out = s_row[b * NA_ROWS + row];
+        for (uint32_t dz = 0; act && dz < 3; dz++)
+            na_cell(p, S, c, o, 3 * row + dz, [&](uint32_t j) {
+                if (j == i && row == 4 && dz == 1) return;
+                if (n < NA_ROW_CAP) out[n] = j | (3 * row + dz) << 16;
+                n++;
+            });
+        if (n > NA_ROW_CAP) {
+            s_long[b] = 1u;
+            n = 0;
+        }
+        s_pre[b * NA_ROWS + row] = n;
+    }
+    __syncthreads();
+    if (tid < 32) {  // exclusive prefix of the rows' counts
+        uint32_t carry = 0;
+        for (int r0 = 0; r0 < NA_BEADS * NA_ROWS; r0 += 32) {
+            const int r = r0 + tid;
+            const uint32_t n = r < NA_BEADS * NA_ROWS ? s_pre[r] : 0u;
+            uint32_t inc = n;
+            for (int off = 1; off < 32; off <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, inc, off);
+                if (tid >= off) inc += y;
+            }
+            if (r < NA_BEADS * NA_ROWS) s_pre[r] = carry + inc - n;
+            carry += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (tid == 0) s_pre[NA_BEADS * NA_ROWS] = carry;
+    }
+    __syncthreads();
     const uint64_t th = t_hash((uint32_t)p.t, p.seed);
     const uint32_t th_lo = (uint32_t)th, th_hi = (uint32_t)(th >> 32);
-    const uint32_t key = S->keyrank[i].x;
-    const int c[3] = {(int)(key / ((uint32_t)p.L[1] * (uint32_t)p.L[2])),
-                      (int)((key / (uint32_t)p.L[2]) % (uint32_t)p.L[1]), (int)(key % (uint32_t)p.L[2])};
-    const double xh[3] = {x[3 * i], x[3 * i + 1], x[3 * i + 2]};
-    const double vh[3] = {v[3 * i], v[3 * i + 1], v[3 * i + 2]};
-    const uint32_t hh = hash[i];
-    const uint32_t ti = min(hh >> 28, p.nt - 1u);
-    const double min2 = (double)min_dist_sqr_f();
-    double F[3] = {0.0, 0.0, 0.0};
-    int dir[3];
-    for (dir[0] = -1; dir[0] <= 1; dir[0]++)
-        for (dir[1] = -1; dir[1] <= 1; dir[1]++)
-            for (dir[2] = -1; dir[2] <= 1; dir[2]++) {
-                int op[3];
-                double delta[3];
-                for (int k = 0; k < 3; k++) {
-                    const int raw = c[k] + dir[k];
-                    const int is_left = raw < 0;
-                    const int is_right = raw == p.L[k];
-                    op[k] = raw + (is_left - is_right) * p.L[k];
-                    delta[k] = (double)(is_right - is_left) * (double)p.L[k];
-                }
-                const uint32_t nc = ((uint32_t)op[0] * (uint32_t)p.L[1] + (uint32_t)op[1]) * (uint32_t)p.L[2] + (uint32_t)op[2];
-                const uint32_t k1 = S->start[nc + 1];
-                for (uint32_t k = S->start[nc]; k < k1; k++) {
-                    const uint32_t j = S->order[k];
-                    const double obx = x[3 * j] + delta[0], oby = x[3 * j + 1] + delta[1], obz = x[3 * j + 2] + delta[2];
-                    const double dx0 = xh[0] - obx, dx1 = xh[1] - oby, dx2 = xh[2] - obz;
-                    const double dr2 = dx0 * dx0 + dx1 * dx1 + dx2 * dx2;
-                    if (dr2 >= 1 || dr2 < min2) continue;
-                    const double dr = sqrt(dr2);
-                    const uint32_t hj = hash[j];
-                    const uint32_t tj = min(hj >> 28, p.nt - 1u);
-                    const double con_strength = p.pair[ti * p.nt + tj][0];
-                    const double sqrt_diss = p.pair[ti * p.nt + tj][1];
-                    const double kappa = 0.0, r0 = 0.5;
-                    const double inv_dr = 1.0 / dr;
-                    const double dv0 = vh[0] - v[3 * j], dv1 = vh[1] - v[3 * j + 1], dv2 = vh[2] - v[3 * j + 2];
-                    const double wr = 1.0 - dr;
-                    const double con_force = con_strength * wr;
-                    const double e0 = dx0 * inv_dr, e1 = dx1 * inv_dr, e2 = dx2 * inv_dr;
-                    const double rdotv = e0 * dv0 + e1 * dv1 + e2 * dv2;
-                    const double sqrt_gammap = sqrt_diss * wr;
-                    const double diss_force = -sqrt_gammap * sqrt_gammap * rdotv;
-                    const double u = (double)hash_u(th_lo, th_hi, hh, hj);
-                    const double rand_scale = sqrt_gammap * p.scale_inv_sqrt_dt;
-                    const double rand_force = rand_scale * u;
-                    const double dr0 = r0 - dr;
-                    const double hookean_force = kappa * dr0;
-                    const double scaled = con_force + diss_force + rand_force + hookean_force;
-                    F[0] = F[0] + e0 * scaled;
-                    F[1] = F[1] + e1 * scaled;
-                    F[2] = F[2] + e2 * scaled;
-                }
-            }
-    f[3 * i] = F[0];
-    f[3 * i + 1] = F[1];
-    f[3 * i + 2] = F[2];
+    const uint32_t total = s_pre[NA_BEADS * NA_ROWS];
+    const int sb = tid % NA_BEADS, axis = tid / NA_BEADS;  // the summing threads' bead and axis
+    const uint32_t b0 = s_pre[sb * NA_ROWS], b1 = s_pre[(sb + 1) * NA_ROWS];
+    double F = 0.0;
+    for (uint32_t c0 = 0; c0 < total; c0 += NA_TERMS) {
+        const uint32_t c1 = min(total, c0 + NA_TERMS);
+        for (uint32_t e = c0 + tid; e < c1; e += NA_THREADS) {
+            uint32_t r = 0;  // the entry's row: the last with s_pre[r] <= e
+            for (uint32_t step = 128; step > 0; step >>= 1)
+                if (r + step < NA_BEADS * NA_ROWS && s_pre[r + step] <= e) r += step;
+            const uint32_t ent = s_row[r][e - s_pre[r]], eb = r / NA_ROWS;
+            double t[3] = {0.0, 0.0, 0.0};
+            na_pair(p, s_pair, x, v, hash, s_id[eb], ent & 0xffffu, s_c[eb], ent >> 16, th_lo, th_hi, t);
+            for (int k = 0; k < 3; k++) s_t[k][e - c0] = t[k];
+        }
+        __syncthreads();
+        if (axis < 3)
+            for (uint32_t e = max(b0, c0); e < min(b1, c1); e++) F = F + s_t[axis][e - c0];
+        __syncthreads();
+    }
+    if (axis < 3 && blockIdx.x * NA_BEADS + sb < p.n && !s_long[sb]) f[3 * s_id[sb] + axis] = F;
+    if (sub == 0 && act && s_long[b]) {  // a bead among very many: its pairs one by one
+        double G[3] = {0.0, 0.0, 0.0};
+        for (uint32_t dir = 0; dir < 27; dir++)
+            na_cell(p, S, c, o, dir, [&](uint32_t j) {
+                double t[3];
+                if ((j == i && dir == 13) || !na_pair(p, s_pair, x, v, hash, i, j, c, dir, th_lo, th_hi, t)) return;
+                for (int k = 0; k < 3; k++) G[k] = G[k] + t[k];
+            });
+        for (int k = 0; k < 3; k++) f[3 * i + k] = G[k];
+    }
 }
 
 // update_mom (dpd_maths_core_half_step.hpp:51-61).
@@ -1081,16 +1176,16 @@ extern "C" int pdpd_step_noalloc(const pdpd_world *w, double *d_x, double *d_v, 
         p.pair[k][1] = sqrt(w->dissipative[k]);
     }
     const uint32_t gb = (p.n + 255) / 256, gc = (p.n_cells + 255) / 256;
+    k_na_clear<<<gc, 256, 0, s>>>(S, p.n_cells);
     for (uint32_t step = 0; step < n_steps; step++) {
         p.t = w->t + (int64_t)step;
-        k_na_clear<<<gc, 256, 0, s>>>(S, p.n_cells, step == 0 ? 1 : 0);
-        k_na_update_pos<<<gb, 256, 0, s>>>(p, S, d_x, d_v, d_f);
+        k_na_update_pos<<<gb, 256, 0, s>>>(p, S, d_x, d_v, d_f, step > 0 ? 1 : 0);
         k_na_scan<<<1, 1024, 0, s>>>(S, p.n_cells, p.n);
         k_na_place<<<gb, 256, 0, s>>>(S, p.n);
-        k_na_canon<<<gb, 256, 0, s>>>(S, p.n);
-        k_na_forces<<<gb, 256, 0, s>>>(p, S, d_x, d_v, d_f, d_hash);
-        k_na_update_mom<<<gb, 256, 0, s>>>(p, d_v, d_f);
+        k_na_canon<<<gb, 256, 0, s>>>(S, p.n, d_x);
+        k_na_forces<<<(p.n + NA_BEADS - 1) / NA_BEADS, NA_THREADS, 0, s>>>(p, S, d_x, d_v, d_f, d_hash);
     }
+    k_na_update_mom<<<gb, 256, 0, s>>>(p, d_v, d_f);
     uint32_t err = 0;
     ce = cudaGetLastError();
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(&err, &S->err, sizeof err, cudaMemcpyDeviceToHost, s);
