@@ -277,7 +277,7 @@ const ConfigEntry kConfig[] = {
     {"grid_blocks", "Persistent grid size of the tile kernels (0 = 16 blocks per SM)."},
     {"graph_steps", "Timesteps captured per CUDA graph replay (0 = automatic)."},
     {"use_graphs", "Replay captured CUDA graphs (1) or launch kernels directly (0)."},
-    {"force_kernel", "FP32 force kernel (default by size: 8 from about 1,300 cells per SM, else 6): "
+    {"force_kernel", "FP32 force kernel (default 8): "
                      "1 = thread per bead from global memory, "
                      "6 = shared-memory brick, full shell, neighbour rows walked into lists, "
                      "128-thread blocks; 8 = as 6 with 512-thread blocks for larger bricks; "
@@ -286,8 +286,8 @@ const ConfigEntry kConfig[] = {
                      "384-thread blocks.  1, 6 and 8 give the same forces to the bit; 9 gives the "
                      "same forces to the bit whatever its brick shape, grid or batch, within the "
                      "FP32 tolerance of the others."},
-    {"brick_x", "Brick extent in cells along x (FP32 brick kernel; default by size: 5x8x8, "
-                "3x4x6 from about 200 cells per SM, 2x4x4 below)."},
+    {"brick_x", "Brick extent in cells along x (FP32 brick kernel; default by the batch's cells per "
+                "SM, from 2x4x4 to 5x8x8)."},
     {"brick_y", "Brick extent in cells along y (FP32 brick kernel)."},
     {"brick_z", "Brick extent in cells along z (FP32 brick kernel)."},
     {"autotune", "FP32: time the force-kernel variants and brick shapes on the first steps of "
@@ -336,7 +336,8 @@ struct pdpd_engine {
     // device arena
     DevBuf d_worlds, d_tiles, d_bricks, d_start, d_cnt, d_blocksums;
     DevBuf d_posA, d_velA, d_frc, d_posB, d_velB, d_frcB;
-    DevBuf d_ids, d_cellg, d_slot_of_id, d_key, d_bucket, d_over_node, d_over_head;
+    DevBuf d_ids, d_cellg, d_slot_of_id, d_key;
+    DevBuf d_buckets;  // the cells' overflow heads and buckets, the overflow nodes
     DevBuf d_bond_row, d_bond_terms, d_bond_params, d_pair, d_hash, d_bonded, d_fbond, d_cellpair, d_posf, d_bterm, d_zlo, d_brick_next, d_hash_old;
     DevBuf d_lists;   // FP64 pair lists (List64Room)
     DevBuf d_row_of;  // FP64: CSR row of each end of the flat bond lists
@@ -399,7 +400,7 @@ struct pdpd_engine {
         drop_graph();
         DevBuf *bufs[] = {&d_worlds, &d_tiles, &d_bricks, &d_start, &d_cnt, &d_blocksums, &d_posA, &d_velA,
                           &d_frc, &d_posB, &d_velB, &d_frcB, &d_ids, &d_cellg, &d_slot_of_id,
-                          &d_key, &d_bucket, &d_over_node, &d_over_head, &d_bond_row, &d_bond_terms, &d_bond_params,
+                          &d_key, &d_buckets, &d_bond_row, &d_bond_terms, &d_bond_params,
                           &d_pair, &d_hash, &d_bonded, &d_fbond, &d_staging[0], &d_staging[1],
                           &d_v2err, &d_cellpair, &d_posf, &d_bterm, &d_zlo, &d_brick_next, &d_hash_old,
                           &d_hostio, &d_inv, &d_blist, &d_scan, &d_lists, &d_row_of};
@@ -493,28 +494,51 @@ struct pdpd_engine {
         return PDPD_OK;
     }
 
+    // Brick shape for the 512-thread kernels (FP32 variant 8, the FP64 list kernel) by the batch's
+    // cells per SM: the largest bricks stage the fewest halo beads per home bead, but the
+    // persistent blocks (two per SM) want several bricks each, and a small batch has too few.
+    // Whole FP32 steps of polymer boxes, us (sides 20, 32, 40, 52, 64, 80; cells per SM 53, 216,
+    // 421, 925, 1725, 3368): 5x8x8 36.4, 41.0, 60.4, 93.5, 160.2, 279; 4x5x8 (480 home beads, one
+    // turn of the block) 27.9, 37.5, 53.5, 91.5, 154.2, 281; 4x4x8 26.9, 35.1, 56.5, 98.7, 158.3,
+    // 298; 4x4x6 26.0, 41.3, 59.4, 106, 182, 345; 2x4x4 25.5, 58.1, 94.8, 183, 336, 665 (sides 9
+    // and 16: 2x4x4 23.2 and 24.1, 4x4x6 23.7 and 26.0).  Smaller bricks where the halo of the
+    // batch's densest world would not fit the staging capacity 5 Poisson deviations above its
+    // mean.
+    template <class Limit> void wide_shape(int shape[3], Limit limit) const
+    {
+        static const int table[][3] = {{5, 8, 8}, {4, 5, 8}, {4, 4, 8}, {4, 4, 6}, {2, 4, 4}, {2, 2, 4}, {1, 2, 2}};
+        static const uint64_t from[] = {2500, 350, 110, 40, 0, 0, 0};  // cells per SM
+        const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
+        int k = 0;
+        while (per_sm < from[k]) k++;
+        for (; k < 6; k++) {
+            const uint32_t hc = (uint32_t)(table[k][0] + 2) * (table[k][1] + 2) * (table[k][2] + 2);
+            const double mean = max_density * hc;
+            if (mean + 5.0 * std::sqrt(mean) <= (double)limit(hc)) break;
+        }
+        for (int d = 0; d < 3; d++) shape[d] = table[k][d];
+    }
+
     // Default kernel variant and brick shape for the attached batch, where the config does not
-    // name them.  The persistent brick kernels want several bricks per SM: the 512-thread row
-    // walk on 5x8x8 bricks is fastest from about 1,300 cells per SM (a 58^3 box on 152 SMs),
-    // the 128-thread row walk on 3x4x6 bricks from about 200, and on 2x4x4 bricks below that.
-    // All of them give the same trajectory.
+    // name them: the 512-thread row walk.  All of them give the same trajectory.
     void default_shape()
     {
-        uint64_t cells = 0;
-        for (const WorldHost &wh : worlds)
-            cells += (uint64_t)wh.dev.L[0] * (uint64_t)wh.dev.L[1] * (uint64_t)wh.dev.L[2];
-        const uint64_t per_sm = cells / (uint64_t)std::max(1, sm_count);
-        if (!kernel_user) cfg_force_kernel = per_sm >= 1300 ? 8 : 6;
+        if (!kernel_user) cfg_force_kernel = 8;
         if (brick_user) return;
+        uint32_t npair = 1;
+        for (const WorldHost &wh : worlds) npair = std::max(npair, wh.dev.n_types * wh.dev.n_types);
+        if (cfg_force_kernel == 8 || cfg_force_kernel == 1) {
+            wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0); });
+            return;
+        }
+        // variant 9: the largest of these with at most 256 home cells whose halo fits; variant 6:
+        // its own shapes below about 1,300 cells per SM, else the largest
+        const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
         static const int big[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {4, 4, 6}, {3, 4, 4}};
         static const int mid[3] = {3, 4, 6}, small[3] = {2, 4, 4};
         const int *b = per_sm >= 200 ? mid : small;
-        if (cfg_force_kernel == 8 || cfg_force_kernel == 9 || per_sm >= 1300) {
-            // the largest brick whose halo (at the batch's highest density) fits the staging
-            // capacity 5 Poisson deviations above its mean, so dense boxes do not overflow it
+        if (cfg_force_kernel == 9 || per_sm >= 1300) {
             const int v = cfg_force_kernel == 9 ? 9 : 8;
-            uint32_t npair = 1;
-            for (const WorldHost &wh : worlds) npair = std::max(npair, wh.dev.n_types * wh.dev.n_types);
             b = big[4];
             for (const auto &c : big) {
                 if (v == 9 && c[0] * c[1] * c[2] > 256) continue;  // the half shell's home sums
@@ -528,29 +552,6 @@ struct pdpd_engine {
             }
         }
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];
-    }
-
-    // Brick shape and block size of the FP64 list kernel, by the batch's cells per SM as for the
-    // FP32 kernels.
-    void list64_shape(int shape[3])
-    {
-        const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
-        static const int big[3] = {5, 8, 8}, mid[3] = {3, 4, 6}, small[3] = {2, 4, 4};
-        const int *b = per_sm >= 1300 ? big : (per_sm >= 200 ? mid : small);
-        args.block_threads = b == big ? 512 : 128;
-        if (b == big) {  // (a denser batch: smaller bricks, as default_shape)
-            static const int less[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {4, 4, 6}, {3, 4, 4}};
-            b = less[4];
-            for (const auto &c : less) {
-                const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
-                const double mean = max_density * hc;
-                if (mean + 5.0 * std::sqrt(mean) <= (double)list64_maxb_limit(512, hc)) {
-                    b = c;
-                    break;
-                }
-            }
-        }
-        for (int d = 0; d < 3; d++) shape[d] = b[d];
     }
 
     // Staged beads a brick of hc halo cells should have room for: the mean halo population
@@ -583,7 +584,7 @@ struct pdpd_engine {
         a.n_bricks = 0;
         if (fp64() ? !a.list : a.force_kernel == 1) return PDPD_OK;
         int shape[3] = {cfg_brick[0], cfg_brick[1], cfg_brick[2]};
-        if (fp64()) list64_shape(shape);
+        if (fp64()) wide_shape(shape, [](uint32_t hc) { return list64_maxb_limit(hc); });
         // Each axis of a world is cut into ceil(L / b) bricks of as equal extents as possible
         // (e.g. a side of 9 with b = 4 into 3 + 3 + 3, not 4 + 4 + 1): no extent exceeds the
         // configured one, and no thin remainder brick stages a halo for a few home cells.
@@ -616,9 +617,9 @@ struct pdpd_engine {
         a.n_bricks = (uint32_t)bricks.size();
         a.brick_hc_max = (uint32_t)(shape[0] + 2) * (shape[1] + 2) * (shape[2] + 2);
         if (fp64()) {
-            const double most = (double)list64_maxb_limit(a.block_threads, a.brick_hc_max);
+            const double most = (double)list64_maxb_limit(a.brick_hc_max);
             a.brick_maxb = (uint32_t)std::min(most, std::max(64.0, staging_want(a.brick_hc_max)));
-            const int rc = list64_setup(sm_count, a.block_threads, a.brick_hc_max, a.brick_maxb, &a.brick_grid);
+            const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, &a.brick_grid);
             if (rc) return fail(PDPD_E_CUDA, "list kernel setup: %s", cudaGetErrorString((cudaError_t)rc));
             if (cfg_grid_blocks > 0) a.brick_grid = cfg_grid_blocks;
             drop_graph();
@@ -1339,9 +1340,9 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     A(e->d_cellg, sizeof(uint32_t) * nb);
     A(e->d_slot_of_id, sizeof(uint32_t) * nb);
     A(e->d_key, sizeof(uint32_t) * nb);
-    A(e->d_bucket, sizeof(uint32_t) * bucket_k * (size_t)nc);
-    A(e->d_over_head, sizeof(uint64_t) * (size_t)nc);
-    A(e->d_over_node, sizeof(uint2) * nb);
+    const size_t head_bytes = (sizeof(uint64_t) * (size_t)nc + 255) & ~size_t(255);
+    const size_t bucket_bytes = sizeof(uint32_t) * bucket_k * (size_t)nc;
+    A(e->d_buckets, head_bytes + bucket_bytes + sizeof(uint2) * nb);
     A(e->d_bond_row, sizeof(uint32_t) * (nb + 1));
     A(e->d_bond_terms, sizeof(BondTerm) * std::max<uint64_t>(1, n_terms));
     A(e->d_bond_params, (f64 ? sizeof(double) : sizeof(float)) * 4 * std::max<uint64_t>(1, n_bparams));
@@ -1355,7 +1356,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     A(e->d_fbond, f64 ? 16 : sizeof(float4) * std::max<uint64_t>(1, nb));
     A(e->d_posf, f64 ? sizeof(float4) * std::max<uint64_t>(1, nb) : 16);
     A(e->d_bterm, f64 ? sizeof(double) * 4 * std::max<uint64_t>(1, n_terms) : 16);
-    A(e->d_row_of, f64 ? sizeof(uint32_t) * std::max<uint64_t>(1, n_terms) : 16);
+    if (f64 && n_terms) A(e->d_row_of, sizeof(uint32_t) * n_terms);
     A(e->d_staging[0], sizeof(double) * 9 * nb);
     if (ce != cudaSuccess) {
         cudaGetLastError();
@@ -1497,7 +1498,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         ce = cudaMemcpyAsync(e->h_small.p, e->d_scan.as<uint32_t>() + scan_blocks((uint32_t)nb), sizeof(uint32_t),
                              cudaMemcpyDeviceToHost, s);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_cnt.p, 0, sizeof(uint32_t) * nc, s);
-    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_over_head.p, 0, sizeof(uint64_t) * nc, s);
+    if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_buckets.p, 0, sizeof(uint64_t) * nc, s);
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_brick_next.p, 0, 64, s);
     uint32_t total = (uint32_t)nb;  // start[n_cells] = total beads, fixed for the attach
     if (ce == cudaSuccess)
@@ -1530,11 +1531,11 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.cellg = e->d_cellg.as<uint32_t>();
     a.slot_of_id = e->d_slot_of_id.as<uint32_t>();
     a.key = e->d_key.as<uint32_t>();
-    a.bucket = e->d_bucket.as<uint32_t>();
+    a.over_head = e->d_buckets.as<unsigned long long>();
+    a.bucket = (uint32_t *)(e->d_buckets.as<char>() + head_bytes);
+    a.over_node = (uint2 *)(e->d_buckets.as<char>() + head_bytes + bucket_bytes);
     a.bucket_k = bucket_k;
     a.over = (Overflow *)(e->d_brick_next.as<char>() + 32);
-    a.over_head = e->d_over_head.as<unsigned long long>();
-    a.over_node = e->d_over_node.as<uint2>();
     a.bond_row = e->d_bond_row.as<uint32_t>();
     a.bond_terms = e->d_bond_terms.as<BondTerm>();
     a.bond_params = e->d_bond_params.p;
@@ -1564,8 +1565,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         a.list_cap = (uint32_t)room.entries;
         a.pair_cap = (uint32_t)room.pairs;
     }
-    a.block_threads = 128;
-    a.pair_blocks = 32 * e->sm_count;
+    a.pair_blocks = 400 * e->sm_count;  // (many times what can reside: the last turns even out)
     int gb = e->cfg_grid_blocks > 0 ? e->cfg_grid_blocks : 16 * e->sm_count;
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;

@@ -431,6 +431,7 @@ __device__ __forceinline__ void bonds32(const KArgs &a, uint32_t k)
 template <bool ONE_PASS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_cells32(KArgs a, uint32_t nb, int tick)
 {
+    step_kernel_begin();
     if (blockIdx.x < nb) scan_cells<ONE_PASS>(a, tick);
     else bonds32(a, (blockIdx.x - nb) * SCAN_THREADS + threadIdx.x);
 }
@@ -702,6 +703,7 @@ __device__ __forceinline__ void pair_forces32(const KArgs &a, const WorldDev &w,
 template <int FINAL>
 __global__ void __launch_bounds__(TILE_BEADS) k_force32(KArgs a)
 {
+    step_kernel_wait();
     __shared__ float2 s_pair[MAX_PAIR];
     __shared__ uint32_t s_j[LIST_MAX * TILE_BEADS];
     __shared__ uint8_t s_dir[LIST_MAX * TILE_BEADS];
@@ -733,6 +735,7 @@ __global__ void __launch_bounds__(TILE_BEADS) k_force32(KArgs a)
 // First update_pos of a run, from the rest state x(t), v(t), f(t).
 __global__ void __launch_bounds__(TILE_BEADS) k_begin32(KArgs a)
 {
+    step_kernel_begin();
     for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
         const Tile tl = a.tiles[tile];
         const uint32_t s = tl.slot_begin + threadIdx.x;
@@ -804,6 +807,7 @@ __global__ void k_bin32(KArgs a, const uint32_t *__restrict__ hash_in)
 
 __global__ void k_finish32(KArgs a)
 {
+    step_kernel_begin();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < a.n_beads) ((float4 *)a.velA)[s] = ((const float4 *)a.velB)[s];
     if (blockIdx.x == 0)
@@ -824,7 +828,7 @@ int launch_bin32(const KArgs &a, const uint32_t *hash_in, cudaStream_t s)
 
 int launch_begin32(const KArgs &a, cudaStream_t s)
 {
-    k_begin32<<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+    launch_step_kernel(k_begin32, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     return 1;
 }
 
@@ -879,8 +883,8 @@ int launch_cells32(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
     const uint32_t nb = scan_blocks(a.n_cells);
     const uint32_t bb = bonds ? (a.n_bonded + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
-    if (scan_one_pass(a.n_cells)) k_cells32<true><<<nb + bb, SCAN_THREADS, 0, s>>>(a, nb, tick);
-    else k_cells32<false><<<nb + bb, SCAN_THREADS, 0, s>>>(a, nb, tick);
+    if (scan_one_pass(a.n_cells)) launch_step_kernel(k_cells32<true>, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
+    else launch_step_kernel(k_cells32<false>, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
     return 1;
 }
 
@@ -899,13 +903,13 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
             break;
         default: k = final_step ? k_force32_brick<1, BRICK_THREADS> : k_force32_brick<0, BRICK_THREADS>; break;
         }
-        k<<<grid, brick_variant_threads(v), L.bytes, s>>>(a, L);
+        launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), L.bytes, s, a, L);
         return 1;
     }
     if (final_step)
-        k_force32<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+        launch_step_kernel(k_force32<1>, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     else
-        k_force32<0><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+        launch_step_kernel(k_force32<0>, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     return 1;
 }
 
@@ -919,7 +923,7 @@ int launch_pair_log32(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const
 
 int launch_finish32(const KArgs &a, cudaStream_t s)
 {
-    k_finish32<<<(a.n_beads + 255) / 256 + 1, 256, 0, s>>>(a);
+    launch_step_kernel(k_finish32, (a.n_beads + 255) / 256 + 1, 256, 0, s, a);
     return 1;
 }
 

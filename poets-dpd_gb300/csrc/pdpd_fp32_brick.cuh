@@ -373,6 +373,7 @@ __device__ __forceinline__ void brick_fallback_bead(const KArgs &a, const WorldD
 template <int FINAL, int T>
 __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_brick(KArgs a, BrickLayout lay)
 {
+    step_kernel_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BrickHeader &H = *reinterpret_cast<BrickHeader *>(smem_raw);
     float2 *spair = reinterpret_cast<float2 *>(smem_raw + lay.off_pair);
@@ -604,6 +605,7 @@ __device__ __forceinline__ void half_walk(const float4 *__restrict__ spos, const
 template <int FINAL>
 __global__ void __launch_bounds__(HALF_THREADS, 2) k_force32_half(KArgs a, BrickLayout lay)
 {
+    step_kernel_wait();
     constexpr int T = HALF_THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BrickHeader &H = *reinterpret_cast<BrickHeader *>(smem_raw);

@@ -485,16 +485,20 @@ __device__ __forceinline__ void bonds64(const KArgs &a, uint32_t k, bool angle)
 }
 
 // The cells' prefix sum (blocks [0, nb)), the Hookean bonds (the next bb) and the angle bonds (no
-// warp mixes the two).
+// warp mixes the two), 64 to a block: an FP64 instruction holds its pipe for 64 cycles, so the
+// warps should be spread over the SMs.
+constexpr int BOND64_BLOCK = 64;
 template <bool ONE_PASS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_cells64(KArgs a, uint32_t nb, uint32_t bb, int tick)
 {
+    step_kernel_begin();
     if (blockIdx.x < nb) {
         scan_cells<ONE_PASS>(a, tick);
         return;
     }
+    if (threadIdx.x >= BOND64_BLOCK) return;
     const bool angle = blockIdx.x - nb >= bb;
-    bonds64(a, (blockIdx.x - nb - (angle ? bb : 0u)) * SCAN_THREADS + threadIdx.x, angle);
+    bonds64(a, (blockIdx.x - nb - (angle ? bb : 0u)) * BOND64_BLOCK + threadIdx.x, angle);
 }
 
 // Bonds, update_mom and either the final write or the next update_pos with its cell count, for
@@ -559,6 +563,7 @@ __device__ __forceinline__ void integrate64(const KArgs &a, const WorldDev &w, u
 template <int FINAL>
 __global__ void __launch_bounds__(TILE_BEADS) k_force64(KArgs a)
 {
+    step_kernel_wait();
     __shared__ Vec2d s_pair[MAX_PAIR];
     __shared__ uint32_t s_j[LIST_MAX * TILE_BEADS];
     __shared__ uint8_t s_dir[LIST_MAX * TILE_BEADS];
@@ -629,6 +634,7 @@ __global__ void __launch_bounds__(TILE_BEADS) k_force64(KArgs a)
 
 __global__ void __launch_bounds__(TILE_BEADS) k_begin64(KArgs a)
 {
+    step_kernel_begin();
     for (uint32_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
         const Tile tl = a.tiles[tile];
         const uint32_t s = tl.slot_begin + threadIdx.x;
@@ -697,6 +703,7 @@ __global__ void k_bin64(KArgs a, const uint32_t *__restrict__ hash_in)
 
 __global__ void k_finish64(KArgs a)
 {
+    step_kernel_begin();
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < a.n_beads) ((Vec4d *)a.velA)[s] = ((const Vec4d *)a.velB)[s];
     if (blockIdx.x == 0)
@@ -714,7 +721,7 @@ int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s)
 
 int launch_begin64(const KArgs &a, cudaStream_t s)
 {
-    k_begin64<<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+    launch_step_kernel(k_begin64, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     return 1;
 }
 
@@ -729,56 +736,51 @@ int launch_pair_log64(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const
 int launch_cells64(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
     const uint32_t nb = scan_blocks(a.n_cells);
-    const uint32_t bb = bonds ? (a.n_bonds + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
-    const uint32_t ab = bonds ? (a.n_angles + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
-    if (scan_one_pass(a.n_cells)) k_cells64<true><<<nb + bb + ab, SCAN_THREADS, 0, s>>>(a, nb, bb, tick);
-    else k_cells64<false><<<nb + bb + ab, SCAN_THREADS, 0, s>>>(a, nb, bb, tick);
+    const uint32_t bb = bonds ? (a.n_bonds + BOND64_BLOCK - 1) / BOND64_BLOCK : 0u;
+    const uint32_t ab = bonds ? (a.n_angles + BOND64_BLOCK - 1) / BOND64_BLOCK : 0u;
+    if (scan_one_pass(a.n_cells)) launch_step_kernel(k_cells64<true>, nb + bb + ab, SCAN_THREADS, 0, s, a, nb, bb, tick);
+    else launch_step_kernel(k_cells64<false>, nb + bb + ab, SCAN_THREADS, 0, s, a, nb, bb, tick);
     return 1;
 }
 
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
 {
     if (a.list) {  // each pair once
-        const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb, (uint32_t)a.block_threads);
+        const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb);
         const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
-        if (a.block_threads == LIST64_WIDE)
-            k_list64<LIST64_WIDE><<<grid, LIST64_WIDE, L.bytes, s>>>(a, L);
-        else
-            k_list64<LIST64_NARROW><<<grid, LIST64_NARROW, L.bytes, s>>>(a, L);
+        launch_step_kernel(k_list64, (uint32_t)grid, LIST64_THREADS, L.bytes, s, a, L);
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
-        k_pairs64<<<std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s>>>(a);
+        launch_step_kernel(k_pairs64, std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s, a);
         const uint32_t parts = a.n_tiles * (TILE_BEADS / SUM64_BEADS);
         if (a.n_tiles == 0) return 2;
-        if (final_step) k_sum64<1><<<parts, SUM64_THREADS, 0, s>>>(a);
-        else k_sum64<0><<<parts, SUM64_THREADS, 0, s>>>(a);
+        if (final_step) launch_step_kernel(k_sum64<1>, parts, SUM64_THREADS, 0, s, a);
+        else launch_step_kernel(k_sum64<0>, parts, SUM64_THREADS, 0, s, a);
         return 3;
     }
     if (final_step)
-        k_force64<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+        launch_step_kernel(k_force64<1>, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     else
-        k_force64<0><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+        launch_step_kernel(k_force64<0>, (uint32_t)a.grid_blocks, TILE_BEADS, 0, s, a);
     return 1;
 }
 
-// Largest staged-bead capacity of a k_list64 brick with two blocks per SM (large bricks).
-uint32_t list64_maxb_limit(int threads, uint32_t hc_max)
+// Largest staged-bead capacity of a k_list64 brick with two blocks per SM.
+uint32_t list64_maxb_limit(uint32_t hc_max)
 {
     int dev = 0, smem_sm = 0;
-    if (threads != LIST64_WIDE) return 2046u;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
         return 2046u;
-    const int budget = smem_sm / 2 - 1024 - (int)list64_layout(hc_max, 0, (uint32_t)threads).bytes - 128;
+    const int budget = smem_sm / 2 - 1024 - (int)list64_layout(hc_max, 0).bytes - 128;
     return (uint32_t)std::max(64, std::min((int)FULL_MAX_STAGED, budget / (int)LIST64_BEAD_BYTES)) & ~1u;
 }
 
-int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int *grid)
+int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int *grid)
 {
-    const int bytes = (int)list64_layout(hc_max, maxb, (uint32_t)threads).bytes;
-    void (*k)(KArgs, List64Layout) = threads == LIST64_WIDE ? k_list64<LIST64_WIDE> : k_list64<LIST64_NARROW>;
+    const int bytes = (int)list64_layout(hc_max, maxb).bytes;
     int nb = 0;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, bytes);
+    cudaError_t e = cudaFuncSetAttribute(k_list64, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_list64, LIST64_THREADS, bytes);
     if (e != cudaSuccess) return (int)e;
     if (nb < 1) return (int)cudaErrorInvalidConfiguration;
     *grid = nb * sm_count;
@@ -787,7 +789,7 @@ int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int 
 
 int launch_finish64(const KArgs &a, cudaStream_t s)
 {
-    k_finish64<<<(a.n_beads + 255) / 256 + 1, 256, 0, s>>>(a);
+    launch_step_kernel(k_finish64, (a.n_beads + 255) / 256 + 1, 256, 0, s, a);
     return 1;
 }
 

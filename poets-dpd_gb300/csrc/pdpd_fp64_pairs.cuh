@@ -80,9 +80,12 @@ struct List64Layout {
 };
 
 constexpr uint32_t LIST64_BEAD_BYTES = 20;
-constexpr int LIST64_WIDE = 512, LIST64_NARROW = 128;  // threads per block: large and small bricks
+constexpr int LIST64_THREADS = 512;
+// Walk segments per thread: a bead whose segments do not fit takes the slow global walk (at 9, one for
+// each row, 0.1% of the beads of a box of density 3, and 35 of 50 us of the kernel at 27^3)
+constexpr int LIST64_SEGS = 18;
 
-__host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t maxb, uint32_t threads)
+__host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t maxb)
 {
     List64Layout L{};
     L.hc_max = hc_max;
@@ -100,7 +103,7 @@ __host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t 
     L.off_xy = take(8 * maxb);
     L.off_zf = take(4 * maxb);
     L.off_sc = take(8 * maxb);
-    L.off_segs = take(4 * (SEG_MAX + 1) * threads);
+    L.off_segs = take(4 * (LIST64_SEGS + 1) * LIST64_THREADS);
     L.bytes = off;
     return L;
 }
@@ -110,9 +113,10 @@ __host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t 
 // faster: 164 us against 161 for the 64^3 box); where there is none left, its beads are marked
 // (lrec.x) and k_sum64 evaluates all their pairs itself.  The order in which warps take room
 // changes where a list lies, not what is in it.  Bound by instruction issue; no FP64 work.
-template <int T>
-__global__ void __launch_bounds__(T, T == LIST64_WIDE ? 2 : 6) k_list64(KArgs a, List64Layout lay)
+__global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Layout lay)
 {
+    step_kernel_wait();
+    constexpr int T = LIST64_THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     List64Header &H = *reinterpret_cast<List64Header *>(smem_raw);
     uint16_t *hstart = reinterpret_cast<uint16_t *>(smem_raw + lay.off_hstart);
@@ -123,7 +127,7 @@ __global__ void __launch_bounds__(T, T == LIST64_WIDE ? 2 : 6) k_list64(KArgs a,
     uint2 *sc = reinterpret_cast<uint2 *>(smem_raw + lay.off_sc);
     const int tid = threadIdx.x, lane = tid & 31;
     uint32_t *segs = reinterpret_cast<uint32_t *>(smem_raw + lay.off_segs) + tid;
-    const int cap = (a.list_capacity > 0 && a.list_capacity < SEG_MAX) ? max(3, a.list_capacity) : SEG_MAX;
+    const int cap = (a.list_capacity > 0 && a.list_capacity < LIST64_SEGS) ? max(3, a.list_capacity) : LIST64_SEGS;
     uint32_t world = L64_NONE;
     for (uint32_t bi = blockIdx.x; bi < a.n_bricks;) {
         const Brick br = a.bricks[bi];
@@ -285,6 +289,7 @@ __device__ __forceinline__ bool pair_term64(const KArgs &a, const WorldDev &w, u
 constexpr int PAIRS64_THREADS = 64;
 __global__ void __launch_bounds__(PAIRS64_THREADS) k_pairs64(KArgs a)
 {
+    step_kernel_wait();
     const unsigned long long n_all = a.list_cursor[1];
     const uint32_t n = (uint32_t)min(n_all, (unsigned long long)a.pair_cap);
     uint32_t world = L64_NONE, th_lo = 0, th_hi = 0;
@@ -356,8 +361,9 @@ __device__ __noinline__ void single_term64(const KArgs &a, const WorldDev &w, ui
 // integrates.
 constexpr int SUM64_THREADS = 128, SUM64_BEADS = 32, SUM64_ENTRIES = 512;
 template <int FINAL>
-__global__ void __launch_bounds__(SUM64_THREADS, 8) k_sum64(KArgs a)
+__global__ void __launch_bounds__(SUM64_THREADS, 12) k_sum64(KArgs a)
 {
+    step_kernel_wait();
     constexpr int PARTS = TILE_BEADS / SUM64_BEADS;
     __shared__ double s_t[3][SUM64_ENTRIES];
     __shared__ uint32_t s_pre[SUM64_BEADS + 1], s_at[SUM64_BEADS];

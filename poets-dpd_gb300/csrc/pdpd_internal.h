@@ -136,7 +136,6 @@ struct KArgs {
     double *staging;
     uint32_t staging_fields;
     uint32_t staging_n;
-    int block_threads;
     int grid_blocks;     // persistent grid size for the tile kernels
     int list_capacity;   // neighbour-list capacity per bead (0 = the kernel's default)
     int force_kernel;    // FP32: 9 = half-shell brick kernel (Newton's third law inside a
@@ -173,8 +172,8 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish32(const KArgs &a, cudaStream_t s);
 int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
 // FP64 list kernel: staged-bead capacity of a brick, and its persistent grid (0 or a cudaError_t).
-uint32_t list64_maxb_limit(int threads, uint32_t hc_max);
-int list64_setup(int sm_count, int threads, uint32_t hc_max, uint32_t maxb, int *grid);
+uint32_t list64_maxb_limit(uint32_t hc_max);
+int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int *grid);
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);

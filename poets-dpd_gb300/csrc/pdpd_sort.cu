@@ -48,13 +48,14 @@ __device__ __forceinline__ void reduce_chunk(const uint32_t *__restrict__ cnt, u
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_cells_reduce(KArgs a, int tick)
 {
+    step_kernel_begin();
     if (blockIdx.x == 0) rebuild_begin(a, tick);
     reduce_chunk(a.cnt, a.n_cells, a.blocksums);
 }
 
 void launch_cells_reduce(const KArgs &a, int tick, cudaStream_t s)
 {
-    k_cells_reduce<<<scan_blocks(a.n_cells), SCAN_THREADS, 0, s>>>(a, tick);
+    launch_step_kernel(k_cells_reduce, scan_blocks(a.n_cells), SCAN_THREADS, 0, s, a, tick);
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan_reduce(const uint32_t *__restrict__ cnt, uint32_t n,
@@ -109,6 +110,7 @@ __device__ __forceinline__ void put_shadow(const KArgs &a, uint32_t dst, const V
 template <class P>
 __global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
 {
+    step_kernel_begin();
     const uint32_t s = blockIdx.x * 256 + threadIdx.x;
     if (s < a.n_cells) a.cnt[s] = 0u;
     if (s >= a.n_beads) return;
@@ -168,8 +170,8 @@ int launch_sort(const KArgs &a, int fp64, int tick, int with_force, int bonds, c
     n += fp64 ? launch_cells64(a, tick, bonds, s) : launch_cells32(a, tick, bonds, s);
     if (a.n_beads == 0) return n;
     const uint32_t g = (std::max(a.n_beads, a.n_cells) + 255) / 256;
-    if (fp64) k_move<Vec4d><<<g, 256, 0, s>>>(a, with_force);
-    else k_move<float4><<<g, 256, 0, s>>>(a, with_force);
+    if (fp64) launch_step_kernel(k_move<Vec4d>, g, 256, 0, s, a, with_force);
+    else launch_step_kernel(k_move<float4>, g, 256, 0, s, a, with_force);
     return n + 1;
 }
 
