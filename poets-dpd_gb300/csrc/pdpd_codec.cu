@@ -11,9 +11,9 @@
 //   where e is the largest frexp exponent of the non-zero components (e + 1 if a mantissa
 //   rounds to +-256); zero and subnormal components count as zero, e < -14 gives the zero
 //   vector, e > 15 or a non-finite component is an error.
-// Every step is exact in IEEE double (frexp, ldexp, round), so the bytes equal the reference
-// writer's for the same state.  Records start at even offsets (headers are 2 bytes, deltas 4,
-// records 20) and are written as 16-bit words.
+// Every step is exact in IEEE double (frexp, ldexp, round), and for the FP32 engine's state in
+// single precision, so the bytes equal the reference writer's for the same state.  Records start
+// at even offsets (headers are 2 bytes, deltas 4, records 20) and are put together as 16-bit words.
 #include <cfloat>
 
 #include "pdpd_device.cuh"
@@ -22,6 +22,7 @@ namespace pdpd {
 
 namespace {
 
+constexpr int V2_TILE = 512;  // records of a block of the encoder
 constexpr uint32_t V2_ERR_VECTOR = 1u;  // non-finite component or magnitude >= 2^15
 constexpr uint32_t V2_ERR_BOX = 2u;     // a position outside [0, L)
 
@@ -71,13 +72,29 @@ __device__ __forceinline__ void cvec3half_decode(uint32_t w, double out[3])
     }
 }
 
-__device__ __forceinline__ void store_words(uint8_t *dst, const uint32_t w[5])
+// The same for a vector held in single precision: scaling by a power of two and rounding are
+// exact there too (a component that underflows rounds to 0 either way; FP32 subnormals are below
+// 2^-15, where the vector is zero).
+__device__ __forceinline__ bool cvec3half_encode(const float p[3], uint32_t &word)
 {
-    uint16_t *d = reinterpret_cast<uint16_t *>(dst);  // even offset
-    for (int k = 0; k < 5; k++) {
-        d[2 * k] = (uint16_t)(w[k] & 0xFFFFu);
-        d[2 * k + 1] = (uint16_t)(w[k] >> 16);
+    const float m = fmaxf(fmaxf(fabsf(p[0]), fabsf(p[1])), fabsf(p[2]));
+    if (!(isfinite(p[0]) && isfinite(p[1]) && isfinite(p[2]))) return false;
+    word = 0u;
+    if (m < 0x1p-15f) return true;
+    int e = (int)(__float_as_uint(m) >> 23) - 126;  // m = f 2^e, f in [0.5, 1)
+    if (e > 15) return false;
+    float scale = __uint_as_float((uint32_t)(8 - e + 127) << 23);
+    float fr[3];
+    for (int i = 0; i < 3; i++) fr[i] = roundf(p[i] * scale);
+    if (fabsf(fr[0]) == 256.0f || fabsf(fr[1]) == 256.0f || fabsf(fr[2]) == 256.0f) {
+        e += 1;
+        if (e > 15) return false;
+        scale *= 0.5f;
+        for (int i = 0; i < 3; i++) fr[i] = roundf(p[i] * scale);
     }
+    word = ((uint32_t)(e + 15) & 0x1Fu) | (((uint32_t)(int)fr[0] & 0x1FFu) << 5) |
+           (((uint32_t)(int)fr[1] & 0x1FFu) << 14) | (((uint32_t)(int)fr[2] & 0x1FFu) << 23);
+    return true;
 }
 
 __device__ __forceinline__ void load_words(const uint8_t *src, uint32_t w[5])
@@ -86,49 +103,85 @@ __device__ __forceinline__ void load_words(const uint8_t *src, uint32_t w[5])
     for (int k = 0; k < 5; k++) w[k] = (uint32_t)s[2 * k] | ((uint32_t)s[2 * k + 1] << 16);
 }
 
-template <int FP64>
-__global__ void k_v2_encode(KArgs a, uint32_t world, uint32_t n, uint8_t *__restrict__ buf,
-                            const uint32_t *__restrict__ off, uint32_t *err)
+// The five words of slot s's record; the error bits.
+template <int FP64> __device__ __forceinline__ uint32_t encode_record(const KArgs &a, const WorldDev &w, uint32_t s,
+                                                                      uint32_t word[5])
 {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const WorldDev &w = a.worlds[world];
-    const uint32_t s = w.bead_base + k;        // walk the world's slots (coalesced reads)
-    const uint32_t i = a.ids[s] - w.bead_base;  // the bead in slot s: its record
-    double x[3], v[3], f[3];
+    uint32_t bad = 0;
     if (FP64) {
         const Vec4d p = ((const Vec4d *)a.posA)[s], vv = ((const Vec4d *)a.velA)[s],
                     ff = ((const Vec4d *)a.frc)[s];
-        x[0] = p.x; x[1] = p.y; x[2] = p.z;
-        v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
-        f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
+        const double x[3] = {p.x, p.y, p.z}, v[3] = {vv.x, vv.y, vv.z}, f[3] = {ff.x, ff.y, ff.z};
+        for (int d = 0; d < 3; d++) {
+            const double side = (double)w.L[d] * 65536.0;
+            double rr = round(x[d] * 65536.0);
+            if (rr == side) rr = 0.0;
+            if (!(rr >= 0.0 && rr < side)) {
+                bad |= V2_ERR_BOX;
+                rr = 0.0;
+            }
+            word[d] = (uint32_t)rr;
+        }
+        if (!cvec3half_encode(v, word[3])) bad |= V2_ERR_VECTOR;
+        if (!cvec3half_encode(f, word[4])) bad |= V2_ERR_VECTOR;
     } else {
         const float4 p = ((const float4 *)a.posA)[s], vv = ((const float4 *)a.velA)[s],
                      ff = ((const float4 *)a.frc)[s];
         int c[3];
         decode_cell(a.cellg[s] - w.cell_base, w.L, c[0], c[1], c[2]);
-        x[0] = (double)c[0] + (double)p.x;
-        x[1] = (double)c[1] + (double)p.y;
-        x[2] = (double)c[2] + (double)p.z;
-        v[0] = vv.x; v[1] = vv.y; v[2] = vv.z;
-        f[0] = ff.x; f[1] = ff.y; f[2] = ff.z;
-    }
-    uint32_t word[5];
-    uint32_t bad = 0;
-    for (int d = 0; d < 3; d++) {
-        const double side = (double)w.L[d] * 65536.0;
-        double rr = round(x[d] * 65536.0);
-        if (rr == side) rr = 0.0;
-        if (!(rr >= 0.0 && rr < side)) {
-            bad |= V2_ERR_BOX;
-            rr = 0.0;
+        const float o[3] = {p.x, p.y, p.z}, v[3] = {vv.x, vv.y, vv.z}, f[3] = {ff.x, ff.y, ff.z};
+        for (int d = 0; d < 3; d++) {
+            // x = c + o: round(x 65536) = c 65536 + round(o 65536), both products exact
+            uint32_t rr = (uint32_t)c[d] * 65536u;
+            if (o[d] >= 0.0f && o[d] < 1.0f) rr += (uint32_t)roundf(o[d] * 65536.0f);
+            else bad |= V2_ERR_BOX;
+            word[d] = rr == (uint32_t)w.L[d] * 65536u ? 0u : rr;
         }
-        word[d] = (uint32_t)rr;
+        if (!cvec3half_encode(v, word[3])) bad |= V2_ERR_VECTOR;
+        if (!cvec3half_encode(f, word[4])) bad |= V2_ERR_VECTOR;
     }
-    if (!cvec3half_encode(v, word[3])) bad |= V2_ERR_VECTOR;
-    if (!cvec3half_encode(f, word[4])) bad |= V2_ERR_VECTOR;
-    store_words(buf + off[i], word);
-    if (bad) atomicOr(err, bad);
+    return bad;
+}
+
+// The section of V2_TILE records, in record order: each thread gathers its bead (inv: the slot of
+// each global bead id), puts its record and the structure bytes before it together in shared
+// memory, and the block writes the tile's run of bytes back in 16-byte words (the structure bytes
+// unchanged).  One thread per slot, writing its record as ten 16-bit words wherever it lies and
+// encoding FP32 values in FP64, took 194 us for the 64^3 box against 25 us.
+template <int FP64>
+__global__ void __launch_bounds__(V2_TILE) k_v2_encode(KArgs a, uint32_t world, uint32_t n, const uint2 *__restrict__ rec,
+                                                       const uint32_t *__restrict__ inv, uint8_t *buf,
+                                                       uint32_t *err)
+{
+    extern __shared__ __align__(16) uint8_t s_run[];
+    const WorldDev &w = a.worlds[world];
+    const uint32_t r0 = blockIdx.x * V2_TILE, r1 = min(n, r0 + V2_TILE), r = r0 + threadIdx.x;
+    const uint32_t b0 = r0 ? rec[r0 - 1].y + 20u : 0u, b1 = rec[r1 - 1].y + 20u;
+    const uint32_t pad = (uint32_t)((uintptr_t)(buf + b0) & 15u);  // the run's place in its first 16-byte word
+    if (r < r1) {
+        const uint2 me = rec[r];
+        const uint32_t gap = r ? rec[r - 1].y + 20u : 0u;  // the structure bytes [gap, me.y)
+        uint32_t word[5];
+        const uint32_t bad = encode_record<FP64>(a, w, inv[w.bead_base + me.x], word);
+        if (bad) atomicOr(err, bad);
+        uint16_t *out = reinterpret_cast<uint16_t *>(s_run + pad + (gap - b0));
+        for (uint32_t k = gap; k < me.y; k += 2) *out++ = *reinterpret_cast<const uint16_t *>(buf + k);
+        for (int k = 0; k < 5; k++) {
+            *out++ = (uint16_t)(word[k] & 0xFFFFu);
+            *out++ = (uint16_t)(word[k] >> 16);
+        }
+    }
+    __syncthreads();
+    uint8_t *base = buf + b0 - pad;  // 16-byte aligned
+    const uint32_t end = pad + (b1 - b0);
+    for (uint32_t k = 16 * threadIdx.x; k < end; k += 16 * V2_TILE) {
+        if (k >= pad && k + 16 <= end) {
+            *reinterpret_cast<uint4 *>(base + k) = *reinterpret_cast<const uint4 *>(s_run + k);
+        } else {
+            for (uint32_t q = max(k, pad); q < min(k + 16, end); q += 2)
+                *reinterpret_cast<uint16_t *>(base + q) = *reinterpret_cast<const uint16_t *>(s_run + q);
+        }
+    }
 }
 
 // Decode one world's records into the id-ordered staging rows (x, v, f per bead).
@@ -153,15 +206,16 @@ __global__ void k_v2_decode(KArgs a, uint32_t world, uint32_t n, const uint8_t *
 
 }  // namespace
 
-int launch_v2_encode(const KArgs &a, int fp64, uint32_t world, uint32_t n, uint8_t *buf,
-                     const uint32_t *off, uint32_t *err, cudaStream_t s)
+int launch_v2_encode(const KArgs &a, int fp64, uint32_t world, uint32_t n, const uint2 *rec, const uint32_t *inv,
+                     uint8_t *buf, uint32_t *err, cudaStream_t s)
 {
     if (n == 0) return 0;
-    const uint32_t g = (n + 255) / 256;
+    const uint32_t g = (n + V2_TILE - 1) / V2_TILE;
+    const uint32_t smem = V2_TILE * 30 + 32;  // a record, its delta and its polymer's header and delta
     if (fp64)
-        k_v2_encode<1><<<g, 256, 0, s>>>(a, world, n, buf, off, err);
+        k_v2_encode<1><<<g, V2_TILE, smem, s>>>(a, world, n, rec, inv, buf, err);
     else
-        k_v2_encode<0><<<g, 256, 0, s>>>(a, world, n, buf, off, err);
+        k_v2_encode<0><<<g, V2_TILE, smem, s>>>(a, world, n, rec, inv, buf, err);
     return 1;
 }
 

@@ -211,6 +211,7 @@ struct HostPinned {
 // record, and the (offset, length) runs of structure bytes (for checking a stream to decode).
 struct V2Layout {
     DevBuf d_buf, d_off;
+    DevBuf d_rec;  // per record in section order: bead, byte offset
     size_t bytes = 0;
     std::vector<uint8_t> tmpl;
     std::vector<std::pair<uint32_t, uint32_t>> structure;
@@ -218,8 +219,11 @@ struct V2Layout {
     {
         d_buf.release();
         d_off.release();
+        d_rec.release();
     }
 };
+
+constexpr int V2_PIECES = 4;
 
 struct WorldHost {
     WorldDev dev;
@@ -355,6 +359,7 @@ struct pdpd_engine {
     DevBuf d_scan;    // attach: scan block sums, then the number of polymer beads
     cudaEvent_t ev_snap[2] = {nullptr, nullptr};
     cudaEvent_t ev_copied[2] = {nullptr, nullptr};
+    cudaEvent_t ev_piece[V2_PIECES] = {};  // of a v2binary section on its way to the host
 
     // graphs
     cudaGraphExec_t graph = nullptr;
@@ -1022,6 +1027,8 @@ void pdpd_destroy(pdpd_engine *e)
         if (e->ev_snap[i]) cudaEventDestroy(e->ev_snap[i]);
         if (e->ev_copied[i]) cudaEventDestroy(e->ev_copied[i]);
     }
+    for (cudaEvent_t ev : e->ev_piece)
+        if (ev) cudaEventDestroy(ev);
     if (e->stream) cudaStreamDestroy(e->stream);
     if (e->side) cudaStreamDestroy(e->side);
     delete e;
@@ -2295,6 +2302,8 @@ int pdpd_v2binary_prepare(pdpd_engine *e, uint32_t world, uint32_t n_polymers,
     if (n_polymers && polymer_start[0] != 0) return e->fail(PDPD_E_INVALID, "polymer_start[0] must be 0");
     auto L = std::make_shared<V2Layout>();
     std::vector<uint32_t> off(n, 0xFFFFFFFFu);
+    std::vector<std::pair<uint32_t, uint32_t>> rec;  // (bead, offset), as the device's uint2
+    rec.reserve(n);
     std::vector<uint8_t> &t = L->tmpl;
     auto put16 = [&](uint32_t v) {
         t.push_back((uint8_t)(v & 0xFF));
@@ -2329,6 +2338,7 @@ int pdpd_v2binary_prepare(pdpd_engine *e, uint32_t world, uint32_t n_polymers,
             prev_bid = bid;
             mark(begin);
             off[bid] = (uint32_t)t.size();
+            rec.push_back({bid, (uint32_t)t.size()});
             t.resize(t.size() + 20, 0);
             begin = t.size();
         }
@@ -2340,11 +2350,15 @@ int pdpd_v2binary_prepare(pdpd_engine *e, uint32_t world, uint32_t n_polymers,
     cudaSetDevice(e->device);
     if (L->d_buf.alloc(std::max<size_t>(L->bytes, 16)) != cudaSuccess ||
         L->d_off.alloc(sizeof(uint32_t) * std::max<uint32_t>(n, 1)) != cudaSuccess ||
+        L->d_rec.alloc(sizeof(uint2) * std::max<uint32_t>(n, 1)) != cudaSuccess ||
         e->d_v2err.alloc(16) != cudaSuccess)
         return e->fail(PDPD_E_NOMEM, "v2binary layout allocation failed");
     cudaError_t ce = cudaMemcpyAsync(L->d_buf.p, t.data(), L->bytes, cudaMemcpyHostToDevice, e->stream);
     if (ce == cudaSuccess && n)
         ce = cudaMemcpyAsync(L->d_off.p, off.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice, e->stream);
+    static_assert(sizeof(rec[0]) == sizeof(uint2), "record layout");
+    if (ce == cudaSuccess && n)
+        ce = cudaMemcpyAsync(L->d_rec.p, rec.data(), sizeof(uint2) * n, cudaMemcpyHostToDevice, e->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) return e->cuda_fail(ce, "v2binary layout upload");
     e->worlds[world].v2 = L;
@@ -2365,21 +2379,40 @@ int pdpd_v2binary_encode(pdpd_engine *e, uint32_t world, uint8_t *out, size_t ca
     if (capacity < L->bytes) return e->fail(PDPD_E_INVALID, "output buffer too small (%zu < %zu bytes)", capacity, L->bytes);
     cudaSetDevice(e->device);
     const WorldDev &wd = e->worlds[world].dev;
-    uint32_t herr = 0;
+    if (e->d_inv.alloc(sizeof(uint32_t) * std::max<uint32_t>(1, e->n_beads)) != cudaSuccess)
+        return e->fail(PDPD_E_NOMEM, "device allocation failed");
     cudaError_t ce = cudaMemsetAsync(e->d_v2err.p, 0, sizeof(uint32_t), e->stream);
-    e->launches += launch_v2_encode(e->args, e->fp64(), world, wd.n_beads, L->d_buf.as<uint8_t>(),
-                                    L->d_off.as<uint32_t>(), e->d_v2err.as<uint32_t>(), e->stream);
+    e->launches += launch_slot_of_id(e->args, wd.bead_base, wd.n_beads, e->d_inv.as<uint32_t>(), e->stream);
+    e->launches += launch_v2_encode(e->args, e->fp64(), world, wd.n_beads, (const uint2 *)L->d_rec.p,
+                                    e->d_inv.as<uint32_t>(), L->d_buf.as<uint8_t>(), e->d_v2err.as<uint32_t>(),
+                                    e->stream);
     if (ce == cudaSuccess) ce = cudaGetLastError();
-    // through pinned staging (a copy to pageable memory would be staged by the driver)
+    // Through pinned staging in pieces, each copied on by the host while the next crosses the link.
+    // (Written by the kernel straight into the caller's array, the 64^3 box takes 170 us where its
+    // pages are known to the GPU, against 330 us so, but 4 ms in a new array.)
     if (e->h_staging[1].alloc(L->bytes + 16) != cudaSuccess) return e->fail(PDPD_E_NOMEM, "pinned allocation failed");
-    uint32_t *herr_p = (uint32_t *)((uint8_t *)e->h_staging[1].p + ((L->bytes + 3) & ~size_t(3)));
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(e->h_staging[1].p, L->d_buf.p, L->bytes, cudaMemcpyDeviceToHost, e->stream);
+    uint8_t *src = (uint8_t *)e->h_staging[1].p;
+    uint32_t *herr_p = (uint32_t *)(src + ((L->bytes + 3) & ~size_t(3)));
+    const size_t pieces = std::min<size_t>(V2_PIECES, L->bytes / (1 << 20) + 1), per = (L->bytes + pieces - 1) / pieces;
+    for (cudaEvent_t &ev : e->ev_piece)
+        if (ce == cudaSuccess && !ev) ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(herr_p, e->d_v2err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream);
-    if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
-    if (ce != cudaSuccess) return e->cuda_fail(ce, "v2binary encode");
-    herr = *herr_p;
-    const uint8_t *src = (const uint8_t *)e->h_staging[1].p;
-    parallel_for(L->bytes, 1 << 22, [&](size_t b, size_t en) { memcpy(out + b, src + b, en - b); });
+    for (size_t k = 0; k < pieces && ce == cudaSuccess; k++) {
+        const size_t b = std::min(L->bytes, k * per), en = std::min(L->bytes, b + per);
+        if (en > b) ce = cudaMemcpyAsync(src + b, L->d_buf.as<uint8_t>() + b, en - b, cudaMemcpyDeviceToHost, e->stream);
+        if (ce == cudaSuccess) ce = cudaEventRecord(e->ev_piece[k], e->stream);
+    }
+    for (size_t k = 0; k < pieces && ce == cudaSuccess; k++) {
+        const size_t b = std::min(L->bytes, k * per), en = std::min(L->bytes, b + per);
+        ce = cudaEventSynchronize(e->ev_piece[k]);
+        if (ce == cudaSuccess)
+            parallel_for(en - b, 1 << 17, [&](size_t p, size_t q) { memcpy(out + b + p, src + b + p, q - p); });
+    }
+    if (ce != cudaSuccess) {
+        cudaStreamSynchronize(e->stream);
+        return e->cuda_fail(ce, "v2binary encode");
+    }
+    const uint32_t herr = *herr_p;
     if (herr & 2u) return e->fail(PDPD_E_INVALID, "Bead is out of bounds.");
     if (herr & 1u)
         return e->fail(PDPD_E_INVALID, "A velocity or force is not finite or has magnitude 65536 or more "

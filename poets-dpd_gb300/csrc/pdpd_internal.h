@@ -273,11 +273,13 @@ int launch_observe(const KArgs &a, int fp64, uint32_t world, uint32_t n_beads, u
                    unsigned long long *rdf, uint32_t n_bond_bins, unsigned long long *bond_hist,
                    ObsPartial *part, cudaStream_t s);
 
-// v2binary codec (pdpd_codec.cu): encode one world's bead records into a prepared section
-// buffer at the given per-bead byte offsets, or decode them into the id-ordered staging rows.
+// v2binary codec (pdpd_codec.cu): encode one world's section from its records in section order
+// (bead, byte offset) and the slot of each bead (inv, launch_slot_of_id) into a buffer that holds
+// its structure bytes, or decode bead records at per-bead byte offsets into the id-ordered
+// staging rows.
 // err (device) collects 1 = unrepresentable vector, 2 = position outside the box.
-int launch_v2_encode(const KArgs &a, int fp64, uint32_t world, uint32_t n, uint8_t *buf,
-                     const uint32_t *off, uint32_t *err, cudaStream_t s);
+int launch_v2_encode(const KArgs &a, int fp64, uint32_t world, uint32_t n, const uint2 *rec, const uint32_t *inv,
+                     uint8_t *buf, uint32_t *err, cudaStream_t s);
 int launch_v2_decode(const KArgs &a, uint32_t world, uint32_t n, const uint8_t *buf,
                      const uint32_t *off, double *staging, uint32_t *err, cudaStream_t s);
 

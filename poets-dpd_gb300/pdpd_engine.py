@@ -596,12 +596,14 @@ class GB300DPDEngine:
 
 
 def _rows(ptr, n, stride_bytes):
-    """Copy n vectors of 3 doubles, stride_bytes apart, out of a callback's pointer."""
+    """Copy n vectors of 3 doubles, stride_bytes apart, out of a callback's pointer (as items of
+    24 bytes: a copy of (n, 3) doubles would loop over each row's three)."""
     if n == 0:
         return np.empty((0, 3))
     step = stride_bytes // 8
     flat = np.ctypeslib.as_array(ptr, shape=((n - 1) * step + 3,))
-    return np.lib.stride_tricks.as_strided(flat, shape=(n, 3), strides=(stride_bytes, 8)).copy()
+    items = np.lib.stride_tricks.as_strided(flat[:3].view("V24"), shape=(n,), strides=(stride_bytes,))
+    return items.copy().view(np.float64).reshape(n, 3)
 
 
 class GB300DPDServer:
@@ -613,8 +615,8 @@ class GB300DPDServer:
     thread after every ``interval_steps`` steps of the job; returning ``False`` ends the job at
     that snapshot.  ``drain()`` waits for every queued job and raises the first error.  The
     final state of job ``i`` is ``results[i] = (x, v, f, t)``; failed jobs are in ``failed``.
-    With ``keep_results=False`` the final states are not copied (``results[i] = t`` only) and
-    snapshots are copied only for jobs with an ``on_interval`` handler.
+    Snapshots are copied only for jobs with an ``on_interval`` handler; with
+    ``keep_results=False`` the final states are not copied either (``results[i] = t`` only).
     """
 
     def __init__(self, precision="fp32", device=-1, memory_budget_bytes=40 << 30,
@@ -644,11 +646,11 @@ class GB300DPDServer:
                 self._handlers.pop(job, None)
                 return 0
             h = self._handlers.get(job)
+            if h is None and status != 1:  # a snapshot nobody looks at: counted, not copied
+                self.snapshots[job] = self.snapshots.get(job, 0) + 1
+                return 1
             if not self.keep_results and h is None:
-                if status == 1:
-                    self.results[job] = int(t)
-                else:
-                    self.snapshots[job] = self.snapshots.get(job, 0) + 1
+                self.results[job] = int(t)
                 return 1
             xs, vs, fs = _rows(x, n, stride), _rows(v, n, stride), _rows(f, n, stride)
             if status == 1:
