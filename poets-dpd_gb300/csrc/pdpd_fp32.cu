@@ -110,79 +110,77 @@ __device__ __forceinline__ void min_image(const WorldDev &w, float d[3])
     }
 }
 
-// Bond forces on one bead from its CSR row (update_hookean_bond / update_angle_bond,
+// One bond term on a bead from row r of its CSR (update_hookean_bond / update_angle_bond,
 // naive_dpd_engine_half_step.hpp:426-483; calc_angle_force dpd_maths_core_half_step.hpp:177-229).
-__device__ __noinline__ void bond_forces32(const KArgs &a, const WorldDev &w, uint32_t id, const int c[3],
-                              const float o[3], float F[3], uint32_t &err)
+__device__ __forceinline__ void bond_term32(const KArgs &a, const WorldDev &w, uint32_t r, const int c[3],
+                                            const float o[3], float t[3], uint32_t &err)
 {
     const float4 *pos = (const float4 *)a.posB;
     const float4 *prm_tab = (const float4 *)a.bond_params;
-    const uint32_t r0 = a.bond_row[id], r1 = a.bond_row[id + 1];
-    for (uint32_t r = r0; r < r1; r++) {
-        const BondTerm bt = a.bond_terms[r];
-        const float4 prm = prm_tab[bt.param];
-        const uint32_t kind = bt.meta & 0xffu, role = bt.meta >> 8;
-        float ra[3], rb[3] = {0.f, 0.f, 0.f};
-        rel_pos(w, pos, a.key, a.slot_of_id[bt.a], c, o, ra);
-        if (kind == 0) {
-            // Hookean: dx = tail - head; head gets -f, tail +f, f = dx * kappa (r0 - r) / r.
-            float dx[3];
+    t[0] = t[1] = t[2] = 0.0f;
+    const BondTerm bt = a.bond_terms[r];
+    const float4 prm = prm_tab[bt.param];
+    const uint32_t kind = bt.meta & 0xffu, role = bt.meta >> 8;
+    float ra[3], rb[3] = {0.f, 0.f, 0.f};
+    rel_pos(w, pos, a.key, a.slot_of_id[bt.a], c, o, ra);
+    if (kind == 0) {
+        // Hookean: dx = tail - head; head gets -f, tail +f, f = dx * kappa (r0 - r) / r.
+        float dx[3];
 #pragma unroll
-            for (int d = 0; d < 3; d++) dx[d] = role == 0 ? ra[d] : -ra[d];
-            min_image(w, dx);
-            float dr = sqrtf(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
-            if (dr > 2.0f) err |= ERR_BOND_SNAPPED;
-            float s = (prm.x * (prm.y - dr)) / dr;
-            float sign = role == 0 ? -1.0f : 1.0f;
+        for (int d = 0; d < 3; d++) dx[d] = role == 0 ? ra[d] : -ra[d];
+        min_image(w, dx);
+        float dr = sqrtf(dx[0] * dx[0] + dx[1] * dx[1] + dx[2] * dx[2]);
+        if (dr > 2.0f) err |= ERR_BOND_SNAPPED;
+        float s = (prm.x * (prm.y - dr)) / dr;
+        float sign = role == 0 ? -1.0f : 1.0f;
 #pragma unroll
-            for (int d = 0; d < 3; d++) F[d] += sign * (dx[d] * s);
-        } else {
-            rel_pos(w, pos, a.key, a.slot_of_id[bt.b], c, o, rb);
-            float xh[3], xm[3], xt[3];
+        for (int d = 0; d < 3; d++) t[d] = sign * (dx[d] * s);
+    } else {
+        rel_pos(w, pos, a.key, a.slot_of_id[bt.b], c, o, rb);
+        float xh[3], xm[3], xt[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            xh[d] = role == 0 ? 0.f : ra[d];
+            xm[d] = role == 0 ? ra[d] : (role == 1 ? 0.f : rb[d]);
+            xt[d] = role == 2 ? 0.f : rb[d];
+        }
+        float b1[3], b2[3];
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            b1[d] = xm[d] - xh[d];
+            b2[d] = xt[d] - xm[d];
+        }
+        min_image(w, b1);
+        min_image(w, b2);
+        float r01 = sqrtf(b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2]);
+        float r12 = sqrtf(b2[0] * b2[0] + b2[1] * b2[1] + b2[2] * b2[2]);
+        float mag = r01 * r12;
+        if (mag > 0.0001f) {
+            float dot = b1[0] * b2[0] + b1[1] * b2[1] + b1[2] * b2[2];
+            float p1 = dot / (r01 * r01);
+            float p2 = dot / (r12 * r12);
+            float fm = prm.x / mag;
+            if (fabsf(dot) > 0.000001f && prm.z > 0.0f) {
+                // 1/sqrt(1/cos^2 phi - 1) loses all precision in FP32 as the bonds turn
+                // collinear: evaluate the normalisation in FP64.
+                double b1d[3] = {b1[0], b1[1], b1[2]}, b2d[3] = {b2[0], b2[1], b2[2]};
+                double dd = b1d[0] * b2d[0] + b1d[1] * b2d[1] + b1d[2] * b2d[2];
+                double n1 = b1d[0] * b1d[0] + b1d[1] * b1d[1] + b1d[2] * b1d[2];
+                double n2 = b2d[0] * b2d[0] + b2d[1] * b2d[1] + b2d[2] * b2d[2];
+                double cos_phi_sq = (dd * dd) / (n1 * n2);
+                double ip = 1.0 / sqrt(1.0 / cos_phi_sq - 1.0);
+                fm = (float)((double)fm * ((double)prm.y - (double)prm.z * ip));
+            }
+            float hf[3], tf[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                xh[d] = role == 0 ? 0.f : ra[d];
-                xm[d] = role == 0 ? ra[d] : (role == 1 ? 0.f : rb[d]);
-                xt[d] = role == 2 ? 0.f : rb[d];
+                hf[d] = (b1[d] * p1 - b2[d]) * fm;
+                tf[d] = (b1[d] - b2[d] * p2) * fm;
             }
-            float b1[3], b2[3];
 #pragma unroll
             for (int d = 0; d < 3; d++) {
-                b1[d] = xm[d] - xh[d];
-                b2[d] = xt[d] - xm[d];
-            }
-            min_image(w, b1);
-            min_image(w, b2);
-            float r01 = sqrtf(b1[0] * b1[0] + b1[1] * b1[1] + b1[2] * b1[2]);
-            float r12 = sqrtf(b2[0] * b2[0] + b2[1] * b2[1] + b2[2] * b2[2]);
-            float mag = r01 * r12;
-            if (mag > 0.0001f) {
-                float dot = b1[0] * b2[0] + b1[1] * b2[1] + b1[2] * b2[2];
-                float p1 = dot / (r01 * r01);
-                float p2 = dot / (r12 * r12);
-                float fm = prm.x / mag;
-                if (fabsf(dot) > 0.000001f && prm.z > 0.0f) {
-                    // 1/sqrt(1/cos^2 phi - 1) loses all precision in FP32 as the bonds turn
-                    // collinear: evaluate the normalisation in FP64.
-                    double b1d[3] = {b1[0], b1[1], b1[2]}, b2d[3] = {b2[0], b2[1], b2[2]};
-                    double dd = b1d[0] * b2d[0] + b1d[1] * b2d[1] + b1d[2] * b2d[2];
-                    double n1 = b1d[0] * b1d[0] + b1d[1] * b1d[1] + b1d[2] * b1d[2];
-                    double n2 = b2d[0] * b2d[0] + b2d[1] * b2d[1] + b2d[2] * b2d[2];
-                    double cos_phi_sq = (dd * dd) / (n1 * n2);
-                    double ip = 1.0 / sqrt(1.0 / cos_phi_sq - 1.0);
-                    fm = (float)((double)fm * ((double)prm.y - (double)prm.z * ip));
-                }
-                float hf[3], tf[3];
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    hf[d] = (b1[d] * p1 - b2[d]) * fm;
-                    tf[d] = (b1[d] - b2[d] * p2) * fm;
-                }
-#pragma unroll
-                for (int d = 0; d < 3; d++) {
-                    float add = role == 0 ? hf[d] : (role == 2 ? tf[d] : -(hf[d] + tf[d]));
-                    F[d] += add;
-                }
+                float add = role == 0 ? hf[d] : (role == 2 ? tf[d] : -(hf[d] + tf[d]));
+                t[d] = add;
             }
         }
     }
@@ -400,40 +398,68 @@ __device__ __forceinline__ void integrate32(const KArgs &a, const WorldDev &w, u
     }
 }
 
-// Bond forces of every polymer bead (monomer bit of the hash clear), one thread per bead, by id
-// for the force kernel to add: on a compact list of the few bonded beads, so that their
-// dependent partner lookups stay out of the pair kernel's warps, and from the advanced, not yet
-// re-sorted state (slot_of_id is that of the sorted state it came from), so that it runs in the
-// launch of the cells' prefix sum.
-__device__ __forceinline__ void bonds32(const KArgs &a, uint32_t k)
+// Bond forces of every polymer bead (monomer bit of the hash clear), by id for the force kernel to
+// add: on a compact list of the few bonded beads, so that their dependent partner lookups stay
+// out of the pair kernel's warps, and from the advanced, not yet re-sorted state (slot_of_id is
+// that of the sorted state it came from), so that it runs in the launch of the cells' prefix
+// sum.  BOND_LANES lanes per bead, a term each, added in row order.  Few beads leave the launch
+// bound by the latency of the lookups, which one lane goes through once per term: eight lanes
+// take the launch of the 32^3 polymer box (9,828 polymer beads) from 12.3 to 9.7 us; many fill
+// the GPU with one lane each, and eight take that of the 128^3 box (314,568) from 43 to 87 us.
+// The line lies where eight lanes per bead fill half the SMs' threads.
+constexpr uint32_t BOND_LANES_FEW = 8, BOND_BEADS_FEW = 20000;
+template <uint32_t BOND_LANES>
+__device__ __forceinline__ void bonds32(const KArgs &a, uint32_t thread)
 {
-    if (k >= a.n_bonded) return;
-    const uint32_t id = a.bonded_ids[k];
-    uint32_t lo = 0, hi = a.n_worlds;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) / 2;
-        if (a.worlds[mid].bead_base <= id) lo = mid; else hi = mid;
+    const uint32_t k = thread / BOND_LANES, lane = thread % BOND_LANES;
+    const bool act = k < a.n_bonded;
+    uint32_t id = 0, r0 = 0, r1 = 0, lo = 0, err = 0;
+    int c[3] = {0, 0, 0};
+    float o[3] = {0.f, 0.f, 0.f}, F[3] = {0.f, 0.f, 0.f};
+    if (act) {
+        id = a.bonded_ids[k];
+        r0 = a.bond_row[id];
+        r1 = a.bond_row[id + 1];
+        uint32_t hi = a.n_worlds;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) / 2;
+            if (a.worlds[mid].bead_base <= id) lo = mid; else hi = mid;
+        }
     }
     const WorldDev &w = a.worlds[lo];
-    const uint32_t s = a.slot_of_id[id];
-    const float4 p = ((const float4 *)a.posB)[s];
-    int c[3];
-    decode_cell(a.key[s] - w.cell_base, w.L, c[0], c[1], c[2]);
-    const float o[3] = {p.x, p.y, p.z};
-    float F[3] = {0.f, 0.f, 0.f};
-    uint32_t err = 0;
-    bond_forces32(a, w, id, c, o, F, err);
-    a.fbond[id] = make_float4(F[0], F[1], F[2], 0.f);
+    if (act) {
+        const uint32_t s = a.slot_of_id[id];
+        const float4 p = ((const float4 *)a.posB)[s];
+        decode_cell(a.key[s] - w.cell_base, w.L, c[0], c[1], c[2]);
+        o[0] = p.x;
+        o[1] = p.y;
+        o[2] = p.z;
+    }
+    for (uint32_t r = r0; __any_sync(0xffffffffu, r < r1); r += BOND_LANES) {
+        float t[3] = {0.f, 0.f, 0.f};
+        if (r + lane < r1) bond_term32(a, w, r + lane, c, o, t, err);
+#pragma unroll
+        for (uint32_t q = 0; q < BOND_LANES; q++) {
+            const float x = __shfl_sync(0xffffffffu, t[0], q, BOND_LANES), y = __shfl_sync(0xffffffffu, t[1], q, BOND_LANES),
+                        z = __shfl_sync(0xffffffffu, t[2], q, BOND_LANES);
+            if (r + q < r1) {
+                F[0] = __fadd_rn(F[0], x);
+                F[1] = __fadd_rn(F[1], y);
+                F[2] = __fadd_rn(F[2], z);
+            }
+        }
+    }
+    if (act && lane == 0) a.fbond[id] = make_float4(F[0], F[1], F[2], 0.f);
     if (err) atomicOr(&a.worlds[lo].err, err);
 }
 
 // The cells' prefix sum (blocks [0, nb)) and the bond forces.
-template <bool ONE_PASS>
+template <bool ONE_PASS, uint32_t BOND_LANES>
 __global__ void __launch_bounds__(SCAN_THREADS) k_cells32(KArgs a, uint32_t nb, int tick)
 {
     step_kernel_begin();
     if (blockIdx.x < nb) scan_cells<ONE_PASS>(a, tick);
-    else bonds32(a, (blockIdx.x - nb) * SCAN_THREADS + threadIdx.x);
+    else bonds32<BOND_LANES>(a, (blockIdx.x - nb) * SCAN_THREADS + threadIdx.x);
 }
 
 // Thread-per-bead pair forces straight from global memory, summed one pair at a time in the
@@ -882,9 +908,12 @@ int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint3
 int launch_cells32(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
     const uint32_t nb = scan_blocks(a.n_cells);
-    const uint32_t bb = bonds ? (a.n_bonded + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
-    if (scan_one_pass(a.n_cells)) launch_step_kernel(k_cells32<true>, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
-    else launch_step_kernel(k_cells32<false>, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
+    const bool few = a.n_bonded <= BOND_BEADS_FEW;
+    const uint32_t bb = bonds ? (a.n_bonded * (few ? BOND_LANES_FEW : 1u) + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    void (*k)(KArgs, uint32_t, int);
+    if (scan_one_pass(a.n_cells)) k = few ? k_cells32<true, BOND_LANES_FEW> : k_cells32<true, 1>;
+    else k = few ? k_cells32<false, BOND_LANES_FEW> : k_cells32<false, 1>;
+    launch_step_kernel(k, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
     return 1;
 }
 

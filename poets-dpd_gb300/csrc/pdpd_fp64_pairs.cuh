@@ -71,6 +71,7 @@ struct List64Header {
     WorldDev w;
     uint32_t home_rows[65];
     uint32_t total, next;
+    uint16_t halo_row[64];
 };
 
 // Shared memory of k_list64: header, hstart, hslot, row bases, then per staged bead offsets
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
         const WorldDev &w = H.w;
         const int HY = br.by + 2, HZ = br.bz + 2;
         uint32_t total = 0, n_home = 0;
-        brick_stage_rows<T>(a, w, br, a.posf, H.home_rows, &H.total, hstart, hslot, rowbase, xy, zf, lay.maxb, total,
+        brick_stage_rows<T>(a, w, br, a.posf, H.home_rows, H.halo_row, &H.total, hstart, hslot, rowbase, xy, zf, lay.maxb, total,
                             n_home, [&](uint32_t j, uint32_t slot, const float4 &, uint32_t code) {
                                 sc[j] = make_uint2(slot, code);
                             });
@@ -153,8 +154,7 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
             bool dense = !staged;
             int c[3] = {0, 0, 0};
             if (act) {
-                const int lx = r / br.by, ly = r - lx * br.by;
-                const int row = (lx + 1) * HY + (ly + 1);
+                const int row = H.halo_row[r];
                 const uint32_t k = t - H.home_rows[r];
                 s = hslot[row * HZ + 1] + k;
                 if (staged) {

@@ -187,7 +187,8 @@ template <int T> struct SegReader {
 // filler far away pads an odd row), so a pair of staged beads never spans two rows:
 //   hstart[row * (HZ + 1) + z] = first staged index of halo cell (row, z), the last entry the
 //   row's end; hslot[row * HZ + z] = the cell's first slot in the sorted state;
-//   home_rows[r] = first home index of home row r; total = staged beads with the fillers.
+//   home_rows[r] = first home index of home row r, halo_row[r] its halo row; total = staged beads
+//   with the fillers.
 // If the halo fits (total <= maxb) the beads are staged; else hstart holds nothing of use.  Halo
 // coordinates lie in [-1, L] (bricks are cut at the box faces), so each wraps with one
 // conditional add or subtract.
@@ -198,7 +199,7 @@ template <int T> struct SegReader {
 template <int T, class Put>
 __device__ __forceinline__ void brick_stage_rows(const KArgs &a, const WorldDev &w, const Brick &br,
                                                  const float4 *__restrict__ pos, uint32_t *home_rows,
-                                                 uint32_t *staged_total, uint16_t *hstart, uint32_t *hslot,
+                                                 uint16_t *halo_row, uint32_t *staged_total, uint16_t *hstart, uint32_t *hslot,
                                                  uint32_t *rowbase, float *xy, float *zf, uint32_t maxb,
                                                  uint32_t &total, uint32_t &n_home, Put put)
 {
@@ -251,8 +252,11 @@ __device__ __forceinline__ void brick_stage_rows(const KArgs &a, const WorldDev 
                 if (zz == HZ - 1) rowbase[row] = inc;
             }
             if (z0 == 0) first_home = __shfl_sync(0xffffffffu, inc, HZ > 32 ? 0 : sub * HZ);
-            if (on && zz == br.bz && hx >= 1 && hx <= br.bx && hy >= 1 && hy <= br.by)
-                home_rows[(hx - 1) * br.by + (hy - 1)] = inc - first_home;
+            if (on && zz == br.bz && hx >= 1 && hx <= br.bx && hy >= 1 && hy <= br.by) {
+                const int r = (hx - 1) * br.by + (hy - 1);
+                home_rows[r] = inc - first_home;
+                halo_row[r] = (uint16_t)row;
+            }
             carry = HZ > 32 ? __shfl_sync(0xffffffffu, inc, 31) : 0u;
         }
     }
