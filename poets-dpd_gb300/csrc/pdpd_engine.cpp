@@ -499,29 +499,81 @@ struct pdpd_engine {
         return PDPD_OK;
     }
 
-    // Brick shape for the 512-thread kernels (FP32 variant 8, the FP64 list kernel) by the batch's
+    // Estimated time of a pass of the 512-thread brick kernels over the batch cut into bricks of
+    // this shape, us: a brick costs 1.8, 6.0 per turn of the block over its home beads (512 of
+    // them) and 0.024 per home bead; two blocks per SM take bricks in turn, nearly in step (0.9 of
+    // the way to whole rounds), and a block alone on its SM takes 0.66 of that.  Fitted to FP32
+    // force passes of 24 water boxes of sides 10 to 96 in 13 shapes each (5.7% rms).
+    double shape_cost(const int shape[3]) const
+    {
+        double total = 0, most = 0, n = 0;
+        for (const WorldHost &wh : worlds) {
+            const int32_t *L = wh.dev.L;
+            const double rho = (double)wh.dev.n_beads / std::max(1.0, (double)L[0] * L[1] * L[2]);
+            int k[3], lo[3], more[3];  // bricks per axis, their smaller extent, how many are one longer
+            for (int d = 0; d < 3; d++) {
+                k[d] = (L[d] + shape[d] - 1) / shape[d];
+                lo[d] = L[d] / k[d];
+                more[d] = L[d] - lo[d] * k[d];
+            }
+            for (int q = 0; q < 8; q++) {
+                double count = 1, cells = 1;
+                for (int d = 0; d < 3; d++) {
+                    const bool longer = q >> d & 1;
+                    count *= longer ? more[d] : k[d] - more[d];
+                    cells *= lo[d] + (longer ? 1 : 0);
+                }
+                if (count == 0) continue;
+                const double beads = rho * cells;
+                double turns = 1;  // expected: Poisson home beads
+                for (int t = 1; t <= 4; t++) turns += 0.5 * std::erfc((512.0 * t - beads) / std::sqrt(2 * beads + 1e-9));
+                const double c = 1.8 + 0.024 * beads + 6.0 * turns;
+                total += count * c;
+                most = std::max(most, c);
+                n += count;
+            }
+        }
+        const double rounds = n / (2.0 * std::max(1, sm_count));
+        if (rounds <= 0.5) return 10 + 0.66 * most;
+        if (rounds <= 1) return 10 + most;
+        return 10 + total / n * (0.9 * std::ceil(rounds) + 0.1 * rounds);
+    }
+
+    // Brick shape for the 512-thread kernels (FP32 variant 8, the FP64 list kernel).  By the batch's
     // cells per SM: the largest bricks stage the fewest halo beads per home bead, but the
     // persistent blocks (two per SM) want several bricks each, and a small batch has too few.
     // Whole FP32 steps of polymer boxes, us (sides 20, 32, 40, 52, 64, 80; cells per SM 53, 216,
     // 421, 925, 1725, 3368): 5x8x8 36.4, 41.0, 60.4, 93.5, 160.2, 279; 4x5x8 (480 home beads, one
     // turn of the block) 27.9, 37.5, 53.5, 91.5, 154.2, 281; 4x4x8 26.9, 35.1, 56.5, 98.7, 158.3,
     // 298; 4x4x6 26.0, 41.3, 59.4, 106, 182, 345; 2x4x4 25.5, 58.1, 94.8, 183, 336, 665 (sides 9
-    // and 16: 2x4x4 23.2 and 24.1, 4x4x6 23.7 and 26.0).  Smaller bricks where the halo of the
-    // batch's densest world would not fit the staging capacity 5 Poisson deviations above its
-    // mean.
+    // and 16: 2x4x4 23.2 and 24.1, 4x4x6 23.7 and 26.0).  In between, how the bricks of a box
+    // divide into rounds of the blocks matters more (36^3: 4x4x8 44.7, 4x6x8 37.6; 39^3: 4x5x8
+    // 49.5, 5x6x8 40.5): another shape is taken where shape_cost puts it 6% below.  Smaller bricks
+    // where the halo of the batch's densest world would not fit the staging capacity 5 Poisson
+    // deviations above its mean.
     template <class Limit> void wide_shape(int shape[3], Limit limit) const
     {
         static const int table[][3] = {{5, 8, 8}, {4, 5, 8}, {4, 4, 8}, {4, 4, 6}, {2, 4, 4}, {2, 2, 4}, {1, 2, 2}};
+        static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
+                                       {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
         static const uint64_t from[] = {2500, 350, 110, 40, 0, 0, 0};  // cells per SM
+        auto fits = [&](const int c[3]) {
+            const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
+            const double mean = max_density * hc;
+            return mean + 5.0 * std::sqrt(mean) <= (double)limit(hc);
+        };
         const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
         int k = 0;
         while (per_sm < from[k]) k++;
-        for (; k < 6; k++) {
-            const uint32_t hc = (uint32_t)(table[k][0] + 2) * (table[k][1] + 2) * (table[k][2] + 2);
-            const double mean = max_density * hc;
-            if (mean + 5.0 * std::sqrt(mean) <= (double)limit(hc)) break;
-        }
-        for (int d = 0; d < 3; d++) shape[d] = table[k][d];
+        while (k < 6 && !fits(table[k])) k++;
+        const int *best = table[k];
+        double cost = 0.94 * shape_cost(best);
+        for (const auto &c : other)
+            if (k < 5 && fits(c) && shape_cost(c) < cost) {
+                best = c;
+                cost = shape_cost(c);
+            }
+        for (int d = 0; d < 3; d++) shape[d] = best[d];
     }
 
     // Default kernel variant and brick shape for the attached batch, where the config does not
