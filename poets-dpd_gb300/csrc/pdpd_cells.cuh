@@ -120,7 +120,7 @@ template <bool ONE_PASS> __device__ __forceinline__ void scan_cells(const KArgs 
         if (blockIdx.x == 0) rebuild_begin(a, tick);
         const uint4 *c = (const uint4 *)a.cnt;
         const uint32_t before = blockIdx.x * (SCAN_CHUNK / 4);
-#pragma unroll 4
+#pragma unroll 8
         for (uint32_t k = threadIdx.x; k < before; k += SCAN_THREADS) {
             const uint4 v = c[k];
             off += v.x + v.y + v.z + v.w;

@@ -376,7 +376,6 @@ __device__ __forceinline__ void brick_fallback_bead(const KArgs &a, const WorldD
 template <int FINAL, int T>
 __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_brick(KArgs a, BrickLayout lay)
 {
-    step_kernel_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BrickHeader &H = *reinterpret_cast<BrickHeader *>(smem_raw);
     float2 *spair = reinterpret_cast<float2 *>(smem_raw + lay.off_pair);
@@ -396,15 +395,24 @@ __global__ void __launch_bounds__(T, T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_
     // Bricks come from the shared counter, the next one fetched while this one is computed (128^3
     // box, 20 steps with the read-back: 22.4 -> 21.8 ms: two of a brick's dependent trips to memory
     // are off its path).
+    // The first brick and its world's tables, which no step changes, are read before the wait for
+    // the kernel in front; the world's time after it.
     uint32_t bi = blockIdx.x;
     if (tid == 0 && bi < a.n_bricks) H.ahead = a.bricks[bi];
     __syncthreads();
+    if (bi < a.n_bricks) load_world(a, H.ahead.world, H.wc, spair);
+    step_kernel_wait();
+    if (tid == 0 && bi < a.n_bricks) {
+        const int64_t t = __ldcg(&a.worlds[H.wc.world].t);
+        const uint64_t th = t_hash((uint32_t)t, H.wc.w.seed);
+        H.th = make_uint2((uint32_t)th, (uint32_t)(th >> 32));
+    }
     while (bi < a.n_bricks) {
         const Brick br = H.ahead;
         if (H.wc.world != br.world) {  // (block-uniform)
             load_world(a, br.world, H.wc, spair);
             if (tid == 0) {
-                const uint64_t th = t_hash((uint32_t)H.wc.w.t, H.wc.w.seed);
+                const uint64_t th = t_hash((uint32_t)__ldcg(&a.worlds[br.world].t), H.wc.w.seed);
                 H.th = make_uint2((uint32_t)th, (uint32_t)(th >> 32));
             }
         }

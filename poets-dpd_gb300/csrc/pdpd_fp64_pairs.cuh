@@ -116,7 +116,6 @@ __host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t 
 // changes where a list lies, not what is in it.  Bound by instruction issue; no FP64 work.
 __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Layout lay)
 {
-    step_kernel_wait();
     constexpr int T = LIST64_THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     List64Header &H = *reinterpret_cast<List64Header *>(smem_raw);
@@ -130,8 +129,16 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
     uint32_t *segs = reinterpret_cast<uint32_t *>(smem_raw + lay.off_segs) + tid;
     const int cap = (a.list_capacity > 0 && a.list_capacity < LIST64_SEGS) ? max(3, a.list_capacity) : LIST64_SEGS;
     uint32_t world = L64_NONE;
+    Brick first{};
+    if (blockIdx.x < a.n_bricks) {  // (what no step changes is read before the wait)
+        first = a.bricks[blockIdx.x];
+        if (tid == 0) H.w = a.worlds[first.world];
+        world = first.world;
+    }
+    step_kernel_wait();
+    __syncthreads();
     for (uint32_t bi = blockIdx.x; bi < a.n_bricks;) {
-        const Brick br = a.bricks[bi];
+        const Brick br = bi == blockIdx.x ? first : a.bricks[bi];
         if (br.world != world) {
             if (tid == 0) H.w = a.worlds[br.world];
             world = br.world;
