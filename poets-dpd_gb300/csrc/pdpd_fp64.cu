@@ -106,8 +106,8 @@ __device__ __forceinline__ void load_x(const Vec4d *__restrict__ pos, uint32_t s
     x[2] = p.z;
 }
 
-// Bond forces, one thread per Hookean bond or angle bond, from the advanced, not yet re-sorted
-// state (slot_of_id is that of the sorted state it came from): each evaluated once, exactly as
+// Bond forces, one thread per Hookean bond or angle bond, from the positions pos of the beads'
+// slots (slot_of_id): each evaluated once, exactly as
 // update_hookean_bond / update_angle_bond (naive_dpd_engine_half_step.hpp:426-483) and
 // calc_angle_force (dpd_maths_core_half_step.hpp:177-229) do, and stored with the sign it is
 // added with at the CSR row of each of its beads (row_of): the force kernel adds a bead's rows in
@@ -119,10 +119,9 @@ __device__ __forceinline__ void store_term64(const KArgs &a, uint32_t row, doubl
     ((Vec4d *)a.bterm)[a.row_of[row]] = Vec4d{x, y, z, 0.0};
 }
 
-__device__ __forceinline__ void hookean64(const KArgs &a, const WorldDev &w, uint32_t k, uint32_t head,
-                                          uint32_t tail, uint32_t &err)
+__device__ __forceinline__ void hookean64(const KArgs &a, const Vec4d *pos, const WorldDev &w, uint32_t k,
+                                          uint32_t head, uint32_t tail, uint32_t &err)
 {
-    const Vec4d *pos = (const Vec4d *)a.posB;
     const Vec4d prm = ((const Vec4d *)a.bond_params)[k];
     double xh[3], xt[3], dx[3];
     load_x(pos, a.slot_of_id[head], xh);
@@ -138,9 +137,9 @@ __device__ __forceinline__ void hookean64(const KArgs &a, const WorldDev &w, uin
     store_term64(a, 2 * k + 1, f[0], f[1], f[2]);
 }
 
-__device__ __forceinline__ void angle64(const KArgs &a, const WorldDev &w, uint32_t g, const uint32_t *hmt)
+__device__ __forceinline__ void angle64(const KArgs &a, const Vec4d *pos, const WorldDev &w, uint32_t g,
+                                        const uint32_t *hmt)
 {
-    const Vec4d *pos = (const Vec4d *)a.posB;
     const Vec4d prm = ((const Vec4d *)a.bond_params)[a.n_bonds + g];
     double xh[3], xm[3], xt[3];
     load_x(pos, a.slot_of_id[hmt[0]], xh);
@@ -465,7 +464,7 @@ struct Balance64 {
 };
 
 // Thread k's bond or angle bond.
-__device__ __forceinline__ void bonds64(const KArgs &a, uint32_t k, bool angle)
+__device__ __forceinline__ void bonds64(const KArgs &a, const Vec4d *pos, uint32_t k, bool angle)
 {
     if (k >= (angle ? a.n_angles : a.n_bonds)) return;
     const uint32_t *ids = angle ? a.bond_list + 2 * (size_t)a.n_bonds + 3 * (size_t)k : a.bond_list + 2 * (size_t)k;
@@ -479,15 +478,14 @@ __device__ __forceinline__ void bonds64(const KArgs &a, uint32_t k, bool angle)
     }
     const WorldDev &w = a.worlds[lo];
     uint32_t err = 0;
-    if (angle) angle64(a, w, k, ids);
-    else hookean64(a, w, k, ids[0], ids[1], err);
+    if (angle) angle64(a, pos, w, k, ids);
+    else hookean64(a, pos, w, k, ids[0], ids[1], err);
     if (err) atomicOr(&a.worlds[lo].err, err);
 }
 
-// The cells' prefix sum (blocks [0, nb)), the Hookean bonds (the next bb) and the angle bonds (no
-// warp mixes the two), 64 to a block: an FP64 instruction holds its pipe for 64 cycles, so the
-// warps should be spread over the SMs.
-constexpr int BOND64_BLOCK = 64;
+// The cells' prefix sum (blocks [0, nb)) and, without pair lists (whose kernel takes them else),
+// the Hookean bonds (the next bb) and the angle bonds, from the advanced, not yet re-sorted state
+// (slot_of_id is that of the sorted state it came from).
 template <bool ONE_PASS>
 __global__ void __launch_bounds__(SCAN_THREADS) k_cells64(KArgs a, uint32_t nb, uint32_t bb, int tick)
 {
@@ -496,9 +494,8 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_cells64(KArgs a, uint32_t nb, 
         scan_cells<ONE_PASS>(a, tick);
         return;
     }
-    if (threadIdx.x >= BOND64_BLOCK) return;
     const bool angle = blockIdx.x - nb >= bb;
-    bonds64(a, (blockIdx.x - nb - (angle ? bb : 0u)) * BOND64_BLOCK + threadIdx.x, angle);
+    bonds64(a, (const Vec4d *)a.posB, (blockIdx.x - nb - (angle ? bb : 0u)) * SCAN_THREADS + threadIdx.x, angle);
 }
 
 // Bonds, update_mom and either the final write or the next update_pos with its cell count, for
@@ -736,8 +733,8 @@ int launch_pair_log64(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const
 int launch_cells64(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
     const uint32_t nb = scan_blocks(a.n_cells);
-    const uint32_t bb = bonds ? (a.n_bonds + BOND64_BLOCK - 1) / BOND64_BLOCK : 0u;
-    const uint32_t ab = bonds ? (a.n_angles + BOND64_BLOCK - 1) / BOND64_BLOCK : 0u;
+    const uint32_t bb = bonds && !a.list ? (a.n_bonds + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    const uint32_t ab = bonds && !a.list ? (a.n_angles + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
     if (scan_one_pass(a.n_cells)) launch_step_kernel(k_cells64<true>, nb + bb + ab, SCAN_THREADS, 0, s, a, nb, bb, tick);
     else launch_step_kernel(k_cells64<false>, nb + bb + ab, SCAN_THREADS, 0, s, a, nb, bb, tick);
     return 1;
@@ -747,8 +744,10 @@ int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
 {
     if (a.list) {  // each pair once
         const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb);
-        const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
-        launch_step_kernel(k_list64, (uint32_t)grid, LIST64_THREADS, L.bytes, s, a, L);
+        const uint32_t bb = (a.n_bonds + BOND64_CHUNK - 1) / BOND64_CHUNK;
+        const uint32_t work = a.n_bricks + bb + (a.n_angles + BOND64_CHUNK - 1) / BOND64_CHUNK;
+        const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, work));
+        launch_step_kernel(k_list64, grid, LIST64_THREADS, L.bytes, s, a, L, bb, work);
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
         launch_step_kernel(k_pairs64, std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s, a);
         const uint32_t parts = a.n_tiles * (TILE_BEADS / SUM64_BEADS);

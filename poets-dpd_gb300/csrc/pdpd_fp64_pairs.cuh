@@ -114,7 +114,12 @@ __host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t 
 // faster: 164 us against 161 for the 64^3 box); where there is none left, its beads are marked
 // (lrec.x) and k_sum64 evaluates all their pairs itself.  The order in which warps take room
 // changes where a list lies, not what is in it.  Bound by instruction issue; no FP64 work.
-__global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Layout lay)
+//
+// The queue's entries after the bricks are chunks of the bond forces: FP64 work, which the pipe
+// has nothing else of meanwhile, in a few warps (64^3 polymer box: 25 us in the prefix sum's
+// launch).
+constexpr uint32_t BOND64_CHUNK = 128;
+__global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Layout lay, uint32_t bb, uint32_t work)
 {
     constexpr int T = LIST64_THREADS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -137,7 +142,18 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
     }
     step_kernel_wait();
     __syncthreads();
-    for (uint32_t bi = blockIdx.x; bi < a.n_bricks;) {
+    for (uint32_t bi = blockIdx.x; bi < work;) {
+        if (bi >= a.n_bricks) {  // Hookean bonds, then angle bonds
+            const uint32_t c = bi - a.n_bricks;
+            const bool angle = c >= bb;
+            if (tid < BOND64_CHUNK)
+                bonds64(a, (const Vec4d *)a.posA, (c - (angle ? bb : 0u)) * BOND64_CHUNK + tid, angle);
+            __syncthreads();
+            if (tid == 0) H.next = gridDim.x + atomicAdd(a.brick_next, 1u);
+            __syncthreads();
+            bi = H.next;
+            continue;
+        }
         const Brick br = bi == blockIdx.x ? first : a.bricks[bi];
         if (br.world != world) {
             if (tid == 0) H.w = a.worlds[br.world];
