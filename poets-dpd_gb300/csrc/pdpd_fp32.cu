@@ -406,8 +406,11 @@ __device__ __forceinline__ void integrate32(const KArgs &a, const WorldDev &w, u
 // bound by the latency of the lookups, which one lane goes through once per term: eight lanes
 // take the launch of the 32^3 polymer box (9,828 polymer beads) from 12.3 to 9.7 us; many fill
 // the GPU with one lane each, and eight take that of the 128^3 box (314,568) from 43 to 87 us.
-// The line lies where eight lanes per bead fill half the SMs' threads.
+// A step of boxes with 5% polymer beads, us with 1, 2, 4, 8 lanes: 16,588 of them 74.6, 73.5, 72.6,
+// 71.8; 26,342 108.3, 105.9, 105.9, 107.1; 39,321 140.7, 138.5, 140.4, 141.4; 55,987 202.6, 201.6,
+// 204.3, 206.7; 76,800 261.1, 261.0, 264.7, 269.6; 132,710 424.4, 427.6, 433.6, 441.8.
 constexpr uint32_t BOND_LANES_FEW = 8, BOND_BEADS_FEW = 20000;
+constexpr uint32_t BOND_LANES_MORE = 2, BOND_BEADS_MORE = 70000;
 template <uint32_t BOND_LANES>
 __device__ __forceinline__ void bonds32(const KArgs &a, uint32_t thread)
 {
@@ -908,11 +911,15 @@ int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint3
 int launch_cells32(const KArgs &a, int tick, int bonds, cudaStream_t s)
 {
     const uint32_t nb = scan_blocks(a.n_cells);
-    const bool few = a.n_bonded <= BOND_BEADS_FEW;
-    const uint32_t bb = bonds ? (a.n_bonded * (few ? BOND_LANES_FEW : 1u) + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
-    void (*k)(KArgs, uint32_t, int);
-    if (scan_one_pass(a.n_cells)) k = few ? k_cells32<true, BOND_LANES_FEW> : k_cells32<true, 1>;
-    else k = few ? k_cells32<false, BOND_LANES_FEW> : k_cells32<false, 1>;
+    const uint32_t lanes = a.n_bonded <= BOND_BEADS_FEW ? BOND_LANES_FEW : a.n_bonded <= BOND_BEADS_MORE ? BOND_LANES_MORE : 1u;
+    const uint32_t bb = bonds ? (a.n_bonded * lanes + SCAN_THREADS - 1) / SCAN_THREADS : 0u;
+    auto pick = [&](auto one_pass) -> void (*)(KArgs, uint32_t, int) {
+        constexpr bool P = decltype(one_pass)::value;
+        if (lanes == BOND_LANES_FEW) return k_cells32<P, BOND_LANES_FEW>;
+        if (lanes == BOND_LANES_MORE) return k_cells32<P, BOND_LANES_MORE>;
+        return k_cells32<P, 1>;
+    };
+    const auto k = scan_one_pass(a.n_cells) ? pick(std::true_type{}) : pick(std::false_type{});
     launch_step_kernel(k, nb + bb, SCAN_THREADS, 0, s, a, nb, tick);
     return 1;
 }

@@ -59,3 +59,15 @@ def test_prefix_sum_edges(box):
     o.run(2, nthreads=8)
     _run([w], "fp64", 2)
     assert np.array_equal(w.x, o.x) and np.array_equal(w.f, o.f)
+
+
+@pytest.mark.parametrize("copies", [4, 12])
+def test_bond_lanes_per_bead(copies):
+    """6,144 polymer beads alone (eight lanes each), four and twelve times that in one batch (two
+    lanes, one): the same state to the bit."""
+    a = W.make_polymer_box(16, chain_fraction=0.5, seed=75, dt=0.001, theta0=0.3)
+    batch = [a.copy() for _ in range(copies)]
+    _run([a], "fp32", 3)
+    _run(batch, "fp32", 3)
+    for b in batch:
+        assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
