@@ -3,10 +3,12 @@
 // The step kernels have already counted each bead into its new cell and entered it in the
 // cell's bucket (cell_arrive, pdpd_cells.cuh).  Here:
 //   1. an exclusive prefix sum of the counts -> start[]: one kernel for up to 32K cells, two
-//      above; the launch also holds the bond forces of the next force pass (they need only the
-//      advanced positions, so their blocks run beside the few of the prefix sum);
+//      above; the launch also holds the bond forces of the next force pass (FP32, and FP64 without
+//      pair lists; they need only the advanced positions, so their blocks run beside the few of
+//      the prefix sum);
 //   2. k_move: each bead ranks itself by (z half, bead id) among its cell's bucket and moves
 //      its payload to start[cell] + that rank; the counts are cleared for the next step.
+// Small boxes without bond blocks do both in one kernel (k_rebuild_small).
 // The result is canonical: cells in index order, beads inside a cell in ascending bead id,
 // whatever order the atomics ran in.  That is the order in which the reference's cell lists
 // hold beads (naive_dpd_engine_half_step.hpp:276-293), so the FP64 force kernel adds pair
@@ -102,22 +104,13 @@ __device__ __forceinline__ uint32_t z_half(const Vec4d &) { return 0u; }
 __device__ __forceinline__ void put_shadow(const KArgs &, uint32_t, const float4 &) {}
 __device__ __forceinline__ void put_shadow(const KArgs &a, uint32_t dst, const Vec4d &p) { a.posf[dst] = offset_shadow(p); }
 
-// Bound by memory: reads 8 (cell) + 32 (payload) bytes per bead in the old order, the cell's
-// bucket and start, and writes 40 in the new order, which is nearly the old one (a bead moves
-// little in a step), so both sides are nearly contiguous.  slot_of_id is kept for polymer beads
-// only (monomer bit of the hash clear): the bond kernels look up bond partners through it; the
-// codec walks slots and reads ids instead.
+// Bead s of the old order, its cell, position and velocity given, into its place in the new one.
 template <class P>
-__global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
+__device__ __forceinline__ void move_bead(const KArgs &a, uint32_t s, uint32_t key, const P &p, const P &v,
+                                          const uint32_t *start, uint32_t epoch, int with_force)
 {
-    step_kernel_begin();
-    const uint32_t s = blockIdx.x * 256 + threadIdx.x;
-    if (s < a.n_cells) a.cnt[s] = 0u;
-    if (s >= a.n_beads) return;
-    const uint32_t key = a.key[s];
-    const P p = ((const P *)a.posB)[s], v = ((const P *)a.velB)[s];
     const uint32_t id = payload_id(v), me = id | z_half(p);
-    const uint32_t b = a.start[key], n = a.start[key + 1] - b;
+    const uint32_t b = start[key], n = start[key + 1] - b;
     const uint32_t m = min(n, a.bucket_k);
     const uint4 *bucket = (const uint4 *)(a.bucket + (size_t)key * a.bucket_k);
     uint32_t rank = 0, lo = 0;
@@ -133,7 +126,7 @@ __global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
     }
     if (n > m) {  // the cell's overflowing beads
         const unsigned long long head = a.over_head[key];
-        uint32_t node = (uint32_t)(head >> 32) == a.over->epoch ? (uint32_t)head : 0xffffffffu;
+        uint32_t node = (uint32_t)(head >> 32) == epoch ? (uint32_t)head : 0xffffffffu;
         while (node != 0xffffffffu) {
             const uint2 o = a.over_node[node];
             rank += o.x < me ? 1u : 0u;
@@ -152,6 +145,65 @@ __global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
     put_shadow(a, dst, p);
 }
 
+// Bound by memory: reads 8 (cell) + 32 (payload) bytes per bead in the old order, the cell's
+// bucket and start, and writes 40 in the new order, which is nearly the old one (a bead moves
+// little in a step), so both sides are nearly contiguous.  slot_of_id is kept for polymer beads
+// only (monomer bit of the hash clear): the bond kernels look up bond partners through it; the
+// codec walks slots and reads ids instead.
+template <class P>
+__global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)
+{
+    step_kernel_begin();
+    const uint32_t s = blockIdx.x * 256 + threadIdx.x;
+    if (s < a.n_cells) a.cnt[s] = 0u;
+    if (s >= a.n_beads) return;
+    move_bead(a, s, a.key[s], ((const P *)a.posB)[s], ((const P *)a.velB)[s], a.start, a.over->epoch, with_force);
+}
+
+// The whole rebuild of a small box without bond blocks, by one cluster: every block makes the
+// prefix sum for itself, in shared memory, while its first beads' state is on the way; the counts
+// are cleared once all blocks have read them.  Bound by the latency of its two rounds of loads.
+// The line: cells a block takes in one turn of the prefix sum, and beads it takes in one turn
+// (FP64) or three.  Step of water boxes, us, two kernels and one: FP32 4^3 14.1 and 12.8, 9^3
+// 15.3 and 14.0, 12^3 (5,184 beads) 16.1 and 15.1, 16^3 (12,288) 17.6 and 16.8; FP64 4^3 29.1
+// and 27.4, 8^3 31.8 and 30.4, 10^3 (3,000) 32.9 and 31.1, 12^3 35.3 and 35.1, 14^3 (8,232) 37.7
+// and 38.2, 16^3 42.4 and 43.0.
+constexpr int SMALL_BLOCKS = 8, SMALL_THREADS = 512;
+constexpr uint32_t SMALL_CELLS = SMALL_THREADS * SCAN_ITEMS, SMALL_BEADS = SMALL_BLOCKS * SMALL_THREADS;
+template <class P>
+__global__ void __cluster_dims__(SMALL_BLOCKS) __launch_bounds__(SMALL_THREADS) k_rebuild_small(KArgs a, int tick, int with_force)
+{
+    __shared__ uint32_t start[SMALL_CELLS + 1], sh[32];
+    step_kernel_begin();
+    const uint32_t first = blockIdx.x * SMALL_THREADS + threadIdx.x;
+    const uint32_t epoch = a.over->epoch + 1u;
+    uint32_t key = 0;
+    P p{}, v{};
+    if (first < a.n_beads) {
+        key = a.key[first];
+        p = ((const P *)a.posB)[first];
+        v = ((const P *)a.velB)[first];
+    }
+    scan_chunk(a.cnt, a.n_cells, 0, 0, start, sh);
+    if (threadIdx.x == 0) start[a.n_cells] = a.n_beads;
+    // every block has read the counts and the epoch
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (uint32_t c = first; c < a.n_cells; c += SMALL_BLOCKS * SMALL_THREADS) {
+        a.cnt[c] = 0u;
+        a.start[c] = start[c];
+    }
+    if (blockIdx.x == 0) rebuild_begin(a, tick);
+    for (uint32_t s = first; s < a.n_beads;) {
+        move_bead(a, s, key, p, v, start, epoch, with_force);
+        s += SMALL_BLOCKS * SMALL_THREADS;
+        if (s < a.n_beads) {
+            key = a.key[s];
+            p = ((const P *)a.posB)[s];
+            v = ((const P *)a.velB)[s];
+        }
+    }
+}
+
 void launch_scan(uint32_t *cnt, uint32_t n, uint32_t *blocksums, uint32_t *start, cudaStream_t s)
 {
     if (n == 0) return;
@@ -163,6 +215,13 @@ void launch_scan(uint32_t *cnt, uint32_t n, uint32_t *blocksums, uint32_t *start
 int launch_sort(const KArgs &a, int fp64, int tick, int with_force, int bonds, cudaStream_t s)
 {
     int n = 0;
+    // (the bond blocks look their partners up in the old order: not beside the move)
+    const bool bond_blocks = bonds && (fp64 ? !a.list && a.n_bonds + a.n_angles > 0 : a.n_bonded > 0);
+    if (a.n_beads > 0 && a.n_beads <= SMALL_BEADS * (fp64 ? 1 : 3) && a.n_cells <= SMALL_CELLS && !bond_blocks) {
+        if (fp64) launch_step_kernel(k_rebuild_small<Vec4d>, SMALL_BLOCKS, SMALL_THREADS, 0, s, a, tick, with_force);
+        else launch_step_kernel(k_rebuild_small<float4>, SMALL_BLOCKS, SMALL_THREADS, 0, s, a, tick, with_force);
+        return 1;
+    }
     if (!scan_one_pass(a.n_cells)) {
         launch_cells_reduce(a, tick, s);
         n++;

@@ -71,3 +71,21 @@ def test_bond_lanes_per_bead(copies):
     _run(batch, "fp32", 3)
     for b in batch:
         assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("box,density", [
+    ((3, 3, 3), 3), ((8, 16, 32), 1), ((8, 16, 32), 4097.5 / 4096), ((16, 16, 16), 3), ((16, 16, 16), 12289.5 / 4096),
+    ((2, 5, 409), 0.5), ((2, 5, 410), 0.5), ((2, 3, 2), 60)])
+def test_one_kernel_rebuild_edges(prec, box, density):
+    """The one-kernel rebuild's limits (4,096 cells; 4,096 beads in FP64, 12,288 in FP32) and buckets
+    that overflow, against the same box in a batch too large for it: the same state to the bit."""
+    w = W.make_water(box, seed=76, a=0.5, gamma=0.5, density=density, dt=0.001)
+    a, b, big = w.copy(), w.copy(), W.make_water((16, 16, 17), seed=77, density=0.1)
+    _run([a], prec, 3)
+    _run([b, big], prec, 3)
+    assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
+    if prec == "fp64":
+        o = O.OracleWorld(w)
+        o.run(3, nthreads=8)
+        assert np.array_equal(a.x, o.x) and np.array_equal(a.v, o.v) and np.array_equal(a.f, o.f)
