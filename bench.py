@@ -16,7 +16,7 @@ grid's bead payload (~1 GB) is larger than L2, so no flush is needed.
             512 states) + Run(K) + read-back of x, v, f of every state, timed on the host.
   plain_fp64  the plain FP64 engine run one state at a time (Attach excluded, as the
             reference's bpsExec), and the batched / plain ratio.
-  roofline  the force pass (bond kernel + brick kernel, dominant): algorithmic bytes per launch
+  roofline  the force pass (brick kernel, dominant): algorithmic bytes per launch
             (1,180 B per bead-step x beads) / its average CUDA-event duration, against the
             measured HBM copy bandwidth.
   roofline_run  the 128^3 box (6,291,456 beads, same chain recipe, a_WT = 75, gamma = 4.5):

@@ -576,6 +576,35 @@ struct pdpd_engine {
         for (int d = 0; d < 3; d++) shape[d] = best[d];
     }
 
+    // Brick shape of the kernel with three lanes per home bead, for the smallest batches: one brick
+    // and one turn (160 beads) per SM at most, and terms that fit its pool.  There a step is the
+    // latency of one warp's way through the force pass, and the lanes cut its walk and evaluation
+    // to a third; with more bricks than SMs they only add to the instructions.  Steps of water
+    // boxes, us, one lane and three: 4^3 13.7 and 10.5, 9^3 13.7 and 10.6, 12^3 15.2 and 12.2, 16^3
+    // 16.9 and 15.1, 18^3 18.7 and 16.3; 20^3 (two turns) 20.7 and 21.3, 24^3 24.8 and 22.7.  The
+    // smallest shape that keeps to one brick per SM is the best or within 2% (9^3: 1x2x4 10.6, 2x3x4
+    // 11.4, 4x4x6 12.6; 12^3: 1x2x4 17.6, 2x2x4 12.2, 2x4x4 13.4; 16^3: 2x3x4 21.3, 2x4x4 15.1, 3x4x4
+    // 15.9).
+    bool small_shape(int shape[3], uint32_t npair) const
+    {
+        static const int table[][3] = {{1, 2, 4}, {2, 2, 4}, {2, 3, 4}, {2, 4, 4}, {3, 3, 4}, {3, 4, 4}};
+        for (const auto &c : table) {
+            uint64_t n = 0;
+            for (const WorldHost &wh : worlds) {
+                uint64_t k = 1;
+                for (int d = 0; d < 3; d++) k *= (uint64_t)((wh.dev.L[d] + c[d] - 1) / c[d]);
+                n += k;
+            }
+            if (n > (uint64_t)sm_count) continue;
+            const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
+            if (max_density * c[0] * c[1] * c[2] > 160 || !brick_planes_fit(max_density, hc, (uint32_t)staging_want(hc) + 2, npair))
+                return false;
+            for (int d = 0; d < 3; d++) shape[d] = c[d];
+            return true;
+        }
+        return false;
+    }
+
     // Default kernel variant and brick shape for the attached batch, where the config does not
     // name them: the 512-thread row walk.  All of them give the same trajectory.
     void default_shape()
@@ -585,6 +614,7 @@ struct pdpd_engine {
         uint32_t npair = 1;
         for (const WorldHost &wh : worlds) npair = std::max(npair, wh.dev.n_types * wh.dev.n_types);
         if (cfg_force_kernel == 8 || cfg_force_kernel == 1) {
+            if (cfg_force_kernel == 8 && small_shape(cfg_brick, npair)) return;
             wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0); });
             return;
         }
@@ -692,8 +722,10 @@ struct pdpd_engine {
         a.brick_maxb = (uint32_t)std::min(limit, std::max(64.0, want));
         int grid = 0;
         uint32_t bytes = 0;
+        int small[3];
+        a.brick_planes = a.force_kernel == 8 && !brick_user && small_shape(small, a.brick_npair) && std::equal(small, small + 3, cfg_brick) ? 3 : 1;
         int rc = brick_setup(sm_count, a.force_kernel, a.brick_hc_max, a.brick_maxb, a.brick_npair,
-                             a.brick_home_max, &grid, &bytes);
+                             a.brick_home_max, a.brick_planes, &grid, &bytes);
         if (rc)
             return fail(PDPD_E_CUDA, "brick kernel setup (%u bytes of shared memory): %s", bytes,
                         cudaGetErrorString((cudaError_t)rc));

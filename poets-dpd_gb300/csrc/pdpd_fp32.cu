@@ -220,10 +220,10 @@ __device__ __forceinline__ float pair_r2(float ax, float ay, float az, const flo
 // One DPD pair force on the home bead, added to F (calc_force,
 // dpd_maths_core_half_step.hpp:69-157): conservative a (1-r), dissipative -gamma w^2 (e.dv),
 // random sqrt(gamma) w sqrt(24 kT/dt) u with kT = 1, along e = dx / r.
-__device__ __forceinline__ void pair_accumulate(float dx, float dy, float dz, float r2,
-                                                const float4 vi, const float4 vj, uint32_t hi,
-                                                uint32_t hj, float2 pp, uint32_t th_lo,
-                                                uint32_t th_hi, float scale, float F[3])
+__device__ __forceinline__ float4 pair_term32(float dx, float dy, float dz, float r2,
+                                              const float4 vi, const float4 vj, uint32_t hi,
+                                              uint32_t hj, float2 pp, uint32_t th_lo,
+                                              uint32_t th_hi, float scale)
 {
     float inv_r;  // r2 >= 1e-18: normal, so flushing subnormals changes nothing and saves the scaling around them
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(inv_r) : "f"(r2));
@@ -236,9 +236,18 @@ __device__ __forceinline__ void pair_accumulate(float dx, float dy, float dz, fl
     const float u = hash_u(th_lo, th_hi, hi, hj);
     const float con_m_diss = __fmaf_rn(-__fmul_rn(sg, sg), rdotv, __fmul_rn(pp.x, wr));
     const float scaled = __fmaf_rn(__fmul_rn(sg, scale), u, con_m_diss);
-    F[0] = __fmaf_rn(ex, scaled, F[0]);
-    F[1] = __fmaf_rn(ey, scaled, F[1]);
-    F[2] = __fmaf_rn(ez, scaled, F[2]);
+    return make_float4(ex, ey, ez, scaled);
+}
+
+__device__ __forceinline__ void pair_accumulate(float dx, float dy, float dz, float r2,
+                                                const float4 vi, const float4 vj, uint32_t hi,
+                                                uint32_t hj, float2 pp, uint32_t th_lo,
+                                                uint32_t th_hi, float scale, float F[3])
+{
+    const float4 t = pair_term32(dx, dy, dz, r2, vi, vj, hi, hj, pp, th_lo, th_hi, scale);
+    F[0] = __fmaf_rn(t.x, t.w, F[0]);
+    F[1] = __fmaf_rn(t.y, t.w, F[1]);
+    F[2] = __fmaf_rn(t.z, t.w, F[2]);
 }
 
 // Separation of the pair (i, j), d = cell_j - cell_i, per axis (o_i - [d > 0]) - (o_j - [d < 0]),
@@ -878,22 +887,35 @@ uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t
     return (uint32_t)std::max(64, std::min(most, budget / per_bead)) & ~1u;
 }
 
+// Three lanes per home bead: the bead's terms fit the pool (5 Poisson deviations above the mean of
+// the densest world) and the block's shared memory the SM.
+bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair)
+{
+    int dev = 0, most = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return false;
+    const double near = 4.19 * density;
+    return near + 5 * std::sqrt(near) <= POOL_TERMS &&
+           (int)brick_layout(hc_max, maxb, npair, BRICK_THREADS_WIDE, 0, 3).bytes <= most;
+}
+
 // Set up the brick kernel for a brick shape: opt in to the shared memory it needs and
 // return its persistent grid (resident blocks x SMs) and dynamic shared-memory bytes.
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max,
-                int *grid, uint32_t *smem_bytes)
+                int planes, int *grid, uint32_t *smem_bytes)
 {
     int nb = 0;
     const uint32_t hm = variant == 9 ? home_max : 0u;
-    const BrickLayout L = brick_layout(hc_max, maxb, npair, brick_variant_threads(variant), hm);
+    const BrickLayout L = brick_layout(hc_max, maxb, npair, brick_variant_threads(variant), hm, planes);
     const int bytes = (int)L.bytes;
     void (*k0)(KArgs, BrickLayout) = nullptr;
     void (*k1)(KArgs, BrickLayout) = nullptr;
     switch (variant) {
     case 9: k0 = k_force32_half<0>; k1 = k_force32_half<1>; break;
     case 8:
-        k0 = k_force32_brick<0, BRICK_THREADS_WIDE>;
-        k1 = k_force32_brick<1, BRICK_THREADS_WIDE>;
+        k0 = planes == 3 ? k_force32_brick<0, BRICK_THREADS_WIDE, 3> : k_force32_brick<0, BRICK_THREADS_WIDE>;
+        k1 = planes == 3 ? k_force32_brick<1, BRICK_THREADS_WIDE, 3> : k_force32_brick<1, BRICK_THREADS_WIDE>;
         break;
     default: k0 = k_force32_brick<0, BRICK_THREADS>; k1 = k_force32_brick<1, BRICK_THREADS>; break;
     }
@@ -929,13 +951,16 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
     if (a.force_kernel != 1 && a.n_bricks > 0) {
         const int v = a.force_kernel;
         const BrickLayout L = brick_layout(a.brick_hc_max, a.brick_maxb, a.brick_npair, brick_variant_threads(v),
-                                           v == 9 ? a.brick_home_max : 0u);
+                                           v == 9 ? a.brick_home_max : 0u, a.brick_planes);
         const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
         void (*k)(KArgs, BrickLayout);
         switch (v) {
         case 9: k = final_step ? k_force32_half<1> : k_force32_half<0>; break;
         case 8:
-            k = final_step ? k_force32_brick<1, BRICK_THREADS_WIDE> : k_force32_brick<0, BRICK_THREADS_WIDE>;
+            if (a.brick_planes == 3)
+                k = final_step ? k_force32_brick<1, BRICK_THREADS_WIDE, 3> : k_force32_brick<0, BRICK_THREADS_WIDE, 3>;
+            else
+                k = final_step ? k_force32_brick<1, BRICK_THREADS_WIDE> : k_force32_brick<0, BRICK_THREADS_WIDE>;
             break;
         default: k = final_step ? k_force32_brick<1, BRICK_THREADS> : k_force32_brick<0, BRICK_THREADS>; break;
         }

@@ -16,8 +16,10 @@
 //              enters the pair in the other bead's list;
 //   k_sum64    each bead adds its terms in order, then bonds and integration.
 // 64^3 polymer box, force pass with bonds: 1.78 ms with each bead evaluating all its pairs
-// (k_force64), 0.90 ms so (lists 0.16, pairs 0.44 at 84% of the FP64 pipe, sums 0.27).
-// That kernel stays for batches the lists have no memory for or too many beads for (a list
+// (k_force64), 0.83 ms so (lists and bonds 0.16, pairs 0.44 at 84% of the FP64 pipe, sums 0.21).
+// (Pairs evaluated by the listing blocks themselves, to have the FP64 pipe busy meanwhile: 0.82
+// ms, and 0.092 -> 0.105 at 27^3: two blocks per SM do not keep both halves going.)
+// k_force64 stays for batches the lists have no memory for or too many beads for (a list
 // entry holds a slot in 25 bits).
 
 // A list entry is one of: L64_OWN | q, the bead evaluates pair q; the slot of a lower bead (25

@@ -104,7 +104,7 @@ struct KArgs {
     uint32_t *cellg;     // global cell of each sorted slot
     uint32_t *slot_of_id;   // sorted slot of each polymer bead, by id (monomers: not kept)
     uint16_t *zlo;       // FP32: beads of each cell in its lower z half (offset z < 0.5), which
-                         // the sort places first; not written for empty cells
+                         // the sort places first (half shell); not written for empty cells
     // advanced, not yet sorted state (B), indexed by the A slot it came from
     void *posB, *velB, *frcB;
     uint32_t *key;       // new global cell
@@ -120,7 +120,7 @@ struct KArgs {
     const void *bond_params;   // float4 / Vec4d: (kappa, r0 | cos theta0, sin theta0, 0)
     const void *pair;          // float2 / Vec2d: (a_ij, sqrt(gamma_ij))
     const void *cellpair;      // float2 / Vec2d per (cell, type pair) of spatial worlds
-    const uint32_t *bonded_ids;  // ids of the beads that have bond terms (FP32 bond kernel)
+    const uint32_t *bonded_ids;  // ids of the beads that have bond terms (FP32)
     uint32_t n_bonded;
     const uint32_t *bond_list;   // the batch's flat lists with global ids: n_bonds pairs, n_angles triples
     uint32_t n_bonds, n_angles;
@@ -145,6 +145,7 @@ struct KArgs {
     uint32_t brick_hc_max;  // halo cells of the nominal brick shape
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds
+    int brick_planes;       // variant 8: lanes per home bead (3 in small batches, else 1)
     uint32_t brick_home_max;  // half shell: home-bead capacity of one brick
     uint32_t *brick_next;   // the brick queue's next free entry beyond the first gridDim.x
                             // (zeroed by the sort, which precedes every force pass)
@@ -177,7 +178,8 @@ int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int *grid);
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);
-// bonds: with the bond forces at the beads' new positions, for the force pass that follows.
+// bonds: with the bond forces at the beads' new positions, for the force pass that follows (FP64
+// with pair lists: the list kernel has them).
 int launch_sort(const KArgs &a, int fp64, int tick, int with_force, int bonds, cudaStream_t s);
 // Its prefix sum of the cell counts, with the bond forces in the same launch; over more cells
 // than one kernel takes (scan_one_pass) it needs the chunks' sums first.
@@ -263,7 +265,8 @@ size_t payload_bytes(int fp64);  // bytes of one pos / vel / frc element
 // Largest staged-bead capacity of a brick for force variant `variant` (two blocks per SM of
 // shared memory for variants 8 and 9, the list entries' range for 6).
 uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max);
-int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max,
+bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair);
+int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max, int planes,
                 int *grid, uint32_t *smem_bytes);  // 0 or a cudaError_t
 uint32_t scan_blocks(uint32_t n_cells);
 

@@ -148,7 +148,7 @@ __device__ __forceinline__ void move_bead(const KArgs &a, uint32_t s, uint32_t k
 // Bound by memory: reads 8 (cell) + 32 (payload) bytes per bead in the old order, the cell's
 // bucket and start, and writes 40 in the new order, which is nearly the old one (a bead moves
 // little in a step), so both sides are nearly contiguous.  slot_of_id is kept for polymer beads
-// only (monomer bit of the hash clear): the bond kernels look up bond partners through it; the
+// only (monomer bit of the hash clear): the bond forces look partners up through it; the
 // codec walks slots and reads ids instead.
 template <class P>
 __global__ void __launch_bounds__(256) k_move(KArgs a, int with_force)

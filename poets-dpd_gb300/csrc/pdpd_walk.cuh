@@ -106,23 +106,25 @@ __device__ __forceinline__ uint32_t walk_mask(const ulonglong2 *sxy, const uint6
 //
 // segs holds cap segments (cap >= 3) with stride T; flush(n) is called with the n candidates of
 // the segments so far when more may not fit, and the walk starts filling them anew.  Returns
-// the candidates left in the segments.
-template <int T, class Flush>
+// the candidates left in the segments.  PLANES = 3: only the three rows of dx = plane - 1.
+template <int T, int PLANES = 1, class Flush>
 __device__ __forceinline__ int walk_rows(const ulonglong2 *xy, const uint64_t *zf, uint32_t *__restrict__ segs,
                                          int cap, const uint16_t *__restrict__ hstart, int HY, int HZ1,
-                                         uint32_t code, uint32_t si, float ox, float oy, float oz, Flush flush)
+                                         uint32_t code, uint32_t si, float ox, float oy, float oz, Flush flush,
+                                         int plane = 0)
 {
+    const int dlo = PLANES == 3 ? plane - 1 : -1, dhi = PLANES == 3 ? plane - 1 : 1;
     const int hx = (int)(code & 255u), hy = (int)((code >> 8) & 255u), hz = (int)((code >> 16) & 255u);
     const float gzp = 1.0f - oz;
     const float below = WALK_R2 - oz * oz, above = WALK_R2 - gzp * gzp;
     const float zi = -((const float *)zf)[si];
     const uint64_t nz = f32x2(zi, zi), m_r2 = f32x2(-WALK_R2, -WALK_R2);
-    const uint16_t *h = hstart + ((hx - 1) * HY + (hy - 1)) * HZ1 + hz;
+    const uint16_t *h = hstart + ((hx + dlo) * HY + (hy - 1)) * HZ1 + hz;
     uint32_t *out = segs;
     const uint32_t *const full = segs + (cap - 3) * T;  // room for the first segments of three rows
     int n_cand = 0;
 #pragma unroll 1
-    for (int ddx = -1; ddx <= 1; ddx++) {
+    for (int ddx = dlo; ddx <= dhi; ddx++) {
         const float gx = slab_gap(ox, ddx), nax = (float)ddx - ox;
         const uint64_t nx = f32x2(nax, nax);
 #pragma unroll
@@ -151,7 +153,7 @@ __device__ __forceinline__ int walk_rows(const ulonglong2 *xy, const uint64_t *z
             }
         }
         h += (HY - 3) * HZ1;
-        if (ddx < 1 && out > full) {
+        if (ddx < dhi && out > full) {
             flush(n_cand);
             out = segs;
             n_cand = 0;

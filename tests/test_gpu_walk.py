@@ -62,3 +62,17 @@ def test_walk_of_coincident_and_barely_separated_beads(force_kernel):
     ref = _run(world, 2, force_kernel=1)
     w = _run(world, 2, force_kernel=force_kernel)
     assert np.array_equal(w.x, ref.x) and np.array_equal(w.f, ref.f)
+
+
+@pytest.mark.parametrize("cfg", [{}, {"list_capacity": 3}, {"grid_blocks": 7}])
+@pytest.mark.parametrize("box", [(2, 2, 2), (4, 3, 5), (9, 9, 9), (12, 12, 12), (14, 13, 14), (16, 16, 16),
+                                 (17, 17, 16), (18, 18, 18)])
+def test_three_lanes_per_bead_equal_the_bead_kernel(box, cfg):
+    """The smallest boxes run three lanes per bead (18^3 the largest): with chains, and a clump whose
+    beads have more candidates than a bead's pool holds."""
+    world = W.make_polymer_box(box, chain_fraction=0.2, seed=54, dt=0.0005)
+    free = np.flatnonzero(world.is_monomer)[:60 if world.n_beads > 100 else 0]
+    world.x[free] = 1.0 + 0.8 * np.random.default_rng(55).random((len(free), 3))
+    ref = _run(world, 3, force_kernel=1)
+    w = _run(world, 3, **cfg)
+    assert np.array_equal(w.x, ref.x) and np.array_equal(w.v, ref.v) and np.array_equal(w.f, ref.f)
