@@ -576,8 +576,9 @@ struct pdpd_engine {
         for (int d = 0; d < 3; d++) shape[d] = best[d];
     }
 
-    // Brick shape of the kernel with three lanes per home bead, for the smallest batches: one brick
-    // and one turn (160 beads) per SM at most, and terms that fit its pool.  There a step is the
+    // Brick shape of the kernels with three lanes per home bead, for the smallest batches: one brick
+    // and one turn (160 beads) for each resident block (FP32 one per SM, FP64 two), and terms that
+    // fit FP32's pool.  There a step is the
     // latency of one warp's way through the force pass, and the lanes cut its walk and evaluation
     // to a third; with more bricks than SMs they only add to the instructions.  Steps of water
     // boxes, us, one lane and three: 4^3 13.7 and 10.5, 9^3 13.7 and 10.6, 12^3 15.2 and 12.2, 16^3
@@ -585,6 +586,8 @@ struct pdpd_engine {
     // smallest shape that keeps to one brick per SM is the best or within 2% (9^3: 1x2x4 10.6, 2x3x4
     // 11.4, 4x4x6 12.6; 12^3: 1x2x4 17.6, 2x2x4 12.2, 2x4x4 13.4; 16^3: 2x3x4 21.3, 2x4x4 15.1, 3x4x4
     // 15.9).
+    // FP64, water, us, one lane and three: 4^3 30.4 and 27.0, 8^3 31.5 and 28.5, 12^3 36.9 and 34.3,
+    // 16^3 43.6 and 41.7, 20^3 56.6 and 55.6, 24^3 74.2 and 72.5; 27^3 (441 bricks) 90.5 and 98.1.
     bool small_shape(int shape[3], uint32_t npair) const
     {
         static const int table[][3] = {{1, 2, 4}, {2, 2, 4}, {2, 3, 4}, {2, 4, 4}, {3, 3, 4}, {3, 4, 4}};
@@ -595,10 +598,11 @@ struct pdpd_engine {
                 for (int d = 0; d < 3; d++) k *= (uint64_t)((wh.dev.L[d] + c[d] - 1) / c[d]);
                 n += k;
             }
-            if (n > (uint64_t)sm_count) continue;
+            if (n > (uint64_t)sm_count * (fp64() ? 2 : 1)) continue;
             const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
-            if (max_density * c[0] * c[1] * c[2] > 160 || !brick_planes_fit(max_density, hc, (uint32_t)staging_want(hc) + 2, npair))
-                return false;
+            if (max_density * c[0] * c[1] * c[2] > 160) return false;
+            const uint32_t maxb = (uint32_t)staging_want(hc) + 2;
+            if (fp64() ? maxb > list64_maxb_limit(hc) : !brick_planes_fit(max_density, hc, maxb, npair)) return false;
             for (int d = 0; d < 3; d++) shape[d] = c[d];
             return true;
         }
@@ -671,7 +675,10 @@ struct pdpd_engine {
         a.n_bricks = 0;
         if (fp64() ? !a.list : a.force_kernel == 1) return PDPD_OK;
         int shape[3] = {cfg_brick[0], cfg_brick[1], cfg_brick[2]};
-        if (fp64()) wide_shape(shape, [](uint32_t hc) { return list64_maxb_limit(hc); });
+        if (fp64()) {
+            a.brick_planes = small_shape(shape, 0) ? 3 : 1;
+            if (a.brick_planes == 1) wide_shape(shape, [](uint32_t hc) { return list64_maxb_limit(hc); });
+        }
         // Each axis of a world is cut into ceil(L / b) bricks of as equal extents as possible
         // (e.g. a side of 9 with b = 4 into 3 + 3 + 3, not 4 + 4 + 1): no extent exceeds the
         // configured one, and no thin remainder brick stages a halo for a few home cells.
@@ -706,7 +713,7 @@ struct pdpd_engine {
         if (fp64()) {
             const double most = (double)list64_maxb_limit(a.brick_hc_max);
             a.brick_maxb = (uint32_t)std::min(most, std::max(64.0, staging_want(a.brick_hc_max)));
-            const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, &a.brick_grid);
+            const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, a.brick_planes, &a.brick_grid);
             if (rc) return fail(PDPD_E_CUDA, "list kernel setup: %s", cudaGetErrorString((cudaError_t)rc));
             if (cfg_grid_blocks > 0) a.brick_grid = cfg_grid_blocks;
             drop_graph();

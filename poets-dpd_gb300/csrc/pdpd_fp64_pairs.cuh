@@ -120,7 +120,12 @@ __host__ __device__ inline List64Layout list64_layout(uint32_t hc_max, uint32_t 
 // The queue's entries after the bricks are chunks of the bond forces: FP64 work, which the pipe
 // has nothing else of meanwhile, in a few warps (64^3 polymer box: 25 us in the prefix sum's
 // launch).
+//
+// PLANES = 3, in the smallest batches (small_shape): three lanes per bead, one per plane of
+// neighbour rows, whose parts of the list follow each other.  (8^3 water, step: 31.5 ->
+// 28.5 us; 16^3 43.6 -> 41.7, 24^3 74.2 -> 72.5.)
 constexpr uint32_t BOND64_CHUNK = 128;
+template <int PLANES>
 __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Layout lay, uint32_t bb, uint32_t work)
 {
     constexpr int T = LIST64_THREADS;
@@ -170,10 +175,12 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
                                 sc[j] = make_uint2(slot, code);
                             });
         const bool staged = total <= lay.maxb;
-        for (uint32_t t0 = tid & ~31; t0 < n_home; t0 += T) {
-            const uint32_t t = t0 + lane;
+        constexpr uint32_t WARP_BEADS = PLANES == 3 ? 10u : 32u;
+        for (uint32_t t0 = (tid >> 5) * WARP_BEADS; t0 < n_home; t0 += (T / 32) * WARP_BEADS) {
+            const int plane = PLANES == 3 ? lane % 3 : 0;
+            const uint32_t t = t0 + (PLANES == 3 ? lane / 3 : lane);
             const int r = home_row_near(H.home_rows, br.bx * br.by, t0, t);
-            const bool act = t < n_home;
+            const bool act = t < n_home && (PLANES == 1 || lane < 30);
             uint32_t s = 0, code = 0;
             uint32_t n = 0, own = 0;
             bool dense = !staged;
@@ -186,8 +193,9 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
                     const uint32_t si = hstart[row * (HZ + 1) + 1] + k;
                     const float *q = xy + 2 * si - (si & 1u);
                     code = sc[si].y;
-                    n = (uint32_t)walk_rows<T>((const ulonglong2 *)xy, (const uint64_t *)zf, segs, cap, hstart, HY, HZ + 1,
-                                               code, si, q[0], q[2], a.posf[s].z, [&](int) { dense = true; });
+                    n = (uint32_t)walk_rows<T, PLANES>((const ulonglong2 *)xy, (const uint64_t *)zf, segs, cap, hstart, HY,
+                                                       HZ + 1, code, si, q[0], q[2], a.posf[s].z,
+                                                       [&](int) { dense = true; }, plane);
                     if (!dense) {
                         SegReader<T> seg(segs);
                         for (uint32_t e = 0; e < n; e++) {
@@ -196,8 +204,15 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
                         }
                     }
                 }
-                if (dense) {
-                    n = 0;
+            }
+            if (PLANES == 3) {  // a bead of whose lanes one has too many is left to the first
+                const uint32_t any = __ballot_sync(0xffffffffu, dense) >> (lane - plane) & 7u;
+                dense = any != 0u;
+                if (dense && plane != 0) n = own = 0;
+            }
+            if (act) {
+                if (dense && plane == 0) {
+                    n = own = 0;
                     decode_cell(a.cellg[s] - w.cell_base, w.L, c[0], c[1], c[2]);
                     walk_global64(a, w, s, c, a.posf[s], [&](uint32_t j, uint32_t, bool image) {
                         n++;
@@ -227,14 +242,17 @@ __global__ void __launch_bounds__(LIST64_THREADS, 2) k_list64(KArgs a, List64Lay
                 // no room left: what the warp took of the pairs' holds none
                 for (unsigned long long q = pfirst + lane; q < pfirst + own_all && q < a.pair_cap; q += 32)
                     a.pair_i[q] = L64_NONE;
-                if (act) a.lrec[s] = make_uint2(L64_NONE, 0u);
+                if (act && plane == 0) a.lrec[s] = make_uint2(L64_NONE, 0u);
                 continue;
             }
             const uint32_t at = (uint32_t)first + n_inc - n;
             uint32_t q = (uint32_t)pfirst + own_inc - own;
+            uint32_t all = n;
+            if (PLANES == 3) all += __shfl_down_sync(0xffffffffu, n, 1) + __shfl_down_sync(0xffffffffu, n, 2);
             if (!act) continue;
             uint32_t *list = a.list + at;
-            a.lrec[s] = make_uint2(at, n);
+            if (plane == 0) a.lrec[s] = make_uint2(at, all);
+            if (PLANES == 3 && dense && plane != 0) continue;
             auto emit = [&](uint32_t j, uint32_t dir, bool both) {
                 if (both || j > s) {
                     *list++ = L64_OWN | q;

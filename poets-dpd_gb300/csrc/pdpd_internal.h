@@ -145,7 +145,7 @@ struct KArgs {
     uint32_t brick_hc_max;  // halo cells of the nominal brick shape
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds
-    int brick_planes;       // variant 8: lanes per home bead (3 in small batches, else 1)
+    int brick_planes;       // variant 8, FP64 lists: lanes per home bead (3 in small batches, else 1)
     uint32_t brick_home_max;  // half shell: home-bead capacity of one brick
     uint32_t *brick_next;   // the brick queue's next free entry beyond the first gridDim.x
                             // (zeroed by the sort, which precedes every force pass)
@@ -174,7 +174,7 @@ int launch_finish32(const KArgs &a, cudaStream_t s);
 int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
 // FP64 list kernel: staged-bead capacity of a brick, and its persistent grid (0 or a cudaError_t).
 uint32_t list64_maxb_limit(uint32_t hc_max);
-int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int *grid);
+int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int planes, int *grid);
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);

@@ -69,3 +69,18 @@ def test_pair_lists_of_a_mixed_batch():
     for n, w, o in zip(names, worlds, oracles):
         o.run(3)
         assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f), n
+
+
+@pytest.mark.parametrize("side", [14, 20, 24, 27])
+def test_lanes_per_bead_of_small_and_larger_boxes(side):
+    """Three lanes per bead up to 24^3, each shape of brick; one above.  The small worlds beside a
+    larger box, one lane per bead for all of them."""
+    names = [n for n in sorted(WORLDS) if n not in ("large_bricks", "dense")] if side == 27 else []
+    worlds = [WORLDS[n]() for n in names] + [W.make_polymer_box(side, chain_fraction=0.1, seed=69, dt=0.005)]
+    oracles = [O.OracleWorld(w) for w in worlds]
+    eng = E.GB300DPDEngine("fp64")
+    eng.AttachBatch(worlds)
+    eng.Run(2)
+    for w, o in zip(worlds, oracles):
+        o.run(2, nthreads=8)
+        assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
