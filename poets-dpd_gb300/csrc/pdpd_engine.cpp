@@ -2439,7 +2439,7 @@ int pdpd_v2binary_prepare(pdpd_engine *e, uint32_t world, uint32_t n_polymers,
         if (off[i] == 0xFFFFFFFFu) return e->fail(PDPD_E_INVALID, "bead %u belongs to no polymer", i);
     L->bytes = t.size();
     cudaSetDevice(e->device);
-    if (L->d_buf.alloc(std::max<size_t>(L->bytes, 16)) != cudaSuccess ||
+    if (L->d_buf.alloc(L->bytes + 32) != cudaSuccess ||
         L->d_off.alloc(sizeof(uint32_t) * std::max<uint32_t>(n, 1)) != cudaSuccess ||
         L->d_rec.alloc(sizeof(uint2) * std::max<uint32_t>(n, 1)) != cudaSuccess ||
         e->d_v2err.alloc(16) != cudaSuccess)
@@ -2472,38 +2472,38 @@ int pdpd_v2binary_encode(pdpd_engine *e, uint32_t world, uint8_t *out, size_t ca
     const WorldDev &wd = e->worlds[world].dev;
     if (e->d_inv.alloc(sizeof(uint32_t) * std::max<uint32_t>(1, e->n_beads)) != cudaSuccess)
         return e->fail(PDPD_E_NOMEM, "device allocation failed");
-    cudaError_t ce = cudaMemsetAsync(e->d_v2err.p, 0, sizeof(uint32_t), e->stream);
+    const size_t err_at = (L->bytes + 15) & ~size_t(15);  // the error word crosses with the section
+    uint32_t *const d_err = (uint32_t *)(L->d_buf.as<uint8_t>() + err_at);
+    cudaError_t ce = cudaMemsetAsync(d_err, 0, sizeof(uint32_t), e->stream);
     e->launches += launch_slot_of_id(e->args, wd.bead_base, wd.n_beads, e->d_inv.as<uint32_t>(), e->stream);
     e->launches += launch_v2_encode(e->args, e->fp64(), world, wd.n_beads, (const uint2 *)L->d_rec.p,
-                                    e->d_inv.as<uint32_t>(), L->d_buf.as<uint8_t>(), e->d_v2err.as<uint32_t>(),
-                                    e->stream);
+                                    e->d_inv.as<uint32_t>(), L->d_buf.as<uint8_t>(), d_err, e->stream);
     if (ce == cudaSuccess) ce = cudaGetLastError();
     // Through pinned staging in pieces, each copied on by the host while the next crosses the link.
     // (Written by the kernel straight into the caller's array, the 64^3 box takes 170 us where its
     // pages are known to the GPU, against 330 us so, but 4 ms in a new array.)
-    if (e->h_staging[1].alloc(L->bytes + 16) != cudaSuccess) return e->fail(PDPD_E_NOMEM, "pinned allocation failed");
+    if (e->h_staging[1].alloc(err_at + 16) != cudaSuccess) return e->fail(PDPD_E_NOMEM, "pinned allocation failed");
     uint8_t *src = (uint8_t *)e->h_staging[1].p;
-    uint32_t *herr_p = (uint32_t *)(src + ((L->bytes + 3) & ~size_t(3)));
     const size_t pieces = std::min<size_t>(V2_PIECES, L->bytes / (1 << 20) + 1), per = (L->bytes + pieces - 1) / pieces;
     for (cudaEvent_t &ev : e->ev_piece)
         if (ce == cudaSuccess && !ev) ce = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(herr_p, e->d_v2err.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream);
     for (size_t k = 0; k < pieces && ce == cudaSuccess; k++) {
-        const size_t b = std::min(L->bytes, k * per), en = std::min(L->bytes, b + per);
-        if (en > b) ce = cudaMemcpyAsync(src + b, L->d_buf.as<uint8_t>() + b, en - b, cudaMemcpyDeviceToHost, e->stream);
-        if (ce == cudaSuccess) ce = cudaEventRecord(e->ev_piece[k], e->stream);
+        const size_t b = std::min(L->bytes, k * per), en = k + 1 < pieces ? std::min(L->bytes, b + per) : err_at + 4;
+        ce = cudaMemcpyAsync(src + b, L->d_buf.as<uint8_t>() + b, en - b, cudaMemcpyDeviceToHost, e->stream);
+        if (ce == cudaSuccess && k + 1 < pieces) ce = cudaEventRecord(e->ev_piece[k], e->stream);
     }
     for (size_t k = 0; k < pieces && ce == cudaSuccess; k++) {
         const size_t b = std::min(L->bytes, k * per), en = std::min(L->bytes, b + per);
-        ce = cudaEventSynchronize(e->ev_piece[k]);
+        ce = k + 1 < pieces ? cudaEventSynchronize(e->ev_piece[k]) : cudaStreamSynchronize(e->stream);
         if (ce == cudaSuccess)
-            parallel_for(en - b, 1 << 17, [&](size_t p, size_t q) { memcpy(out + b + p, src + b + p, q - p); });
+            // (several host threads from half a megabyte: 320 KB take 9 us longer with them, 720 KB 12 less)
+            parallel_for(en - b, en - b < (1 << 19) ? en - b : 1 << 17, [&](size_t p, size_t q) { memcpy(out + b + p, src + b + p, q - p); });
     }
     if (ce != cudaSuccess) {
         cudaStreamSynchronize(e->stream);
         return e->cuda_fail(ce, "v2binary encode");
     }
-    const uint32_t herr = *herr_p;
+    const uint32_t herr = *(const uint32_t *)(src + err_at);
     if (herr & 2u) return e->fail(PDPD_E_INVALID, "Bead is out of bounds.");
     if (herr & 1u)
         return e->fail(PDPD_E_INVALID, "A velocity or force is not finite or has magnitude 65536 or more "

@@ -1,5 +1,5 @@
 """v2binary snapshots at the encoder's edges, byte for byte against the codec's restatement: worlds
-of one record, of a tile's 512 records and one more, boxes whose positions round up to the box
+of one record, of a tile's 64 records and one more, boxes whose positions round up to the box
 side, vectors at the format's limits in FP32 (exponents at both ends, mantissas that round up to
 256, subnormals), and polymers that put their headers between the records."""
 
@@ -28,7 +28,7 @@ def _world(kind, seed):
     if kind == "polymers":
         w = W.make_polymer_box((7, 5, 9), chain_fraction=0.4, seed=seed)
     else:
-        n = {"one": 1, "tile": 512, "tile_and_one": 513, "many": 4000}[kind]
+        n = {"one": 1, "tile": 64, "tile_and_one": 65, "many": 4000}[kind]
         w = W.make_water((11, 13, 4), seed=seed, density=n / (11 * 13 * 4.0) + 1e-9)
         assert w.n_beads == n
     w.v, w.f = _edge_vectors(w, rng), _edge_vectors(w, rng)
