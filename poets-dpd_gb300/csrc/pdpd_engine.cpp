@@ -749,8 +749,8 @@ struct pdpd_engine {
     uint32_t autotune(uint32_t n_steps)
     {
         // (variant 9 is left out: its forces are not bit-identical with these)
-        static const int cand[][4] = {{8, 5, 8, 8}, {8, 4, 10, 8}, {8, 4, 8, 10}, {8, 4, 8, 8},
-                                      {8, 6, 8, 6}, {6, 3, 4, 6}, {6, 4, 4, 6}, {1, 4, 4, 4}};
+        int cand[][4] = {{8, 5, 8, 8}, {8, 4, 10, 8}, {8, 4, 8, 10}, {8, 4, 8, 8},
+                         {8, 6, 8, 6}, {6, 3, 4, 6}, {6, 4, 4, 6}, {1, 4, 4, 4}};
         const int n_cand = (int)(sizeof cand / sizeof cand[0]);
         const uint32_t timed = 3;  // steps timed per candidate, after one warm step
         const uint32_t warm = 8;   // steps of the untimed warm-up run
@@ -759,6 +759,9 @@ struct pdpd_engine {
             n_steps < warm + 1 + (timed + 2) * n_cand + 1)
             return 0;
         const int keep[4] = {cfg_force_kernel, cfg_brick[0], cfg_brick[1], cfg_brick[2]};
+        // (a size-aware default that is none of them runs against them in place of the slowest)
+        if (std::none_of(cand, cand + n_cand, [&](const int *c) { return std::equal(c, c + 4, keep); }))
+            std::copy(keep, keep + 4, cand[n_cand - 2]);
         cudaEvent_t e0, e1;
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
