@@ -542,34 +542,46 @@ struct pdpd_engine {
     // Brick shape for the 512-thread kernels (FP32 variant 8, the FP64 list kernel).  By the batch's
     // cells per SM: the largest bricks stage the fewest halo beads per home bead, but the
     // persistent blocks (two per SM) want several bricks each, and a small batch has too few.
-    // Whole FP32 steps of polymer boxes, us (sides 20, 32, 40, 52, 64, 80; cells per SM 53, 216,
-    // 421, 925, 1725, 3368): 5x8x8 36.4, 41.0, 60.4, 93.5, 160.2, 279; 4x5x8 (480 home beads, one
-    // turn of the block) 27.9, 37.5, 53.5, 91.5, 154.2, 281; 4x4x8 26.9, 35.1, 56.5, 98.7, 158.3,
-    // 298; 4x4x6 26.0, 41.3, 59.4, 106, 182, 345; 2x4x4 25.5, 58.1, 94.8, 183, 336, 665 (sides 9
-    // and 16: 2x4x4 23.2 and 24.1, 4x4x6 23.7 and 26.0).  In between, how the bricks of a box
-    // divide into rounds of the blocks matters more (36^3: 4x4x8 44.7, 4x6x8 37.6; 39^3: 4x5x8
-    // 49.5, 5x6x8 40.5): another shape is taken where shape_cost puts it 6% below.  Smaller bricks
-    // where the halo of the batch's densest world would not fit the staging capacity 5 Poisson
-    // deviations above its mean.
+    // Whole FP32 steps of polymer boxes, us (sides 24, 32, 40, 48, 56, 64, 72, 80, 96; cells per SM 91,
+    // 216, 421, 728, 1155, 1725, 2456, 3368, 5821): 5x8x8 31.9, 48.7, 51.3, 90.3, 95.2, 139.7, 199.1,
+    // 254.7, 414.5; 4x8x10 29.8, 43.8, 51.4, 89.6, 93.4, 133.4, 189.2, 256.5, 414.3; 4x5x8 (480 home
+    // beads, one turn of the block) 28.0, 31.0, 53.1, 63.0, 103.2, 134.4, 196.2, 263.4, 444.7; 4x4x8
+    // 26.1, 29.0, 49.4, 69.3, 105.2, 144.0, 209.7, 279.1, 469.6; 3x4x6 20.9, 35.9, 59.7, 82.3, 132.5,
+    // 185.3, 258.7, 361.3, 591.1 (sides 9 and 16, an earlier kernel: 2x4x4 23.2 and 24.1, 4x4x6 23.7
+    // and 26.0).  Up to two bricks for each block, how they divide into rounds matters more (36^3:
+    // 4x4x8 45.5, 4x6x8 38.9; 40^3: 4x5x8 53.1, 5x6x8 43.2): there another shape is taken where
+    // shape_cost puts it 6% below; above 500 cells per SM the estimate is no better than the table
+    // (45^3: it puts 4x6x8, 67.0, before 4x5x8, 58.8).  From 1,000 on 4x8x10 against 4x5x8 and the
+    // estimate, 20 steps: 56^3 2,412 and 2,216; 56x57x52 2,366 and 2,245; 100x55x41 3,001 and 2,833;
+    // 72x70x73 4,554 and 4,375; 14 boxes of 16 to 24 2,000 and 1,840; but 61x57x55 2,482 and 2,640
+    // (52x50x55, 940 cells per SM: 1,864 and 2,000).  The list kernel keeps the line it was measured
+    // with.  Smaller bricks where the halo of the batch's densest world would not fit the staging
+    // capacity 5 Poisson deviations above its mean.
     template <class Limit> void wide_shape(int shape[3], Limit limit) const
     {
-        static const int table[][3] = {{5, 8, 8}, {4, 5, 8}, {4, 4, 8}, {4, 4, 6}, {2, 4, 4}, {2, 2, 4}, {1, 2, 2}};
+        struct Row {
+            uint64_t from32, from64;  // cells per SM
+            int c[3];
+        };
+        constexpr uint64_t never = ~0ull;
+        static const Row table[] = {{2500, 2500, {5, 8, 8}}, {1000, never, {4, 8, 10}}, {350, 350, {4, 5, 8}}, {110, 110, {4, 4, 8}},
+                                    {never, 40, {4, 4, 6}}, {40, never, {3, 4, 6}}, {0, 0, {2, 4, 4}}, {0, 0, {2, 2, 4}}, {0, 0, {1, 2, 2}}};
         static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
                                        {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
-        static const uint64_t from[] = {2500, 350, 110, 40, 0, 0, 0};  // cells per SM
         auto fits = [&](const int c[3]) {
             const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
             const double mean = max_density * hc;
             return mean + 5.0 * std::sqrt(mean) <= (double)limit(hc);
         };
         const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
+        const int last = (int)(sizeof table / sizeof table[0]) - 1;
         int k = 0;
-        while (per_sm < from[k]) k++;
-        while (k < 6 && !fits(table[k])) k++;
-        const int *best = table[k];
+        while (per_sm < (fp64() ? table[k].from64 : table[k].from32)) k++;
+        while (k < last && !fits(table[k].c)) k++;
+        const int *best = table[k].c;
         double cost = 0.94 * shape_cost(best);
         for (const auto &c : other)
-            if (k < 5 && fits(c) && shape_cost(c) < cost) {
+            if (k < last - 1 && (fp64() || per_sm < 500) && fits(c) && shape_cost(c) < cost) {
                 best = c;
                 cost = shape_cost(c);
             }
