@@ -590,10 +590,9 @@ struct pdpd_engine {
 
     // Brick shape of the kernels with three lanes per home bead, for the smallest batches: one brick
     // and one turn (160 beads) for each resident block (FP32 one per SM, FP64 two), and terms that
-    // fit FP32's pool.  There a step is the
-    // latency of one warp's way through the force pass, and the lanes cut its walk and evaluation
-    // to a third; with more bricks than SMs they only add to the instructions.  Steps of water
-    // boxes, us, one lane and three: 4^3 13.7 and 10.5, 9^3 13.7 and 10.6, 12^3 15.2 and 12.2, 16^3
+    // fit FP32's pool.  There a step is the latency of one warp's way through the force pass, and
+    // the lanes cut its walk and evaluation to a third; with more bricks they only add to the
+    // instructions.  Steps of water boxes, us, one lane and three: 4^3 13.7 and 10.5, 9^3 13.7 and 10.6, 12^3 15.2 and 12.2, 16^3
     // 16.9 and 15.1, 18^3 18.7 and 16.3; 20^3 (two turns) 20.7 and 21.3, 24^3 24.8 and 22.7.  The
     // smallest shape that keeps to one brick per SM is the best or within 2% (9^3: 1x2x4 10.6, 2x3x4
     // 11.4, 4x4x6 12.6; 12^3: 1x2x4 17.6, 2x2x4 12.2, 2x4x4 13.4; 16^3: 2x3x4 21.3, 2x4x4 15.1, 3x4x4
