@@ -34,7 +34,7 @@ __device__ __forceinline__ void step_kernel_begin()
 }
 
 template <class... P, class... A>
-inline void launch_step_kernel(void (*k)(P...), uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t s, A... args)
+inline cudaError_t launch_step_kernel(void (*k)(P...), uint32_t grid, uint32_t block, uint32_t smem, cudaStream_t s, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
@@ -46,7 +46,23 @@ inline void launch_step_kernel(void (*k)(P...), uint32_t grid, uint32_t block, u
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, P(args)...);  // (an error is seen by the caller's cudaGetLastError)
+    return cudaLaunchKernelEx(&cfg, k, P(args)...);  // (an error is also seen by the caller's cudaGetLastError)
+}
+
+// Opt a kernel in to all the dynamic shared memory that a block may have on the current device.  The
+// limit belongs to the kernel, for every engine of the process: set to the need of one batch,
+// it would refuse the launches of another engine whose batch needs more.  What a launch takes
+// (and its occupancy) follows from the bytes it names, not from the limit.
+inline cudaError_t allow_dynamic_smem(const void *k)
+{
+    int dev = 0, most = 0;
+    cudaFuncAttributes at{};
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    return e;
 }
 
 // riscv_mix64_m2 (reference include/dpd/core/hash.hpp:20-30), full 64-bit form.

@@ -900,7 +900,7 @@ bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t n
            (int)brick_layout(hc_max, maxb, npair, BRICK_THREADS_WIDE, 0, 3).bytes <= most;
 }
 
-// Set up the brick kernel for a brick shape: opt in to the shared memory it needs and
+// Set up the brick kernel for a brick shape: opt in to large shared memory and
 // return its persistent grid (resident blocks x SMs) and dynamic shared-memory bytes.
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max,
                 int planes, int *grid, uint32_t *smem_bytes)
@@ -919,8 +919,8 @@ int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint3
         break;
     default: k0 = k_force32_brick<0, BRICK_THREADS>; k1 = k_force32_brick<1, BRICK_THREADS>; break;
     }
-    cudaError_t e = cudaFuncSetAttribute(k0, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = allow_dynamic_smem((const void *)k0);
+    if (e == cudaSuccess) e = allow_dynamic_smem((const void *)k1);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k0, (int)brick_variant_threads(variant), bytes);
     if (e != cudaSuccess) return (int)e;

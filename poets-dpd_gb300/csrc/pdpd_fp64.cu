@@ -747,7 +747,10 @@ int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
         const uint32_t bb = (a.n_bonds + BOND64_CHUNK - 1) / BOND64_CHUNK;
         const uint32_t work = a.n_bricks + bb + (a.n_angles + BOND64_CHUNK - 1) / BOND64_CHUNK;
         const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, work));
-        launch_step_kernel(a.brick_planes == 3 ? k_list64<3> : k_list64<1>, grid, LIST64_THREADS, L.bytes, s, a, L, bb, work);
+        // (a list that was not made is not read: the error reaches the caller)
+        if (launch_step_kernel(a.brick_planes == 3 ? k_list64<3> : k_list64<1>, grid, LIST64_THREADS, L.bytes, s, a, L,
+                               bb, work) != cudaSuccess)
+            return 0;
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
         launch_step_kernel(k_pairs64, std::min<uint32_t>((uint32_t)a.pair_blocks, std::max(1u, pb)), PAIRS64_THREADS, 0, s, a);
         const uint32_t parts = a.n_tiles * (TILE_BEADS / SUM64_BEADS);
@@ -779,7 +782,7 @@ int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int planes, int *
     const auto k = planes == 3 ? k_list64<3> : k_list64<1>;
     const int bytes = (int)list64_layout(hc_max, maxb).bytes;
     int nb = 0;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    cudaError_t e = allow_dynamic_smem((const void *)k);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, LIST64_THREADS, bytes);
     if (e != cudaSuccess) return (int)e;
     if (nb < 1) return (int)cudaErrorInvalidConfiguration;
