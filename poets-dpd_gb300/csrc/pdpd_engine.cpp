@@ -301,6 +301,9 @@ const ConfigEntry kConfig[] = {
                     "pageable host memory through the host's page tables, as Grace-Blackwell does "
                     "over NVLink-C2C, and the arrays are 8-byte aligned), or through pinned "
                     "staging buffers and DMA (0).  The results are the same."},
+    {"pair_lists", "FP64: each pair evaluated once, through lists (1, default: where there is room for "
+                   "them), or by each of its beads, without (0).  The results are the same.  Applies "
+                   "from the next attach."},
 };
 
 }  // namespace
@@ -324,6 +327,7 @@ struct pdpd_engine {
     int cfg_brick[3] = {BRICK_X, BRICK_Y, BRICK_Z};
     int cfg_autotune = 0;
     int cfg_host_direct = 1;
+    int cfg_pair_lists = 1;
     bool host_access = false;  // the device reaches pageable host memory through the host's page tables
     bool kernel_user = false;  // force_kernel set through the config
     bool brick_user = false;   // a brick_* entry set through the config
@@ -1478,7 +1482,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     // FP64: the pair lists, where they are addressable and there is memory for them (else the
     // force pass runs without: same results, slower)
     List64Room room;
-    bool lists = f64 && nb > 0 && nb < (1u << 25);
+    bool lists = f64 && e->cfg_pair_lists && nb > 0 && nb < (1u << 25);
     for (uint32_t i = 0; lists && i < n_worlds; i++)
         if (ws[i].n_beads) room.add((double)ws[i].n_beads, ws[i].box, wdev[i].asym != 0);
     lists = lists && room.entries < 2e9 && room.pairs < 1e9;
@@ -2095,7 +2099,7 @@ int pdpd_get_config(pdpd_engine *e, uint32_t index, char *name, size_t name_len,
     if (index >= sizeof(kConfig) / sizeof(kConfig[0])) return PDPD_E_INVALID;
     int vals[] = {e->cfg_list_capacity, e->cfg_grid_blocks, e->cfg_graph_steps, e->cfg_use_graphs,
                   e->cfg_force_kernel, e->cfg_brick[0], e->cfg_brick[1], e->cfg_brick[2],
-                  e->cfg_autotune, e->cfg_host_direct};
+                  e->cfg_autotune, e->cfg_host_direct, e->cfg_pair_lists};
     static_assert(sizeof(vals) / sizeof(vals[0]) == sizeof(kConfig) / sizeof(kConfig[0]), "config values");
     if (name && name_len) snprintf(name, name_len, "%s", kConfig[index].name);
     if (desc && desc_len) snprintf(desc, desc_len, "%s", kConfig[index].desc);
@@ -2140,6 +2144,9 @@ int pdpd_set_config(pdpd_engine *e, const char *key, const char *value)
     } else if (k == "host_direct") {
         e->cfg_host_direct = v ? 1 : 0;
         return PDPD_OK;  // no bearing on the captured graphs or the kernels
+    } else if (k == "pair_lists") {
+        e->cfg_pair_lists = v ? 1 : 0;
+        return PDPD_OK;  // (applies from the next attach)
     }
     else return e->fail(PDPD_E_INVALID, "Unknown engine config name '%s'", key);
     e->drop_graph();  // graphs are captured again at the next run
