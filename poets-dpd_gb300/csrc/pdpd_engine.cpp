@@ -617,7 +617,7 @@ struct pdpd_engine {
             const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
             if (max_density * c[0] * c[1] * c[2] > 160) return false;
             const uint32_t maxb = (uint32_t)staging_want(hc) + 2;
-            if (fp64() ? maxb > list64_maxb_limit(hc) : !brick_planes_fit(max_density, hc, maxb, npair)) return false;
+            if (fp64() ? maxb > list64_maxb_limit(hc) : !brick_planes_fit(max_density, hc, maxb, npair, segs())) return false;
             for (int d = 0; d < 3; d++) shape[d] = c[d];
             return true;
         }
@@ -634,7 +634,7 @@ struct pdpd_engine {
         for (const WorldHost &wh : worlds) npair = std::max(npair, wh.dev.n_types * wh.dev.n_types);
         if (cfg_force_kernel == 8 || cfg_force_kernel == 1) {
             if (cfg_force_kernel == 8 && small_shape(cfg_brick, npair)) return;
-            wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0); });
+            wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0, segs()); });
             return;
         }
         // variant 9: the largest of these with at most 256 home cells whose halo fits; variant 6:
@@ -651,7 +651,7 @@ struct pdpd_engine {
                 const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
                 const double mean = max_density * hc;
                 const uint32_t hm = home_want((uint32_t)(c[0] * c[1] * c[2]));
-                if (mean + 5.0 * std::sqrt(mean) <= (double)brick_maxb_limit(v, hc, npair, hm)) {
+                if (mean + 5.0 * std::sqrt(mean) <= (double)brick_maxb_limit(v, hc, npair, hm, segs())) {
                     b = c;
                     break;
                 }
@@ -659,6 +659,8 @@ struct pdpd_engine {
         }
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];
     }
+
+    BrickSegs segs() const { return brick_segs(max_density, args.list_capacity); }
 
     // Staged beads a brick of hc halo cells should have room for: the mean halo population
     // of the densest world + 6 standard deviations (Poisson), at least 1.2x the mean, + 32.
@@ -734,20 +736,21 @@ struct pdpd_engine {
             drop_graph();
             return PDPD_OK;
         }
+        a.segs = segs();
         a.brick_npair = 1;
         for (const WorldHost &wh : worlds) a.brick_npair = std::max(a.brick_npair, wh.dev.n_types * wh.dev.n_types);
         // staged-bead capacity (staging_want) within the variant's limit; a fuller brick takes
         // the (bit-identical) global path
         a.brick_home_max = a.force_kernel == 9 ? home_want((uint32_t)(cfg_brick[0] * cfg_brick[1] * cfg_brick[2])) : 0u;
         const double want = staging_want(a.brick_hc_max);
-        const double limit = (double)brick_maxb_limit(a.force_kernel, a.brick_hc_max, a.brick_npair, a.brick_home_max);
+        const double limit = (double)brick_maxb_limit(a.force_kernel, a.brick_hc_max, a.brick_npair, a.brick_home_max, a.segs);
         a.brick_maxb = (uint32_t)std::min(limit, std::max(64.0, want));
         int grid = 0;
         uint32_t bytes = 0;
         int small[3];
         a.brick_planes = a.force_kernel == 8 && !brick_user && small_shape(small, a.brick_npair) && std::equal(small, small + 3, cfg_brick) ? 3 : 1;
         int rc = brick_setup(sm_count, a.force_kernel, a.brick_hc_max, a.brick_maxb, a.brick_npair,
-                             a.brick_home_max, a.brick_planes, &grid, &bytes);
+                             a.brick_home_max, a.brick_planes, a.segs, &grid, &bytes);
         if (rc)
             return fail(PDPD_E_CUDA, "brick kernel setup (%u bytes of shared memory): %s", bytes,
                         cudaGetErrorString((cudaError_t)rc));

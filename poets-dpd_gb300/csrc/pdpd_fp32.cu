@@ -872,7 +872,7 @@ int launch_begin32(const KArgs &a, cudaStream_t s)
 
 // Largest staged-bead capacity of a brick for a force variant: what leaves room for two
 // blocks per SM (variants 8 and 9), within the 16-bit staged indices of the list entries.
-uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max)
+uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max, BrickSegs segs)
 {
     if (variant != 8 && variant != 9) return 2046u;  // variant 6: its bricks stay far below
     int dev = 0, smem_sm = 0;
@@ -880,16 +880,30 @@ uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess)
         return 2046u;
     const uint32_t hm = variant == 9 ? home_max : 0u;
-    const BrickLayout L = brick_layout(hc_max, 0, npair, brick_variant_threads(variant), hm);
+    const BrickLayout L = brick_layout(hc_max, 0, npair, brick_variant_threads(variant), hm, 1, segs);
     const int per_bead = (int)(variant == 9 ? HALF_BEAD_BYTES : FULL_BEAD_BYTES);
     const int budget = smem_sm / 2 - 1024 - (int)L.bytes - 128;  // (each part is rounded up to 16 bytes)
     const int most = variant == 9 ? 65535 : (int)FULL_MAX_STAGED;
     return (uint32_t)std::max(64, std::min(most, budget / per_bead)) & ~1u;
 }
 
+// A bead of a box of this density meets about 3 density candidates in a neighbour row: SEG_BEADS to a
+// segment, with two Poisson deviations.
+BrickSegs brick_segs(double density, int list_capacity)
+{
+    const double row = 3 * density;
+    const int per_row = std::max(1, (int)std::ceil((row + 2 * std::sqrt(row)) / SEG_BEADS));
+    BrickSegs s{SEG_MIN, 3 * per_row};
+    if (density > 4) s.cap = 9 * per_row <= 28 ? 9 * per_row : 3 * per_row + 1;
+    if (list_capacity > 0) s.cap = list_capacity;
+    s.cap = std::min(SEG_MAX, std::max(3, s.cap));
+    s.spare = std::min(s.spare, s.cap);
+    return s;
+}
+
 // Three lanes per home bead: the bead's terms fit the pool (5 Poisson deviations above the mean of
 // the densest world) and the block's shared memory the SM.
-bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair)
+bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair, BrickSegs segs)
 {
     int dev = 0, most = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -897,27 +911,34 @@ bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t n
         return false;
     const double near = 4.19 * density;
     return near + 5 * std::sqrt(near) <= POOL_TERMS &&
-           (int)brick_layout(hc_max, maxb, npair, BRICK_THREADS_WIDE, 0, 3).bytes <= most;
+           (int)brick_layout(hc_max, maxb, npair, BRICK_THREADS_WIDE, 0, 3, segs).bytes <= most;
+}
+
+// Variant 8's kernel.
+template <int FINAL> static auto wide_kernel(int planes, BrickSegs segs)
+{
+    if (planes == 3) return k_force32_brick<FINAL, BRICK_THREADS_WIDE, 3>;
+    return segs.cap > SEG_MIN ? k_force32_brick<FINAL, BRICK_THREADS_WIDE, 1, true> : k_force32_brick<FINAL, BRICK_THREADS_WIDE>;
 }
 
 // Set up the brick kernel for a brick shape: opt in to large shared memory and
 // return its persistent grid (resident blocks x SMs) and dynamic shared-memory bytes.
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max,
-                int planes, int *grid, uint32_t *smem_bytes)
+                int planes, BrickSegs segs, int *grid, uint32_t *smem_bytes)
 {
     int nb = 0;
     const uint32_t hm = variant == 9 ? home_max : 0u;
-    const BrickLayout L = brick_layout(hc_max, maxb, npair, brick_variant_threads(variant), hm, planes);
+    const BrickLayout L = brick_layout(hc_max, maxb, npair, brick_variant_threads(variant), hm, planes, segs);
     const int bytes = (int)L.bytes;
     void (*k0)(KArgs, BrickLayout) = nullptr;
     void (*k1)(KArgs, BrickLayout) = nullptr;
     switch (variant) {
     case 9: k0 = k_force32_half<0>; k1 = k_force32_half<1>; break;
     case 8:
-        k0 = planes == 3 ? k_force32_brick<0, BRICK_THREADS_WIDE, 3> : k_force32_brick<0, BRICK_THREADS_WIDE>;
-        k1 = planes == 3 ? k_force32_brick<1, BRICK_THREADS_WIDE, 3> : k_force32_brick<1, BRICK_THREADS_WIDE>;
+        k0 = wide_kernel<0>(planes, segs);
+        k1 = wide_kernel<1>(planes, segs);
         break;
-    default: k0 = k_force32_brick<0, BRICK_THREADS>; k1 = k_force32_brick<1, BRICK_THREADS>; break;
+    default: k0 = k_force32_brick<0, BRICK_THREADS, 1, true>; k1 = k_force32_brick<1, BRICK_THREADS, 1, true>; break;
     }
     cudaError_t e = allow_dynamic_smem((const void *)k0);
     if (e == cudaSuccess) e = allow_dynamic_smem((const void *)k1);
@@ -951,18 +972,13 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
     if (a.force_kernel != 1 && a.n_bricks > 0) {
         const int v = a.force_kernel;
         const BrickLayout L = brick_layout(a.brick_hc_max, a.brick_maxb, a.brick_npair, brick_variant_threads(v),
-                                           v == 9 ? a.brick_home_max : 0u, a.brick_planes);
+                                           v == 9 ? a.brick_home_max : 0u, a.brick_planes, a.segs);
         const int grid = (int)std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, a.n_bricks));
         void (*k)(KArgs, BrickLayout);
         switch (v) {
         case 9: k = final_step ? k_force32_half<1> : k_force32_half<0>; break;
-        case 8:
-            if (a.brick_planes == 3)
-                k = final_step ? k_force32_brick<1, BRICK_THREADS_WIDE, 3> : k_force32_brick<0, BRICK_THREADS_WIDE, 3>;
-            else
-                k = final_step ? k_force32_brick<1, BRICK_THREADS_WIDE> : k_force32_brick<0, BRICK_THREADS_WIDE>;
-            break;
-        default: k = final_step ? k_force32_brick<1, BRICK_THREADS> : k_force32_brick<0, BRICK_THREADS>; break;
+        case 8: k = final_step ? wide_kernel<1>(a.brick_planes, a.segs) : wide_kernel<0>(a.brick_planes, a.segs); break;
+        default: k = final_step ? k_force32_brick<1, BRICK_THREADS, 1, true> : k_force32_brick<0, BRICK_THREADS, 1, true>; break;
         }
         launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), L.bytes, s, a, L);
         return 1;

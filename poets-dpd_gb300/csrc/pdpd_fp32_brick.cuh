@@ -65,7 +65,7 @@ __device__ __forceinline__ uint32_t brick_fetch(const KArgs &a, BrickHeader &H)
 //   Full shell (variants 6 and 8): header, pair table, hstart[rows][HZ + 1] (16 bits), hslot[HC],
 //   then per staged bead, beads in pairs (2k, 2k + 1): xy = {x, x', y, y'} per pair, zf = the
 //   bead's z in brick coordinates, vel = {v, hash}, zc = {z offset, halo cell}; then
-//   seg[SEG_MAX][threads].
+//   seg[seg_cap + 1][threads].
 //   Half shell: header, pair table, hstart[HC+1], hslot[HC], hlo[HC], pos[maxb], vel[maxb],
 //   list[cap][threads], hidx[maxb] (home index of a staged bead, NOT_HOME for a halo bead),
 //   hsi[home_max] (staged index of a home bead) and acc[6][home_max] (fixed-point force sums of
@@ -73,6 +73,7 @@ __device__ __forceinline__ uint32_t brick_fetch(const KArgs &a, BrickHeader &H)
 //   that 32-bit atomics add them exactly).
 struct BrickLayout {
     uint32_t hc_max, maxb, home_max;
+    int seg_cap, seg_spare;  // full shell: walk segments per thread, and of a plane of rows
     uint32_t off_pair, off_hstart, off_hslot, off_hlo, off_pos, off_vel, off_list, off_hidx, off_hsi,
         off_acc, off_zf, off_zc, off_pool, bytes;
 };
@@ -88,9 +89,11 @@ constexpr uint32_t FULL_BEAD_BYTES = 36, HALF_BEAD_BYTES = 34;
 // npair: the largest n_types^2 of the attached worlds (the staged pair table); home_max: the
 // home-bead capacity of the half-shell variant (0 for the full-shell variants).
 __host__ __device__ inline BrickLayout brick_layout(uint32_t hc_max, uint32_t maxb, uint32_t npair,
-                                                    uint32_t threads, uint32_t home_max, int planes = 1)
+                                                    uint32_t threads, uint32_t home_max, int planes, BrickSegs segs)
 {
     BrickLayout L{};
+    L.seg_cap = segs.cap;
+    L.seg_spare = segs.spare;
     L.hc_max = hc_max;
     L.maxb = maxb;
     L.home_max = home_max;
@@ -120,7 +123,7 @@ __host__ __device__ inline BrickLayout brick_layout(uint32_t hc_max, uint32_t ma
         L.off_zf = take(4 * maxb);
         L.off_vel = take(16 * maxb);
         L.off_zc = take(8 * maxb);
-        L.off_list = take(4 * (SEG_MAX + 1) * threads);
+        L.off_list = take(4 * (uint32_t)(segs.cap + 1) * threads);
         if (planes == 3) L.off_pool = take(16 * POOL_TERMS * (threads / 32) * POOL_WARP_BEADS);
     }
     L.bytes = off;
@@ -337,13 +340,13 @@ __device__ __noinline__ float3 segs_eval_call(Staged st, const uint32_t *segs, i
 
 // Full-shell pair forces of one staged home bead (variants 6 and 8), at staged index si: the
 // walk's segments (pdpd_walk.cuh) evaluated in order.
-template <int T>
-__device__ __forceinline__ void rows_forces(const Staged &st, uint32_t *__restrict__ segs, int cap,
-                                            const uint16_t *__restrict__ hstart, int HY, int HZ1, uint32_t code,
+template <int T, bool TOGETHER = false>
+__device__ __forceinline__ void rows_forces(const Staged &st, uint32_t *__restrict__ segs, int cap, const uint16_t *__restrict__ hstart, int HY, int HZ1, uint32_t code,
                                             uint32_t si, const float4 pi, const float4 vi, const float2 *pair,
-                                            uint32_t nt, uint32_t th_lo, uint32_t th_hi, float scale, float F[3])
+                                            uint32_t nt, uint32_t th_lo, uint32_t th_hi, float scale, float F[3],
+                                            int spare = 3, uint32_t lanes = 0u)
 {
-    const int left = walk_rows<T>(st.xy, st.zf, segs, cap, hstart, HY, HZ1, code, si, pi.x, pi.y, pi.z,
+    const int left = walk_rows<T, 1, TOGETHER>(st.xy, st.zf, segs, cap, hstart, HY, HZ1, code, si, pi.x, pi.y, pi.z,
                                   [&](int n_cand) {
                                       const float3 G = segs_eval_call<T>(st, segs, n_cand, pi, vi, code, pair, nt,
                                                                          th_lo, th_hi, scale,
@@ -351,7 +354,7 @@ __device__ __forceinline__ void rows_forces(const Staged &st, uint32_t *__restri
                                       F[0] = G.x;
                                       F[1] = G.y;
                                       F[2] = G.z;
-                                  });
+                                  }, 0, lanes, spare);
     segs_eval<T>(st, segs, left, pi, vi, code, pair, nt, th_lo, th_hi, scale, F);
 }
 
@@ -447,7 +450,9 @@ __device__ __forceinline__ void brick_fallback_bead(const KArgs &a, const WorldD
 }
 
 // Full-shell brick kernel (variants 6 and 8): one thread per home bead, or three lanes (PLANES = 3).
-template <int FINAL, int T, int PLANES = 1>
+// DENSE: the lanes of a warp flush their segments together (walk_rows); in boxes whose beads keep all
+// of theirs the votes would cost 1% of the pass.
+template <int FINAL, int T, int PLANES = 1, bool DENSE = false>
 __global__ void __launch_bounds__(T, PLANES == 3 ? 1 : T == BRICK_THREADS_WIDE ? 2 : 6) k_force32_brick(KArgs a, BrickLayout lay)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -462,7 +467,7 @@ __global__ void __launch_bounds__(T, PLANES == 3 ? 1 : T == BRICK_THREADS_WIDE ?
     float2 *zc = reinterpret_cast<float2 *>(smem_raw + lay.off_zc);
     const int tid = threadIdx.x;
     uint32_t *segs = reinterpret_cast<uint32_t *>(smem_raw + lay.off_list) + tid;
-    const int cap = (a.list_capacity > 0 && a.list_capacity < SEG_MAX) ? max(3, a.list_capacity) : SEG_MAX;
+    const int cap = DENSE ? lay.seg_cap : (a.list_capacity > 0 && a.list_capacity < SEG_MIN) ? max(3, a.list_capacity) : SEG_MIN;
     const Staged st{reinterpret_cast<const ulonglong2 *>(xy), reinterpret_cast<const uint64_t *>(zf), svel, zc};
     if (tid == 0) H.wc.world = 0xffffffffu;
     __syncthreads();
@@ -521,6 +526,7 @@ __global__ void __launch_bounds__(T, PLANES == 3 ? 1 : T == BRICK_THREADS_WIDE ?
             const bool act = t < n_home && (PLANES == 1 || lane < 30u);
             if (PLANES == 3) t = min(t, n_home - 1u);  // (all lanes stay for the shuffles)
             const int r = home_row_near(H.home_rows, br.bx * br.by, t0, t);
+            const uint32_t lanes = DENSE ? __ballot_sync(0xffffffffu, act) : 0u;
             if (PLANES == 1 && !act) continue;
             const int row = H.halo_row[r];
             const uint32_t k = t - H.home_rows[r];
@@ -539,6 +545,9 @@ __global__ void __launch_bounds__(T, PLANES == 3 ? 1 : T == BRICK_THREADS_WIDE ?
             if constexpr (PLANES == 3)
                 planes_forces<T>(st, segs, cap, hstart, HY, HZ + 1, code, si, pi, vi, spair, nt, th_lo, th_hi, scale,
                                  act, plane, reinterpret_cast<float4 *>(smem_raw + lay.off_pool) + (tid >> 5) * WARP_BEADS + lane / 3u, F);
+            else if constexpr (DENSE)
+                rows_forces<T, true>(st, segs, cap, hstart, HY, HZ + 1, code, si, pi, vi, spair, nt, th_lo, th_hi, scale, F,
+                                     lay.seg_spare, lanes);
             else
                 rows_forces<T>(st, segs, cap, hstart, HY, HZ + 1, code, si, pi, vi, spair, nt, th_lo, th_hi, scale, F);
             if (PLANES == 3 && !(act && plane == 0)) continue;

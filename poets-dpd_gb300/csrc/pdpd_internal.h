@@ -58,6 +58,12 @@ struct Brick {
     uint32_t pad;
 };
 
+// Walk segments (pdpd_walk.cuh) a thread of the FP32 full-shell kernels keeps, and how many of them
+// a plane of three neighbour rows should find free.
+struct BrickSegs {
+    int cap, spare;
+};
+
 // Default brick shape (cells), the autotuner's usual pick on GB300; bx * by <= 64.
 constexpr int BRICK_X = 4, BRICK_Y = 8, BRICK_Z = 8;
 
@@ -145,6 +151,7 @@ struct KArgs {
     uint32_t brick_hc_max;  // halo cells of the nominal brick shape
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds
+    BrickSegs segs;         // variants 6 and 8
     int brick_planes;       // variant 8, FP64 lists: lanes per home bead (3 in small batches, else 1)
     uint32_t brick_home_max;  // half shell: home-bead capacity of one brick
     uint32_t *brick_next;   // the brick queue's next free entry beyond the first gridDim.x
@@ -264,10 +271,12 @@ int launch_rng_eval(size_t n, const uint32_t *t, const uint64_t *seed, const uin
 size_t payload_bytes(int fp64);  // bytes of one pos / vel / frc element
 // Largest staged-bead capacity of a brick for force variant `variant` (two blocks per SM of
 // shared memory for variants 8 and 9, the list entries' range for 6).
-uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max);
-bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair);
+uint32_t brick_maxb_limit(int variant, uint32_t hc_max, uint32_t npair, uint32_t home_max, BrickSegs segs);
+bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t npair, BrickSegs segs);
+// The segments for a box of this density (list_capacity: the config entry, 0 = automatic).
+BrickSegs brick_segs(double density, int list_capacity);
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max, int planes,
-                int *grid, uint32_t *smem_bytes);  // 0 or a cudaError_t
+                BrickSegs segs, int *grid, uint32_t *smem_bytes);  // 0 or a cudaError_t
 uint32_t scan_blocks(uint32_t n_cells);
 
 // Observables of one world (pdpd_observe.cu): per-block FP64 partial sums.

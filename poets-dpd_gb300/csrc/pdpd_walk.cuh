@@ -7,7 +7,7 @@
 namespace pdpd {
 namespace {
 
-constexpr int SEG_MAX = 9;              // walk segments kept per thread (one for each row)
+constexpr int SEG_MIN = 9, SEG_MAX = 40;  // walk segments kept per thread: one for each row, or more in dense boxes
 constexpr float WALK_R2 = 1.0001f;
 constexpr uint32_t SEG_BEADS = 20;      // candidates of one walk segment
 constexpr uint32_t SEG_BASE = 0xfffu;   // low 12 bits of a segment: its first pair
@@ -107,11 +107,17 @@ __device__ __forceinline__ uint32_t walk_mask(const ulonglong2 *sxy, const uint6
 // segs holds cap segments (cap >= 3) with stride T; flush(n) is called with the n candidates of
 // the segments so far when more may not fit, and the walk starts filling them anew.  Returns
 // the candidates left in the segments.  PLANES = 3: only the three rows of dx = plane - 1.
-template <int T, int PLANES = 1, class Flush>
+//
+// TOGETHER: between planes of rows, the lanes of the mask `lanes` (those that walk) flush together
+// as soon as one of them has fewer than `spare` segments left: each on its own, in dense
+// boxes, they would flush at different rows, one after the other (24^3 boxes, step, us, with nine
+// segments each on its own and with brick_segs' number together: density 7 127 and 53, 10 298 and
+// 90, 14 571 and 120, 20 1,089 and 277).
+template <int T, int PLANES = 1, bool TOGETHER = false, class Flush>
 __device__ __forceinline__ int walk_rows(const ulonglong2 *xy, const uint64_t *zf, uint32_t *__restrict__ segs,
                                          int cap, const uint16_t *__restrict__ hstart, int HY, int HZ1,
                                          uint32_t code, uint32_t si, float ox, float oy, float oz, Flush flush,
-                                         int plane = 0)
+                                         int plane = 0, uint32_t lanes = 0u, int spare = 3)
 {
     const int dlo = PLANES == 3 ? plane - 1 : -1, dhi = PLANES == 3 ? plane - 1 : 1;
     const int hx = (int)(code & 255u), hy = (int)((code >> 8) & 255u), hz = (int)((code >> 16) & 255u);
@@ -153,7 +159,7 @@ __device__ __forceinline__ int walk_rows(const ulonglong2 *xy, const uint64_t *z
             }
         }
         h += (HY - 3) * HZ1;
-        if (ddx < dhi && out > full) {
+        if (ddx < dhi && (TOGETHER ? __any_sync(lanes, out > segs + (cap - spare) * T) : out > full)) {
             flush(n_cand);
             out = segs;
             n_cand = 0;

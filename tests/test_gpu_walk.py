@@ -76,3 +76,26 @@ def test_three_lanes_per_bead_equal_the_bead_kernel(box, cfg):
     ref = _run(world, 3, force_kernel=1)
     w = _run(world, 3, **cfg)
     assert np.array_equal(w.x, ref.x) and np.array_equal(w.v, ref.v) and np.array_equal(w.f, ref.f)
+
+
+@pytest.mark.parametrize("list_capacity", [0, 10, 40])
+@pytest.mark.parametrize("force_kernel", [6, 8])
+@pytest.mark.parametrize("density", [4.5, 11, 30])
+def test_dense_boxes_equal_the_bead_kernel(density, force_kernel, list_capacity):
+    """Boxes dense enough for the lanes to keep more segments and flush them together: room for all
+    of a bead's, for a plane of rows, for less; bricks that are staged, and a clump that is not.
+    A list_capacity set later applies from the next attach."""
+    world = W.make_water((7, 9, 8), seed=56, dt=0.0005, density=density, a=0.5)
+    n = world.n_beads // 8
+    world.x[:n] = 2.0 + 2.5 * np.random.default_rng(57).random((n, 3))
+    ref = _run(world, 3, force_kernel=1)
+    w = world.copy()
+    eng = E.GB300DPDEngine("fp32")
+    eng.SetConfigEntry("force_kernel", force_kernel)
+    eng.SetConfigEntry("list_capacity", list_capacity)
+    eng.Attach(w)
+    eng.Run(1)
+    eng.SetConfigEntry("list_capacity", 3)
+    eng.SetConfigEntry("grid_blocks", 50)
+    eng.Run(2)
+    assert np.array_equal(w.x, ref.x) and np.array_equal(w.v, ref.v) and np.array_equal(w.f, ref.f)
