@@ -253,6 +253,23 @@ struct List64Room {
     }
 };
 
+// What the lists save over the force pass without them (k_force64), us a step, for a world of n
+// beads in `cells` cells: the list kernel goes through all cells, at 0.088 ns each; without lists
+// the FP64 work grows with the density, and beyond about 4 beads a cell its candidate lists
+// overflow.  Steps of water boxes, us, with lists and without: 64^3 of density 0.05 54 and 41, 0.1 59
+// and 49, 0.2 65 and 73, 3 833 and 1,771; 90^3, 0.2 149 and 116, 0.25 159 and 133, 0.3 172 and 176;
+// 128^3, 0.05 267 and 89, 0.2 370 and 275, 0.25 405 and 345, 0.3 447 and 466; 160^3, 0.25 775 and 679,
+// 0.3 837 and 878; 24^3, 10 657 and 14,400.
+double lists64_saving_us(double n, double cells)
+{
+    const double rho = n / cells;
+    const double bead_ns = rho > 3 ? 1.2 * std::pow(rho / 3, 3) : std::min(1.2, 1.1 * rho);
+    return 1e-3 * (n * bead_ns - 0.088 * cells);
+}
+// Small batches gain at any density: a bead's walk on global memory is a long chain (32^3 of
+// density 0.005 to 0.1 30 to 33 with lists, 34 to 40 without; 50^3, 0.05 43 and 39).
+constexpr double LISTS64_BASE_US = 12;
+
 uint32_t bucket_room(double density)
 {
     return (uint32_t)std::min(64.0, std::max(8.0, 4 * std::ceil((density + 5.5 * std::sqrt(density) + 3) / 4)));
@@ -301,9 +318,9 @@ const ConfigEntry kConfig[] = {
                     "pageable host memory through the host's page tables, as Grace-Blackwell does "
                     "over NVLink-C2C, and the arrays are 8-byte aligned), or through pinned "
                     "staging buffers and DMA (0).  The results are the same."},
-    {"pair_lists", "FP64: each pair evaluated once, through lists (1, default: where there is room for "
-                   "them), or by each of its beads, without (0).  The results are the same.  Applies "
-                   "from the next attach."},
+    {"pair_lists", "FP64: each pair evaluated once, through lists, or by each of its beads, without (0); "
+                   "1 (default): lists where they pay and there is room for them; 2: wherever there is "
+                   "room.  The results are the same.  Applies from the next attach."},
 };
 
 }  // namespace
@@ -1486,8 +1503,12 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     // force pass runs without: same results, slower)
     List64Room room;
     bool lists = f64 && e->cfg_pair_lists && nb > 0 && nb < (1u << 25);
-    for (uint32_t i = 0; lists && i < n_worlds; i++)
+    double saving = LISTS64_BASE_US;
+    for (uint32_t i = 0; lists && i < n_worlds; i++) {
+        saving += lists64_saving_us((double)ws[i].n_beads, (double)wdev[i].n_cells);
         if (ws[i].n_beads) room.add((double)ws[i].n_beads, ws[i].box, wdev[i].asym != 0);
+    }
+    lists = lists && (saving > 0 || e->cfg_pair_lists == 2);
     lists = lists && room.entries < 2e9 && room.pairs < 1e9;
     if (lists) {
         lists = e->d_lists.alloc(room.bytes(nb)) == cudaSuccess;
@@ -2148,7 +2169,7 @@ int pdpd_set_config(pdpd_engine *e, const char *key, const char *value)
         e->cfg_host_direct = v ? 1 : 0;
         return PDPD_OK;  // no bearing on the captured graphs or the kernels
     } else if (k == "pair_lists") {
-        e->cfg_pair_lists = v ? 1 : 0;
+        e->cfg_pair_lists = (int)std::min(v, 2l);
         return PDPD_OK;  // (applies from the next attach)
     }
     else return e->fail(PDPD_E_INVALID, "Unknown engine config name '%s'", key);

@@ -35,3 +35,12 @@ def test_dense_boxes_fp32(box, density):
     flushed its walk segments on its own."""
     w = [_water(box, density)]
     assert _step_us("fp32", w) < 0.45 * _step_us("fp32", w, force_kernel=1)
+
+
+@pytest.mark.parametrize("box,density", [(64, 0.05), (128, 0.05), (200, 0.01), (128, 0.5), (20, 0.3), (24, 6)])
+def test_sparse_and_dense_boxes_fp64(box, density):
+    """With pair lists and without, whichever is the faster; with lists at any density, 128^3 of
+    density 0.05 took 3 times as long as without."""
+    w = [_water(box, density)]
+    best = min(_step_us("fp64", w, pair_lists=0), _step_us("fp64", w, pair_lists=2))
+    assert _step_us("fp64", w) < 1.25 * best
