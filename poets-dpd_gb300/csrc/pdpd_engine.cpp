@@ -576,38 +576,73 @@ struct pdpd_engine {
     // estimate, 20 steps: 56^3 2,412 and 2,216; 56x57x52 2,366 and 2,245; 100x55x41 3,001 and 2,833;
     // 72x70x73 4,554 and 4,375; 14 boxes of 16 to 24 2,000 and 1,840; but 61x57x55 2,482 and 2,640
     // (52x50x55, 940 cells per SM: 1,864 and 2,000).  The list kernel keeps the line it was measured
-    // with.  Smaller bricks where the halo of the batch's densest world would not fit the staging
-    // capacity 5 Poisson deviations above its mean.
+    // with.
+    struct ShapeRow {
+        uint64_t from32, from64;  // cells per SM
+        int c[3];
+    };
+    static constexpr uint64_t NEVER = ~0ull;
+    static constexpr ShapeRow SHAPES[] = {{2500, 2500, {5, 8, 8}}, {1000, NEVER, {4, 8, 10}}, {350, 350, {4, 5, 8}}, {110, 110, {4, 4, 8}},
+                                          {NEVER, 40, {4, 4, 6}}, {40, NEVER, {3, 4, 6}}, {0, 0, {2, 4, 4}}, {0, 0, {2, 2, 4}}, {0, 0, {1, 2, 2}}};
+    static constexpr int LAST_SHAPE = (int)(sizeof SHAPES / sizeof SHAPES[0]) - 1;
+
+    int shape_row() const
+    {
+        const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
+        int k = 0;
+        while (per_sm < (fp64() ? SHAPES[k].from64 : SHAPES[k].from32)) k++;
+        return k;
+    }
+
+    static uint32_t halo_cells(const int c[3]) { return (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2); }
+
+    // A halo of hc cells fits room for `room` staged beads 5 Poisson deviations above its mean in a
+    // box of density rho.
+    static bool halo_fits(uint32_t hc, double rho, uint32_t room)
+    {
+        const double mean = rho * hc;
+        return mean + 5.0 * std::sqrt(mean) <= (double)room;
+    }
+
     template <class Limit> void wide_shape(int shape[3], Limit limit) const
     {
-        struct Row {
-            uint64_t from32, from64;  // cells per SM
-            int c[3];
-        };
-        constexpr uint64_t never = ~0ull;
-        static const Row table[] = {{2500, 2500, {5, 8, 8}}, {1000, never, {4, 8, 10}}, {350, 350, {4, 5, 8}}, {110, 110, {4, 4, 8}},
-                                    {never, 40, {4, 4, 6}}, {40, never, {3, 4, 6}}, {0, 0, {2, 4, 4}}, {0, 0, {2, 2, 4}}, {0, 0, {1, 2, 2}}};
         static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
                                        {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
-        auto fits = [&](const int c[3]) {
-            const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
-            const double mean = max_density * hc;
-            return mean + 5.0 * std::sqrt(mean) <= (double)limit(hc);
-        };
+        double least = max_density, most = 0;  // the sparsest world, and the densest that the shape fits
+        for (const WorldHost &wh : worlds)
+            if (wh.dev.n_beads) least = std::min(least, density(wh.dev));
         const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
-        const int last = (int)(sizeof table / sizeof table[0]) - 1;
-        int k = 0;
-        while (per_sm < (fp64() ? table[k].from64 : table[k].from32)) k++;
-        while (k < last && !fits(table[k].c)) k++;
-        const int *best = table[k].c;
+        int k = shape_row();
+        while (k < LAST_SHAPE && !halo_fits(halo_cells(SHAPES[k].c), least, limit(halo_cells(SHAPES[k].c)))) k++;
+        const int *best = SHAPES[k].c;
+        const uint32_t room = limit(halo_cells(best));
+        for (const WorldHost &wh : worlds)
+            if (halo_fits(halo_cells(best), density(wh.dev), room)) most = std::max(most, density(wh.dev));
         double cost = 0.94 * shape_cost(best);
         for (const auto &c : other)
-            if (k < last - 1 && (fp64() || per_sm < 500) && fits(c) && shape_cost(c) < cost) {
+            if (k < LAST_SHAPE - 1 && (fp64() || per_sm < 500) && halo_fits(halo_cells(c), most, limit(halo_cells(c))) &&
+                shape_cost(c) < cost) {
                 best = c;
                 cost = shape_cost(c);
             }
         for (int d = 0; d < 3; d++) shape[d] = best[d];
     }
+
+    // The brick shape of a world of density rho in a batch of bricks of `shape`: smaller ones where the
+    // halo would not fit.  (The shape of the densest world for all: a 6^3 box of density 30 beside
+    // a 100^3 one of density 0.1, FP32, step 2,560 us against 158.)
+    template <class Limit> const int *world_shape(const int shape[3], uint32_t room, double rho, Limit limit) const
+    {
+        if (halo_fits(halo_cells(shape), rho, room)) return shape;
+        int k = shape_row();
+        auto fits = [&](const int c[3]) {  // (the launch's layout has room for the largest halo)
+            return halo_fits(halo_cells(c), rho, limit(std::max(halo_cells(shape), halo_cells(c))));
+        };
+        while (k < LAST_SHAPE && !fits(SHAPES[k].c)) k++;
+        return SHAPES[k].c;
+    }
+
+    static double density(const WorldDev &d) { return (double)d.n_beads / ((double)d.L[0] * d.L[1] * d.L[2]); }
 
     // Brick shape of the kernels with three lanes per home bead, for the smallest batches: one brick
     // and one turn (160 beads) for each resident block (FP32 one per SM, FP64 two), and terms that
@@ -633,7 +668,7 @@ struct pdpd_engine {
             if (n > (uint64_t)sm_count * (fp64() ? 2 : 1)) continue;
             const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
             if (max_density * c[0] * c[1] * c[2] > 160) return false;
-            const uint32_t maxb = (uint32_t)staging_want(hc) + 2;
+            const uint32_t maxb = (uint32_t)staging_want(hc, max_density) + 2;
             if (fp64() ? maxb > list64_maxb_limit(hc) : !brick_planes_fit(max_density, hc, maxb, npair, segs())) return false;
             for (int d = 0; d < 3; d++) shape[d] = c[d];
             return true;
@@ -679,11 +714,11 @@ struct pdpd_engine {
 
     BrickSegs segs() const { return brick_segs(max_density, args.list_capacity); }
 
-    // Staged beads a brick of hc halo cells should have room for: the mean halo population
-    // of the densest world + 6 standard deviations (Poisson), at least 1.2x the mean, + 32.
-    double staging_want(uint32_t hc) const
+    // Staged beads a brick of hc halo cells should have room for: its mean halo population
+    // at density rho + 6 standard deviations (Poisson), at least 1.2x the mean, + 32.
+    static double staging_want(uint32_t hc, double rho)
     {
-        const double mean = max_density * hc;
+        const double mean = rho * hc;
         return std::max(mean + 6.0 * std::sqrt(mean), 1.2 * mean) + 32;
     }
 
@@ -711,8 +746,19 @@ struct pdpd_engine {
         int shape[3] = {cfg_brick[0], cfg_brick[1], cfg_brick[2]};
         if (fp64()) {
             a.brick_planes = small_shape(shape, 0) ? 3 : 1;
-            if (a.brick_planes == 1) wide_shape(shape, [](uint32_t hc) { return list64_maxb_limit(hc); });
+            if (a.brick_planes == 1) wide_shape(shape, list64_maxb_limit);
+        } else {
+            int small[3];
+            a.segs = segs();
+            a.brick_npair = 1;
+            for (const WorldHost &wh : worlds) a.brick_npair = std::max(a.brick_npair, wh.dev.n_types * wh.dev.n_types);
+            a.brick_planes = a.force_kernel == 8 && !brick_user && small_shape(small, a.brick_npair) && std::equal(small, small + 3, cfg_brick) ? 3 : 1;
         }
+        auto limit = [&](uint32_t hc) {
+            return fp64() ? list64_maxb_limit(hc) : brick_maxb_limit(8, hc, a.brick_npair, 0, a.segs);
+        };
+        const uint32_t room = limit(halo_cells(shape));
+        const bool per_world = a.brick_planes == 1 && (fp64() || (a.force_kernel == 8 && !brick_user));
         // Each axis of a world is cut into ceil(L / b) bricks of as equal extents as possible
         // (e.g. a side of 9 with b = 4 into 3 + 3 + 3, not 4 + 4 + 1): no extent exceeds the
         // configured one, and no thin remainder brick stages a halo for a few home cells.
@@ -723,9 +769,16 @@ struct pdpd_engine {
             for (int k = 0; k <= n; k++) c.push_back((int)((int64_t)L * k / n));
             return c;
         };
+        uint32_t hc_max = 0;
+        double want = 64;
         for (uint32_t i = 0; i < worlds.size(); i++) {
             const int32_t *L = worlds[i].dev.L;
-            const std::vector<int> cx = cuts(L[0], shape[0]), cy = cuts(L[1], shape[1]), cz = cuts(L[2], shape[2]);
+            const double rho = density(worlds[i].dev);
+            const int *c = per_world ? world_shape(shape, room, rho, limit) : shape;
+            const uint32_t hc = halo_cells(c);
+            hc_max = std::max(hc_max, hc);
+            want = std::max(want, staging_want(hc, rho));
+            const std::vector<int> cx = cuts(L[0], c[0]), cy = cuts(L[1], c[1]), cz = cuts(L[2], c[2]);
             for (size_t a0 = 0; a0 + 1 < cx.size(); a0++)
                 for (size_t a1 = 0; a1 + 1 < cy.size(); a1++)
                     for (size_t a2 = 0; a2 + 1 < cz.size(); a2++)
@@ -743,29 +796,22 @@ struct pdpd_engine {
         if (ce != cudaSuccess) return cuda_fail(ce, "brick table upload");
         a.bricks = d_bricks.as<Brick>();
         a.n_bricks = (uint32_t)bricks.size();
-        a.brick_hc_max = (uint32_t)(shape[0] + 2) * (shape[1] + 2) * (shape[2] + 2);
+        a.brick_hc_max = hc_max;
         if (fp64()) {
-            const double most = (double)list64_maxb_limit(a.brick_hc_max);
-            a.brick_maxb = (uint32_t)std::min(most, std::max(64.0, staging_want(a.brick_hc_max)));
+            a.brick_maxb = (uint32_t)std::min((double)list64_maxb_limit(hc_max), want);
             const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, a.brick_planes, &a.brick_grid);
             if (rc) return fail(PDPD_E_CUDA, "list kernel setup: %s", cudaGetErrorString((cudaError_t)rc));
             if (cfg_grid_blocks > 0) a.brick_grid = cfg_grid_blocks;
             drop_graph();
             return PDPD_OK;
         }
-        a.segs = segs();
-        a.brick_npair = 1;
-        for (const WorldHost &wh : worlds) a.brick_npair = std::max(a.brick_npair, wh.dev.n_types * wh.dev.n_types);
         // staged-bead capacity (staging_want) within the variant's limit; a fuller brick takes
         // the (bit-identical) global path
         a.brick_home_max = a.force_kernel == 9 ? home_want((uint32_t)(cfg_brick[0] * cfg_brick[1] * cfg_brick[2])) : 0u;
-        const double want = staging_want(a.brick_hc_max);
-        const double limit = (double)brick_maxb_limit(a.force_kernel, a.brick_hc_max, a.brick_npair, a.brick_home_max, a.segs);
-        a.brick_maxb = (uint32_t)std::min(limit, std::max(64.0, want));
+        const double most = (double)brick_maxb_limit(a.force_kernel, hc_max, a.brick_npair, a.brick_home_max, a.segs);
+        a.brick_maxb = (uint32_t)std::min(most, want);
         int grid = 0;
         uint32_t bytes = 0;
-        int small[3];
-        a.brick_planes = a.force_kernel == 8 && !brick_user && small_shape(small, a.brick_npair) && std::equal(small, small + 3, cfg_brick) ? 3 : 1;
         int rc = brick_setup(sm_count, a.force_kernel, a.brick_hc_max, a.brick_maxb, a.brick_npair,
                              a.brick_home_max, a.brick_planes, a.segs, &grid, &bytes);
         if (rc)

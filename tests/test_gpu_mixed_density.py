@@ -1,0 +1,44 @@
+"""Batches of worlds of very different densities, whose bricks have different shapes: each world as
+it is alone."""
+
+import numpy as np
+import pytest
+
+import oracle as O
+import pdpd_engine as E
+import pdpd_world as W
+
+pytestmark = pytest.mark.gpu
+
+BATCHES = {
+    "dense_beside_sparse": [((6, 6, 6), 30), ((40, 41, 39), 0.1)],
+    "dense_among_many": [((20, 21, 19), 3), ((9, 8, 10), 14), ((22, 20, 24), 3), ((5, 4, 5), 45), ((20, 20, 20), 3)],
+    "sparse_among_dense": [((12, 11, 12), 12), ((30, 30, 31), 0.02), ((12, 12, 13), 12)],
+    "empty_and_dense": [((5, 6, 5), 20), ((16, 16, 16), 1.0 / 4096), ((2, 2, 2), 60)],
+}
+
+
+@pytest.mark.parametrize("config", [{}, {"force_kernel": 8}, {"brick_x": 3, "brick_y": 4, "brick_z": 5}, {"autotune": 1}])
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+@pytest.mark.parametrize("name", sorted(BATCHES))
+def test_batches_of_mixed_density(name, prec, config):
+    worlds = [W.make_water(box, seed=90 + k, density=rho, a=0.5, dt=0.001) for k, (box, rho) in enumerate(BATCHES[name])]
+    ref = [w.copy() for w in worlds]
+    steps = 40 if "autotune" in config else 3  # (the trials are steps of the run)
+    if prec == "fp64":
+        ref = [O.OracleWorld(w) for w in ref]
+        for o in ref:
+            o.run(steps, nthreads=8)
+    else:
+        for w in ref:
+            eng = E.GB300DPDEngine("fp32")
+            eng.SetConfigEntry("force_kernel", 1)
+            eng.Attach(w)
+            eng.Run(steps)
+    eng = E.GB300DPDEngine(prec)
+    for k, v in config.items():
+        eng.SetConfigEntry(k, v)
+    eng.AttachBatch(worlds)
+    eng.Run(steps)
+    for w, o in zip(worlds, ref):
+        assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
