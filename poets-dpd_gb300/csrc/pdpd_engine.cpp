@@ -689,24 +689,20 @@ struct pdpd_engine {
             wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0, segs()); });
             return;
         }
-        // variant 9: the largest of these with at most 256 home cells whose halo fits; variant 6:
-        // its own shapes below about 1,300 cells per SM, else the largest
+        // variant 9: the largest of these with at most 256 home cells whose halo fits; variant 6: the
+        // first of its own that fits, from 3x4x6 at about 200 cells per SM and more (64^3, step, us:
+        // 3x4x6 174, 2x4x4 189, 4x8x8 274; 5x8x8, whose halo does not fit it, 802)
         const uint64_t per_sm = n_cells / (uint64_t)std::max(1, sm_count);
         static const int big[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {4, 4, 6}, {3, 4, 4}};
-        static const int mid[3] = {3, 4, 6}, small[3] = {2, 4, 4};
-        const int *b = per_sm >= 200 ? mid : small;
-        if (cfg_force_kernel == 9 || per_sm >= 1300) {
-            const int v = cfg_force_kernel == 9 ? 9 : 8;
-            b = big[4];
-            for (const auto &c : big) {
-                if (v == 9 && c[0] * c[1] * c[2] > 256) continue;  // the half shell's home sums
-                const uint32_t hc = (uint32_t)(c[0] + 2) * (c[1] + 2) * (c[2] + 2);
-                const double mean = max_density * hc;
-                const uint32_t hm = home_want((uint32_t)(c[0] * c[1] * c[2]));
-                if (mean + 5.0 * std::sqrt(mean) <= (double)brick_maxb_limit(v, hc, npair, hm, segs())) {
-                    b = c;
-                    break;
-                }
+        static const int narrow[][3] = {{3, 4, 6}, {2, 4, 4}, {2, 2, 4}, {1, 2, 2}};
+        const int *b = cfg_force_kernel == 9 ? big[4] : narrow[3];
+        const int *const from = cfg_force_kernel == 9 ? big[0] : narrow[per_sm >= 200 ? 0 : 1];
+        for (const int *c = from; c != b; c += 3) {
+            if (cfg_force_kernel == 9 && c[0] * c[1] * c[2] > 256) continue;  // the half shell's home sums
+            const uint32_t hm = home_want((uint32_t)(c[0] * c[1] * c[2]));
+            if (halo_fits(halo_cells(c), max_density, brick_maxb_limit(cfg_force_kernel, halo_cells(c), npair, hm, segs()))) {
+                b = c;
+                break;
             }
         }
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];

@@ -53,3 +53,10 @@ def test_a_dense_world_beside_a_large_sparse_one(prec):
     dense, sparse = _water(6, 30, 1), _water(100, 0.1, 2)
     apart = _step_us(prec, [dense]) + _step_us(prec, [sparse])
     assert _step_us(prec, [dense, sparse]) < 1.4 * apart
+
+
+def test_default_shape_of_the_narrow_kernel():
+    """force_kernel 6 against itself on the bricks that suit it; 4.5 times as long on the largest, whose
+    halo does not fit its blocks."""
+    w = [_water(64, 3)]
+    assert _step_us("fp32", w, force_kernel=6) < 1.3 * _step_us("fp32", w, force_kernel=6, brick_x=3, brick_y=4, brick_z=6)
