@@ -298,7 +298,7 @@ const ConfigEntry kConfig[] = {
     {"grid_blocks", "Persistent grid size of the tile kernels (0 = 16 blocks per SM)."},
     {"graph_steps", "Timesteps captured per CUDA graph replay (0 = automatic)."},
     {"use_graphs", "Replay captured CUDA graphs (1) or launch kernels directly (0)."},
-    {"force_kernel", "FP32 force kernel (default 8): "
+    {"force_kernel", "FP32 force kernel (default 8, or 6 for many bricks of few beads): "
                      "1 = thread per bead from global memory, "
                      "6 = shared-memory brick, full shell, neighbour rows walked into lists, "
                      "128-thread blocks; 8 = as 6 with 512-thread blocks for larger bricks; "
@@ -676,17 +676,45 @@ struct pdpd_engine {
         return false;
     }
 
+    // More bricks than variant 8's resident blocks, of at most 128 home beads each (a turn of variant
+    // 6's blocks) on average: bricks of tiny worlds, of sparse boxes, or small ones that the config
+    // names.  Most threads of variant 8's blocks would idle.  Steps, us, with 8 and with 6: 600 boxes
+    // of 2^3 31.9 and 22.4, 2,000 of 3^3 100 and 64, 32^3 of density 3 in bricks of 3x3x3 68 and 52; 48^3
+    // of density 0.3 in 4x4x8 38 and 27; but 300 boxes of 3^3 (a brick per block) 22.7 and 26.7, 600 of
+    // 4^3 (192 beads each) 45 and 49.
+    bool few_beads_a_brick(const int shape[3]) const
+    {
+        double n = 0;
+        for (const WorldHost &wh : worlds) {
+            double k = 1;
+            for (int d = 0; d < 3; d++) k *= (wh.dev.L[d] + shape[d] - 1) / shape[d];
+            n += k;
+        }
+        return !fp64() && n > 2.0 * sm_count && n_beads <= 128 * n && max_density <= 4;
+    }
+
     // Default kernel variant and brick shape for the attached batch, where the config does not
-    // name them: the 512-thread row walk.  All of them give the same trajectory.
+    // name them: the 512-thread row walk, or the 128-thread one.  All of them give the same trajectory.
     void default_shape()
     {
         if (!kernel_user) cfg_force_kernel = 8;
-        if (brick_user) return;
+        if (brick_user) {
+            if (!kernel_user && few_beads_a_brick(cfg_brick)) cfg_force_kernel = 6;
+            return;
+        }
         uint32_t npair = 1;
         for (const WorldHost &wh : worlds) npair = std::max(npair, wh.dev.n_types * wh.dev.n_types);
         if (cfg_force_kernel == 8 || cfg_force_kernel == 1) {
             if (cfg_force_kernel == 8 && small_shape(cfg_brick, npair)) return;
             wide_shape(cfg_brick, [&](uint32_t hc) { return brick_maxb_limit(8, hc, npair, 0, segs()); });
+            if (!kernel_user && few_beads_a_brick(cfg_brick)) {
+                cfg_force_kernel = 6;
+                for (int d = 0; d < 3; d++) {  // (no larger than the worlds: small blocks, more of them on an SM)
+                    int most = 1;
+                    for (const WorldHost &wh : worlds) most = std::max(most, wh.dev.L[d]);
+                    cfg_brick[d] = std::min(cfg_brick[d], most);
+                }
+            }
             return;
         }
         // variant 9: the largest of these with at most 256 home cells whose halo fits; variant 6: the
