@@ -970,6 +970,27 @@ __device__ __forceinline__ bool na_pair(const NaParams &p, const double (*pair)[
     return true;
 }
 
+// The cell of bead i.
+__device__ __forceinline__ void na_cell_of(const NaParams &p, const NaScratch *S, uint32_t i, int c[3])
+{
+    const uint32_t key = S->keyrank[i].x, yz = (uint32_t)p.L[1] * (uint32_t)p.L[2];
+    c[0] = (int)(key / yz);
+    c[1] = (int)(key / (uint32_t)p.L[2] % (uint32_t)p.L[1]);
+    c[2] = (int)(key % (uint32_t)p.L[2]);
+}
+
+// The cell in direction d of cell c.
+__device__ __forceinline__ uint32_t na_neighbour(const NaParams &p, const int c[3], const int d[3])
+{
+    int op[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const int raw = c[k] + d[k];
+        op[k] = raw < 0 ? raw + p.L[k] : (raw == p.L[k] ? 0 : raw);
+    }
+    return ((uint32_t)op[0] * (uint32_t)p.L[1] + (uint32_t)op[1]) * (uint32_t)p.L[2] + (uint32_t)op[2];
+}
+
 // Visit the beads of direction (dx, dy, dz)'s cell that can be in range of the bead at offset o in
 // cell c: the conservative FP32 test of the engine's lists (walk_global64).
 template <class Visit>
@@ -979,15 +1000,8 @@ __device__ __forceinline__ void na_cell(const NaParams &p, const NaScratch *S, c
     const int d[3] = {(int)(dir / 9) - 1, (int)(dir / 3 % 3) - 1, (int)(dir % 3) - 1};
     const float gx = slab_gap(o.x, d[0]), gy = slab_gap(o.y, d[1]), gz = slab_gap(o.z, d[2]);
     if (gx * gx + gy * gy + gz * gz >= WALK_R2) return;
-    int op[3];
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        const int raw = c[k] + d[k];
-        op[k] = raw < 0 ? raw + p.L[k] : (raw == p.L[k] ? 0 : raw);
-    }
     const float ax = o.x - (float)d[0], ay = o.y - (float)d[1], az = o.z - (float)d[2];
-    const uint32_t nc = ((uint32_t)op[0] * (uint32_t)p.L[1] + (uint32_t)op[1]) * (uint32_t)p.L[2] + (uint32_t)op[2];
-    const uint32_t k1 = S->start[nc + 1];
+    const uint32_t nc = na_neighbour(p, c, d), k1 = S->start[nc + 1];
     for (uint32_t k = S->start[nc]; k < k1; k++) {
         const float4 q = S->pos[k];
         const float ex = ax - q.x, ey = ay - q.y, ez = az - q.z;
@@ -1002,6 +1016,68 @@ __device__ __forceinline__ void na_cell(const NaParams &p, const NaScratch *S, c
 // a serial chain of FP64 latencies on 48 blocks: 458 us for the 16^3 box against 34 us.
 constexpr int NA_BEADS = 16, NA_LANES = 8, NA_THREADS = NA_BEADS * NA_LANES, NA_ROWS = 9;
 constexpr uint32_t NA_ROW_CAP = 24, NA_TERMS = 512;
+
+// A bead among so many that a row of its candidates does not fit: its eight lanes go through the
+// cells together, in order, eight candidates at a time, and evaluate the candidates so far whenever
+// the bead's list (the room of all its rows) is full.  (By the first lane alone, one pair after
+// the other: 10^3 box of density 20, step 3,530 us against 490; 8^3 of density 60 14,700 and 3,640.)
+// (It reads its bead anew, so that the kernel keeps nothing for it through its other work.)
+__device__ __noinline__ void na_long_bead(const NaParams &p, const double (*pair)[2], const NaScratch *S,
+                                          const double *__restrict__ x, const double *__restrict__ v,
+                                          const uint32_t *__restrict__ hash, uint32_t h, uint32_t th_lo, uint32_t th_hi,
+                                          uint32_t *list, double (*terms)[NA_TERMS], double *__restrict__ f)
+{
+    constexpr uint32_t CAP = NA_ROWS * NA_ROW_CAP, CHUNK = NA_TERMS / NA_BEADS;
+    const int b = threadIdx.x / NA_LANES, sub = threadIdx.x % NA_LANES;
+    const uint32_t shift = threadIdx.x & 31u & ~(NA_LANES - 1u), lanes = ((1u << NA_LANES) - 1u) << shift;
+    const float4 o = S->pos[h];
+    const uint32_t i = __float_as_uint(o.w);
+    int c[3];
+    na_cell_of(p, S, i, c);
+    uint32_t n = 0;
+    double F = 0.0;  // of axis `sub`
+    auto evaluate = [&]() {
+        __syncwarp(lanes);
+        for (uint32_t e0 = 0; e0 < n; e0 += CHUNK) {
+            const uint32_t m = min(n - e0, CHUNK);
+            for (uint32_t e = sub; e < m; e += NA_LANES) {
+                const uint32_t ent = list[e0 + e];
+                double t[3] = {0.0, 0.0, 0.0};
+                na_pair(p, pair, x, v, hash, i, ent & 0xffffu, c, ent >> 16, th_lo, th_hi, t);
+                for (int k = 0; k < 3; k++) terms[k][b * CHUNK + e] = t[k];
+            }
+            __syncwarp(lanes);
+            if (sub < 3)
+                for (uint32_t e = 0; e < m; e++) F = F + terms[sub][b * CHUNK + e];
+            __syncwarp(lanes);
+        }
+        n = 0;
+    };
+    for (uint32_t dir = 0; dir < 27; dir++) {
+        const int d[3] = {(int)(dir / 9) - 1, (int)(dir / 3 % 3) - 1, (int)(dir % 3) - 1};
+        const float gx = slab_gap(o.x, d[0]), gy = slab_gap(o.y, d[1]), gz = slab_gap(o.z, d[2]);
+        if (gx * gx + gy * gy + gz * gz >= WALK_R2) continue;
+        const uint32_t nc = na_neighbour(p, c, d), k1 = S->start[nc + 1];
+        const float ax = o.x - (float)d[0], ay = o.y - (float)d[1], az = o.z - (float)d[2];
+        for (uint32_t k0 = S->start[nc]; k0 < k1; k0 += NA_LANES) {
+            uint32_t j = 0;
+            bool in = false;
+            if (k0 + sub < k1) {
+                const float4 q = S->pos[k0 + sub];
+                const float ex = ax - q.x, ey = ay - q.y, ez = az - q.z;
+                j = __float_as_uint(q.w);
+                in = ex * ex + ey * ey + ez * ez < WALK_R2 && !(j == i && dir == 13);
+            }
+            const uint32_t hits = __ballot_sync(lanes, in) >> shift;
+            if (in) list[n + __popc(hits & ((1u << sub) - 1u))] = j | dir << 16;
+            n += __popc(hits);
+            if (n > CAP - NA_LANES) evaluate();
+        }
+    }
+    evaluate();
+    if (sub < 3) f[3 * i + sub] = F;
+}
+
 __global__ void __launch_bounds__(NA_THREADS) k_na_forces(const __grid_constant__ NaParams p, const NaScratch *S,
                                                           const double *__restrict__ x, const double *__restrict__ v,
                                                           double *__restrict__ f, const uint32_t *__restrict__ hash)
@@ -1028,10 +1104,7 @@ __global__ void __launch_bounds__(NA_THREADS) k_na_forces(const __grid_constant_
     if (act) {
         o = S->pos[h];
         i = __float_as_uint(o.w);
-        const uint32_t key = S->keyrank[i].x, yz = (uint32_t)p.L[1] * (uint32_t)p.L[2];
-        c[0] = (int)(key / yz);
-        c[1] = (int)(key / (uint32_t)p.L[2] % (uint32_t)p.L[1]);
-        c[2] = (int)(key % (uint32_t)p.L[2]);
+        na_cell_of(p, S, i, c);
         if (sub == 0) {
             s_id[b] = i;
             for (int k = 0; k < 3; k++) s_c[b][k] = c[k];
@@ -1091,16 +1164,7 @@ __global__ void __launch_bounds__(NA_THREADS) k_na_forces(const __grid_constant_
         __syncthreads();
     }
     if (axis < 3 && blockIdx.x * NA_BEADS + sb < p.n && !s_long[sb]) f[3 * s_id[sb] + axis] = F;
-    if (sub == 0 && act && s_long[b]) {  // a bead among very many: its pairs one by one
-        double G[3] = {0.0, 0.0, 0.0};
-        for (uint32_t dir = 0; dir < 27; dir++)
-            na_cell(p, S, c, o, dir, [&](uint32_t j) {
-                double t[3];
-                if ((j == i && dir == 13) || !na_pair(p, s_pair, x, v, hash, i, j, c, dir, th_lo, th_hi, t)) return;
-                for (int k = 0; k < 3; k++) G[k] = G[k] + t[k];
-            });
-        for (int k = 0; k < 3; k++) f[3 * i + k] = G[k];
-    }
+    if (h < p.n && s_long[b]) na_long_bead(p, s_pair, S, x, v, hash, h, th_lo, th_hi, s_row[b * NA_ROWS], s_t, f);
 }
 
 // update_mom (dpd_maths_core_half_step.hpp:51-61).

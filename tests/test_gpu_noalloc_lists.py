@@ -48,3 +48,26 @@ def test_noalloc_lists_bit_exact(name):
         E.step_noalloc(w, x.data_ptr(), v.data_ptr(), f.data_ptr(), h.data_ptr(), 2, t=2 * k)
     for a, b in ((x, o.x), (v, o.v), (f, o.f)):
         assert np.array_equal(a.cpu().numpy(), b)
+
+
+def _clump(seed, n_in, edge):
+    w = W.make_water((6, 5, 7), seed=seed, density=4, a=0.3, gamma=0.5, dt=0.0005)
+    w.x[:n_in] = 1.3 + edge * np.random.default_rng(seed).random((n_in, 3))
+    return w
+
+
+# (26 candidates in a row; more than the list holds at once; a whole box of such beads)
+CLUMPS = {"few_long": (88, 60, 1.0), "many_refills": (89, 700, 0.9), "spread": (90, 800, 2.5)}
+
+
+@pytest.mark.parametrize("name", sorted(CLUMPS))
+def test_noalloc_long_beads_beside_others(name):
+    torch = pytest.importorskip("torch")
+    w = _clump(*CLUMPS[name])
+    o = O.OracleWorld(w)
+    o.run(3, nthreads=8)
+    x, v, f = (torch.from_numpy(a.copy()).to("cuda:0") for a in (w.x, w.v, w.f))
+    h = torch.from_numpy(w.hashes().view(np.int32).copy()).to("cuda:0")
+    E.step_noalloc(w, x.data_ptr(), v.data_ptr(), f.data_ptr(), h.data_ptr(), 3, t=0)
+    for a, b in ((x, o.x), (v, o.v), (f, o.f)):
+        assert np.array_equal(a.cpu().numpy(), b)

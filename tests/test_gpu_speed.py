@@ -67,3 +67,20 @@ def test_many_bricks_of_few_beads(side, copies, config):
     """Against force_kernel 6, whose blocks have 128 threads; 1.3 to 1.9 times as long with 512."""
     worlds = [_water(side, 3, k) for k in range(copies)]
     assert _step_us("fp32", worlds, **config) < 1.15 * _step_us("fp32", worlds, force_kernel=6, **config)
+
+
+@pytest.mark.parametrize("box,density", [(10, 20), (8, 60)])
+def test_dense_boxes_noalloc(box, density):
+    """pdpd_step_noalloc against the FP64 engine without pair lists, a thread per bead: 0.05-0.15 of its
+    time; 0.4-0.5 when one lane evaluated all pairs of a bead whose candidates did not fit."""
+    torch = pytest.importorskip("torch")
+    w = _water(box, density)
+    x, v, f = (torch.from_numpy(a.copy()).to("cuda:0") for a in (w.x, w.v, w.f))
+    h = torch.from_numpy(w.hashes().view("int32").copy()).to("cuda:0")
+    best = 1e9
+    for k in range(4):
+        t0 = time.perf_counter()
+        E.step_noalloc(w, x.data_ptr(), v.data_ptr(), f.data_ptr(), h.data_ptr(), 4, t=4 * k)
+        best = min(best, (time.perf_counter() - t0) / 4 * 1e6)
+    none = _step_us("fp64", [w], pair_lists=0)
+    assert best < 0.3 * none
