@@ -21,7 +21,8 @@ struct __align__(16) Vec2d {
 // microseconds, and the gaps between them were a good part of it (9^3 water, 40 steps with the
 // read-back: 1.01 -> 0.77 ms).  The short kernels also let the next one's blocks come up at
 // once; the force kernels do not, as those blocks would take room on the SMs for nothing
-// meanwhile (32^3 polymer box, 100 steps: 3.72 ms without any of this, 3.85 with, 3.54 so).
+// meanwhile (32^3 polymer box, 100 steps: 3.72 ms without any of this, 3.85 with, 3.54 so).  The
+// force kernels of one thread per bead are launched plainly (launch_force64, launch_force32).
 __device__ __forceinline__ void step_kernel_wait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

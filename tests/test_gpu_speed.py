@@ -84,3 +84,12 @@ def test_dense_boxes_noalloc(box, density):
         best = min(best, (time.perf_counter() - t0) / 4 * 1e6)
     none = _step_us("fp64", [w], pair_lists=0)
     assert best < 0.3 * none
+
+
+@pytest.mark.parametrize("side,density", [(24, 3), (16, 8)])
+def test_fp64_force_pass_without_lists_of_few_tiles(side, density):
+    """Per bead, against a box of many more tiles than SMs: 2.7 and 3.1 times as long when the blocks of
+    the small box crowded on a few SMs, 1.8 and 1.4 spread evenly."""
+    small, large = _water(side, density), _water(2 * side, density)
+    per_bead = [_step_us("fp64", [w], pair_lists=0, steps=4) / w.n_beads for w in (small, large)]
+    assert per_bead[0] < 2.25 * per_bead[1]
