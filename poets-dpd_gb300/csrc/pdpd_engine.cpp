@@ -259,12 +259,13 @@ struct List64Room {
 // overflow.  Steps of water boxes, us, with lists and without: 64^3 of density 0.05 54 and 41, 0.1 59
 // and 49, 0.2 65 and 73, 3 833 and 1,771; 90^3, 0.2 149 and 116, 0.25 159 and 133, 0.3 172 and 176;
 // 128^3, 0.05 267 and 89, 0.2 370 and 275, 0.25 405 and 345, 0.3 447 and 466; 160^3, 0.25 775 and 679,
-// 0.3 837 and 878; 24^3, 10 657 and 14,400.
+// 0.3 837 and 878; 24^3, 10 657 and 14,400.  A world costs the list kernel a brick at least, about
+// 120 cells' worth: 2,000 boxes of 2^3 of density 0.25 74 and 59, 0.5 82 and 80, 1 94 and 116.
 double lists64_saving_us(double n, double cells)
 {
     const double rho = n / cells;
     const double bead_ns = rho > 3 ? 1.2 * std::pow(rho / 3, 3) : std::min(1.2, 1.1 * rho);
-    return 1e-3 * (n * bead_ns - 0.088 * cells);
+    return 1e-3 * (n * bead_ns - 0.088 * std::max(cells, 120.0));
 }
 // Small batches gain at any density: a bead's walk on global memory is a long chain (32^3 of
 // density 0.005 to 0.1 30 to 33 with lists, 34 to 40 without; 50^3, 0.05 43 and 39).

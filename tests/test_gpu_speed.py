@@ -46,6 +46,12 @@ def test_sparse_and_dense_boxes_fp64(box, density):
     assert _step_us("fp64", w) < 1.25 * best
 
 
+def test_many_tiny_sparse_worlds_fp64():
+    """Without pair lists, which took 1.3 times as long."""
+    worlds = [_water(2, 0.125, k) for k in range(4000)]
+    assert _step_us("fp64", worlds) < 1.12 * _step_us("fp64", worlds, pair_lists=0)
+
+
 @pytest.mark.parametrize("prec", ["fp32", "fp64"])
 def test_a_dense_world_beside_a_large_sparse_one(prec):
     """Against the two one after the other: about as long; FP32 took 5 times as long when the densest
