@@ -5,6 +5,7 @@
 //   force (finish step t, start step t+1) -> scan x2 -> place -> canon
 // which is captured once per attach into a CUDA graph of G consecutive steps and replayed.
 #include <algorithm>
+#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -18,6 +19,7 @@
 #include <memory>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -521,17 +523,47 @@ struct pdpd_engine {
         return PDPD_OK;
     }
 
+    // The batch's worlds of equal size and bead count together; of more than 32 kinds, 32 that stand
+    // for their neighbours in order of size (an estimate over 600 worlds took longer than the rest
+    // of their attach's host work).
+    struct WorldKind {
+        std::array<int32_t, 3> L;
+        uint32_t n_beads;
+        double count;
+    };
+    std::vector<WorldKind> world_kinds() const
+    {
+        std::vector<WorldKind> all, kinds;
+        auto key = [](const WorldKind &w) { return std::make_tuple((int64_t)w.L[0] * w.L[1] * w.L[2], w.L, w.n_beads); };
+        for (const WorldHost &wh : worlds)
+            all.push_back({{wh.dev.L[0], wh.dev.L[1], wh.dev.L[2]}, wh.dev.n_beads, 1});
+        std::sort(all.begin(), all.end(), [&](const WorldKind &x, const WorldKind &y) { return key(x) < key(y); });
+        for (const WorldKind &w : all)
+            if (!kinds.empty() && key(kinds.back()) == key(w)) kinds.back().count += 1;
+            else kinds.push_back(w);
+        const size_t most = 32, n = kinds.size();
+        if (n <= most) return kinds;
+        std::vector<WorldKind> some;
+        for (size_t k = 0; k < most; k++) {
+            const size_t b = n * k / most, e = n * (k + 1) / most;
+            some.push_back(kinds[(b + e) / 2]);
+            some.back().count = 0;
+            for (size_t i = b; i < e; i++) some.back().count += kinds[i].count;
+        }
+        return some;
+    }
+
     // Estimated time of a pass of the 512-thread brick kernels over the batch cut into bricks of
     // this shape, us: a brick costs 1.8, 6.0 per turn of the block over its home beads (512 of
     // them) and 0.024 per home bead; two blocks per SM take bricks in turn, nearly in step (0.9 of
     // the way to whole rounds), and a block alone on its SM takes 0.66 of that.  Fitted to FP32
     // force passes of 24 water boxes of sides 10 to 96 in 13 shapes each (5.7% rms).
-    double shape_cost(const int shape[3]) const
+    double shape_cost(const int shape[3], const std::vector<WorldKind> &kinds) const
     {
         double total = 0, most = 0, n = 0;
-        for (const WorldHost &wh : worlds) {
-            const int32_t *L = wh.dev.L;
-            const double rho = (double)wh.dev.n_beads / std::max(1.0, (double)L[0] * L[1] * L[2]);
+        for (const WorldKind &w : kinds) {
+            const std::array<int32_t, 3> &L = w.L;
+            const double rho = (double)w.n_beads / std::max(1.0, (double)L[0] * L[1] * L[2]);
             int k[3], lo[3], more[3];  // bricks per axis, their smaller extent, how many are one longer
             for (int d = 0; d < 3; d++) {
                 k[d] = (L[d] + shape[d] - 1) / shape[d];
@@ -539,7 +571,7 @@ struct pdpd_engine {
                 more[d] = L[d] - lo[d] * k[d];
             }
             for (int q = 0; q < 8; q++) {
-                double count = 1, cells = 1;
+                double count = w.count, cells = 1;
                 for (int d = 0; d < 3; d++) {
                     const bool longer = q >> d & 1;
                     count *= longer ? more[d] : k[d] - more[d];
@@ -548,7 +580,12 @@ struct pdpd_engine {
                 if (count == 0) continue;
                 const double beads = rho * cells;
                 double turns = 1;  // expected: Poisson home beads
-                for (int t = 1; t <= 4; t++) turns += 0.5 * std::erfc((512.0 * t - beads) / std::sqrt(2 * beads + 1e-9));
+                const double width = std::sqrt(2 * beads + 1e-9);
+                for (int t = 1; t <= 4; t++) {
+                    const double z = (512.0 * t - beads) / width;
+                    if (z > 4) break;  // (below 1e-8, and the next ones)
+                    turns += z < -4 ? 1.0 : 0.5 * std::erfc(z);
+                }
                 const double c = 1.8 + 0.024 * beads + 6.0 * turns;
                 total += count * c;
                 most = std::max(most, c);
@@ -619,13 +656,17 @@ struct pdpd_engine {
         const uint32_t room = limit(halo_cells(best));
         for (const WorldHost &wh : worlds)
             if (halo_fits(halo_cells(best), density(wh.dev), room)) most = std::max(most, density(wh.dev));
-        double cost = 0.94 * shape_cost(best);
-        for (const auto &c : other)
-            if (k < LAST_SHAPE - 1 && (fp64() || per_sm < 500) && halo_fits(halo_cells(c), most, limit(halo_cells(c))) &&
-                shape_cost(c) < cost) {
-                best = c;
-                cost = shape_cost(c);
+        if (k < LAST_SHAPE - 1 && (fp64() || per_sm < 500)) {
+            const std::vector<WorldKind> kinds = world_kinds();
+            double cost = 0.94 * shape_cost(best, kinds);
+            for (const auto &c : other) {
+                const double t = halo_fits(halo_cells(c), most, limit(halo_cells(c))) ? shape_cost(c, kinds) : cost;
+                if (t < cost) {
+                    best = c;
+                    cost = t;
+                }
             }
+        }
         for (int d = 0; d < 3; d++) shape[d] = best[d];
     }
 
@@ -698,6 +739,7 @@ struct pdpd_engine {
     // name them: the 512-thread row walk, or the 128-thread one.  All of them give the same trajectory.
     void default_shape()
     {
+        if (fp64()) return;  // (no entries of the config for its bricks)
         if (!kernel_user) cfg_force_kernel = 8;
         if (brick_user) {
             if (!kernel_user && few_beads_a_brick(cfg_brick)) cfg_force_kernel = 6;
