@@ -50,19 +50,16 @@ inline cudaError_t launch_step_kernel(void (*k)(P...), uint32_t grid, uint32_t b
     return cudaLaunchKernelEx(&cfg, k, P(args)...);  // (an error is also seen by the caller's cudaGetLastError)
 }
 
-// Opt a kernel in to all the dynamic shared memory that a block may have on the current device.  The
-// limit belongs to the kernel, for every engine of the process: set to the need of one batch,
-// it would refuse the launches of another engine whose batch needs more.  What a launch takes
-// (and its occupancy) follows from the bytes it names, not from the limit.
+// Opt a kernel without static shared memory in to all the dynamic shared memory that a block may have
+// on the current device.  The limit belongs to the kernel, for every engine of the process: set to
+// the need of one batch, it would refuse the launches of another engine whose batch needs more.
+// What a launch takes (and its occupancy) follows from the bytes it names, not from the limit.
 inline cudaError_t allow_dynamic_smem(const void *k)
 {
     int dev = 0, most = 0;
-    cudaFuncAttributes at{};
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&at, k);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)at.sharedSizeBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
     return e;
 }
 

@@ -173,7 +173,7 @@ struct KArgs {
 //           final: v(t+1) -> B.vel, f(t+1) -> frc
 //   finish: B.vel -> A.vel and t += 1                           (after a final force pass)
 //   unsort: A rest state -> id-ordered staging (pdpd_hostio.cu)   (download)
-//   sort:   B -> A counting sort (pdpd_sort.cu)
+//   sort:   B -> A counting sort (pdpd_sort.cu); with_force: after a bin (slot = id order, with f)
 int launch_bin32(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
 int launch_begin32(const KArgs &a, cudaStream_t s);
 int launch_force32(const KArgs &a, int final_step, cudaStream_t s);
