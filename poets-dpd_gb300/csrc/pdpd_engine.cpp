@@ -535,11 +535,14 @@ struct pdpd_engine {
     {
         std::vector<WorldKind> all, kinds;
         auto key = [](const WorldKind &w) { return std::make_tuple((int64_t)w.L[0] * w.L[1] * w.L[2], w.L, w.n_beads); };
-        for (const WorldHost &wh : worlds)
-            all.push_back({{wh.dev.L[0], wh.dev.L[1], wh.dev.L[2]}, wh.dev.n_beads, 1});
+        for (const WorldHost &wh : worlds) {  // (runs of equal worlds first: there is less to sort)
+            const WorldKind w{{wh.dev.L[0], wh.dev.L[1], wh.dev.L[2]}, wh.dev.n_beads, 1};
+            if (!all.empty() && all.back().L == w.L && all.back().n_beads == w.n_beads) all.back().count += 1;
+            else all.push_back(w);
+        }
         std::sort(all.begin(), all.end(), [&](const WorldKind &x, const WorldKind &y) { return key(x) < key(y); });
         for (const WorldKind &w : all)
-            if (!kinds.empty() && key(kinds.back()) == key(w)) kinds.back().count += 1;
+            if (!kinds.empty() && key(kinds.back()) == key(w)) kinds.back().count += w.count;
             else kinds.push_back(w);
         const size_t most = 32, n = kinds.size();
         if (n <= most) return kinds;
@@ -700,6 +703,7 @@ struct pdpd_engine {
     bool small_shape(int shape[3], uint32_t npair) const
     {
         static const int table[][3] = {{1, 2, 4}, {2, 2, 4}, {2, 3, 4}, {2, 4, 4}, {3, 3, 4}, {3, 4, 4}};
+        if (worlds.size() > (size_t)sm_count * (fp64() ? 2 : 1)) return false;
         for (const auto &c : table) {
             uint64_t n = 0;
             for (const WorldHost &wh : worlds) {
