@@ -783,6 +783,18 @@ struct pdpd_engine {
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];
     }
 
+    // Shared memory with which a block is alone on its SM.  The blocks of a brick kernel come up while
+    // the cell-list kernel drains, two of them on the SMs that are free first: a batch of no more
+    // bricks than SMs asks for half an SM's memory, so that each brick gets an SM (steps, us,
+    // without and with: 22^3 of density 3 27.4 and 22.9, 24^3 28.5 and 24.0, 25^3 31.8 and 25.0; 16^3 of
+    // density 8 37.7 and 29.8; FP64, 25^3 87.3 and 81.8).
+    uint32_t alone_smem() const
+    {
+        int most = 0;
+        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess) return 0;
+        return (uint32_t)most / 2;
+    }
+
     BrickSegs segs() const { return brick_segs(max_density, args.list_capacity); }
 
     // Staged beads a brick of hc halo cells should have room for: its mean halo population
@@ -868,6 +880,7 @@ struct pdpd_engine {
         a.bricks = d_bricks.as<Brick>();
         a.n_bricks = (uint32_t)bricks.size();
         a.brick_hc_max = hc_max;
+        a.brick_smem = bricks.size() <= (size_t)sm_count ? alone_smem() : 0u;
         if (fp64()) {
             a.brick_maxb = (uint32_t)std::min((double)list64_maxb_limit(hc_max), want);
             const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, a.brick_planes, &a.brick_grid);

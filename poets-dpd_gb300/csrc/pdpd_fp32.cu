@@ -979,7 +979,7 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
         case 8: k = final_step ? wide_kernel<1>(a.brick_planes, a.segs) : wide_kernel<0>(a.brick_planes, a.segs); break;
         default: k = final_step ? k_force32_brick<1, BRICK_THREADS, 1, true> : k_force32_brick<0, BRICK_THREADS, 1, true>; break;
         }
-        launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), L.bytes, s, a, L);
+        launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), std::max(L.bytes, a.brick_smem), s, a, L);
         return 1;
     }
     // Launched when the kernel in front has finished, as k_force64: its blocks spread evenly over the SMs

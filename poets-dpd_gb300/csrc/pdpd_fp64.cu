@@ -747,7 +747,8 @@ int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
         const uint32_t work = a.n_bricks + bb + (a.n_angles + BOND64_CHUNK - 1) / BOND64_CHUNK;
         const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, work));
         // (a list that was not made is not read: the error reaches the caller)
-        if (launch_step_kernel(a.brick_planes == 3 ? k_list64<3> : k_list64<1>, grid, LIST64_THREADS, L.bytes, s, a, L,
+        if (launch_step_kernel(a.brick_planes == 3 ? k_list64<3> : k_list64<1>, grid, LIST64_THREADS,
+                               std::max(L.bytes, a.brick_smem), s, a, L,
                                bb, work) != cudaSuccess)
             return 0;
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;

@@ -148,6 +148,7 @@ struct KArgs {
                          // brick), 8 = full-shell brick kernel with 512-thread blocks, 6 = the
                          // same with 128-thread blocks, 1 = thread per bead (global memory)
     int brick_grid;      // persistent grid size of the brick kernel
+    uint32_t brick_smem;    // bytes of shared memory that a brick kernel's launch asks for at least
     uint32_t brick_hc_max;  // halo cells of the nominal brick shape
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds

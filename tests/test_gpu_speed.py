@@ -99,3 +99,10 @@ def test_fp64_force_pass_without_lists_of_few_tiles(side, density):
     small, large = _water(side, density), _water(2 * side, density)
     per_bead = [_step_us("fp64", [w], pair_lists=0, steps=4) / w.n_beads for w in (small, large)]
     assert per_bead[0] < 2.25 * per_bead[1]
+
+
+def test_bricks_of_a_small_batch_spread_over_the_sms():
+    """A brick per SM, against force_kernel 6 on smaller ones: 0.82 of its time, 1.05 with two bricks on
+    some SMs and none on others."""
+    w = [_water(25, 3)]
+    assert _step_us("fp32", w, steps=20) < 0.93 * _step_us("fp32", w, steps=20, force_kernel=6)
