@@ -26,6 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/pdpd_gpu.h"
+#include "pdpd_footprint.hpp"
 #include "pdpd_internal.h"
 
 using namespace pdpd;
@@ -231,52 +232,6 @@ struct WorldHost {
     WorldDev dev;
     std::shared_ptr<V2Layout> v2;
 };
-
-// Room for the FP64 engine's pair lists of a world: candidates and the pairs its beads evaluate
-// themselves (half of those, and both sides of the pairs across the box's faces), at the world's
-// mean density with a margin for its fluctuations.  Beads that find no room are evaluated without
-// lists, with the same result.
-struct List64Room {
-    double entries = 0, pairs = 0;
-    // one buffer: cursors, a record per bead, entries, pairs, terms
-    size_t off_lrec() const { return 256; }
-    size_t off_list(size_t n_beads) const { return off_lrec() + up(8 * n_beads); }
-    size_t off_pairs(size_t n_beads) const { return off_list(n_beads) + up(4 * (size_t)entries); }
-    size_t off_term(size_t n_beads) const { return off_pairs(n_beads) + up(8 * (size_t)pairs); }
-    size_t bytes(size_t n_beads) const { return off_term(n_beads) + up(24 * (size_t)pairs); }
-    static size_t up(size_t n) { return (n + 255) & ~size_t(255); }
-    void add(double n, const int32_t box[3], bool asym)
-    {
-        const double near = 1.3 * 4.19 * n / ((double)box[0] * box[1] * box[2]);
-        double across = 0;
-        for (int k = 0; k < 3; k++) across += 0.375 / box[k];
-        entries += n * (near + 8);
-        pairs += n * (near * (asym ? 1.0 : 0.5 + 0.5 * std::min(1.0, across)) + 5);
-    }
-};
-
-// What the lists save over the force pass without them (k_force64), us a step, for a world of n
-// beads in `cells` cells: the list kernel goes through all cells, at 0.088 ns each; without lists
-// the FP64 work grows with the density, and beyond about 4 beads a cell its candidate lists
-// overflow.  Steps of water boxes, us, with lists and without: 64^3 of density 0.05 54 and 41, 0.1 59
-// and 49, 0.2 65 and 73, 3 833 and 1,771; 90^3, 0.2 149 and 116, 0.25 159 and 133, 0.3 172 and 176;
-// 128^3, 0.05 267 and 89, 0.2 370 and 275, 0.25 405 and 345, 0.3 447 and 466; 160^3, 0.25 775 and 679,
-// 0.3 837 and 878; 24^3, 10 657 and 14,400.  A world costs the list kernel a brick at least, about
-// 120 cells' worth: 2,000 boxes of 2^3 of density 0.25 74 and 59, 0.5 82 and 80, 1 94 and 116.
-double lists64_saving_us(double n, double cells)
-{
-    const double rho = n / cells;
-    const double bead_ns = rho > 3 ? 1.2 * std::pow(rho / 3, 3) : std::min(1.2, 1.1 * rho);
-    return 1e-3 * (n * bead_ns - 0.088 * std::max(cells, 120.0));
-}
-// Small batches gain at any density: a bead's walk on global memory is a long chain (32^3 of
-// density 0.005 to 0.1 30 to 33 with lists, 34 to 40 without; 50^3, 0.05 43 and 39).
-constexpr double LISTS64_BASE_US = 12;
-
-uint32_t bucket_room(double density)
-{
-    return (uint32_t)std::min(64.0, std::max(8.0, 4 * std::ceil((density + 5.5 * std::sqrt(density) + 3) / 4)));
-}
 
 bool asymmetric(const pdpd_world &w)
 {
@@ -1579,9 +1534,10 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
         put(n_bond_par + g, p);
     });
 
-    // Room for the beads of a cell that a rebuild ranks from its bucket: the densest world's mean
-    // and 5.5 Poisson deviations (cells that hold more go through overflow lists).
-    const uint32_t bucket_k = bucket_room(max_density);
+    BatchSize size;
+    for (uint32_t i = 0; i < n_worlds; i++)
+        size.add(ws[i].n_beads, ws[i].box, ws[i].n_bonds, ws[i].n_angles, wdev[i].asym != 0);
+    const uint32_t bucket_k = size.bucket_k();
 
     // --- allocate
     const size_t P = payload_bytes(f64);
@@ -1631,15 +1587,8 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     }
     // FP64: the pair lists, where they are addressable and there is memory for them (else the
     // force pass runs without: same results, slower)
-    List64Room room;
-    bool lists = f64 && e->cfg_pair_lists && nb > 0 && nb < (1u << 25);
-    double saving = LISTS64_BASE_US;
-    for (uint32_t i = 0; lists && i < n_worlds; i++) {
-        saving += lists64_saving_us((double)ws[i].n_beads, (double)wdev[i].n_cells);
-        if (ws[i].n_beads) room.add((double)ws[i].n_beads, ws[i].box, wdev[i].asym != 0);
-    }
-    lists = lists && (saving > 0 || e->cfg_pair_lists == 2);
-    lists = lists && room.entries < 2e9 && room.pairs < 1e9;
+    const List64Room &room = size.room;
+    bool lists = f64 && e->cfg_pair_lists && size.lists_fit() && (size.lists_pay() || e->cfg_pair_lists == 2);
     if (lists) {
         lists = e->d_lists.alloc(room.bytes(nb)) == cudaSuccess;
         if (!lists) cudaGetLastError();
@@ -2770,7 +2719,7 @@ struct ServerJob {
     pdpd_job_fn cb = nullptr;
     void *user = nullptr;
     double t_submit = 0;
-    size_t bytes = 0;
+    BatchSize size;
     int slot = -1;           // world index in the attached batch, -1 before the first attach
     bool stopped = false;    // no further callbacks: the callback asked to stop, or it failed
     bool ended = false;      // final state delivered or owed; the world leaves the batch at the
@@ -2787,19 +2736,11 @@ struct Delivery {
     int final_state;
 };
 
-size_t job_bytes(const pdpd_world &w, int precision)
+BatchSize job_size(const pdpd_world &w, int precision)
 {
-    // sorted state A and B, ids / cells, two id-ordered staging rows, hashes
-    const size_t per_bead = precision == PDPD_FP64 ? 412 : 284;
-    const size_t cells = (size_t)w.box[0] * w.box[1] * w.box[2];
-    size_t lists = 0;
-    if (precision == PDPD_FP64 && w.n_beads) {
-        List64Room room;
-        room.add((double)w.n_beads, w.box, asymmetric(w));
-        lists = room.bytes(w.n_beads);
-    }
-    return per_bead * w.n_beads + lists + (20 + 4 * bucket_room((double)w.n_beads / (double)cells)) * cells +
-           48 * (2 * (size_t)w.n_bonds + 3 * (size_t)w.n_angles) + 4096;
+    BatchSize size;
+    size.add(w.n_beads, w.box, w.n_bonds, w.n_angles, precision == PDPD_FP64 && asymmetric(w));
+    return size;
 }
 
 }  // namespace
@@ -2969,10 +2910,10 @@ void pdpd_server::run()
                     i++;
                 }
             if (in_phase) {
-                size_t used = 0;
-                for (auto &j : active) used += j->bytes;
-                while (!pending.empty() && (active.empty() || used + pending.front()->bytes <= budget)) {
-                    used += pending.front()->bytes;
+                BatchSize used;
+                for (auto &j : active) used.add(j->size);
+                while (!pending.empty() && job_joins(used, pending.front()->size, eng->fp64(), budget)) {
+                    used.add(pending.front()->size);
                     active.push_back(std::move(pending.front()));
                     pending.pop_front();
                     changed = true;
@@ -3273,7 +3214,7 @@ int pdpd_server_submit(pdpd_server *s, const pdpd_world *w, uint32_t n_steps, pd
     j->t = w->t;
     j->cb = cb;
     j->user = user;
-    j->bytes = job_bytes(*w, s->precision);
+    j->size = job_size(*w, s->precision);
     j->t_submit = now_s();
     {
         std::lock_guard<std::mutex> lk(s->mu);

@@ -42,3 +42,23 @@ def test_batches_of_mixed_density(name, prec, config):
     eng.Run(steps)
     for w, o in zip(worlds, ref):
         assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
+
+
+@pytest.mark.parametrize("prec", ["fp32", "fp64"])
+def test_a_dense_world_does_not_enlarge_the_others(prec):
+    """Device memory of a small dense world and a large sparse one in a batch: what the two take one by
+    one (the buckets of all cells were as large as the densest world's: 200 MB more here)."""
+    torch = pytest.importorskip("torch")
+
+    def taken(worlds):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        eng = E.GB300DPDEngine(prec)
+        eng.AttachBatch(worlds)
+        eng.Run(1)
+        return free - torch.cuda.mem_get_info()[0]
+
+    dense, sparse = W.make_water(6, seed=95, density=30, a=0.5, dt=0.001), W.make_water(100, seed=96, density=0.1, dt=0.001)
+    taken([dense.copy()])  # (the context's own allocations)
+    apart = taken([dense.copy()]) + taken([sparse.copy()])
+    assert taken([dense, sparse]) <= apart + (24 << 20)
