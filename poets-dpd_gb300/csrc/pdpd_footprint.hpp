@@ -114,13 +114,15 @@ struct BatchSize {
     }
 };
 
-// Whether a job joins a running batch (its size, 0 worlds: none) within the budget.
+// Whether a job joins a running batch (its size, 0 worlds: none) within the budget.  An FP64 batch
+// is kept small enough for its pair lists: without them its steps take about twice as long.
 inline bool job_joins(const BatchSize &batch, const BatchSize &job, bool fp64, size_t budget)
 {
     if (batch.worlds == 0) return true;
     BatchSize all = batch;
     all.add(job);
-    return all.bytes(fp64) <= budget;
+    if (all.bytes(fp64) > budget) return false;
+    return !(fp64 && all.lists_pay() && !all.lists_fit() && batch.lists_fit());
 }
 
 }  // namespace pdpd

@@ -40,7 +40,7 @@ int main()
                 if (!fp64 || (b.lists_pay() == x->lists_pay() && b.lists_pay() == y->lists_pay()))
                     CHECK(b.bytes(fp64) <= x->bytes(fp64) + y->bytes(fp64) + 1024);
         }
-    // admission: within the budget; the first job at any size
+    // admission: within the budget; the first job at any size; FP64 not beyond the lists' reach
     const size_t GB = size_t(1) << 30;
     for (bool fp64 : {false, true}) {
         BatchSize b;
@@ -49,6 +49,16 @@ int main()
         for (; n < 100000 && job_joins(b, usual, fp64, 40 * GB); n++) b.add(usual);
         CHECK(n > 0 && n < 100000);
         CHECK(b.bytes(fp64) <= 40 * GB);
+        CHECK(!fp64 || b.lists_fit());
+        CHECK(fp64 || b.beads > (1u << 26));
     }
+    // a job beyond the lists' reach runs, alone or with others
+    const BatchSize giant = world(300, 300, 300, 3);
+    CHECK(!giant.lists_fit() && giant.bytes(true) < 40 * GB);
+    CHECK(job_joins(BatchSize{}, giant, true, GB) && job_joins(giant, usual, true, 80 * GB));
+    CHECK(!job_joins(usual, giant, true, 80 * GB) && job_joins(usual, giant, false, 80 * GB));
+    // a batch that takes no lists has no such limit
+    const BatchSize thin = world(512, 512, 512, 0.2);
+    CHECK(!thin.lists_pay() && job_joins(thin, thin, true, 200 * GB));
     return failed ? 1 : 0;
 }
