@@ -3119,8 +3119,7 @@ int pdpd_server_create(int precision, int device, size_t memory_budget_bytes, ui
     // that fills the budget, at most 16 GiB each.  Pinning host memory is slow: in a 20 s
     // stream whose batch grew to the budget, buffers re-pinned as they grew (by half, then by
     // 4x) held the GPU idle for 7%, then 4.5% of the wall time.
-    const size_t per_bead = precision == PDPD_FP64 ? 424 : 296;  // as job_bytes
-    const size_t full = std::min<size_t>(sizeof(double) * 9 * (memory_budget_bytes / per_bead), size_t(16) << 30);
+    const size_t full = snapshot_reserve(precision == PDPD_FP64, memory_budget_bytes);
     for (HostPinned &h : s->snap)
         if (h.alloc(std::max<size_t>(full, 4096), true) != cudaSuccess) {
             g_last_error = "pinned snapshot buffers: allocation failed";

@@ -125,4 +125,13 @@ inline bool job_joins(const BatchSize &batch, const BatchSize &job, bool fp64, s
     return !(fp64 && all.lists_pay() && !all.lists_fit() && batch.lists_fit());
 }
 
+// Bytes of a host snapshot buffer (rows x, v, f as doubles) for the batches that a budget admits.
+// FP64: no batch with pair lists takes less than 600 bytes a bead, nor has 2^25 beads; a single
+// job that is larger gets a larger buffer when it comes.
+inline size_t snapshot_reserve(bool fp64, size_t budget)
+{
+    const size_t beads = fp64 ? std::min<size_t>(budget / 600, size_t(1) << 25) : budget / BEAD_BYTES32;
+    return std::min<size_t>(9 * sizeof(double) * beads, size_t(16) << 30);
+}
+
 }  // namespace pdpd

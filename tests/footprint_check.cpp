@@ -51,7 +51,11 @@ int main()
         CHECK(b.bytes(fp64) <= 40 * GB);
         CHECK(!fp64 || b.lists_fit());
         CHECK(fp64 || b.beads > (1u << 26));
+        // (the snapshot buffers hold what the budget admits)
+        CHECK(snapshot_reserve(fp64, 40 * GB) >= 72 * b.beads);
+        CHECK(snapshot_reserve(fp64, 4 * GB) <= 72 * (4 * GB / BEAD_BYTES32));
     }
+    CHECK(snapshot_reserve(true, 40 * GB) <= 72 * (size_t(1) << 25));
     // a job beyond the lists' reach runs, alone or with others
     const BatchSize giant = world(300, 300, 300, 3);
     CHECK(!giant.lists_fit() && giant.bytes(true) < 40 * GB);

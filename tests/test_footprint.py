@@ -1,6 +1,6 @@
 """What the engine and the job server take a batch's device memory to be (pdpd_footprint.hpp):
 bucket sizes of batches of mixed density, admission by the budget and by the reach of the FP64
-pair lists."""
+pair lists, the snapshot buffers' reservation."""
 
 import os
 import shutil
