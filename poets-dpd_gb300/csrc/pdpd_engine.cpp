@@ -170,6 +170,7 @@ struct DevBuf {
         if (grow) n += n / 2;
         cudaError_t e = cudaMalloc(&p, n);
         if (e != cudaSuccess) {
+            cudaGetLastError();  // (reported here, not by the next caller of the runtime)
             p = nullptr;
             return e;
         }
@@ -195,6 +196,7 @@ struct HostPinned {
         release();
         cudaError_t e = cudaMallocHost(&p, n);
         if (e != cudaSuccess) {
+            cudaGetLastError();
             p = nullptr;
             return e;
         }
@@ -393,6 +395,20 @@ struct pdpd_engine {
         attached = false;
         tuned = false;
         n_beads = n_cells = n_tiles = 0;
+    }
+
+    // The pair lists' buffer, `need` bytes that leave `spare` free on the device; half as much again
+    // where it grows (as DevBuf) and there is room.
+    bool alloc_lists(size_t need, size_t spare)
+    {
+        if (d_lists.p && d_lists.bytes >= need) return true;
+        const size_t want = d_lists.p ? need + need / 2 : need;
+        d_lists.release();
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+        for (size_t n : {want, need})
+            if (free >= n + spare && d_lists.alloc(n) == cudaSuccess) return true;
+        return false;
     }
 
     bool fp64() const { return precision == PDPD_FP64; }
@@ -1540,59 +1556,66 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     const uint32_t bucket_k = size.bucket_k();
 
     // --- allocate
+    // FP64: the pair lists, where they are addressable, pay and find memory (else the force pass
+    // runs without: same results, slower).  They come last, and give way to the other buffers.
+    const List64Room &room = size.room;
+    bool lists = f64 && e->cfg_pair_lists && size.lists_fit() && (size.lists_pay() || e->cfg_pair_lists == 2);
+    if (!lists) e->d_lists.release();
     const size_t P = payload_bytes(f64);
+    const size_t head_bytes = (sizeof(uint64_t) * (size_t)nc + 255) & ~size_t(255);
+    const size_t bucket_bytes = sizeof(uint32_t) * bucket_k * (size_t)nc;
     cudaError_t ce = cudaSuccess;
     auto A = [&](DevBuf &b, size_t n) {
         if (ce == cudaSuccess) ce = b.alloc(n);
     };
-    A(e->d_worlds, sizeof(WorldDev) * n_worlds);
-    A(e->d_tiles, sizeof(Tile) * std::max<size_t>(1, tiles.size()));
-    A(e->d_start, sizeof(uint32_t) * ((size_t)nc + 1));
-    A(e->d_cnt, sizeof(uint32_t) * (size_t)nc);
-    A(e->d_zlo, f64 ? 16 : sizeof(uint16_t) * std::max<size_t>(1, (size_t)nc));
-    A(e->d_brick_next, 64);  // the brick queue's counter, then the overflow lists' state
-    A(e->d_blocksums, sizeof(uint32_t) * (scan_blocks((uint32_t)nc) + 1));
-    A(e->d_posA, P * nb);
-    A(e->d_velA, P * nb);
-    A(e->d_frc, P * nb);
-    A(e->d_posB, P * nb);
-    A(e->d_velB, P * nb);
-    A(e->d_frcB, P * nb);
-    A(e->d_ids, sizeof(uint32_t) * nb);
-    A(e->d_cellg, sizeof(uint32_t) * nb);
-    A(e->d_slot_of_id, sizeof(uint32_t) * nb);
-    A(e->d_key, sizeof(uint32_t) * nb);
-    const size_t head_bytes = (sizeof(uint64_t) * (size_t)nc + 255) & ~size_t(255);
-    const size_t bucket_bytes = sizeof(uint32_t) * bucket_k * (size_t)nc;
-    A(e->d_buckets, head_bytes + bucket_bytes + sizeof(uint2) * nb);
-    A(e->d_bond_row, sizeof(uint32_t) * (nb + 1));
-    A(e->d_bond_terms, sizeof(BondTerm) * std::max<uint64_t>(1, n_terms));
-    A(e->d_bond_params, (f64 ? sizeof(double) : sizeof(float)) * 4 * std::max<uint64_t>(1, n_bparams));
-    A(e->d_pair, (f64 ? sizeof(double) : sizeof(float)) * 2 * n_pair);
-    A(e->d_cellpair, std::max<size_t>(16, f64 ? sizeof(double) * cp64.size() : sizeof(float) * cp32.size()));
-    A(e->d_hash, sizeof(uint32_t) * nb);
-    A(e->d_bonded, sizeof(uint32_t) * std::max<uint64_t>(1, nb));
-    A(e->d_blist, std::max<size_t>(16, list_bytes));
-    A(e->d_inv, sizeof(uint32_t) * std::max<uint64_t>(1, nb));
-    A(e->d_scan, sizeof(uint32_t) * (scan_blocks((uint32_t)nb) + 1));
-    A(e->d_fbond, f64 ? 16 : sizeof(float4) * std::max<uint64_t>(1, nb));
-    A(e->d_posf, f64 ? sizeof(float4) * std::max<uint64_t>(1, nb) : 16);
-    A(e->d_bterm, f64 ? sizeof(double) * 4 * std::max<uint64_t>(1, n_terms) : 16);
-    if (f64 && n_terms) A(e->d_row_of, sizeof(uint32_t) * n_terms);
-    A(e->d_staging[0], sizeof(double) * 9 * nb);
+    auto allocate = [&]() {
+        ce = cudaSuccess;
+        A(e->d_worlds, sizeof(WorldDev) * n_worlds);
+        A(e->d_tiles, sizeof(Tile) * std::max<size_t>(1, tiles.size()));
+        A(e->d_start, sizeof(uint32_t) * ((size_t)nc + 1));
+        A(e->d_cnt, sizeof(uint32_t) * (size_t)nc);
+        A(e->d_zlo, f64 ? 16 : sizeof(uint16_t) * std::max<size_t>(1, (size_t)nc));
+        A(e->d_brick_next, 64);  // the brick queue's counter, then the overflow lists' state
+        A(e->d_blocksums, sizeof(uint32_t) * (scan_blocks((uint32_t)nc) + 1));
+        A(e->d_posA, P * nb);
+        A(e->d_velA, P * nb);
+        A(e->d_frc, P * nb);
+        A(e->d_posB, P * nb);
+        A(e->d_velB, P * nb);
+        A(e->d_frcB, P * nb);
+        A(e->d_ids, sizeof(uint32_t) * nb);
+        A(e->d_cellg, sizeof(uint32_t) * nb);
+        A(e->d_slot_of_id, sizeof(uint32_t) * nb);
+        A(e->d_key, sizeof(uint32_t) * nb);
+        A(e->d_buckets, head_bytes + bucket_bytes + sizeof(uint2) * nb);
+        A(e->d_bond_row, sizeof(uint32_t) * (nb + 1));
+        A(e->d_bond_terms, sizeof(BondTerm) * std::max<uint64_t>(1, n_terms));
+        A(e->d_bond_params, (f64 ? sizeof(double) : sizeof(float)) * 4 * std::max<uint64_t>(1, n_bparams));
+        A(e->d_pair, (f64 ? sizeof(double) : sizeof(float)) * 2 * n_pair);
+        A(e->d_cellpair, std::max<size_t>(16, f64 ? sizeof(double) * cp64.size() : sizeof(float) * cp32.size()));
+        A(e->d_hash, sizeof(uint32_t) * nb);
+        A(e->d_bonded, sizeof(uint32_t) * std::max<uint64_t>(1, nb));
+        A(e->d_blist, std::max<size_t>(16, list_bytes));
+        A(e->d_inv, sizeof(uint32_t) * std::max<uint64_t>(1, nb));
+        A(e->d_scan, sizeof(uint32_t) * (scan_blocks((uint32_t)nb) + 1));
+        A(e->d_fbond, f64 ? 16 : sizeof(float4) * std::max<uint64_t>(1, nb));
+        A(e->d_posf, f64 ? sizeof(float4) * std::max<uint64_t>(1, nb) : 16);
+        A(e->d_bterm, f64 ? sizeof(double) * 4 * std::max<uint64_t>(1, n_terms) : 16);
+        if (f64 && n_terms) A(e->d_row_of, sizeof(uint32_t) * n_terms);
+        A(e->d_staging[0], sizeof(double) * 9 * nb);
+    };
+    allocate();
+    if (ce != cudaSuccess && e->d_lists.p) {  // (the lists of the batch before)
+        e->d_lists.release();
+        allocate();
+    }
     if (ce != cudaSuccess) {
         cudaGetLastError();
         e->release();
         return e->fail(PDPD_E_NOMEM, "device allocation failed: %s", cudaGetErrorString(ce));
     }
-    // FP64: the pair lists, where they are addressable and there is memory for them (else the
-    // force pass runs without: same results, slower)
-    const List64Room &room = size.room;
-    bool lists = f64 && e->cfg_pair_lists && size.lists_fit() && (size.lists_pay() || e->cfg_pair_lists == 2);
-    if (lists) {
-        lists = e->d_lists.alloc(room.bytes(nb)) == cudaSuccess;
-        if (!lists) cudaGetLastError();
-    }
+    // (not at the cost of the buffers that come later: brick table, read-backs, snapshots)
+    if (lists) lists = e->alloc_lists(room.bytes(nb), 128 * nb + 8 * nc + (64u << 20));
     // Host staging rows of the worlds that come from their descriptors: the whole batch in
     // slot order, or in a re-pack only the new worlds, packed (the kept worlds' rows stay on
     // the device, and the pinned buffer stays the size of what a re-pack brings in).
