@@ -1,6 +1,7 @@
 // Device-side helpers shared by the kernel translation units.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 
 #include "pdpd_internal.h"
@@ -21,8 +22,7 @@ struct __align__(16) Vec2d {
 // microseconds, and the gaps between them were a good part of it (9^3 water, 40 steps with the
 // read-back: 1.01 -> 0.77 ms).  The short kernels also let the next one's blocks come up at
 // once; the force kernels do not, as those blocks would take room on the SMs for nothing
-// meanwhile (32^3 polymer box, 100 steps: 3.72 ms without any of this, 3.85 with, 3.54 so).  The
-// force kernels of one thread per bead are launched plainly (launch_force64, launch_force32).
+// meanwhile (32^3 polymer box, 100 steps: 3.72 ms without any of this, 3.85 with, 3.54 so).
 __device__ __forceinline__ void step_kernel_wait()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -50,17 +50,37 @@ inline cudaError_t launch_step_kernel(void (*k)(P...), uint32_t grid, uint32_t b
     return cudaLaunchKernelEx(&cfg, k, P(args)...);  // (an error is also seen by the caller's cudaGetLastError)
 }
 
-// Opt a kernel without static shared memory in to all the dynamic shared memory that a block may have
-// on the current device.  The limit belongs to the kernel, for every engine of the process: set to
-// the need of one batch, it would refuse the launches of another engine whose batch needs more.
-// What a launch takes (and its occupancy) follows from the bytes it names, not from the limit.
-inline cudaError_t allow_dynamic_smem(const void *k)
+// Opt a kernel in to all the dynamic shared memory that a block may have on the current device
+// (beside `fixed` bytes of static memory).  The limit belongs to the kernel, for every engine of the
+// process: set to the need of one batch, it would refuse the launches of another engine whose batch
+// needs more.  What a launch takes (and its occupancy) follows from the bytes it names, not from
+// the limit.
+inline cudaError_t allow_dynamic_smem(const void *k, size_t fixed = 0)
 {
     int dev = 0, most = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fixed);
     return e;
+}
+
+// Dynamic shared memory with which no more than an even share of `blocks` blocks fits an SM (0 where
+// `resident`, those that fit without it, are no more).  The blocks of a force kernel come up while
+// the cell-list kernel drains: without it they crowd on the SMs that are free first, and a block
+// takes as long as its SM's pipes are shared.  Steps, us, crowded and spread: FP32 bricks, 22^3 of
+// density 3 27.4 and 22.7, 24^3 28.5 and 23.8, 25^3 31.8 and 25.0, 16^3 of density 8 37.7 and 29.6;
+// variant 6, 22^3 29.9 and 24.3; a thread per bead, 22^3 66.5 and 50.7, 14^3 of density 10 285 and 198;
+// the FP64 list kernel, 25^3 87.3 and 81.0.
+inline uint32_t spread_smem(uint32_t blocks, int resident, int sm_count, size_t fixed = 0)
+{
+    int dev = 0, most = 0, opt_in = 0;
+    const uint32_t share = (blocks + (uint32_t)sm_count - 1) / (uint32_t)sm_count;
+    if (share == 0 || share >= (uint32_t)resident || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&opt_in, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
+        return 0;
+    const int want = most / (int)(share + 1) + 1;  // (one block more would not fit)
+    return (uint32_t)std::max(0, std::min(want, opt_in) - (int)fixed);
 }
 
 // riscv_mix64_m2 (reference include/dpd/core/hash.hpp:20-30), full 64-bit form.

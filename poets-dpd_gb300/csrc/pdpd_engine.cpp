@@ -754,18 +754,6 @@ struct pdpd_engine {
         for (int d = 0; d < 3; d++) cfg_brick[d] = b[d];
     }
 
-    // Shared memory with which a block is alone on its SM.  The blocks of a brick kernel come up while
-    // the cell-list kernel drains, two of them on the SMs that are free first: a batch of no more
-    // bricks than SMs asks for half an SM's memory, so that each brick gets an SM (steps, us,
-    // without and with: 22^3 of density 3 27.4 and 22.9, 24^3 28.5 and 24.0, 25^3 31.8 and 25.0; 16^3 of
-    // density 8 37.7 and 29.8; FP64, 25^3 87.3 and 81.8).
-    uint32_t alone_smem() const
-    {
-        int most = 0;
-        if (cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) != cudaSuccess) return 0;
-        return (uint32_t)most / 2;
-    }
-
     BrickSegs segs() const { return brick_segs(max_density, args.list_capacity); }
 
     // Staged beads a brick of hc halo cells should have room for: its mean halo population
@@ -796,7 +784,12 @@ struct pdpd_engine {
         a.force_kernel = any_spatial() ? 1 : cfg_force_kernel;
         a.bricks = nullptr;
         a.n_bricks = 0;
-        if (fp64() ? !a.list : a.force_kernel == 1) return PDPD_OK;
+        if (fp64() ? !a.list : a.force_kernel == 1) {
+            const int gb = cfg_grid_blocks > 0 ? cfg_grid_blocks : 16 * sm_count;
+            const uint32_t blocks = std::min<uint32_t>((uint32_t)gb, n_tiles);
+            const int rc = fp64() ? 0 : force32_setup(sm_count, blocks, &a.tile_smem);
+            return rc ? fail(PDPD_E_CUDA, "force kernel setup: %s", cudaGetErrorString((cudaError_t)rc)) : PDPD_OK;
+        }
         int shape[3] = {cfg_brick[0], cfg_brick[1], cfg_brick[2]};
         if (fp64()) {
             a.brick_planes = small_shape(shape, 0) ? 3 : 1;
@@ -851,10 +844,9 @@ struct pdpd_engine {
         a.bricks = d_bricks.as<Brick>();
         a.n_bricks = (uint32_t)bricks.size();
         a.brick_hc_max = hc_max;
-        a.brick_smem = bricks.size() <= (size_t)sm_count ? alone_smem() : 0u;
         if (fp64()) {
             a.brick_maxb = (uint32_t)std::min((double)list64_maxb_limit(hc_max), want);
-            const int rc = list64_setup(sm_count, a.brick_hc_max, a.brick_maxb, a.brick_planes, &a.brick_grid);
+            const int rc = list64_setup(a, sm_count, &a.brick_grid, &a.brick_smem);
             if (rc) return fail(PDPD_E_CUDA, "list kernel setup: %s", cudaGetErrorString((cudaError_t)rc));
             if (cfg_grid_blocks > 0) a.brick_grid = cfg_grid_blocks;
             drop_graph();
@@ -868,10 +860,11 @@ struct pdpd_engine {
         int grid = 0;
         uint32_t bytes = 0;
         int rc = brick_setup(sm_count, a.force_kernel, a.brick_hc_max, a.brick_maxb, a.brick_npair,
-                             a.brick_home_max, a.brick_planes, a.segs, &grid, &bytes);
+                             a.brick_home_max, a.brick_planes, a.segs, a.n_bricks, &grid, &bytes);
         if (rc)
             return fail(PDPD_E_CUDA, "brick kernel setup (%u bytes of shared memory): %s", bytes,
                         cudaGetErrorString((cudaError_t)rc));
+        a.brick_smem = bytes;
         a.brick_grid = cfg_grid_blocks > 0 ? cfg_grid_blocks : grid;
         drop_graph();
         return PDPD_OK;

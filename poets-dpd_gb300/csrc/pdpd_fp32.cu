@@ -741,6 +741,7 @@ __device__ __forceinline__ void pair_forces32(const KArgs &a, const WorldDev &w,
 template <int FINAL>
 __global__ void __launch_bounds__(TILE_BEADS) k_force32(KArgs a)
 {
+    step_kernel_wait();
     __shared__ float2 s_pair[MAX_PAIR];
     __shared__ uint32_t s_j[LIST_MAX * TILE_BEADS];
     __shared__ uint8_t s_dir[LIST_MAX * TILE_BEADS];
@@ -921,9 +922,9 @@ template <int FINAL> static auto wide_kernel(int planes, BrickSegs segs)
 }
 
 // Set up the brick kernel for a brick shape: opt in to large shared memory and
-// return its persistent grid (resident blocks x SMs) and dynamic shared-memory bytes.
+// return its persistent grid (resident blocks x SMs) and dynamic shared-memory bytes for n_bricks.
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max,
-                int planes, BrickSegs segs, int *grid, uint32_t *smem_bytes)
+                int planes, BrickSegs segs, uint32_t n_bricks, int *grid, uint32_t *smem_bytes)
 {
     int nb = 0;
     const uint32_t hm = variant == 9 ? home_max : 0u;
@@ -946,7 +947,7 @@ int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint3
     if (e != cudaSuccess) return (int)e;
     if (nb < 1) return (int)cudaErrorInvalidConfiguration;
     *grid = nb * sm_count;
-    *smem_bytes = L.bytes;
+    *smem_bytes = std::max(L.bytes, spread_smem(std::min((uint32_t)*grid, n_bricks), nb, sm_count));
     return 0;
 }
 
@@ -979,16 +980,24 @@ int launch_force32(const KArgs &a, int final_step, cudaStream_t s)
         case 8: k = final_step ? wide_kernel<1>(a.brick_planes, a.segs) : wide_kernel<0>(a.brick_planes, a.segs); break;
         default: k = final_step ? k_force32_brick<1, BRICK_THREADS, 1, true> : k_force32_brick<0, BRICK_THREADS, 1, true>; break;
         }
-        launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), std::max(L.bytes, a.brick_smem), s, a, L);
+        launch_step_kernel(k, (uint32_t)grid, brick_variant_threads(v), a.brick_smem, s, a, L);
         return 1;
     }
-    // Launched when the kernel in front has finished, as k_force64: its blocks spread evenly over the SMs
-    // (24^3 of density 3 59 us a step against 67, 14^3 of density 10 242 and 285; 4^3 39.4 and 38.8).
-    if (final_step)
-        k_force32<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
-    else
-        k_force32<0><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
+    launch_step_kernel(final_step ? k_force32<1> : k_force32<0>, (uint32_t)a.grid_blocks, TILE_BEADS, a.tile_smem, s, a);
     return 1;
+}
+
+// Dynamic shared memory of the thread-per-bead kernel's launch for `blocks` blocks.
+int force32_setup(int sm_count, uint32_t blocks, uint32_t *smem)
+{
+    void (*const k[2])(KArgs) = {k_force32<0>, k_force32<1>};
+    cudaFuncAttributes at{};
+    int resident = 0;
+    cudaError_t e = cudaFuncGetAttributes(&at, (const void *)k[0]);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k[0], TILE_BEADS, 0);
+    for (int q = 0; q < 2 && e == cudaSuccess; q++) e = allow_dynamic_smem((const void *)k[q], at.sharedSizeBytes);
+    if (e == cudaSuccess) *smem = spread_smem(blocks, resident, sm_count, at.sharedSizeBytes);
+    return (int)e;
 }
 
 int launch_pair_log32(const KArgs &a, const uint32_t *sel, uint32_t n_sel, const uint32_t *offs,

@@ -739,16 +739,22 @@ int launch_cells64(const KArgs &a, int tick, int bonds, cudaStream_t s)
     return 1;
 }
 
+// Entries of the list kernel's queue: bricks, then chunks of bonds and of angles.
+static uint32_t list64_work(const KArgs &a)
+{
+    return a.n_bricks + (a.n_bonds + BOND64_CHUNK - 1) / BOND64_CHUNK + (a.n_angles + BOND64_CHUNK - 1) / BOND64_CHUNK;
+}
+
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
 {
     if (a.list) {  // each pair once
         const List64Layout L = list64_layout(a.brick_hc_max, a.brick_maxb);
         const uint32_t bb = (a.n_bonds + BOND64_CHUNK - 1) / BOND64_CHUNK;
-        const uint32_t work = a.n_bricks + bb + (a.n_angles + BOND64_CHUNK - 1) / BOND64_CHUNK;
+        const uint32_t work = list64_work(a);
         const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)a.brick_grid, work));
         // (a list that was not made is not read: the error reaches the caller)
         if (launch_step_kernel(a.brick_planes == 3 ? k_list64<3> : k_list64<1>, grid, LIST64_THREADS,
-                               std::max(L.bytes, a.brick_smem), s, a, L,
+                               a.brick_smem, s, a, L,
                                bb, work) != cudaSuccess)
             return 0;
         const uint32_t pb = (a.pair_cap + PAIRS64_THREADS - 1) / PAIRS64_THREADS;
@@ -759,9 +765,9 @@ int launch_force64(const KArgs &a, int final_step, cudaStream_t s)
         else launch_step_kernel(k_sum64<0>, parts, SUM64_THREADS, 0, s, a);
         return 3;
     }
-    // Launched when the kernel in front has finished: blocks that come up while it drains crowd on
-    // the SMs that are free first, and a block takes as long as its SM's FP64 pipe is shared (24^3
-    // of density 3 264 us a step against 173; 16^3 of density 8 7,070 and 3,170).
+    // Launched when the kernel in front has finished: its few blocks then spread evenly over the SMs,
+    // whose FP64 pipe they share (spread_smem; 24^3 of density 3, step, 264 us crowded, 184 spread by
+    // shared memory, 173 so; 16^3 of density 8 7,070, 3,220, 3,170).
     if (final_step)
         k_force64<1><<<a.grid_blocks, TILE_BEADS, 0, s>>>(a);
     else
@@ -780,16 +786,17 @@ uint32_t list64_maxb_limit(uint32_t hc_max)
     return (uint32_t)std::max(64, std::min((int)FULL_MAX_STAGED, budget / (int)LIST64_BEAD_BYTES)) & ~1u;
 }
 
-int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int planes, int *grid)
+int list64_setup(const KArgs &a, int sm_count, int *grid, uint32_t *smem)
 {
-    const auto k = planes == 3 ? k_list64<3> : k_list64<1>;
-    const int bytes = (int)list64_layout(hc_max, maxb).bytes;
+    const auto k = a.brick_planes == 3 ? k_list64<3> : k_list64<1>;
+    const int bytes = (int)list64_layout(a.brick_hc_max, a.brick_maxb).bytes;
     int nb = 0;
     cudaError_t e = allow_dynamic_smem((const void *)k);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, LIST64_THREADS, bytes);
     if (e != cudaSuccess) return (int)e;
     if (nb < 1) return (int)cudaErrorInvalidConfiguration;
     *grid = nb * sm_count;
+    *smem = std::max((uint32_t)bytes, spread_smem(std::min((uint32_t)*grid, list64_work(a)), nb, sm_count));
     return 0;
 }
 

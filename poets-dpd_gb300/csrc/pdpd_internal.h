@@ -148,7 +148,8 @@ struct KArgs {
                          // brick), 8 = full-shell brick kernel with 512-thread blocks, 6 = the
                          // same with 128-thread blocks, 1 = thread per bead (global memory)
     int brick_grid;      // persistent grid size of the brick kernel
-    uint32_t brick_smem;    // bytes of shared memory that a brick kernel's launch asks for at least
+    uint32_t brick_smem;    // dynamic shared memory of the brick or list kernel's launch
+    uint32_t tile_smem;     // ... of the FP32 thread-per-bead kernel's
     uint32_t brick_hc_max;  // halo cells of the nominal brick shape
     uint32_t brick_maxb;    // staged-bead capacity of one brick
     uint32_t brick_npair;   // staged pair-table entries: the largest n_types^2 of the worlds
@@ -180,9 +181,10 @@ int launch_begin32(const KArgs &a, cudaStream_t s);
 int launch_force32(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish32(const KArgs &a, cudaStream_t s);
 int launch_bin64(const KArgs &a, const uint32_t *hash_in, cudaStream_t s);
-// FP64 list kernel: staged-bead capacity of a brick, and its persistent grid (0 or a cudaError_t).
+// FP64 list kernel: staged-bead capacity of a brick, and, for the bricks and bonds of a, its
+// persistent grid and dynamic shared memory (0 or a cudaError_t).
 uint32_t list64_maxb_limit(uint32_t hc_max);
-int list64_setup(int sm_count, uint32_t hc_max, uint32_t maxb, int planes, int *grid);
+int list64_setup(const KArgs &a, int sm_count, int *grid, uint32_t *smem);
 int launch_begin64(const KArgs &a, cudaStream_t s);
 int launch_force64(const KArgs &a, int final_step, cudaStream_t s);
 int launch_finish64(const KArgs &a, cudaStream_t s);
@@ -277,7 +279,9 @@ bool brick_planes_fit(double density, uint32_t hc_max, uint32_t maxb, uint32_t n
 // The segments for a box of this density (list_capacity: the config entry, 0 = automatic).
 BrickSegs brick_segs(double density, int list_capacity);
 int brick_setup(int sm_count, int variant, uint32_t hc_max, uint32_t maxb, uint32_t npair, uint32_t home_max, int planes,
-                BrickSegs segs, int *grid, uint32_t *smem_bytes);  // 0 or a cudaError_t
+                BrickSegs segs, uint32_t n_bricks, int *grid, uint32_t *smem_bytes);  // 0 or a cudaError_t
+// Dynamic shared memory of the FP32 thread-per-bead kernel for `blocks` blocks (0 or a cudaError_t).
+int force32_setup(int sm_count, uint32_t blocks, uint32_t *smem);
 uint32_t scan_blocks(uint32_t n_cells);
 
 // Observables of one world (pdpd_observe.cu): per-block FP64 partial sums.
