@@ -267,8 +267,9 @@ const ConfigEntry kConfig[] = {
                      "384-thread blocks.  1, 6 and 8 give the same forces to the bit; 9 gives the "
                      "same forces to the bit whatever its brick shape, grid or batch, within the "
                      "FP32 tolerance of the others."},
-    {"brick_x", "Brick extent in cells along x (FP32 brick kernel; default by the batch's cells per "
-                "SM, from 2x4x4 to 5x8x8)."},
+    {"brick_x", "Brick extent in cells along x (FP32 brick kernel; default by the batch's size and each "
+                "world's density, from 1x2x2 to 5x8x8, with three lanes per bead in the smallest "
+                "batches; set for all worlds, one lane per bead, where any of the three is set)."},
     {"brick_y", "Brick extent in cells along y (FP32 brick kernel)."},
     {"brick_z", "Brick extent in cells along z (FP32 brick kernel)."},
     {"autotune", "FP32: time the force-kernel variants and brick shapes on the first steps of "
@@ -575,20 +576,19 @@ struct pdpd_engine {
     // Brick shape for the 512-thread kernels (FP32 variant 8, the FP64 list kernel).  By the batch's
     // cells per SM: the largest bricks stage the fewest halo beads per home bead, but the
     // persistent blocks (two per SM) want several bricks each, and a small batch has too few.
-    // Whole FP32 steps of polymer boxes, us (sides 24, 32, 40, 48, 56, 64, 72, 80, 96; cells per SM 91,
-    // 216, 421, 728, 1155, 1725, 2456, 3368, 5821): 5x8x8 31.9, 48.7, 51.3, 90.3, 95.2, 139.7, 199.1,
-    // 254.7, 414.5; 4x8x10 29.8, 43.8, 51.4, 89.6, 93.4, 133.4, 189.2, 256.5, 414.3; 4x5x8 (480 home
-    // beads, one turn of the block) 28.0, 31.0, 53.1, 63.0, 103.2, 134.4, 196.2, 263.4, 444.7; 4x4x8
-    // 26.1, 29.0, 49.4, 69.3, 105.2, 144.0, 209.7, 279.1, 469.6; 3x4x6 20.9, 35.9, 59.7, 82.3, 132.5,
-    // 185.3, 258.7, 361.3, 591.1 (sides 9 and 16, an earlier kernel: 2x4x4 23.2 and 24.1, 4x4x6 23.7
-    // and 26.0).  Up to two bricks for each block, how they divide into rounds matters more (36^3:
-    // 4x4x8 45.5, 4x6x8 38.9; 40^3: 4x5x8 53.1, 5x6x8 43.2): there another shape is taken where
-    // shape_cost puts it 6% below; above 500 cells per SM the estimate is no better than the table
-    // (45^3: it puts 4x6x8, 67.0, before 4x5x8, 58.8).  From 1,000 on 4x8x10 against 4x5x8 and the
-    // estimate, 20 steps: 56^3 2,412 and 2,216; 56x57x52 2,366 and 2,245; 100x55x41 3,001 and 2,833;
-    // 72x70x73 4,554 and 4,375; 14 boxes of 16 to 24 2,000 and 1,840; but 61x57x55 2,482 and 2,640
-    // (52x50x55, 940 cells per SM: 1,864 and 2,000).  The list kernel keeps the line it was measured
-    // with.
+    // Whole FP32 steps of polymer boxes, us (sides 24, 32, 40, 48, 52, 54, 56, 64, 72, 80, 96; cells per SM
+    // 91, 216, 421, 728, 925, 1036, 1155, 1725, 2456, 3368, 5821): 5x8x8 35.3, 37.9, 57.0, 96.3, 94.2, 99.6,
+    // 103.5, 146.8, 210.9, 268.8, 435.0; 4x8x10 32.8, 35.8, 59.5, 95.5, 90.5, 93.2, 99.4, 141.4, 200.0,
+    // 268.5, 435.1; 4x5x8 (480 home beads, one turn of the block) 28.9, 37.4, 62.0, 71.7, 91.0, 100.1,
+    // 112.1, 148.2, 211.5, 280.9, 470.2; 4x4x8 23.5, 32.4, 53.7, 74.6, 92.1, 102.3, 110.0, 151.8, 218.4,
+    // 292.7, 490.4; 3x4x6 23.4, 38.8, 63.7, 86.6, 110.7, 115.1, 138.4, 192.5, 269.1, 375.8, 614.0.  Up to
+    // two bricks for each block, how they divide into rounds matters more (36^3: 4x5x8 54.2, 4x6x8
+    // 42.7; 40^3: 4x5x8 62.0, 5x6x8 48.9): there another shape is taken where shape_cost puts it 6%
+    // below; above 500 cells per SM the estimate is no better than the table.  Around the line at
+    // 1,000 uneven boxes go either way: 4x8x10 and 4x5x8 at 52x50x55 (941 cells per SM) 91.4 and 90.3,
+    // 56x57x52 (1,092) 100.9 and 108.1, 47x66x61 (1,245) 113.6 and 114.8, 61x57x55 (1,258) 120.0 and 114.2,
+    // 59x53x62 (1,275) 112.6 and 114.8, 70x60x50 (1,382) 117.4 and 125.1, 100x55x41 (1,484) 128.3 and
+    // 133.1, 72x70x73 (2,421) 199.7 and 209.3.  The list kernel keeps the line it was measured with.
     struct ShapeRow {
         uint64_t from32, from64;  // cells per SM
         int c[3];
@@ -664,11 +664,10 @@ struct pdpd_engine {
     // and one turn (160 beads) for each resident block (FP32 one per SM, FP64 two), and terms that
     // fit FP32's pool.  There a step is the latency of one warp's way through the force pass, and
     // the lanes cut its walk and evaluation to a third; with more bricks they only add to the
-    // instructions.  Steps of water boxes, us, one lane and three: 4^3 13.7 and 10.5, 9^3 13.7 and 10.6, 12^3 15.2 and 12.2, 16^3
-    // 16.9 and 15.1, 18^3 18.7 and 16.3; 20^3 (two turns) 20.7 and 21.3, 24^3 24.8 and 22.7.  The
-    // smallest shape that keeps to one brick per SM is the best or within 2% (9^3: 1x2x4 10.6, 2x3x4
-    // 11.4, 4x4x6 12.6; 12^3: 1x2x4 17.6, 2x2x4 12.2, 2x4x4 13.4; 16^3: 2x3x4 21.3, 2x4x4 15.1, 3x4x4
-    // 15.9).
+    // instructions.  Steps of water boxes, us, one lane (the best of eight shapes) and three: 4^3 13.7
+    // and 11.3, 9^3 13.9 and 11.5, 12^3 15.8 and 13.6, 14^3 17.4 and 15.3, 16^3 17.9 and 16.2, 17^3 18.4 and
+    // 16.7, 18^3 18.6 and 18.2.  The smallest shape that keeps to one brick per SM was the best or
+    // within 2% of it (9^3: 1x2x4 10.6, 2x3x4 11.4, 4x4x6 12.6; 12^3: 1x2x4 17.6, 2x2x4 12.2, 2x4x4 13.4).
     // FP64, water, us, one lane and three: 4^3 30.4 and 27.0, 8^3 31.5 and 28.5, 12^3 36.9 and 34.3,
     // 16^3 43.6 and 41.7, 20^3 56.6 and 55.6, 24^3 74.2 and 72.5; 27^3 (441 bricks) 90.5 and 98.1.
     bool small_shape(int shape[3], uint32_t npair) const
