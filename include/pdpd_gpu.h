@@ -364,11 +364,12 @@ typedef struct pdpd_server_stats {
 } pdpd_server_stats;
 
 /* Create a server with its own engine (precision, device as pdpd_create) and worker thread.
- * memory_budget_bytes bounds the summed footprint estimate of the admitted jobs (a job larger
- * than the budget still runs, alone); interval_steps >= 1 is the snapshot interval.  The
- * server reserves two pinned host buffers for the snapshots of a batch that fills the budget
- * (72 bytes per bead, at most 16 GiB each): creation takes a moment, later batches do not
- * wait for host memory to be pinned. */
+ * memory_budget_bytes bounds the footprint of the admitted jobs' batch (at density 3 about 330
+ * bytes per bead in FP32, 950 in FP64 with its pair lists; a job larger than the budget still
+ * runs, alone); an FP64 batch is also kept below the 2^25 beads that pair lists reach.
+ * interval_steps >= 1 is the snapshot interval.  The server reserves two pinned host buffers for
+ * the snapshots of a batch that fills the budget (72 bytes per bead, at most 16 GiB each, 2.4 GiB
+ * in FP64): creation takes a moment, later batches do not wait for host memory to be pinned. */
 int pdpd_server_create(int precision, int device, size_t memory_budget_bytes,
                        uint32_t interval_steps, pdpd_server **out);
 /* Queue a job: the world (copied; the caller's arrays may be reused at once) advanced by
