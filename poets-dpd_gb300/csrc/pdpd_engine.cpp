@@ -405,8 +405,8 @@ struct pdpd_engine {
         if (d_lists.p && d_lists.bytes >= need) return true;
         const size_t want = d_lists.p ? need + need / 2 : need;
         d_lists.release();
-        size_t free = 0, total = 0;
-        if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+        size_t free = want + spare, total = 0;
+        if (need > (8u << 20) && cudaMemGetInfo(&free, &total) != cudaSuccess) return false;  // (a call not made for little)
         for (size_t n : {want, need})
             if (free >= n + spare && d_lists.alloc(n) == cudaSuccess) return true;
         return false;
