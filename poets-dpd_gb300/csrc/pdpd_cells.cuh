@@ -104,6 +104,7 @@ __device__ __forceinline__ void rebuild_begin(const KArgs &a, int tick)
     if (threadIdx.x == 0) {
         *a.brick_next = 0u;
         if (a.list_cursor) a.list_cursor[0] = a.list_cursor[1] = 0ull;
+        a.worlds[0].crowded = a.over->count;
         a.over->count = 0u;
         a.over->epoch += 1u;
     }

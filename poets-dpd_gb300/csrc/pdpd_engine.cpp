@@ -313,6 +313,7 @@ struct pdpd_engine {
     bool tuned = false;
     std::string tune_log;
     double max_density = 0;
+    bool crowded = false;  // the density varies over the box (adapt_bricks)
 
     // attached worlds
     bool attached = false;
@@ -470,10 +471,31 @@ struct pdpd_engine {
         return PDPD_OK;
     }
 
+    // FP32: where the last rebuild that the host knows of left 0.5% of the beads without room in their
+    // cells' buckets (5.5 Poisson deviations above the mean), the density varies over the box, and
+    // large bricks overflow where it is high: their beads are gathered from global memory, or by
+    // lanes that wait for one another.  From here on smaller ones, in boxes large enough to have
+    // them by default.  Steps, us, with the default shape and with 4x4x6: 80% of the beads at density
+    // 12, 48^3 457 and 340 (60% at 9), 64^3 1,573 and 825, 80^3 1,324 and 958 (60% at 9); density falling
+    // as 1/sqrt(z), 48^3 460 and 364, 86^3 1,876 and 1,184; but 32^3 172 and 239.
+    static constexpr int CROWDED_SHAPE[3] = {4, 4, 6};
+    int adapt_bricks()
+    {
+        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || args.bucket_k < bucket_room(max_density) ||
+            n_cells / (uint64_t)std::max(1, sm_count) < 350 || !h_err.p)
+            return PDPD_OK;
+        if ((uint64_t)((const WorldDev *)h_err.p)->crowded * 200 <= n_beads) return PDPD_OK;
+        crowded = true;
+        cudaStreamSynchronize(stream);
+        return configure_bricks();
+    }
+
     // Enqueue n steps (n >= 1) on stream s.
     int enqueue_run(uint32_t n, cudaStream_t s)
     {
         if (n == 0) return PDPD_OK;
+        const int adapted = adapt_bricks();
+        if (adapted) return adapted;
         launches += enqueue_begin(s);
         uint32_t mid = n - 1;
         if (cfg_use_graphs && mid > 0 && s == stream) {
@@ -620,6 +642,10 @@ struct pdpd_engine {
     {
         static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
                                        {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
+        if (crowded) {
+            for (int d = 0; d < 3; d++) shape[d] = CROWDED_SHAPE[d];
+            return;
+        }
         double least = max_density, most = 0;  // the sparsest world, and the densest that the shape fits
         for (const WorldHost &wh : worlds)
             if (wh.dev.n_beads) least = std::min(least, density(wh.dev));
@@ -1803,6 +1829,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     int gb = e->cfg_grid_blocks > 0 ? e->cfg_grid_blocks : 16 * e->sm_count;
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;
+    e->crowded = false;
     {
         int rc = e->configure_bricks();
         if (rc) {

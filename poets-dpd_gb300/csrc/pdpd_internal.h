@@ -32,7 +32,8 @@ struct WorldDev {
     int64_t t;
     uint64_t cellpair_base;
     uint32_t asym;        // 1: some strength a_ij or gamma_ij differs from a_ji or gamma_ji
-    uint32_t pad;
+    uint32_t crowded;     // of the first world: the batch's beads that found their cell's bucket full
+                          // in the last rebuild
 };
 
 // A run of consecutive sorted bead slots of one world: the unit of work of the step

@@ -62,3 +62,22 @@ def test_a_dense_world_does_not_enlarge_the_others(prec):
     taken([dense.copy()])  # (the context's own allocations)
     apart = taken([dense.copy()]) + taken([sparse.copy()])
     assert taken([dense, sparse]) <= apart + (24 << 20)
+
+
+def test_an_uneven_box_gets_other_bricks_between_runs():
+    """A box whose density varies over it (its beads overflow their cells' buckets): the same state to the
+    bit as by the thread-per-bead kernel, from the first run on and after the bricks have changed."""
+    a = W.make_water(40, seed=97, a=1.0, dt=0.001)
+    a.x[:, 2] = a.x[:, 2] ** 3 / 1600
+    b = a.copy()
+    eng, ref = E.GB300DPDEngine("fp32"), E.GB300DPDEngine("fp32")
+    ref.SetConfigEntry("force_kernel", 1)
+    eng.Attach(a)
+    ref.Attach(b)
+    shapes = set()
+    for steps in (1, 3, 2):
+        eng.Run(steps)
+        ref.Run(steps)
+        shapes.add(tuple(v for n, _, v in eng.GetConfigEntries() if n.startswith("brick_")))
+        assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
+    assert ("4", "4", "6") in shapes

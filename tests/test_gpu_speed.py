@@ -121,3 +121,14 @@ def test_attach_of_many_worlds():
 
     worlds = [_water((5 + k % 5, 6 + k % 3, 7 + k % 4), 3, k) for k in range(300)]
     assert attach_us("fp64", worlds) < 1.17 * attach_us("fp32", worlds)
+
+
+def test_an_uneven_large_box():
+    """80% of the beads in a fifth of the box, against smaller bricks: 1.9 times as long in the default
+    ones of its mean density."""
+    import numpy as np
+
+    w = _water(64, 3)
+    n, rng = w.n_beads * 4 // 5, np.random.default_rng(1)
+    w.x[:n, 2], w.x[n:, 2] = 12.8 * rng.random(n), 12.8 + 51.2 * rng.random(w.n_beads - n)
+    assert _step_us("fp32", [w]) < 1.35 * _step_us("fp32", [w], brick_x=4, brick_y=4, brick_z=6)
