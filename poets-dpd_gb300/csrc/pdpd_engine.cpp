@@ -471,20 +471,33 @@ struct pdpd_engine {
         return PDPD_OK;
     }
 
-    // FP32: where the last rebuild that the host knows of left 0.5% of the beads without room in their
-    // cells' buckets (5.5 Poisson deviations above the mean), the density varies over the box, and
-    // large bricks overflow where it is high: their beads are gathered from global memory, or by
-    // lanes that wait for one another.  From here on smaller ones, in boxes large enough to have
-    // them by default.  Steps, us, with the default shape and with 4x4x6: 80% of the beads at density
-    // 12, 48^3 457 and 340 (60% at 9), 64^3 1,573 and 825, 80^3 1,324 and 958 (60% at 9); density falling
-    // as 1/sqrt(z), 48^3 460 and 364, 86^3 1,876 and 1,184; but 32^3 172 and 239.
+    // FP32: where the last rebuild that the host knows of left many beads without room in their cells'
+    // buckets (0.5% of them, and half as many again as even worlds would), the density varies over
+    // a box, and large bricks overflow where it is high: their beads are gathered from global
+    // memory, and a few bricks take as long as all the others.  From here on smaller ones, where
+    // the batch and a box in it are large enough to have them by default.  Steps, us, with the default
+    // shape and with 4x4x6: 80% of the beads at density 12, 64^3 1,573 and 825; 60% at 9, 48^3 457 and
+    // 340, 80^3 1,324 and 958; density falling as 1/sqrt(z), 48^3 460 and 364, 86^3 1,876 and 1,184, eight
+    // boxes of 41x33x27 741 and 587, four and 16 of 28^3 292 and 276, 833 and 684; but one of 32^3 172
+    // and 239, two of 28^3 195 and 233, four of 24^3 191 and 239, 32 of 37x25x19 837 and 958.
     static constexpr int CROWDED_SHAPE[3] = {4, 4, 6};
+    uint64_t largest_world() const
+    {
+        uint32_t most = 0;
+        for (const WorldHost &wh : worlds) most = std::max(most, wh.dev.n_cells);
+        return most;
+    }
     int adapt_bricks()
     {
-        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || args.bucket_k < bucket_room(max_density) ||
-            n_cells / (uint64_t)std::max(1, sm_count) < 350 || !h_err.p)
+        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning ||
+            n_cells / (uint64_t)std::max(1, sm_count) < 350 || largest_world() / (uint64_t)std::max(1, sm_count) < 125 || !h_err.p)
             return PDPD_OK;
-        if ((uint64_t)((const WorldDev *)h_err.p)->crowded * 200 <= n_beads) return PDPD_OK;
+        double even = 0;  // what Poisson counts leave
+        for (const WorldHost &wh : worlds) {
+            const double rho = density(wh.dev), s = std::sqrt(rho + 1e-9), z = (args.bucket_k - rho) / s;
+            even += wh.dev.n_cells * s * (std::exp(-0.5 * z * z) / 2.5066 - 0.5 * z * std::erfc(z / 1.4142));
+        }
+        if (((const WorldDev *)h_err.p)->crowded <= 1.5 * even + n_beads / 200.0) return PDPD_OK;
         crowded = true;
         cudaStreamSynchronize(stream);
         return configure_bricks();
