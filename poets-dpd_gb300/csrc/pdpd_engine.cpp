@@ -313,7 +313,8 @@ struct pdpd_engine {
     bool tuned = false;
     std::string tune_log;
     double max_density = 0;
-    bool crowded = false;  // the density varies over the box (adapt_bricks)
+    bool crowded = false;      // the density varies over the box (adapt_bricks)
+    double crowded_from = -1;  // crowd_limit() of the attached batch, -1: not asked for yet
 
     // attached worlds
     bool attached = false;
@@ -481,23 +482,27 @@ struct pdpd_engine {
     // boxes of 41x33x27 741 and 587, four and 16 of 28^3 292 and 276, 833 and 684; but one of 32^3 172
     // and 239, two of 28^3 195 and 233, four of 24^3 191 and 239, 32 of 37x25x19 837 and 958.
     static constexpr int CROWDED_SHAPE[3] = {4, 4, 6};
-    uint64_t largest_world() const
+    // More of the batch's beads than this without room are crowded: found once for an attached batch.
+    double crowd_limit() const
     {
-        uint32_t most = 0;
-        for (const WorldHost &wh : worlds) most = std::max(most, wh.dev.n_cells);
-        return most;
-    }
-    int adapt_bricks()
-    {
-        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning ||
-            n_cells / (uint64_t)std::max(1, sm_count) < 350 || largest_world() / (uint64_t)std::max(1, sm_count) < 125 || !h_err.p)
-            return PDPD_OK;
+        uint32_t largest = 0;
         double even = 0;  // what Poisson counts leave
         for (const WorldHost &wh : worlds) {
             const double rho = density(wh.dev), s = std::sqrt(rho + 1e-9), z = (args.bucket_k - rho) / s;
             even += wh.dev.n_cells * s * (std::exp(-0.5 * z * z) / 2.5066 - 0.5 * z * std::erfc(z / 1.4142));
+            largest = std::max(largest, wh.dev.n_cells);
         }
-        if (((const WorldDev *)h_err.p)->crowded <= 1.5 * even + n_beads / 200.0) return PDPD_OK;
+        return largest / (uint64_t)std::max(1, sm_count) < 125 ? 4e9 : 1.5 * even + n_beads / 200.0;
+    }
+    int adapt_bricks()
+    {
+        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || !h_err.p ||
+            n_cells / (uint64_t)std::max(1, sm_count) < 350)
+            return PDPD_OK;
+        const uint32_t beads = ((const WorldDev *)h_err.p)->crowded;
+        if (beads <= n_beads / 200) return PDPD_OK;
+        if (crowded_from < 0) crowded_from = crowd_limit();
+        if (beads <= crowded_from) return PDPD_OK;
         crowded = true;
         cudaStreamSynchronize(stream);
         return configure_bricks();
@@ -1844,6 +1849,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;
     e->crowded = false;
+    e->crowded_from = -1;
     {
         int rc = e->configure_bricks();
         if (rc) {
