@@ -150,3 +150,12 @@ def test_batches_of_uneven_boxes(box, copies, shape):
         w.x[:, 2] = w.x[:, 2] ** 2 / box[2]
     best = _step_us("fp32", worlds, steps=4, **dict(zip(("brick_x", "brick_y", "brick_z"), shape)))
     assert _step_us("fp32", worlds, steps=4) < 1.1 * best
+
+
+def test_a_dense_uneven_world_beside_others_fp64():
+    """Against the two one after the other: as long; 1.5 times when the dense world had the bricks of the
+    batch's size, and the last of them were waited for."""
+    dense, others = _water((30, 24, 24), 6.28), [_water(24, 1, k) for k in range(8)]
+    dense.x[:, 2] = dense.x[:, 2] ** 2 / 24
+    apart = _step_us("fp64", [dense], steps=3) + _step_us("fp64", others, steps=3)
+    assert _step_us("fp64", [dense] + others, steps=3) < 1.25 * apart
