@@ -894,7 +894,8 @@ struct pdpd_engine {
             const int *c = per_world ? world_shape(shape, room, rho, limit) : shape;
             hc_max = std::max(hc_max, halo_cells(c));
             want = std::max(want, staging_want(halo_cells(c), rho));
-            if (per_world) c = lighter_shape(shape, c, rho, rho2);
+            if (per_world && !brick_user) c = lighter_shape(shape, c, rho, rho2);
+            hc_max = std::max(hc_max, halo_cells(c));
             const std::vector<int> cx = cuts(L[0], c[0]), cy = cuts(L[1], c[1]), cz = cuts(L[2], c[2]);
             for (size_t a0 = 0; a0 + 1 < cx.size(); a0++)
                 for (size_t a1 = 0; a1 + 1 < cy.size(); a1++)
