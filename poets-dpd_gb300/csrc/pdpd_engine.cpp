@@ -15,6 +15,7 @@
 #include <functional>
 #include <condition_variable>
 #include <mutex>
+#include <numeric>
 #include <unistd.h>
 #include <memory>
 #include <string>
@@ -888,7 +889,16 @@ struct pdpd_engine {
         };
         uint32_t hc_max = 0;
         double want = 64;
-        for (uint32_t i = 0; i < worlds.size(); i++) {
+        // Worlds of higher density first, by powers of two: their bricks take longest, and the pass ends
+        // with the last one.  A world of 22^3 of density 10, FP64, behind 50 of 20^3 of density 0.7, step
+        // 694 us, 618 with it first; FP32, 25 boxes of densities 0.07 to 3.6 535 and 481.
+        std::vector<uint32_t> order(worlds.size());
+        std::vector<int> power(worlds.size());
+        std::iota(order.begin(), order.end(), 0u);
+        for (uint32_t i : order) power[i] = worlds[i].dev.n_beads ? std::ilogb(1.414 * density(worlds[i].dev)) : -1000;
+        if (!std::is_sorted(power.begin(), power.end(), std::greater<int>()))
+            std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return power[x] > power[y]; });
+        for (uint32_t i : order) {
             const int32_t *L = worlds[i].dev.L;
             const double rho = density(worlds[i].dev);
             const int *c = per_world ? world_shape(shape, room, rho, limit) : shape;

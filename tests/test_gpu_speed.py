@@ -159,3 +159,9 @@ def test_a_dense_uneven_world_beside_others_fp64():
     dense.x[:, 2] = dense.x[:, 2] ** 2 / 24
     apart = _step_us("fp64", [dense], steps=3) + _step_us("fp64", others, steps=3)
     assert _step_us("fp64", [dense] + others, steps=3) < 1.25 * apart
+
+
+def test_a_dense_world_behind_others_fp64():
+    """Against the dense world in front: the same time; 1.11 times when its bricks were the pass's last."""
+    dense, others = _water(22, 10), [_water(20, 0.7, k) for k in range(50)]
+    assert _step_us("fp64", others + [dense]) < 1.06 * _step_us("fp64", [dense] + others)
