@@ -33,18 +33,25 @@ struct List64Room {
 };
 
 // What the lists save over the force pass without them (k_force64), us a step, for a world of n
-// beads in `cells` cells: the list kernel goes through all cells, at 0.088 ns each; without lists
+// beads: the list kernel goes through all cells, at 0.088 ns each; without lists
 // the FP64 work grows with the density, and beyond about 4 beads a cell its candidate lists
 // overflow.  Steps of water boxes, us, with lists and without: 64^3 of density 0.05 54 and 41, 0.1 59
 // and 49, 0.2 65 and 73, 3 833 and 1,771; 90^3, 0.2 149 and 116, 0.25 159 and 133, 0.3 172 and 176;
 // 128^3, 0.05 267 and 89, 0.2 370 and 275, 0.25 405 and 345, 0.3 447 and 466; 160^3, 0.25 775 and 679,
 // 0.3 837 and 878; 24^3, 10 657 and 14,400.  A world costs the list kernel a brick at least, about
-// 120 cells' worth: 2,000 boxes of 2^3 of density 0.25 74 and 59, 0.5 82 and 80, 1 94 and 116.
-inline double lists64_saving_us(double n, double cells)
+// 120 cells' worth: 2,000 boxes of 2^3 of density 0.25 74 and 59, 0.5 82 and 80, 1 94 and 116.  And
+// bricks that a world does not fill cost more for each of its cells, which the mean of its cells
+// and the cells of its 5x8x8 bricks describes: 100 boxes of 11x9x14 (3,840 for 1,386) of density
+// 0.05 57 and 39, 0.15 62 and 46; 1,000 of 6^3 (640 for 216), 0.15 94 and 68, 0.4 118 and 110; 1,000
+// of 8^3 (640 for 512), 0.25 131 and 111; ten of 24^3 (14,400 for 13,824), 0.05 45 and 41, 0.25 50 and
+// 60.
+inline double lists64_saving_us(double n, const int32_t box[3])
 {
+    const double cells = (double)box[0] * box[1] * box[2];
+    const double padded = 320.0 * ((box[0] + 4) / 5) * ((box[1] + 7) / 8) * ((box[2] + 7) / 8);
     const double rho = n / cells;
     const double bead_ns = rho > 3 ? 1.2 * std::pow(rho / 3, 3) : std::min(1.2, 1.1 * rho);
-    return 1e-3 * (n * bead_ns - 0.088 * std::max(cells, 120.0));
+    return 1e-3 * (n * bead_ns - 0.088 * std::max(std::sqrt(cells * padded), 120.0));
 }
 // Small batches gain at any density: a bead's walk on global memory is a long chain (32^3 of
 // density 0.005 to 0.1 30 to 33 with lists, 34 to 40 without; 50^3, 0.05 43 and 39).
@@ -79,7 +86,7 @@ struct BatchSize {
         bonds += n_bonds;
         angles += n_angles;
         if (n_beads) room.add((double)n_beads, box, asym);
-        saving_us += lists64_saving_us((double)n_beads, (double)c);
+        saving_us += lists64_saving_us((double)n_beads, box);
     }
     void add(const BatchSize &o)
     {

@@ -165,3 +165,10 @@ def test_a_dense_world_behind_others_fp64():
     """Against the dense world in front: the same time; 1.11 times when its bricks were the pass's last."""
     dense, others = _water(22, 10), [_water(20, 0.7, k) for k in range(50)]
     assert _step_us("fp64", others + [dense]) < 1.06 * _step_us("fp64", [dense] + others)
+
+
+@pytest.mark.parametrize("box,copies,density", [((11, 9, 14), 100, 0.05), ((11, 9, 14), 100, 0.15), ((6, 6, 6), 1000, 0.25)])
+def test_sparse_worlds_that_fill_their_bricks_badly_fp64(box, copies, density):
+    """Without pair lists, which took 1.46, 1.34 and 1.24 times as long."""
+    worlds = [_water(box, density, k) for k in range(copies)]
+    assert _step_us("fp64", worlds) < 1.12 * _step_us("fp64", worlds, pair_lists=0)
