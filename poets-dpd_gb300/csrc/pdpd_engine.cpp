@@ -763,21 +763,24 @@ struct pdpd_engine {
     }
 
     // More bricks than variant 8's resident blocks, of at most 128 home beads (a turn of variant 6's
-    // blocks) in the average bead's brick: bricks of tiny worlds, of sparse boxes, or small ones that
-    // the config names.  Most threads of variant 8's blocks would idle.  Steps, us, with 8 and with 6: 600 boxes
+    // blocks) in any world: bricks of tiny worlds, of sparse boxes, or small ones that the config
+    // names.  Most threads of variant 8's blocks would idle.  Steps, us, with 8 and with 6: 600 boxes
     // of 2^3 31.9 and 22.4, 2,000 of 3^3 100 and 64, 32^3 of density 3 in bricks of 3x3x3 68 and 52; 48^3
     // of density 0.3 in 4x4x8 38 and 27; but 300 boxes of 3^3 (a brick per block) 22.7 and 26.7, 600 of
-    // 4^3 (192 beads each) 45 and 49.
+    // 4^3 (192 beads each) 45 and 49; 41x67x65 of density 0.16 beside 11x11x13 of density 3 (393 beads to a
+    // brick) 43 and 69.  At most 80 in bricks of more than 128 cells, whose beads vary most where the
+    // density does: 64x75x100, even and with a density falling as 1/sqrt(z), density 0.2 79 and 57, 106
+    // and 102; 0.3 (96 beads) 81 and 61, 120 and 148; 0.45 85 and 73, 140 and 223.
     bool few_beads_a_brick(const int shape[3]) const
     {
-        double n = 0, home = 0;
+        double n = 0;
         for (const WorldHost &wh : worlds) {
             double k = 1;
             for (int d = 0; d < 3; d++) k *= (wh.dev.L[d] + shape[d] - 1) / shape[d];
+            if (wh.dev.n_beads > (wh.dev.n_cells > 128 * k ? 80 : 128) * k) return false;
             n += k;
-            home += wh.dev.n_beads / k * wh.dev.n_beads;
         }
-        return !fp64() && n > 2.0 * sm_count && home <= 128.0 * n_beads && max_density <= 4;
+        return !fp64() && n > 2.0 * sm_count && max_density <= 4;
     }
 
     // Default kernel variant and brick shape for the attached batch, where the config does not

@@ -172,3 +172,13 @@ def test_sparse_worlds_that_fill_their_bricks_badly_fp64(box, copies, density):
     """Without pair lists, which took 1.46, 1.34 and 1.24 times as long."""
     worlds = [_water(box, density, k) for k in range(copies)]
     assert _step_us("fp64", worlds) < 1.12 * _step_us("fp64", worlds, pair_lists=0)
+
+
+@pytest.mark.parametrize("boxes", [[((41, 67, 65), 0.16), ((11, 11, 13), 3)], [((64, 75, 100), 0.45)]])
+def test_a_few_full_bricks_among_many(boxes):
+    """A box of density 3 beside a sparse one, and a sparse box whose density falls as 1/sqrt(z), against
+    force_kernel 8: 1.6 times as long in blocks of 128 threads."""
+    worlds = [_water(box, density, k) for k, (box, density) in enumerate(boxes)]
+    if len(worlds) == 1:
+        worlds[0].x[:, 2] = worlds[0].x[:, 2] ** 2 / worlds[0].box[2]
+    assert _step_us("fp32", worlds, steps=20) < 1.15 * _step_us("fp32", worlds, steps=20, force_kernel=8)
