@@ -481,7 +481,9 @@ struct pdpd_engine {
     // shape and with 4x4x6: 80% of the beads at density 12, 64^3 1,573 and 825; 60% at 9, 48^3 457 and
     // 340, 80^3 1,324 and 958; density falling as 1/sqrt(z), 48^3 460 and 364, 86^3 1,876 and 1,184, eight
     // boxes of 41x33x27 741 and 587, four and 16 of 28^3 292 and 276, 833 and 684; but one of 32^3 172
-    // and 239, two of 28^3 195 and 233, four of 24^3 191 and 239, 32 of 37x25x19 837 and 958.
+    // and 239, two of 28^3 195 and 233, four of 24^3 191 and 239, 32 of 37x25x19 837 and 958.  Boxes
+    // below a mean density of 1.25 have few beads to a small brick: 64x75x100 falling so, density 1 290
+    // and 322, 1.5 499 and 451.
     static constexpr int CROWDED_SHAPE[3] = {4, 4, 6};
     // More of the batch's beads than this without room are crowded: found once for an attached batch.
     double crowd_limit() const
@@ -498,7 +500,7 @@ struct pdpd_engine {
     int adapt_bricks()
     {
         if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || !h_err.p ||
-            n_cells / (uint64_t)std::max(1, sm_count) < 350)
+            n_cells / (uint64_t)std::max(1, sm_count) < 350 || n_beads < 1.25 * n_cells)
             return PDPD_OK;
         const uint32_t beads = ((const WorldDev *)h_err.p)->crowded;
         if (beads <= n_beads / 200) return PDPD_OK;

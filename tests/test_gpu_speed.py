@@ -182,3 +182,11 @@ def test_a_few_full_bricks_among_many(boxes):
     if len(worlds) == 1:
         worlds[0].x[:, 2] = worlds[0].x[:, 2] ** 2 / worlds[0].box[2]
     assert _step_us("fp32", worlds, steps=20) < 1.15 * _step_us("fp32", worlds, steps=20, force_kernel=8)
+
+
+def test_an_uneven_box_of_low_density():
+    """Density 1 falling as 1/sqrt(z), against the default bricks for even boxes; 1.12 times as long in
+    smaller ones."""
+    w = _water((64, 75, 100), 1)
+    w.x[:, 2] = w.x[:, 2] ** 2 / 100
+    assert _step_us("fp32", [w]) < 1.06 * _step_us("fp32", [w], brick_x=5, brick_y=8, brick_z=8)
