@@ -56,6 +56,13 @@ inline double lists64_saving_us(double n, const int32_t box[3])
 // Small batches gain at any density: a bead's walk on global memory is a long chain (32^3 of
 // density 0.005 to 0.1 30 to 33 with lists, 34 to 40 without; 50^3, 0.05 43 and 39).
 constexpr double LISTS64_BASE_US = 12;
+// And the chain is the longer the denser the densest world, however few its beads: 63x53x91 of density
+// 0.11 and 10x9x8 of density 3, 73 with lists and 99 without, and 6^3 of density 1 67 and 62; 90^3 of
+// density 0.2 and 6^3 of density 3, 153 and 166, and 1 150 and 126.
+inline double lists64_chain_us(double most_density)
+{
+    return 25 * std::min(1.0, std::max(0.0, (most_density - 0.4) / 1.6));
+}
 
 // Entries of a cell's bucket in a world of this density: the mean and 5.5 Poisson deviations (cells
 // that hold more go through overflow lists), a multiple of 4.
@@ -74,7 +81,8 @@ constexpr size_t BEAD_BYTES64 = 6 * 32 + 16 + 144 + 8 + 4 + 4 + 8 + 4 + 16;
 struct BatchSize {
     uint64_t worlds = 0, beads = 0, cells = 0, bucket_entries = 0, bonds = 0, angles = 0;
     List64Room room;
-    double saving_us = LISTS64_BASE_US;  // of the pair lists
+    double saving_us = LISTS64_BASE_US;  // of the pair lists, but for the chain
+    double most_density = 0;
 
     void add(uint32_t n_beads, const int32_t box[3], uint32_t n_bonds, uint32_t n_angles, bool asym)
     {
@@ -87,6 +95,7 @@ struct BatchSize {
         angles += n_angles;
         if (n_beads) room.add((double)n_beads, box, asym);
         saving_us += lists64_saving_us((double)n_beads, box);
+        most_density = std::max(most_density, (double)n_beads / (double)c);
     }
     void add(const BatchSize &o)
     {
@@ -99,6 +108,7 @@ struct BatchSize {
         room.entries += o.room.entries;
         room.pairs += o.room.pairs;
         saving_us += o.saving_us - LISTS64_BASE_US;
+        most_density = std::max(most_density, o.most_density);
     }
 
     // Entries of every bucket of the batch: as many in all as the worlds' own sizes come to, so that a
@@ -109,7 +119,7 @@ struct BatchSize {
     // The pair lists can address the batch (a list entry holds a slot in 25 bits, a pair in 30), and
     // save time.
     bool lists_fit() const { return beads > 0 && beads < (1u << 25) && room.entries < 2e9 && room.pairs < 1e9; }
-    bool lists_pay() const { return saving_us > 0; }
+    bool lists_pay() const { return saving_us + lists64_chain_us(most_density) > 0; }
 
     // Device bytes of the batch.
     size_t bytes(bool fp64) const

@@ -190,3 +190,9 @@ def test_an_uneven_box_of_low_density():
     w = _water((64, 75, 100), 1)
     w.x[:, 2] = w.x[:, 2] ** 2 / 100
     assert _step_us("fp32", [w]) < 1.06 * _step_us("fp32", [w], brick_x=5, brick_y=8, brick_z=8)
+
+
+def test_a_small_dense_world_beside_a_sparse_one_fp64():
+    """With pair lists; 1.37 times as long without, for the few beads of the dense world."""
+    worlds = [_water((63, 53, 91), 0.11), _water((10, 9, 8), 3, 2)]
+    assert _step_us("fp64", worlds) < 1.15 * _step_us("fp64", worlds, pair_lists=2)
