@@ -483,8 +483,11 @@ struct pdpd_engine {
     // boxes of 41x33x27 741 and 587, four and 16 of 28^3 292 and 276, 833 and 684; but one of 32^3 172
     // and 239, two of 28^3 195 and 233, four of 24^3 191 and 239, 32 of 37x25x19 837 and 958.  Boxes
     // below a mean density of 1.25 have few beads to a small brick: 64x75x100 falling so, density 1 290
-    // and 322, 1.5 499 and 451.
-    static constexpr int CROWDED_SHAPE[3] = {4, 4, 6};
+    // and 322, 1.5 499 and 451.  From a mean density of 4 on smaller ones still; so, 4x4x6 and 3x4x4:
+    // density 3, 60^3 524 and 570, 79x69x75 830 and 959; 4, 853 and 799, 1,322 and 1,337; 5.1, 1,348 and 1,026,
+    // 2,058 and 1,726; 80% of the beads in a fifth, 60^3 of density 3 790 and 781, 4 1,222 and 1,068, 5.1
+    // 2,194 and 1,541.
+    static constexpr int CROWDED_SHAPE[3] = {4, 4, 6}, CROWDED_DENSE[3] = {3, 4, 4};
     // More of the batch's beads than this without room are crowded: found once for an attached batch.
     double crowd_limit() const
     {
@@ -664,7 +667,7 @@ struct pdpd_engine {
         static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
                                        {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
         if (crowded) {
-            for (int d = 0; d < 3; d++) shape[d] = CROWDED_SHAPE[d];
+            for (int d = 0; d < 3; d++) shape[d] = n_beads < 4.0 * n_cells ? CROWDED_SHAPE[d] : CROWDED_DENSE[d];
             return;
         }
         double least = max_density, most = 0;  // the sparsest world, and the densest that the shape fits

@@ -196,3 +196,10 @@ def test_a_small_dense_world_beside_a_sparse_one_fp64():
     """With pair lists; 1.37 times as long without, for the few beads of the dense world."""
     worlds = [_water((63, 53, 91), 0.11), _water((10, 9, 8), 3, 2)]
     assert _step_us("fp64", worlds) < 1.15 * _step_us("fp64", worlds, pair_lists=2)
+
+
+def test_an_uneven_box_of_high_density():
+    """Density 5 falling as 1/sqrt(z), against 3x4x4 bricks; 1.3 times as long in 4x4x6."""
+    w = _water(60, 5)
+    w.x[:, 2] = w.x[:, 2] ** 2 / 60
+    assert _step_us("fp32", [w]) < 1.12 * _step_us("fp32", [w], brick_x=3, brick_y=4, brick_z=4)
