@@ -234,6 +234,7 @@ constexpr int V2_PIECES = 4;
 struct WorldHost {
     WorldDev dev;
     std::shared_ptr<V2Layout> v2;
+    bool crowded = false;  // its density varies, and most other worlds' does not (adapt_bricks)
 };
 
 bool asymmetric(const pdpd_world &w)
@@ -315,7 +316,8 @@ struct pdpd_engine {
     std::string tune_log;
     double max_density = 0;
     bool crowded = false;      // the density varies over the box (adapt_bricks)
-    double crowded_from = -1;  // crowd_limit() of the attached batch, -1: not asked for yet
+    double crowded_even = -1;  // the batch's even_overflow(), -1: not asked for yet
+    uint32_t crowded_seen = 0;
 
     // attached worlds
     bool attached = false;
@@ -474,7 +476,7 @@ struct pdpd_engine {
     }
 
     // FP32: where the last rebuild that the host knows of left many beads without room in their cells'
-    // buckets (0.5% of them, and half as many again as even worlds would), the density varies over
+    // buckets (0.5% of a world's, and a quarter more than an even one's), the density varies over
     // a box, and large bricks overflow where it is high: their beads are gathered from global
     // memory, and a few bricks take as long as all the others.  From here on smaller ones, where
     // the batch and a box in it are large enough to have them by default.  Steps, us, with the default
@@ -486,32 +488,55 @@ struct pdpd_engine {
     // and 322, 1.5 499 and 451.  From a mean density of 4 on smaller ones still; so, 4x4x6 and 3x4x4:
     // density 3, 60^3 524 and 570, 79x69x75 830 and 959; 4, 853 and 799, 1,322 and 1,337; 5.1, 1,348 and 1,026,
     // 2,058 and 1,726; 80% of the beads in a fifth, 60^3 of density 3 790 and 781, 4 1,222 and 1,068, 5.1
-    // 2,194 and 1,541.
+    // 2,194 and 1,541.  Where such worlds hold less than half of the batch's beads, they alone have
+    // smaller bricks, of any size, and the first ones: 31x16x29 falling so beside even boxes of 43x44x40,
+    // 34x46x31 and 26x34x41, 285 without and 149; 30 boxes, 1.8M beads, 528 with 4x4x6 for all, 385.
     static constexpr int CROWDED_SHAPE[3] = {4, 4, 6}, CROWDED_DENSE[3] = {3, 4, 4};
-    // More of the batch's beads than this without room are crowded: found once for an attached batch.
-    double crowd_limit() const
+    const int *crowded_shape(double rho) const { return rho < 4 ? CROWDED_SHAPE : CROWDED_DENSE; }
+    // Beads without room in an even world of this many cells and this density (Poisson counts).
+    double even_overflow(double cells, double rho) const
     {
-        uint32_t largest = 0;
-        double even = 0;  // what Poisson counts leave
-        for (const WorldHost &wh : worlds) {
-            const double rho = density(wh.dev), s = std::sqrt(rho + 1e-9), z = (args.bucket_k - rho) / s;
-            even += wh.dev.n_cells * s * (std::exp(-0.5 * z * z) / 2.5066 - 0.5 * z * std::erfc(z / 1.4142));
-            largest = std::max(largest, wh.dev.n_cells);
-        }
-        return largest / (uint64_t)std::max(1, sm_count) < 125 ? 4e9 : 1.5 * even + n_beads / 200.0;
+        double p = std::exp(-rho), left = rho - args.bucket_k;
+        for (uint32_t n = 0; n < args.bucket_k; n++, p *= rho / n) left += (args.bucket_k - n) * p;
+        return cells * std::max(0.0, left);
     }
     int adapt_bricks()
     {
-        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || !h_err.p ||
-            n_cells / (uint64_t)std::max(1, sm_count) < 350 || n_beads < 1.25 * n_cells)
-            return PDPD_OK;
-        const uint32_t beads = ((const WorldDev *)h_err.p)->crowded;
-        if (beads <= n_beads / 200) return PDPD_OK;
-        if (crowded_from < 0) crowded_from = crowd_limit();
-        if (beads <= crowded_from) return PDPD_OK;
-        crowded = true;
-        cudaStreamSynchronize(stream);
-        return configure_bricks();
+        const uint64_t sms = (uint64_t)std::max(1, sm_count);
+        if (fp64() || crowded || kernel_user || brick_user || tuned || tuning || !h_err.p || n_cells / sms < 350) return PDPD_OK;
+        const uint32_t beads = std::min(((const WorldDev *)h_err.p)->crowded, n_beads);
+        if (beads <= crowded_seen) return PDPD_OK;
+        if (crowded_even < 0) {
+            crowded_even = 0;
+            for (const WorldHost &wh : worlds) crowded_even += even_overflow(wh.dev.n_cells, density(wh.dev));
+        }
+        if (beads <= 1.25 * crowded_even + n_beads / 1500.0) return PDPD_OK;
+        crowded_seen = (uint32_t)std::min<uint64_t>(2ull * beads, n_beads);  // (looked at again when twice as many)
+        // the worlds that these beads are of
+        std::vector<uint2> node(beads);
+        cudaError_t ce = cudaMemcpyAsync(node.data(), args.over_node, sizeof(uint2) * beads, cudaMemcpyDeviceToHost, stream);
+        if (ce == cudaSuccess) ce = cudaStreamSynchronize(stream);
+        if (ce != cudaSuccess) return cuda_fail(ce, "overflow list read");
+        std::vector<uint32_t> in(worlds.size());
+        for (const uint2 &o : node) {
+            auto after = std::upper_bound(worlds.begin(), worlds.end(), o.x & 0x7fffffffu,
+                                          [](uint32_t id, const WorldHost &wh) { return id < wh.dev.bead_base; });
+            in[after - worlds.begin() - 1]++;
+        }
+        uint64_t uneven = 0, largest = 0;
+        for (size_t i = 0; i < worlds.size(); i++) {
+            const WorldDev &d = worlds[i].dev;
+            worlds[i].crowded = d.n_beads >= 1.25 * d.n_cells && in[i] > 1.25 * even_overflow(d.n_cells, density(d)) + d.n_beads / 200.0;
+            if (!worlds[i].crowded) continue;
+            uneven += d.n_beads;
+            largest = std::max<uint64_t>(largest, d.n_cells);
+        }
+        if (2 * uneven >= n_beads) {
+            for (WorldHost &wh : worlds) wh.crowded = false;
+            crowded = largest / sms >= 125;
+            if (!crowded) return PDPD_OK;
+        }
+        return uneven ? configure_bricks() : PDPD_OK;
     }
 
     // Enqueue n steps (n >= 1) on stream s.
@@ -667,7 +692,7 @@ struct pdpd_engine {
         static const int other[][3] = {{5, 8, 8}, {4, 8, 8}, {4, 6, 8}, {5, 6, 8}, {4, 5, 8}, {4, 4, 8},
                                        {3, 5, 8}, {4, 4, 6}, {3, 4, 8}, {3, 4, 6}, {2, 4, 8}, {2, 4, 4}};
         if (crowded) {
-            for (int d = 0; d < 3; d++) shape[d] = n_beads < 4.0 * n_cells ? CROWDED_SHAPE[d] : CROWDED_DENSE[d];
+            for (int d = 0; d < 3; d++) shape[d] = crowded_shape((double)n_beads / (double)n_cells)[d];
             return;
         }
         double least = max_density, most = 0;  // the sparsest world, and the densest that the shape fits
@@ -897,19 +922,19 @@ struct pdpd_engine {
         };
         uint32_t hc_max = 0;
         double want = 64;
-        // Worlds of higher density first, by powers of two: their bricks take longest, and the pass ends
+        // Worlds of higher density first, by powers of two (uneven ones as if 8 times as dense): their bricks take longest, and the pass ends
         // with the last one.  A world of 22^3 of density 10, FP64, behind 50 of 20^3 of density 0.7, step
         // 694 us, 618 with it first; FP32, 25 boxes of densities 0.07 to 3.6 535 and 481.
         std::vector<uint32_t> order(worlds.size());
         std::vector<int> power(worlds.size());
         std::iota(order.begin(), order.end(), 0u);
-        for (uint32_t i : order) power[i] = worlds[i].dev.n_beads ? std::ilogb(1.414 * density(worlds[i].dev)) : -1000;
+        for (uint32_t i : order) power[i] = worlds[i].dev.n_beads ? std::ilogb((worlds[i].crowded ? 11.3 : 1.414) * density(worlds[i].dev)) : -1000;
         if (!std::is_sorted(power.begin(), power.end(), std::greater<int>()))
             std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return power[x] > power[y]; });
         for (uint32_t i : order) {
             const int32_t *L = worlds[i].dev.L;
             const double rho = density(worlds[i].dev);
-            const int *c = per_world ? world_shape(shape, room, rho, limit) : shape;
+            const int *c = per_world ? world_shape(worlds[i].crowded ? crowded_shape(rho) : shape, room, rho, limit) : shape;
             hc_max = std::max(hc_max, halo_cells(c));
             want = std::max(want, staging_want(halo_cells(c), rho));
             if (per_world && !brick_user) c = lighter_shape(shape, c, rho, rho2);
@@ -1894,7 +1919,8 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;
     e->crowded = false;
-    e->crowded_from = -1;
+    e->crowded_even = -1;
+    e->crowded_seen = (uint32_t)nb / 1500;
     {
         int rc = e->configure_bricks();
         if (rc) {

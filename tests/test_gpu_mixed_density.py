@@ -81,3 +81,21 @@ def test_an_uneven_box_gets_other_bricks_between_runs():
         shapes.add(tuple(v for n, _, v in eng.GetConfigEntries() if n.startswith("brick_")))
         assert np.array_equal(a.x, b.x) and np.array_equal(a.v, b.v) and np.array_equal(a.f, b.f)
     assert ("4", "4", "6") in shapes
+
+
+def test_an_uneven_world_gets_other_bricks_among_even_ones():
+    """The same as the thread-per-bead kernel's to the bit, before and after the host has seen which world
+    is uneven."""
+    boxes = [(20, 21, 19), (41, 40, 39), (3, 4, 3), (26, 25, 27), (40, 38, 41)]
+    a = [W.make_water(box, seed=60 + k, a=1.0, dt=0.001) for k, box in enumerate(boxes)]
+    a[3].x[:, 2] = a[3].x[:, 2] ** 3 / 27**2
+    b = [w.copy() for w in a]
+    eng, ref = E.GB300DPDEngine("fp32"), E.GB300DPDEngine("fp32")
+    ref.SetConfigEntry("force_kernel", 1)
+    eng.AttachBatch(a)
+    ref.AttachBatch(b)
+    for steps in (1, 3, 2):
+        eng.Run(steps)
+        ref.Run(steps)
+        for w, o in zip(a, b):
+            assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
