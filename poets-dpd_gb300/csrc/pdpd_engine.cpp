@@ -1919,6 +1919,7 @@ static int attach_impl(pdpd_engine *e, const pdpd_world *ws, uint32_t n_worlds, 
     a.list_capacity = e->cfg_list_capacity;
     e->max_density = max_density;
     e->crowded = false;
+    if (e->h_err.p) ((WorldDev *)e->h_err.p)->crowded = 0;  // (what was read back of the batch before)
     e->crowded_even = -1;
     e->crowded_seen = (uint32_t)nb / 1500;
     {

@@ -99,3 +99,22 @@ def test_an_uneven_world_gets_other_bricks_among_even_ones():
         ref.Run(steps)
         for w, o in zip(a, b):
             assert np.array_equal(w.x, o.x) and np.array_equal(w.v, o.v) and np.array_equal(w.f, o.f)
+
+
+def test_an_uneven_batch_leaves_no_mark_on_the_next():
+    """An even box attached after an uneven one has the bricks of an even box."""
+    def shape(eng):
+        return tuple(v for n, _, v in eng.GetConfigEntries() if n.startswith("brick_"))
+
+    even = [W.make_water(40, seed=k, a=1.0, dt=0.001) for k in range(2)]
+    uneven = even[0].copy()
+    uneven.x[:, 2] = uneven.x[:, 2] ** 3 / 1600
+    fresh, eng = E.GB300DPDEngine("fp32"), E.GB300DPDEngine("fp32")
+    fresh.Attach(even[0])
+    fresh.Run(1)
+    fresh.Run(1)
+    for w in (uneven, even[1]):
+        eng.Attach(w)
+        eng.Run(1)
+        eng.Run(1)
+    assert shape(eng) == shape(fresh)
