@@ -491,8 +491,16 @@ struct pdpd_engine {
     // 2,194 and 1,541.  Where such worlds hold less than half of the batch's beads, they alone have
     // smaller bricks, of any size, and the first ones: 31x16x29 falling so beside even boxes of 43x44x40,
     // 34x46x31 and 26x34x41, 285 without and 149; 30 boxes, 1.8M beads, 528 with 4x4x6 for all, 385.
-    static constexpr int CROWDED_SHAPE[3] = {4, 4, 6}, CROWDED_DENSE[3] = {3, 4, 4};
+    // Below 1,000 cells per SM 3x4x6, and only where they hold less than a fifth; uneven beside
+    // even boxes, default, 4x4x6 and 3x4x6: 24^3 beside 40^3 174, 185, 150; 20x30x25 beside 44^3 173, 182,
+    // 145; but 37x28x33 (27% of the beads) beside 58x35x46 200, 249, 247, 30^3 (22%) beside two of 36^3
+    // 196, 205, 222.
+    static constexpr int CROWDED_SHAPE[3] = {4, 4, 6}, CROWDED_DENSE[3] = {3, 4, 4}, CROWDED_FEW[3] = {3, 4, 6};
     const int *crowded_shape(double rho) const { return rho < 4 ? CROWDED_SHAPE : CROWDED_DENSE; }
+    const int *uneven_shape(double rho) const
+    {
+        return rho < 4 && n_cells / (uint64_t)std::max(1, sm_count) < 1000 ? CROWDED_FEW : crowded_shape(rho);
+    }
     // Beads without room in an even world of this many cells and this density (Poisson counts).
     double even_overflow(double cells, double rho) const
     {
@@ -531,12 +539,11 @@ struct pdpd_engine {
             uneven += d.n_beads;
             largest = std::max<uint64_t>(largest, d.n_cells);
         }
-        if (2 * uneven >= n_beads) {
+        crowded = 2 * uneven >= n_beads && largest / sms >= 125;
+        if (2 * uneven >= n_beads || (n_cells / sms < 1000 && 5 * uneven >= n_beads))
             for (WorldHost &wh : worlds) wh.crowded = false;
-            crowded = largest / sms >= 125;
-            if (!crowded) return PDPD_OK;
-        }
-        return uneven ? configure_bricks() : PDPD_OK;
+        else if (uneven) return configure_bricks();
+        return crowded ? configure_bricks() : PDPD_OK;
     }
 
     // Enqueue n steps (n >= 1) on stream s.
@@ -934,7 +941,7 @@ struct pdpd_engine {
         for (uint32_t i : order) {
             const int32_t *L = worlds[i].dev.L;
             const double rho = density(worlds[i].dev);
-            const int *c = per_world ? world_shape(worlds[i].crowded ? crowded_shape(rho) : shape, room, rho, limit) : shape;
+            const int *c = per_world ? world_shape(worlds[i].crowded ? uneven_shape(rho) : shape, room, rho, limit) : shape;
             hc_max = std::max(hc_max, halo_cells(c));
             want = std::max(want, staging_want(halo_cells(c), rho));
             if (per_world && !brick_user) c = lighter_shape(shape, c, rho, rho2);

@@ -211,3 +211,11 @@ def test_an_uneven_world_among_even_ones():
     worlds = [_water(box, 3, k) for k, box in enumerate([(43, 44, 40), (34, 46, 31), (26, 34, 41), (31, 16, 29)])]
     worlds[3].x[:, 2] = worlds[3].x[:, 2] ** 2 / 29
     assert _step_us("fp32", worlds) < 1.2 * _step_us("fp32", worlds, brick_x=4, brick_y=4, brick_z=6)
+
+
+@pytest.mark.parametrize("uneven,even,copies", [((37, 28, 33), (58, 35, 46), 1), ((30, 30, 30), (36, 36, 36), 2), ((24, 24, 24), (40, 40, 40), 1)])
+def test_a_batch_of_a_few_boxes_with_an_uneven_one(uneven, even, copies):
+    """Against 4x5x8 bricks; the first two 1.15 to 1.25 times as long when the uneven box had smaller ones."""
+    worlds = [_water(uneven, 3)] + [_water(even, 3, 2 + k) for k in range(copies)]
+    worlds[0].x[:, 2] = worlds[0].x[:, 2] ** 2 / uneven[2]
+    assert _step_us("fp32", worlds) < 1.1 * _step_us("fp32", worlds, brick_x=4, brick_y=5, brick_z=8)
